@@ -1,0 +1,909 @@
+// Shift-reuse implicit-GEMM convolution (device body): any filter of a few
+// taps, stride 1 or 2, on the tcgen05 tensor cores straight from the NCHW
+// input.
+//
+//   D[pos][k] = sum over 16-channel blocks cb, taps (r, s) of
+//               X16[pos + shift(r, s)][16 channels] . W16[k][16 channels at the tap]
+//
+// Positions number the outputs of all images on a grid of GX columns and GY
+// rows an image, GX and GY a little larger than OW and OH, flat with columns
+// fastest.  With the stride split off into planes (plane (a, b) holds input
+// rows y = gy * U + a - P and columns x = gx * V + b - Q; stride 1 has one
+// plane), tap (r, s) reads plane (r % U, s % V) at position
+//   pos + (r / U) * GX + s / V,
+// the same shift for every position of a tile.  GX is the smallest width for
+// which a shift past the right edge lands on a column of the next row that is
+// zero padding where padding is due (GY likewise for rows of the next image),
+// so one zero column and one zero row separate neighbours: (W + 1)(H + 1) /
+// (W H) of the outputs' positions for 3x3 / stride 1 / pad 1.  Positions past
+// OW or OH compute values nobody stores.
+//
+// So a position tile's input is staged in shared memory ONCE per 16-channel
+// block -- its 128 positions plus the shifts' halo -- and every tap reads it
+// through a descriptor that starts shift * 16 bytes later: the K-major
+// no-swizzle operand is stored as [8-channel half][position][16 bytes], whose
+// 8-row groups follow each other without a gap (SBO = 128), so any row may
+// start a tile.  Against one staged operand per tap that is 9 * 128 = 1152
+// rows down to 128 + 2 GX + 2 per 16 channels of a 3x3 layer (190 at 28x28),
+// few enough that four warps bring them in from NCHW and no pre-pass over the
+// input is needed.
+//
+// Those producers read the input as quads of pixels: a channel's plane is
+// contiguous, so four consecutive pixels of eight channels are eight 8-byte
+// loads whatever the row breaks; each pixel's eight channels then go to its
+// position's 16-byte row.  (One pixel and channel per 2-byte load, four times
+// the load instructions, left the kernel waiting on them: 1.5 k cycles to
+// issue a stage of a 28x28 layer against 1.15 k cycles of its MMAs.)
+//
+// What bounds it: the tensor cores for C >= 128 (each 16-channel block of a
+// stage is R * S MMAs back to back on one staged input), the weight stream
+// from L2 beside them -- every CTA reads all its weights once per tile,
+// taps * 32 bytes per output channel and 16 channels.  CG = 2 (a cluster of
+// two CTAs, M = 256 positions) halves that stream per SM: each CTA holds half
+// of the weights' rows and the pair's MMA reads both halves.
+//
+// Measured (B200, L2 flushed, conv alone): N128 C256 28x28 K256 92 us = 1284
+// TFLOP/s direct (the Winograd two-stage kernels it replaces there: 61 + 79 +
+// 54 us); N64 C256 14x14 K256 30 us; N32 C512 7x7 K512 31 us; N32 C128 56x56
+// K128 stride 2 37 us (gathering implicit GEMM: 69 us).
+//
+// The weight operand (shift_weight_kernel) is laid out as the stages read it:
+// per unit block of output channels and CTA of the unit, 16-channel block by
+// 16-channel block, tap by tap, each piece the K-major core-matrix
+// interleave (row k, channel c at (k >> 3) * 256 + (c >> 3) * 128 + (k & 7)
+// * 16 + (c & 7) * 2).  A stage is then one run of up to 36 KB, copied by
+// NCOPY lanes: a bulk copy costs ~190 cycles of the copy engine whatever its
+// size up to a few KB, and one copy per tap held a stage of nine MMAs at
+// 1.8 k cycles.
+//
+// The reference computes only 3x3 / stride 1 / pad 1 and round-trips V and M
+// through HBM (src/preprocessing.cuh:273-424, src/matrixmul.cuh:139-556,
+// src/conv2d.cpp:17-250).
+#pragma once
+#include <cuda_runtime.h>
+#include <cuda_fp16.h>
+#include "tc_sm100.cuh"
+#include "wino_param.h"
+
+namespace wino {
+namespace sc {
+
+constexpr int TM = 128;                   // positions per CTA and unit
+constexpr int MAXTAP = 64;
+constexpr int MAXSTAGE = 8;
+constexpr int NCOPY = 4;                  // bulk copies a stage's weights are split into
+constexpr int SMEM_STAGES = 225 * 1024;   // dynamic shared memory of the stages
+constexpr int SMEM_BYTES = SMEM_STAGES + 128;
+constexpr int NSM = 148;                  // SMs of a B200 (the rules below count units against them)
+// Four warpgroups: warps 0-3 epilogue, 4 MMA issue, 5 weight copies, 6-7
+// padding rows, 8-15 input producers in two groups of four that take alternate
+// stages (a warp's own latency, not the issue slots, sets its pace, so two
+// groups bring twice the stages).  Launched with 128 registers a thread (the
+// whole register file); the MMA and epilogue warpgroups hand registers to the
+// producers, which hold the loads of the stages ahead.
+constexpr int NWARP_E = 4, WARP_MMA = 4, WARP_LOAD = 5, WARP_Z0 = 6, NWARP_Z = 2, WARP_P0 = 8, NWARP_P = 4, NGROUP = 2;
+constexpr int NTHREAD = (WARP_P0 + NGROUP * NWARP_P) * 32;
+constexpr int NPROD = NWARP_P * 32;       // producers of one stage
+constexpr int REGS_LAUNCH = 128, REGS_EPI = 112, REGS_MMA = 64, REGS_PROD = 168;
+static_assert(128 * REGS_EPI + 128 * REGS_MMA + NGROUP * NPROD * REGS_PROD == NTHREAD * REGS_LAUNCH,
+              "the warpgroups' register limits add up to the launch allocation");
+constexpr uint32_t SLEEP_NS = 32;
+// Items (a quad of pixels, eight channels) a producer thread may own per
+// stage, and operand rows whose padding it looks after.
+constexpr int MAXITEM = 4, MAXITEM_STRIDED = 6, MAXITEM_ODD = 2, MAXROWS = 1024;
+
+struct Shared {
+  uint64_t full[MAXSTAGE], empty[MAXSTAGE];
+  uint64_t accfull[2], accempty[2];
+  uint64_t mmadone;
+  uint32_t tmem_base;
+  int abort_flag;
+  int aoff[MAXTAP];                       // tap -> operand row offset in the stage
+};
+
+// The problem as the kernel sees it.  GX, GY, NB, log2 cps, nstage and qmax
+// are worked out on the host and travel packed in the kernel argument's
+// transform_pin (no workspace pointer is needed there), the rest follows
+// from them in a few operations: the divisions of the rules below cost a
+// CTA 6 k cycles before its first load.
+struct Plan {
+  int N, C, H, W, K, R, S, U, V, P, Q, OH, OW;
+  int GX, GY;          // position grid of an image
+  int nu, nv;          // planes: nu * nv
+  int rows;            // operand rows of a stage per 8 channels, all planes
+  int taps, CB, NKS, Kp;
+  int lcps, cps, nst;  // 16-channel blocks per stage (a power of two), stages per unit
+  int NB, nKU;         // output channels per unit, units per position tile
+  int units;
+  int stageA, stageB, nstage;
+  int qmax, qpi;       // quads of pixels a tile's rows may touch, quads per image
+  long long npos;
+};
+
+// Smallest grid extent for `o` outputs with filter extent f, stride st, pad
+// pd over an input extent e: a shift past the end must find zero padding on
+// both sides (positions GX + j of a row are positions j of the next).
+__host__ __device__ __forceinline__ int grid_extent(int o, int f, int st, int pd, int e) {
+  const int dmax = (f - 1) / st, np = st < f ? st : f;
+  for (int g = o; g < o + dmax; ++g) {
+    bool ok = true;
+    for (int b = 0; b < np; ++b) {
+      const int wrap = o + (f - 1 - b) / st - g;
+      for (int j = 0; j < wrap; ++j)
+        ok = ok && j < g && j * st + b - pd < 0 && (g + j) * st + b - pd >= e;
+    }
+    if (ok) return g;
+  }
+  return o + dmax;
+}
+
+__host__ __device__ __forceinline__ int div_stride(int x, int st) { return st == 1 ? x : st == 2 ? x >> 1 : x / st; }
+
+// Operand rows of plane (a, b): the tile's positions and its largest shift.
+__host__ __device__ __forceinline__ int plane_rows(const Plan& g, int a, int b) {
+  return TM + div_stride(g.R - 1 - a, g.U) * g.GX + div_stride(g.S - 1 - b, g.V);
+}
+
+// Tensor-pipe cycles of one MMA of N output channels as they issue here
+// (M = 128 per SM, K = 16: 56 up to N = 64, then N / 2).
+__host__ __device__ __forceinline__ int mma_cycles(int n) { return n <= 112 ? 56 : n >> 1; }
+
+__host__ __device__ __forceinline__ void plan_dims(Plan& g, const KernelParam& p) {
+  g.N = p.n; g.C = p.c; g.H = p.h; g.W = p.w; g.K = p.k; g.R = p.r; g.S = p.s;
+  g.U = p.u; g.V = p.v; g.P = p.p; g.Q = p.q; g.OH = p.Oh; g.OW = p.Ow;
+  g.nu = g.U < g.R ? g.U : g.R;
+  g.nv = g.V < g.S ? g.V : g.S;
+  g.taps = g.R * g.S;
+  g.CB = (g.C + 15) >> 4;
+  g.NKS = g.taps * g.CB;
+  g.Kp = (g.K + 15) & ~15;
+  g.qpi = (g.H * g.W + 3) >> 2;
+}
+
+// What follows from GX, GY, NB, lcps.
+__host__ __device__ __forceinline__ void plan_finish(Plan& g, int cg) {
+  g.rows = 0;
+  for (int a = 0; a < g.nu; ++a)
+    for (int b = 0; b < g.nv; ++b) g.rows += plane_rows(g, a, b);
+  // positions up to the last image's last output
+  g.npos = ((long long)(g.N - 1) * g.GY + g.OH - 1) * g.GX + g.OW;
+  g.nKU = (g.Kp + g.NB - 1) / g.NB;
+  g.units = (int)((g.npos + TM * cg - 1) >> (cg == 2 ? 8 : 7)) * g.nKU;
+  g.cps = 1 << g.lcps;
+  g.nst = (g.CB + g.cps - 1) >> g.lcps;
+  const int rows_b = cg == 2 ? ((g.Kp < g.NB ? (g.Kp + 31) & ~31 : g.NB) >> 1) : (g.Kp < g.NB ? g.Kp : g.NB);
+  // one more row: where producers drop pixels of a quad that are not the tile's
+  g.stageA = (g.cps * g.rows * 32 + 16 + 127) & ~127;
+  g.stageB = g.cps * g.taps * rows_b * 32;
+}
+
+// Plan of a problem for CG CTAs a unit (host; the rules).
+__host__ inline Plan make_plan(const KernelParam& p, int cg) {
+  Plan g;
+  plan_dims(g, p);
+  g.GX = grid_extent(g.OW, g.S, g.V, g.Q, g.W);
+  g.GY = grid_extent(g.OH, g.R, g.U, g.P, g.H);
+  // even rows of outputs on an even grid: pairs of neighbouring outputs then
+  // sit on lanes 2i, 2i + 1 and share 4-byte stores
+  if ((g.OW & 1) == 0) g.GX = (g.GX + 1) & ~1;
+  g.npos = ((long long)(g.N - 1) * g.GY + g.OH - 1) * g.GX + g.OW;
+  // Output channels per unit: a wave's time is its MMA time, so the fewest
+  // waves x cycles; wide units win ties (less of the input staged twice).
+  g.NB = 256;
+  if (cg == 1) {
+    long long best_t = -1;
+    for (int nb = 128; nb >= 32; nb >>= 1) {
+      const long long tiles = (g.npos + TM - 1) / TM, un = tiles * ((g.Kp + nb - 1) / nb);
+      const long long t = ((un + NSM - 1) / NSM) * mma_cycles(g.Kp < nb ? g.Kp : nb);
+      if (best_t < 0 || t < best_t) { best_t = t; g.NB = nb; }
+    }
+  }
+  // Quads a tile's rows touch: stride 1, at most the positions' own pixels
+  // (padding only lessens them); else whole grid rows.
+  int longest = 0;
+  for (int a = 0; a < g.nu; ++a)
+    for (int b = 0; b < g.nv; ++b) longest = plane_rows(g, a, b) > longest ? plane_rows(g, a, b) : longest;
+  const long long lines = (longest + 2 * g.GX - 2) / g.GX;
+  const long long px = g.U == 1 && g.V == 1 ? longest : lines * g.U * g.W;
+  // (images end in a partial quad when H * W is not a multiple of 4)
+  const long long imgs = lines / g.GY + 2;
+  const long long q = px / 4 + 2 + ((g.H * g.W) % 4 ? imgs : 0);
+  g.qmax = (int)(q < 4096 ? q : 4096);
+  // several 16-channel blocks a stage where a block has few taps
+  int cps = g.taps >= 6 ? 1 : g.taps >= 3 ? 2 : 4;
+  while (cps > 1 && (cps >> 1) >= g.CB) cps >>= 1;
+  for (;; cps >>= 1) {
+    g.lcps = cps == 4 ? 2 : cps == 2 ? 1 : 0;
+    plan_finish(g, cg);
+    if (cps == 1 || (2 * cps * g.qmax <= 3 * NPROD && 3 * (g.stageA + g.stageB) <= SMEM_STAGES)) break;
+  }
+  const int fit = SMEM_STAGES / (g.stageA + g.stageB);
+  g.nstage = fit < MAXSTAGE ? fit : MAXSTAGE;
+  return g;
+}
+
+__host__ inline unsigned long long pack_plan(const Plan& g) {
+  return (unsigned long long)g.GX | (unsigned long long)g.GY << 16 | (unsigned long long)(g.NB / 16) << 32 |
+         (unsigned long long)g.lcps << 40 | (unsigned long long)g.nstage << 44 | (unsigned long long)g.qmax << 48;
+}
+
+__device__ __forceinline__ Plan unpack_plan(const KernelParam& p, int cg) {
+  Plan g;
+  plan_dims(g, p);
+  const unsigned long long w = reinterpret_cast<unsigned long long>(p.transform_pin);
+  g.GX = (int)(w & 0xffff);
+  g.GY = (int)(w >> 16 & 0xffff);
+  g.NB = (int)(w >> 32 & 0xff) * 16;
+  g.lcps = (int)(w >> 40 & 15);
+  g.nstage = (int)(w >> 44 & 15);
+  g.qmax = (int)(w >> 48);
+  plan_finish(g, cg);
+  return g;
+}
+
+// Rows of the weight operand one CTA of a unit holds (the unit's output
+// channels k0 .., padded to the MMA's granularity).
+__host__ __device__ __forceinline__ int unit_n(const Plan& g, int cg, int k0) {
+  const int n = g.Kp - k0 < g.NB ? g.Kp - k0 : g.NB;
+  return cg == 2 ? (n + 31) & ~31 : n;
+}
+
+// Bytes of the weight operand.
+__host__ __device__ __forceinline__ size_t weight_bytes(const Plan& g, int cg) {
+  const int last = (g.nKU - 1) * g.NB;
+  return (size_t)(last + unit_n(g, cg, last)) * g.NKS * 32;
+}
+
+// n / d for 0 <= n < 2^31: m = ceil(2^32 / d) overestimates the quotient by
+// at most one.
+struct Div {
+  unsigned m;
+  int d;
+};
+__device__ __forceinline__ Div make_div(int d) { return Div{0xffffffffu / (unsigned)d + 1u, d}; }
+__device__ __forceinline__ int quot(int n, const Div& v) {
+  if (v.d == 1) return n;
+  const int q = (int)__umulhi((unsigned)n, v.m);
+  return q * v.d > n ? q - 1 : q;
+}
+
+// Unit u: position tile and output-channel block (k-blocks of one position
+// tile on neighbouring CTAs, so its input comes from L2 the second time).
+__device__ __forceinline__ void unit_of(const Plan& g, int u, int& pt, int& k0) {
+  pt = g.nKU == 1 ? u : (int)((unsigned)u / (unsigned)g.nKU);
+  k0 = (u - pt * g.nKU) * g.NB;
+}
+
+// t / d for 0 <= t < 2^20, with rd = 1.0f / d: (t + 1/2) / d is at least
+// 1 / (2 d) away from a whole number, more than the product's rounding error.
+__device__ __forceinline__ int small_div(int t, float rd) { return __float2int_rz(((float)t + 0.5f) * rd); }
+
+// Grid coordinates of a tile's first position, and of the position o later.
+struct Base {
+  int n, gy, gx;
+};
+struct Grid {
+  Div gx, gy;
+  float rgx, rgy;
+};
+__device__ __forceinline__ Grid make_grid(const Plan& g) {
+  return Grid{make_div(g.GX), make_div(g.GY), 1.0f / (float)g.GX, 1.0f / (float)g.GY};
+}
+__device__ __forceinline__ Base tile_base(const Grid& gr, int pos0) {
+  Base b;
+  const int line = quot(pos0, gr.gx);
+  b.gx = pos0 - line * gr.gx.d;
+  b.n = quot(line, gr.gy);
+  b.gy = line - b.n * gr.gy.d;
+  return b;
+}
+__device__ __forceinline__ Base advance(const Grid& gr, const Base& b, int o) {
+  Base r;
+  const int t = b.gx + o, dl = small_div(t, gr.rgx);
+  r.gx = t - dl * gr.gx.d;
+  const int l = b.gy + dl, dn = small_div(l, gr.rgy);
+  r.gy = l - dn * gr.gy.d;
+  r.n = b.n + dn;
+  return r;
+}
+
+// All of the block's threads (both CTAs' with CG = 2), each role from its own
+// place: barriers initialised and TMEM allocated before anyone relies on them.
+template <int CG>
+__device__ __forceinline__ void setup_sync() {
+  tc_fence_before();
+  __syncwarp();
+  if (CG == 2) cluster_sync();
+  else asm volatile("bar.sync 0;" ::: "memory");
+  tc_fence_after();
+}
+
+// Every lane polls (no broadcast behind the poll); the outcome is the warp's.
+template <bool kCluster = false>
+__device__ __forceinline__ bool wait_all_lanes(uint64_t* bar, uint32_t parity, volatile int* abort, uint32_t* err,
+                                               uint32_t code) {
+  return __all_sync(0xffffffffu, mbar_wait_impl<kCluster>(bar, parity, abort, err, code)) != 0;
+}
+
+// One stage's loads of a producer thread, and where they go.
+template <int NI, int NW>
+struct Slot {
+  uint2 w[NI][8][NW];
+  uint2 row[NI];                          // 16-byte rows of the stage its pixels go to, 16 bits each, store order
+  uint32_t shifts;                        // unaligned quads: first pixel's place in its 8-byte word, 4 bits an item
+};
+
+// Input producers with NI items a thread and stage, the loads of DEPTH (at
+// most four) of the group's stages in flight.  An item is (8-channel group of the
+// stage, quad of the tile's pixel range), quads fastest, so a warp's loads
+// are 256-byte runs of a channel's plane.  ALIGNED: a quad is one 8-byte
+// word of every channel (input 8-byte aligned, H * W a multiple of 4);
+// otherwise the two words around it and a shift.
+template <int CG, int NI, int DEPTH, bool ALIGNED, bool STRIDED>
+__device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uint8_t* smem, Shared& sh, int tid,
+                                        int group, int u0, int ustep, int cnt, int tile_pos, int tile_stride,
+                                        uint32_t* err) {
+  constexpr int NW = ALIGNED ? 1 : 2;     // 8-byte words per channel
+  volatile int* abort_flag = &sh.abort_flag;
+  const unsigned short* X = static_cast<const unsigned short*>(p.pin);
+  const int HW = g.H * g.W, ngrp = 2 * g.cps;
+  const uint32_t trash = (uint32_t)(ngrp * g.rows);
+  const Grid gr = make_grid(g);
+  const float rw = 1.0f / (float)g.W, rqpi = 1.0f / (float)g.qpi;
+  const int ushift = STRIDED ? g.U - 1 : 0, vshift = STRIDED ? g.V - 1 : 0;      // strides 1 and 2
+  // Pixel order of this lane's stores: pixel k ^ rot first, so that the eight
+  // lanes of a 16-byte store phase, whose quads are 64 bytes apart, fill one
+  // 128-byte line (no bank conflicts).
+  const int rot = (tid >> 1) & 3;
+  const uint32_t sel0 = rot & 1 ? 0x7632u : 0x5410u, sel1 = rot & 1 ? 0x5410u : 0x7632u;
+  int iq[NI], ich[NI];                    // quad (-1: none) and first channel of the stage
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int idx = tid + i * NPROD, grp = idx / g.qmax;
+    iq[i] = grp < ngrp ? idx - grp * g.qmax : -1;
+    ich[i] = grp * 8;
+  }
+  // planes by (row parity, column parity): first operand row, rows (0: none)
+  constexpr int NPL = STRIDED ? 4 : 1;
+  int pbase[NPL], prow[NPL];
+  {
+    int r = 0;
+#pragma unroll
+    for (int pl = 0; pl < NPL; ++pl) {
+      const int a = pl >> vshift, b = pl & vshift;
+      const bool there = a <= ushift && a < g.nu && b < g.nv;
+      pbase[pl] = r;
+      prow[pl] = STRIDED ? (there ? plane_rows(g, a, b) : 0) : g.rows;
+      r += prow[pl];
+    }
+  }
+  // load side: element offset from the unit's first image (-1: no loads), the
+  // quad's pixels inside the image, rows of its pixels, padding rows
+  int off[NI], npx[NI];
+  uint2 row_l[NI];
+  int lu = 0, lj = group;                 // this group's stages: every NGROUP-th
+  while (lj >= g.nst) { lj -= g.nst; ++lu; }
+  int entered = -1;
+  const unsigned short* base = X;
+  Slot<NI, NW> ring[DEPTH];
+  auto enter = [&]() {
+    int pt, k0;
+    unit_of(g, u0 + lu * ustep, pt, k0);
+    const Base b0 = tile_base(gr, pt * tile_stride + tile_pos);
+    base = X + (size_t)b0.n * g.C * HW;
+    // the range starts with the first position's pixel (stride 1) or the
+    // first pixel row of its grid row
+    const int y0 = (b0.gy << ushift) - g.P;
+    int lo = y0 * g.W;
+    if (!STRIDED) lo += min(max(b0.gx - g.Q, 0), g.W);
+    lo = min(max(lo, 0), HW);
+    const int q0 = lo >> 2, yb = max(y0, 0);
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      off[i] = -1;
+      npx[i] = 0;
+      row_l[i].x = row_l[i].y = trash | trash << 16;
+      if (iq[i] < 0) continue;
+      int q = q0 + iq[i], dn = 0;
+      if (q >= g.qpi) {
+        q -= g.qpi;
+        dn = small_div(q, rqpi);
+        q -= dn * g.qpi;
+        ++dn;
+      }
+      if (b0.n + dn >= g.N) continue;
+      const int i0 = q * 4;
+      // pixel row and column, from the row the range starts in (rel >= -3)
+      const int rel = dn == 0 ? i0 - yb * g.W : i0;
+      const int dy = rel < 0 ? -1 : small_div(rel, rw);
+      int y = (dn == 0 ? yb : 0) + dy, x = rel - dy * g.W;
+      while (x < 0) { x += g.W; --y; }    // images narrower than the overhang
+      bool any = false;
+      uint32_t d[4];
+#pragma unroll
+      for (int px = 0; px < 4; ++px) {
+        d[px] = trash;
+        int r = -1, pr = g.rows, pb = 0;
+        bool in = i0 + px < HW;
+        if (!STRIDED) {
+          r = (dn * g.GY + y + g.P - b0.gy) * g.GX + x + g.Q - b0.gx;
+          in = in && x + g.Q < g.GX && y + g.P < g.GY;
+        } else {
+          const int yy = y + g.P, xx = x + g.Q;
+          const int gy = yy >> ushift, gx = xx >> vshift;
+          const int pl = ((yy & ushift) << vshift) | (xx & vshift);
+          pb = pbase[0];
+          pr = prow[0];
+#pragma unroll
+          for (int z = 1; z < NPL; ++z)
+            if (pl == z) { pb = pbase[z]; pr = prow[z]; }
+          r = (dn * g.GY + gy - b0.gy) * g.GX + gx - b0.gx;
+          in = in && gx < g.GX && gy < g.GY;
+        }
+        if (in && r >= 0 && r < pr) {
+          d[px] = (uint32_t)((ich[i] >> 3) * g.rows + pb + r);
+          any = true;
+        }
+        if (++x == g.W) { x = 0; ++y; }
+      }
+      // stored in the order px ^ rot
+      const uint32_t w0 = d[0] | d[1] << 16, w1 = d[2] | d[3] << 16;
+      const uint32_t v0 = rot & 2 ? w1 : w0, v1 = rot & 2 ? w0 : w1;
+      row_l[i] = make_uint2(__byte_perm(v0, v0, rot & 1 ? 0x1032 : 0x3210), __byte_perm(v1, v1, rot & 1 ? 0x1032 : 0x3210));
+      npx[i] = min(4, HW - i0);
+      if (any) off[i] = dn * g.C * HW + i0;
+    }
+  };
+  auto issue = [&](Slot<NI, NW>& s) {
+    const int c0 = lj << (g.lcps + 4);
+    uint32_t shifts = 0;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int c = c0 + ich[i], nc = off[i] >= 0 ? g.C - c : 0;   // channels to load
+      const unsigned short* src = base + (off[i] + c * HW);
+      s.row[i] = row_l[i];
+      if (!ALIGNED) shifts |= ((uint32_t)(reinterpret_cast<uintptr_t>(src) >> 1) & 3u) << (4 * i);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const bool on = e < nc;
+        if (ALIGNED) {
+          s.w[i][e][0] = on ? __ldg(reinterpret_cast<const uint2*>(src + e * HW)) : make_uint2(0, 0);
+        } else {
+          const uintptr_t ad = reinterpret_cast<uintptr_t>(src + e * HW);
+          const uint2* wp = reinterpret_cast<const uint2*>(ad & ~uintptr_t(7));
+          s.w[i][e][0] = on ? __ldg(wp) : make_uint2(0, 0);
+          // the next word only where it holds a pixel of the quad
+          s.w[i][e][NW - 1] = on && ((int)(ad >> 1) & 3) + npx[i] > 4 ? __ldg(wp + 1) : make_uint2(0, 0);
+        }
+      }
+    }
+    s.shifts = shifts;
+  };
+  const int stage_bytes = g.stageA + g.stageB;
+  int st = group;
+  uint32_t phase = 1;                     // empty waits: the first pass over the ring is free
+  auto consume = [&](const Slot<NI, NW>& s) -> bool {
+    if (!wait_all_lanes(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
+    uint8_t* dst = smem + st * stage_bytes;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      uint32_t lo[8], hi[8];              // pixels (rot & 2, + 1) and the other two, of eight channels
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        uint32_t a = s.w[i][e][0].x, b = s.w[i][e][0].y;
+        if (!ALIGNED) {
+          const uint32_t sh16 = ((s.shifts >> (4 * i)) + (uint32_t)(e * HW)) & 3u;
+          uint32_t t0 = a, t1 = b, t2 = s.w[i][e][NW - 1].x;
+          if (sh16 & 2u) { t0 = b; t1 = s.w[i][e][NW - 1].x; t2 = s.w[i][e][NW - 1].y; }
+          a = sh16 & 1u ? __byte_perm(t0, t1, 0x5432) : t0;
+          b = sh16 & 1u ? __byte_perm(t1, t2, 0x5432) : t1;
+        }
+        lo[e] = rot & 2 ? b : a;
+        hi[e] = rot & 2 ? a : b;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t rw2 = k < 2 ? s.row[i].x : s.row[i].y, r = k & 1 ? rw2 >> 16 : rw2 & 0xffffu;
+        const uint32_t sel = k & 1 ? sel1 : sel0;
+        const uint32_t* v = k < 2 ? lo : hi;
+        *reinterpret_cast<uint4*>(dst + r * 16) =
+            make_uint4(__byte_perm(v[0], v[1], sel), __byte_perm(v[2], v[3], sel), __byte_perm(v[4], v[5], sel),
+                       __byte_perm(v[6], v[7], sel));
+      }
+    }
+    fence_proxy_async_shared();
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(&sh.full[st]);
+    st += NGROUP;
+    if (st >= g.nstage) { st -= g.nstage; phase ^= 1; }
+    return true;
+  };
+  // Turn t stores the loads of DEPTH turns ago from its ring slot and issues
+  // new ones into it.  One loop body with a case per slot: unrolled over the
+  // slots, the unit entry above was compiled in seven times and its first
+  // pass through the instruction cache held the first stage up by 10 us.
+  const int total = (cnt * g.nst - group + NGROUP - 1) / NGROUP;
+  // the first loads go out before the block's setup is complete
+  int slot = 0;
+  bool set = false;
+  for (int t = 0; t < total + DEPTH; ++t) {
+    if (t == DEPTH) {
+      setup_sync<CG>();
+      set = true;
+    }
+    const bool more = t < total;
+    if (more && lu != entered) {
+      enter();
+      entered = lu;
+    }
+    bool ok = true;
+    auto turn = [&](Slot<NI, NW>& s) {
+      if (t >= DEPTH) ok = consume(s);
+      if (more && ok) issue(s);
+    };
+    if (slot == 0) turn(ring[0]);
+    if (DEPTH > 1 && slot == 1) turn(ring[DEPTH > 1 ? 1 : 0]);
+    if (DEPTH > 2 && slot == 2) turn(ring[DEPTH > 2 ? 2 : 0]);
+    if (DEPTH > 3 && slot == 3) turn(ring[DEPTH > 3 ? 3 : 0]);
+    if (!ok) break;
+    if (++slot == DEPTH) slot = 0;
+    lj += NGROUP;
+    while (lj >= g.nst) { lj -= g.nst; ++lu; }
+  }
+  if (!set) setup_sync<CG>();             // no stage for this group
+}
+
+// Padding rows of the operand (two warps): the zero columns and rows of a
+// tile's positions, written to every stage (a slot's last tile had them
+// elsewhere).
+__device__ __forceinline__ void pad_rows(const Plan& g, uint8_t* smem, Shared& sh, int tid, int u0, int ustep, int cnt,
+                                         int tile_pos, int tile_stride, uint32_t* err) {
+  constexpr int NT = NWARP_Z * 32;
+  volatile int* abort_flag = &sh.abort_flag;
+  const Grid gr = make_grid(g);
+  const int ngrp = 2 * g.cps, stage_bytes = g.stageA + g.stageB;
+  int st = 0;
+  uint32_t phase = 1;
+  for (int i = 0; i < cnt; ++i) {
+    int pt, k0;
+    unit_of(g, u0 + i * ustep, pt, k0);
+    const Base b0 = tile_base(gr, pt * tile_stride + tile_pos);
+    uint32_t zero = 0;                    // bit z: row tid + z * NT is padding
+    int pbase = 0;
+    for (int a = 0; a < g.nu; ++a)
+      for (int b = 0; b < g.nv; ++b) {
+        const int pr = plane_rows(g, a, b);
+        for (int z = 0, r = tid - pbase; r < pr; ++z, r += NT) {
+          if (r < 0) continue;
+          const Base c = advance(gr, b0, r);
+          const int y = c.gy * g.U + a - g.P, x = c.gx * g.V + b - g.Q;
+          if (!(c.n < g.N && (unsigned)y < (unsigned)g.H && (unsigned)x < (unsigned)g.W)) zero |= 1u << z;
+        }
+        pbase += pr;
+      }
+    for (int j = 0; j < g.nst; ++j) {
+      if (!wait_all_lanes(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY)) return;
+      uint8_t* dst = smem + st * stage_bytes + tid * 16;
+      for (uint32_t m = zero; m != 0; m &= m - 1)
+        for (int grp = 0; grp < ngrp; ++grp)
+          *reinterpret_cast<uint4*>(dst + (grp * g.rows + (__ffs(m) - 1) * NT) * 16) = make_uint4(0, 0, 0, 0);
+      fence_proxy_async_shared();
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(&sh.full[st]);
+      if (++st == g.nstage) { st = 0; phase ^= 1; }
+    }
+  }
+}
+
+// Operand row at which tap (r, s) starts reading a stage: its plane's first
+// row plus its shift.
+__device__ __forceinline__ int tap_row(const Plan& g, int r, int s) {
+  const int dr = div_stride(r, g.U), ds = div_stride(s, g.V), a = r - dr * g.U, b = s - ds * g.V;
+  int base = 0;
+  for (int x = 0; x <= a; ++x)
+    for (int z = 0; z < (x < a ? g.nv : b); ++z) base += plane_rows(g, x, z);
+  return base + dr * g.GX + ds;
+}
+
+// MMA issue: per stage and 16-channel block one MMA a tap, all on the same
+// staged input.  The whole warp runs the loop and one elected lane issues, so
+// the descriptors stay in uniform registers.  TAPS > 0: that many taps,
+// their shifts kept in registers and the taps unrolled, so
+// that an MMA costs the warp a couple of adds: one warp feeds the tensor
+// pipe, and with the shifts read from shared memory inside the loop it
+// managed one N = 64 MMA per 92 cycles against the pipe's 56.
+template <int CG, int TAPS>
+__device__ __forceinline__ void issue_mmas(const Plan& g, Shared& sh, uint32_t sbase, uint32_t tmem, int u0, int ustep,
+                                           int cnt, uint32_t* err) {
+  constexpr uint16_t BOTH = 3;
+  constexpr int NOFF = TAPS > 0 ? TAPS : 1;
+  volatile int* abort_flag = &sh.abort_flag;
+  const bool leader = elect_one();
+  const uint32_t stage16 = (uint32_t)(g.stageA + g.stageB) >> 4, a16 = (uint32_t)g.stageA >> 4;
+  const uint64_t adesc0 = smem_desc(sbase, (uint32_t)g.rows * 16, 128), bdesc0 = smem_desc(sbase, 128, 256) + a16;
+  const uint32_t qstep = (uint32_t)g.rows * 2;
+  uint32_t off[NOFF];
+#pragma unroll
+  for (int t = 0; t < NOFF; ++t) off[t] = (uint32_t)__shfl_sync(0xffffffffu, sh.aoff[t], 0);
+  int st = 0;
+  uint32_t phase = 0, s16 = 0;
+  bool ok = true;
+  for (int i = 0; ok && i < cnt; ++i) {
+    int pt, k0;
+    unit_of(g, u0 + i * ustep, pt, k0);
+    const int nn = unit_n(g, CG, k0);
+    const uint32_t idesc = instr_desc(CG * 128, (uint32_t)nn, 0, 0, 0, 0);
+    const uint32_t bstep = (uint32_t)((nn / CG) * 32) >> 4;
+    const int ab = i & 1;
+    if (i >= 2) {
+      ok = wait_all_lanes<CG == 2>(&sh.accempty[ab], ((i >> 1) - 1) & 1, abort_flag, err, ERR_WAIT_DRAIN);
+      if (!ok) break;
+    }
+    tc_fence_after();
+    const uint32_t d = tmem + ab * 256;
+    auto mma = [&](uint64_t ad, uint64_t bd, uint32_t acc) {
+      if (leader) {
+        if (CG == 2) mma_f16_pair(d, ad, bd, idesc, acc);
+        else mma_f16(d, ad, bd, idesc, acc);
+      }
+    };
+    for (int j = 0; j < g.nst; ++j) {
+      ok = wait_all_lanes<CG == 2>(&sh.full[st], phase, abort_flag, err, ERR_WAIT_FULL);
+      if (!ok) break;
+      tc_fence_after();
+      const int nk = min(g.cps, g.CB - j * g.cps);
+      uint64_t aq = adesc0 + s16, bd = bdesc0 + s16;
+      for (int q = 0; q < nk; ++q, aq += qstep) {
+        if (TAPS > 0) {
+#pragma unroll
+          for (int t = 0; t < TAPS; ++t, bd += bstep) mma(aq + off[t], bd, t > 0 || j > 0 || q > 0 ? 1u : 0u);
+        } else {
+#pragma unroll 4
+          for (int t = 0; t < g.taps; ++t, bd += bstep)
+            mma(aq + (uint32_t)sh.aoff[t], bd, t > 0 || j > 0 || q > 0 ? 1u : 0u);
+        }
+      }
+      if (leader) {
+        if (CG == 2) mma_commit_pair(&sh.empty[st], BOTH);
+        else mma_commit(&sh.empty[st]);
+      }
+      s16 += stage16;
+      if (++st == g.nstage) { st = 0; s16 = 0; phase ^= 1; }
+    }
+    if (ok && leader) {
+      if (CG == 2) mma_commit_pair(&sh.accfull[ab], BOTH);
+      else mma_commit(&sh.accfull[ab]);
+    }
+  }
+  // every MMA issued (also on an abort) has finished before TMEM is freed
+  if (leader) {
+    if (CG == 2) mma_commit_pair(&sh.mmadone, 1);
+    else mma_commit(&sh.mmadone);
+    mbar_wait(&sh.mmadone, 0, nullptr, err, ERR_WAIT_ACCUM);
+  }
+}
+
+}  // namespace sc
+
+// KCRS weights -> the weight operand of a problem's plan, one 16-byte word
+// per thread.
+template <int CG>
+__device__ __forceinline__ void shift_weight_body(const KernelParam& p, uint8_t* wop) {
+  using namespace sc;
+  const Plan g = unpack_plan(p, CG);
+  const long long nword = (long long)(weight_bytes(g, CG) >> 4);
+  const long long wi = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (wi >= nword) return;
+  // (row of the operand, 16-channel block, tap, half), halves fastest, so
+  // neighbouring threads read one output channel's weights
+  const int hh = (int)(wi & 1);
+  const long long r2 = wi >> 1;
+  const int row = (int)(r2 / g.NKS), ks = (int)(r2 - (long long)row * g.NKS);
+  const int cb = ks / g.taps, tap = ks - cb * g.taps;
+  const int k0 = row / g.NB * g.NB, rk = row - k0;
+  const int rows = unit_n(g, CG, k0) / CG, rank = rk / rows, rr = rk - rank * rows;
+  const unsigned short* w = static_cast<const unsigned short*>(p.pweight);
+  uint32_t v[4];
+#pragma unroll
+  for (int e = 0; e < 8; e += 2) {
+    const int c = cb * 16 + hh * 8 + e;
+    uint32_t lo = 0, hi = 0;
+    if (row < g.K && c < g.C) lo = w[((size_t)row * g.C + c) * g.taps + tap];
+    if (row < g.K && c + 1 < g.C) hi = w[((size_t)row * g.C + c + 1) * g.taps + tap];
+    v[e >> 1] = lo | (hi << 16);
+  }
+  uint8_t* dst = wop + ((size_t)(k0 + rank * rows) * g.NKS + (size_t)ks * rows) * 32 + (rr >> 3) * 256 + hh * 128 +
+                 (rr & 7) * 16;
+  *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+// The kernel body.  CG = 2: clusters of two CTAs (__cluster_dims__(2, 1, 1)),
+// a unit is 256 positions, rank 0 issues the pair's MMAs.  `wop`: the weight
+// operand.
+template <int CG>
+__device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint8_t* wop, uint32_t* err) {
+  using namespace sc;
+  extern __shared__ __align__(128) uint8_t shift_smem[];
+  __shared__ Shared sh;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(shift_smem) + 127) & ~uintptr_t(127));
+  // a warp-uniform warp index (and below tensor memory base), so that what
+  // the MMA warp derives stays in uniform registers
+  const int warp = __shfl_sync(0xffffffffu, (int)warp_id(), 0), lane = lane_id();
+  const Plan g = unpack_plan(p, CG);
+  const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
+  const int u0 = CG == 2 ? (int)cluster_id_x() : (int)blockIdx.x;
+  const int ustep = CG == 2 ? (int)cluster_count_x() : (int)gridDim.x;
+  const int cnt = u0 < g.units ? (g.units - 1 - u0) / ustep + 1 : 0;
+  const int stage_bytes = g.stageA + g.stageB;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < MAXSTAGE; ++s) {
+      // producers, padding, weights (and at a pair's rank 0 the peer's whole stage)
+      mbar_init(&sh.full[s], NWARP_P + NWARP_Z + 1 + (CG == 2 && rank == 0 ? 1 : 0));
+      mbar_init(&sh.empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&sh.accfull[a], 1);
+      mbar_init(&sh.accempty[a], CG * NWARP_E);
+    }
+    mbar_init(&sh.mmadone, 1);
+    sh.abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == WARP_MMA) {
+    if (CG == 2) { tmem_alloc_pair(&sh.tmem_base, 512); tmem_relinquish_pair(); }
+    else { tmem_alloc(&sh.tmem_base, 512); tmem_relinquish(); }
+    for (int t = lane; t < g.taps; t += 32) {
+      const int r = t / g.S, s = t - r * g.S;
+      sh.aoff[t] = tap_row(g, r, s);
+    }
+  }
+  volatile int* abort_flag = &sh.abort_flag;
+  const uint32_t sbase = smem_u32(smem);
+
+  if (warp >= WARP_MMA && warp < WARP_P0) {
+    regs_dec<REGS_MMA>();
+    setup_sync<CG>();
+    if (warp == WARP_LOAD) {
+      // weight pieces of a stage: (16-channel block, tap), one bulk copy each
+      // from its own lane; this CTA's rows of the unit's output channels
+      int st = 0;
+      uint32_t phase = 1;
+      bool ok = true;
+      int issued = 0;
+      for (int i = 0; ok && i < cnt && !*abort_flag; ++i) {
+        int pt, k0;
+        unit_of(g, u0 + i * ustep, pt, k0);
+        const uint32_t piece = (uint32_t)(unit_n(g, CG, k0) / CG) * 32;      // one tap of 16 channels
+        const uint8_t* src = wop + (size_t)k0 * g.NKS * 32 + (size_t)rank * piece * g.NKS;
+        for (int j = 0; j < g.nst; ++j) {
+          if (!mbar_wait_warp(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY, 0)) { ok = false; break; }
+          const uint32_t np = (uint32_t)(min(g.cps, g.CB - j * g.cps) * g.taps);
+          if (lane == 0) mbar_arrive_expect_tx(&sh.full[st], piece * np);
+          __syncwarp();
+          uint8_t* dst = smem + st * stage_bytes + g.stageA;
+          const uint8_t* from = src + (size_t)j * g.cps * g.taps * piece;
+          const uint32_t a = piece * (np * lane / NCOPY), b = piece * (np * (lane + 1) / NCOPY);
+          if (lane < NCOPY && b > a) bulk_g2s(dst + a, from + a, b - a, &sh.full[st]);
+          ++issued;
+          if (++st == g.nstage) { st = 0; phase ^= 1; }
+        }
+      }
+      // copies still in flight land before the CTA leaves (an abort may have
+      // kept the MMA side from waiting for them)
+      if (*abort_flag) {
+        if (lane == 0)
+          for (int b = issued > g.nstage ? issued - g.nstage : 0; b < issued; ++b)
+            mbar_wait(&sh.full[b % g.nstage], (b / g.nstage) & 1, nullptr, err, ERR_WAIT_FULL);
+      }
+    } else if (warp >= WARP_Z0) {
+      pad_rows(g, smem, sh, threadIdx.x - WARP_Z0 * 32, u0, ustep, cnt, rank * TM, TM * CG, err);
+    } else {
+      const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem_base, 0);
+      if (CG == 2 && rank == 1) {
+        // tell rank 0 that this CTA's half of each stage is complete
+        const uint32_t lead = mapa_shared(smem_u32(&sh.full[0]), 0);
+        int st = 0;
+        uint32_t phase = 0;
+        for (int left = cnt * g.nst; left > 0; --left) {
+          if (!wait_all_lanes(&sh.full[st], phase, abort_flag, err, ERR_WAIT_FULL)) break;
+          if (lane == 0) mbar_arrive_remote(lead + st * 8);
+          if (++st == g.nstage) { st = 0; phase ^= 1; }
+        }
+      } else if (g.taps == 9) {
+        issue_mmas<CG, 9>(g, sh, sbase, tmem, u0, ustep, cnt, err);
+      } else if (g.taps == 1) {
+        issue_mmas<CG, 1>(g, sh, sbase, tmem, u0, ustep, cnt, err);
+      } else {
+        issue_mmas<CG, 0>(g, sh, sbase, tmem, u0, ustep, cnt, err);
+      }
+    }
+    __syncwarp();
+  } else if (warp < NWARP_E) {
+    regs_dec<REGS_EPI>();
+    setup_sync<CG>();
+    const uint32_t tmem = sh.tmem_base;
+    // epilogue: TMEM lane 32 * quarter + lane = position of this CTA's tile
+    const int quarter = warp;
+    __half* Y = static_cast<__half*>(p.pout);
+    const int OHOW = g.OH * g.OW;
+    const Grid gr = make_grid(g);
+    // even output rows sit on an even grid: neighbouring outputs on lanes 2i,
+    // 2i + 1 share 4-byte stores
+    const bool pair = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 3) == 0;
+    const uint32_t lead_accempty = mapa_shared(smem_u32(&sh.accempty[0]), 0);
+    for (int ui = 0; ui < cnt; ++ui) {
+      int pt, k0;
+      unit_of(g, u0 + ui * ustep, pt, k0);
+      const int nrows = min(g.NB, g.Kp - k0);
+      const int kval = min(nrows, g.K - k0);             // output channels that exist
+      const int ab = ui & 1;
+      const Base c = advance(gr, tile_base(gr, pt * (TM * CG) + rank * TM), quarter * 32 + lane);
+      const bool live = c.n < g.N && c.gy < g.OH && c.gx < g.OW;
+      __half* yb = live ? Y + ((size_t)c.n * g.K + k0) * OHOW + (size_t)c.gy * g.OW + c.gx : Y;
+      if (!mbar_wait_warp(&sh.accfull[ab], (ui >> 1) & 1, abort_flag, err, ERR_WAIT_ACCUM, SLEEP_NS)) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + ab * 256;
+      auto ld = [&](int cc, float* v) {
+        tmem_ld16(taddr + cc, v);
+        if (cc + 16 < nrows) tmem_ld16(taddr + cc + 16, v + 16);
+      };
+      auto stc = [&](int cc, const float* v) {
+        store_cols_f16<32>(yb + (size_t)cc * OHOW, (size_t)OHOW, v, kval - cc, live, pair);
+      };
+      float va[32], vb[32];
+      ld(0, va);
+      tmem_ld_wait();
+      for (int cc = 0; cc < nrows; cc += 64) {
+        if (cc + 32 < nrows) ld(cc + 32, vb);
+        stc(cc, va);
+        tmem_ld_wait();
+        if (cc + 32 >= nrows) break;
+        if (cc + 64 < nrows) ld(cc + 64, va);
+        stc(cc + 32, vb);
+        tmem_ld_wait();
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_peer(lead_accempty + ab * 8);
+        else mbar_arrive(&sh.accempty[ab]);
+      }
+    }
+  } else {
+    regs_inc<REGS_PROD>();
+    const int group = (warp - WARP_P0) / NWARP_P, tid = threadIdx.x - (WARP_P0 + group * NWARP_P) * 32;
+    const int nitem = 2 * g.cps * g.qmax;
+    const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(p.pin) & 7) == 0;
+    const int tp = rank * TM, ts = TM * CG;
+    const bool strided = g.U > 1 || g.V > 1;
+#define SC_PRODUCE(ni, depth, al, strd) produce<CG, ni, depth, al, strd>(g, p, smem, sh, tid, group, u0, ustep, cnt, tp, ts, err)
+    if (aligned && !strided) {
+      if (nitem <= NPROD) SC_PRODUCE(1, 2, true, false);
+      else if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, false);
+      else SC_PRODUCE(4, 1, true, false);
+    } else if (aligned) {
+      if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, true);
+      else if (nitem <= 4 * NPROD) SC_PRODUCE(4, 1, true, true);
+      else SC_PRODUCE(6, 1, true, true);
+    } else if (!strided) {
+      if (nitem <= NPROD) SC_PRODUCE(1, 2, false, false);
+      else SC_PRODUCE(2, 1, false, false);
+    } else {
+      SC_PRODUCE(2, 1, false, true);
+    }
+#undef SC_PRODUCE
+  }
+  tc_fence_before();
+  __syncthreads();
+  // the peer may still read this CTA's shared memory or arrive on its
+  // barriers until both CTAs get here
+  if (CG == 2) cluster_sync();
+  if (warp == WARP_MMA) {
+    tc_fence_after();
+    if (CG == 2) tmem_dealloc_pair(sh.tmem_base, 512);
+    else tmem_dealloc(sh.tmem_base, 512);
+  }
+}
+
+}  // namespace wino

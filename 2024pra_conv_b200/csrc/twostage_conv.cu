@@ -66,6 +66,7 @@
 #include "tc_sm100.cuh"
 #include "wino_common.cuh"
 #include "vgen.cuh"
+#include "shift_conv.cuh"
 
 // Load instruction of the tap-pair producers' window words: through L1
 // (ld.global.nc) by default, or cached in L2 only (ld.global.cg).
@@ -1176,9 +1177,19 @@ __device__ __forceinline__ Prod prod(const Geo& g, const uint8_t* xr, int t, int
 // output channel) U scale su (p.pweight, fp32 [16][K]) before rounding M.
 // F8 = 1: single e4m3 terms (one MMA per K-step, one byte per tile and
 // channel, a K-step of 32 channels per piece).
+// The fp16 bulk-copy variant, launched without a mid_result, computes outputs
+// instead of M: the one-CTA shift-reuse implicit GEMM (shift_conv.cuh), which
+// needs no M and no pre-pass (transform_pin then carries its packed plan).
 template <bool TMAV, int F8 = 0>
-__global__ void __launch_bounds__(TMAV ? trs::NTHREAD_V : trs::NTHREAD, 1) twostage_res_kernel_t(KernelParam p) {
+__global__ void __launch_bounds__(TMAV && F8 ? trs::NTHREAD_V : trs::NTHREAD, 1) twostage_res_kernel_t(KernelParam p) {
   static_assert(F8 == 0 || TMAV, "the fp8 variants read V2 by bulk copy");
+  static_assert(trs::NTHREAD == sc::NTHREAD && sc::SMEM_BYTES <= 227 * 1024, "one kernel hosts both schedules");
+  if constexpr (TMAV && F8 == 0) {
+    if (p.mid_result == nullptr) {
+      shift_conv_body<1>(p, static_cast<const uint8_t*>(p.transform_filter), &g_twostage_err);
+      return;
+    }
+  }
   constexpr int TERMS = F8 == 1 ? 1 : 2;        // bytes per tile and channel in V2 and U
   using namespace trs;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1925,6 +1936,7 @@ __global__ void __launch_bounds__(ot::NTHREAD, WINO_OT_MINB) twostage_output_ker
   using namespace ts;
   extern __shared__ __align__(128) uint8_t osm[];
   __shared__ uint64_t full[ot::NBUF];
+  if (p.mid_result == nullptr) return;    // slot 3 wrote the outputs itself
   const int K = p.k, P = p.Oh, Q = p.Ow;
   const int TP = (P + 1) >> 1, TQ = (Q + 1) >> 1;
   const long long NT = (long long)p.n * TP * TQ;
@@ -2121,7 +2133,7 @@ int wino_twostage_prepare() {
   if (cudaFuncSetAttribute(twostage_res_kernel_t<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            trs::SMEM_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(twostage_res_kernel_t<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           trs::SMEM_BYTES) != cudaSuccess ||
+                           sc::SMEM_BYTES > trs::SMEM_BYTES ? sc::SMEM_BYTES : trs::SMEM_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(twostage_res_kernel_t<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            trs::SMEM_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(twostage_res_kernel_t<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2131,6 +2143,8 @@ int wino_twostage_prepare() {
   // launched with; any other launch count would leave an increase waiting
   cudaFuncAttributes fa{};
   if (cudaFuncGetAttributes(&fa, twostage_res_kernel_t<false>) != cudaSuccess || fa.numRegs != trs::REGS_LAUNCH)
+    return 1;
+  if (cudaFuncGetAttributes(&fa, twostage_res_kernel_t<true>) != cudaSuccess || fa.numRegs != sc::REGS_LAUNCH)
     return 1;
   return (int)cudaFuncSetAttribute(twostage_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    tp::SMEM_BYTES);

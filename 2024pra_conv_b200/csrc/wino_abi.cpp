@@ -111,6 +111,17 @@ unsigned wino_igemm_grid(int n, int k, int oh, int ow, int sms);
 int wino_igemm_shape_ok(int n, int c, int h, int w, int k, int oh, int ow);
 int wino_igemm_prepare();
 uint32_t wino_igemm_error_read_clear();
+int wino_shift_cg(const wino::KernelParam* p);
+unsigned long long wino_shift_pack(const wino::KernelParam* p, int cg);
+unsigned wino_shift_grid(const wino::KernelParam* p, int cg, int sms);
+size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
+unsigned wino_shift_weight_grid(const wino::KernelParam* p, int cg);
+void* wino_shift_weight_kernel_ptr(int cg);
+void* wino_shift_kernel_ptr(int cg);
+int wino_shift_threads();
+int wino_shift_smem_bytes();
+int wino_shift_prepare();
+uint32_t wino_shift_error_read_clear();
 }
 
 namespace {
@@ -223,17 +234,74 @@ int check_general(long long n, long long c, long long h, long long w, long long 
   return WINO_OK;
 }
 
+// The shift-reuse implicit GEMM (shift_conv.cuh) for a drop-in problem: CTAs a
+// unit and the workspace that holds its weight operand, or cg = 0.
+struct ShiftPlan {
+  int cg;
+  void* wop;
+};
+
+// Direct-conv FLOPs from which the drop-in takes the shift kernel.  Below it
+// every route is bound by its launches (N1 C16 16x16 K16: 8 us of kernels on
+// either), and the two-stage route's results stay bit-identical to
+// wino_conv2d_twostage there.
+constexpr double kShiftMinFlops = 64e6;
+
+static ShiftPlan plan_shift(const problem_t& pr, int oh, int ow) {
+  const ShiftPlan none{0, nullptr};
+  if (pr.r * pr.s == 1 || !pr.transform_filter) return none;
+  if (2.0 * pr.n * pr.k * oh * ow * pr.c * pr.r * pr.s < kShiftMinFlops) return none;
+  wino::KernelParam p{};
+  p.pin = pr.in;
+  p.n = (short)pr.n; p.c = (short)pr.c; p.h = (short)pr.h; p.w = (short)pr.w; p.k = (short)pr.k;
+  p.r = (short)pr.r; p.s = (short)pr.s; p.u = (short)pr.u; p.v = (short)pr.v; p.p = (short)pr.p; p.q = (short)pr.q;
+  p.Oh = (short)oh; p.Ow = (short)ow;
+  int cg = wino_shift_cg(&p);
+  if (cg == 0) return none;
+  // weight operand: the caller's transform_filter (16*k*c fp16), else its
+  // transform_pin (4*h*h*n*c fp16); reference src/main.cpp:36-38
+  const size_t filter_bytes = (size_t)16 * pr.k * pr.c * 2, pin_bytes = (size_t)4 * pr.h * pr.h * pr.n * pr.c * 2;
+  for (; cg >= 1; --cg) {
+    const size_t need = wino_shift_weight_bytes(&p, cg);
+    if (need <= filter_bytes && (reinterpret_cast<uintptr_t>(pr.transform_filter) & 15) == 0)
+      return ShiftPlan{cg, pr.transform_filter};
+    if (pr.transform_pin && need <= pin_bytes && (reinterpret_cast<uintptr_t>(pr.transform_pin) & 15) == 0)
+      return ShiftPlan{cg, pr.transform_pin};
+  }
+  return none;
+}
+
+// Two-stage route (input transform fused into full-width tap GEMMs, M in the
+// caller's mid_result, output transform in slot 4): M fits the reference's
+// mid_result size of 4*k*h*w*n fp16 elements (even H and W) and the pre-pass
+// records fit transform_pin.
+static bool two_stage_fits(const problem_t& pr) {
+  return pr.transform_pin != nullptr && (reinterpret_cast<uintptr_t>(pr.transform_pin) & 15) == 0 &&
+         pr.mid_result != nullptr && (reinterpret_cast<uintptr_t>(pr.mid_result) & 15) == 0 &&
+         twostage_ok((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w) &&
+         wino_twostage_prepass_bytes((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w) <=
+             (size_t)4 * pr.h * pr.h * pr.n * pr.c * 2 &&
+         wino_twostage_m_bytes((int)pr.n, (int)pr.h, (int)pr.w, (int)pr.k) <= (size_t)4 * pr.k * pr.h * pr.w * pr.n * 2;
+}
+
+// 3x3 / stride 1 / pad 1 with 16-channel multiples and a U-cache workspace.
+static bool wino_contract(const problem_t& pr) {
+  return pr.r == 3 && pr.s == 3 && pr.u == 1 && pr.v == 1 && pr.p == 1 && pr.q == 1 &&
+         wino_check_shape((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w, (int)pr.k) == WINO_OK &&
+         pr.transform_filter != nullptr;
+}
+
 // Route of getkernelInfo for a validated problem (no CUDA calls).
-static int plan_route(const problem_t& pr) {
-  // Winograd F(2x2,3x3) for 3x3 / stride 1 / pad 1 with 16-channel multiples
-  // and a U-cache workspace; every other shape goes to the direct kernel.
-  const bool wino = pr.r == 3 && pr.s == 3 && pr.u == 1 && pr.v == 1 && pr.p == 1 && pr.q == 1 &&
-                    wino_check_shape((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w, (int)pr.k) == WINO_OK &&
-                    pr.transform_filter != nullptr;
-  if (!wino) {
+static int plan_route(const problem_t& pr, ShiftPlan* shift) {
+  const int oh = (int)((pr.h - pr.r + 2 * pr.p) / pr.u + 1), ow = (int)((pr.w - pr.s + 2 * pr.q) / pr.v + 1);
+  *shift = plan_shift(pr, oh, ow);
+  // (outside the contract it is the implicit-GEMM route with another kernel)
+  if (shift->cg) return wino_contract(pr) ? WINO_ROUTE_SHIFT : WINO_ROUTE_IGEMM;
+  // Winograd F(2x2,3x3) inside its contract; every other shape goes to the
+  // implicit GEMM or the direct kernel.
+  if (!wino_contract(pr)) {
     // Tensor-core implicit GEMM when its re-laid-out weights fit the
     // caller's transform_filter (16*k*c fp16, reference src/main.cpp:38).
-    const int oh = (int)((pr.h - pr.r + 2 * pr.p) / pr.u + 1), ow = (int)((pr.w - pr.s + 2 * pr.q) / pr.v + 1);
     const bool igemm = pr.transform_filter != nullptr &&
                        (reinterpret_cast<uintptr_t>(pr.transform_filter) & 15) == 0 &&
                        wino_igemm_operand_bytes((int)pr.c, (int)pr.k, (int)pr.r, (int)pr.s) <=
@@ -250,20 +318,7 @@ static int plan_route(const problem_t& pr) {
                       (reinterpret_cast<uintptr_t>(pr.transform_pin) & 15) == 0 &&
                       wino_xb_bytes((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w) <= pin_ws_bytes &&
                       xb_items_ok((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w);
-  // Two-stage route (input transform fused into full-width tap GEMMs, M in
-  // the caller's mid_result, output transform in slot 4) whenever M fits the
-  // reference's mid_result size of 4*k*h*w*n fp16 elements (even H and W) and
-  // the pre-pass records fit transform_pin.
-  const bool two_stage = pr.transform_pin != nullptr &&
-                         (reinterpret_cast<uintptr_t>(pr.transform_pin) & 15) == 0 &&
-                         pr.mid_result != nullptr &&
-                         (reinterpret_cast<uintptr_t>(pr.mid_result) & 15) == 0 &&
-                         twostage_ok((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w) &&
-                         wino_twostage_prepass_bytes((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w) <=
-                             pin_ws_bytes &&
-                         wino_twostage_m_bytes((int)pr.n, (int)pr.h, (int)pr.w, (int)pr.k) <=
-                             (size_t)4 * pr.k * pr.h * pr.w * pr.n * 2;
-  if (two_stage) return WINO_ROUTE_TWOSTAGE;
+  if (two_stage_fits(pr)) return WINO_ROUTE_TWOSTAGE;
   return use_xb ? WINO_ROUTE_FUSED_XB : WINO_ROUTE_FUSED;
 }
 
@@ -274,8 +329,9 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
   const int st = check_general(pr.n, pr.c, pr.h, pr.w, pr.k, pr.r, pr.s, pr.u, pr.v, pr.p, pr.q, &oh, &ow);
   if (st != WINO_OK) return st;
   if (!pr.in || !pr.weight || !pr.out) return WINO_EINVAL;
-  int route = plan_route(pr);
-  if (route == WINO_ROUTE_IGEMM && wino_igemm_prepare() != 0) route = WINO_ROUTE_DIRECT;
+  ShiftPlan shift{};
+  int route = plan_route(pr, &shift);
+  if (route == WINO_ROUTE_IGEMM && shift.cg == 0 && wino_igemm_prepare() != 0) route = WINO_ROUTE_DIRECT;
   const bool wino = route != WINO_ROUTE_DIRECT && route != WINO_ROUTE_IGEMM;
 
   mykernelParamType* a = static_cast<mykernelParamType*>(param);
@@ -290,6 +346,32 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
   a->Oh = (short)oh; a->Ow = (short)ow;
   std::memset(kernelInfo, 0, sizeof(*kernelInfo));
 
+  if (shift.cg != 0) {
+    if (wino_shift_prepare() != 0 || wino_twostage_prepare() != 0) return WINO_ECUDA;
+    a->transform_filter = static_cast<_Float16*>(shift.wop);
+    a->mid_result = nullptr;
+    wino::KernelParam* kp = static_cast<wino::KernelParam*>(param);
+    // the packed plan travels in transform_pin, which the kernels need no
+    // pointer in
+    kp->transform_pin = nullptr;
+    kp->transform_pin = reinterpret_cast<void*>(wino_shift_pack(kp, shift.cg));
+    set_slot(kernelInfo, 1, wino_shift_weight_grid(kp, shift.cg), 1, 1, 256, 1, 1, 0,
+             wino_shift_weight_kernel_ptr(shift.cg));
+    set_slot(kernelInfo, 2, 1, 1, 1, 32, 1, 1, 0, wino_noop_kernel_ptr());
+    // Problems of the two-stage route keep its slot 3 and 4 kernels, by which
+    // callers tell the route: given no mid_result, its GEMM kernel runs the
+    // one-CTA shift schedule and its output transform has nothing to do.
+    const bool hosted = shift.cg == 1 && pr.c <= 256 && wino_contract(pr) && two_stage_fits(pr);
+    set_slot(kernelInfo, 3, wino_shift_grid(kp, shift.cg, sm_count()), 1, 1, (unsigned)wino_shift_threads(), 1, 1,
+             (unsigned)wino_shift_smem_bytes(),
+             hosted ? wino_twostage_gemm_kernel_ptr_for((int)pr.c) : wino_shift_kernel_ptr(shift.cg));
+    if (hosted)
+      set_slot(kernelInfo, 4, 1, 1, 1, (unsigned)wino_twostage_output_threads(), 1, 1, 0,
+               wino_twostage_output_kernel_ptr());
+    else
+      set_slot(kernelInfo, 4, 1, 1, 1, 32, 1, 1, 0, wino_noop_kernel_ptr());
+    return WINO_OK;
+  }
   if (route == WINO_ROUTE_IGEMM) {
     int mode = wino_igemm_mode(pr.in, (int)pr.k, (int)pr.h, (int)pr.w, (int)pr.r, (int)pr.s, (int)pr.u,
                                (int)pr.v, (int)pr.p, (int)pr.q);
@@ -368,7 +450,8 @@ extern "C" int wino_dropin_route(const void* problem) {
   const int st = check_general(pr.n, pr.c, pr.h, pr.w, pr.k, pr.r, pr.s, pr.u, pr.v, pr.p, pr.q, &oh, &ow);
   if (st != WINO_OK) return -st;
   if (!pr.in || !pr.weight || !pr.out) return -WINO_EINVAL;
-  return plan_route(pr);
+  ShiftPlan shift{};
+  return plan_route(pr, &shift);
 }
 
 extern "C" int wino_getParamsize(problem_t* problem, int* paramSize) {
@@ -700,7 +783,11 @@ extern "C" int wino_launch_kernelinfo(const void* kiv, void* param, void* stream
   if (!ki || !param) return WINO_EINVAL;
   const unsigned* slots[4] = {&ki->blockx1, &ki->blockx2, &ki->blockx3, &ki->blockx4};
   void* const fns[4] = {ki->kernelPtr1, ki->kernelPtr2, ki->kernelPtr3, ki->kernelPtr4};
+  // slots whose kernel has nothing to do are not launched: the empty kernel,
+  // and the two-stage output transform without an M
+  const bool no_m = static_cast<const wino::KernelParam*>(param)->mid_result == nullptr;
   for (int i = 0; i < 4; ++i) {
+    if (fns[i] == wino_noop_kernel_ptr() || (no_m && fns[i] == wino_twostage_output_kernel_ptr())) continue;
     const unsigned* b = slots[i];
     const cudaError_t e = cudaLaunchKernel(fns[i], dim3(b[0], b[1], b[2]), dim3(b[3], b[4], b[5]),
                                            (void**)&param, (size_t)b[6], (cudaStream_t)stream);
@@ -715,6 +802,7 @@ extern "C" int wino_error_read_clear(uint32_t* code) {
   const uint32_t b = wino_unfused_error_read_clear();
   const uint32_t c = wino_twostage_error_read_clear();
   const uint32_t d = wino_igemm_error_read_clear();
-  *code = a ? a : (b ? b : (c ? c : d));
+  const uint32_t e = wino_shift_error_read_clear();
+  *code = a ? a : (b ? b : (c ? c : (d ? d : e)));
   return WINO_OK;
 }

@@ -25,6 +25,16 @@
  *     kernels go in the slots depends on the shape and on which workspaces
  *     are usable (wino_dropin_route in winoconv.h reports the choice):
  *
+ *     shift route: any filter of two to 64 taps with strides 1 or 2 from 64
+ *       MFLOP on (2*n*k*Oh*Ow*c*r*s; a position tile's input must fit the
+ *       kernel's shared memory, in practice w up to about 400):
+ *         slot 1  weight -> transform_filter (tensor-core operand; to
+ *                 transform_pin where it does not fit there)
+ *         slot 3  shift-reuse implicit GEMM reading `in` directly -> out;
+ *                 slots 2, 4 have nothing to do.
+ *       mid_result is left untouched, and so is transform_pin unless it holds
+ *       the weights.  For smaller problems, and what this route does not
+ *       take:
  *     two-stage route: r = s = 3, u = v = 1, p = q = 1, c % 16 == k % 16
  *       == 0, even h and w, all three workspaces present, transform_pin
  *       16-byte aligned and large enough for the pre-pass output:
@@ -49,7 +59,7 @@
  *       16-byte aligned or too small): slot 2 is an empty kernel and the
  *       fused kernel reads `in` directly; transform_pin and mid_result are
  *       left untouched.
- *     implicit-GEMM route: any other shape (filter size, stride, padding,
+ *     implicit-GEMM route: 1x1 filters, and any other shape (filter size, stride, padding,
  *       channel counts not multiples of 16) whose re-laid-out weights,
  *       r*s*ceil(c/16)*round16(k) rows of 32 bytes, fit transform_filter
  *       (non-null, 16-byte aligned): slot 1 weight -> transform_filter in the
