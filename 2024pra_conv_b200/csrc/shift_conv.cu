@@ -59,7 +59,7 @@ int wino_shift_cg(const KernelParam* p) {
   const int n2 = g2.Kp < 256 ? (g2.Kp + 31) / 32 * 32 : 256;
   // a pair needs work for every pair of SMs
   if (g2.units < sc::NSM / 2) return 1;
-  const long long t1 = w1 * sc::mma_cycles(g1.Kp < g1.NB ? g1.Kp : g1.NB), t2 = w2 * sc::mma_cycles(n2);
+  const long long t1 = w1 * sc::mma_cycles(1, g1.Kp < g1.NB ? g1.Kp : g1.NB), t2 = w2 * sc::mma_cycles(2, n2);
   return t2 <= t1 ? 2 : 1;
 }
 

@@ -51,10 +51,9 @@
 // per unit block of output channels and CTA of the unit, 16-channel block by
 // 16-channel block, tap by tap, each piece the K-major core-matrix
 // interleave (row k, channel c at (k >> 3) * 256 + (c >> 3) * 128 + (k & 7)
-// * 16 + (c & 7) * 2).  A stage is then one run of up to 36 KB, copied by
-// NCOPY lanes: a bulk copy costs ~190 cycles of the copy engine whatever its
-// size up to a few KB, and one copy per tap held a stage of nine MMAs at
-// 1.8 k cycles.
+// * 16 + (c & 7) * 2).  A stage is then one run of up to 36 KB
+// and one bulk copy (one per tap issued no faster than a stage per 1.8 k
+// cycles; splitting the run over lanes gained nothing).
 //
 // The reference computes only 3x3 / stride 1 / pad 1 and round-trips V and M
 // through HBM (src/preprocessing.cuh:273-424, src/matrixmul.cuh:139-556,
@@ -71,7 +70,6 @@ namespace sc {
 constexpr int TM = 128;                   // positions per CTA and unit
 constexpr int MAXTAP = 64;
 constexpr int MAXSTAGE = 8;
-constexpr int NCOPY = 4;                  // bulk copies a stage's weights are split into
 constexpr int SMEM_STAGES = 225 * 1024;   // dynamic shared memory of the stages
 constexpr int SMEM_BYTES = SMEM_STAGES + 128;
 constexpr int NSM = 148;                  // SMs of a B200 (the rules below count units against them)
@@ -144,9 +142,12 @@ __host__ __device__ __forceinline__ int plane_rows(const Plan& g, int a, int b) 
   return TM + div_stride(g.R - 1 - a, g.U) * g.GX + div_stride(g.S - 1 - b, g.V);
 }
 
-// Tensor-pipe cycles of one MMA of N output channels as they issue here
-// (M = 128 per SM, K = 16: 56 up to N = 64, then N / 2).
-__host__ __device__ __forceinline__ int mma_cycles(int n) { return n <= 112 ? 56 : n >> 1; }
+// Cycles of one MMA of N output channels (issue_mmas): its arithmetic, or its
+// shared-memory reads; a pair's CTAs read half of B each.
+__host__ __device__ __forceinline__ int mma_cycles(int cg, int n) {
+  const int reads = 64 + n / (4 * cg), math = n >> 1;
+  return reads > math ? reads : math;
+}
 
 __host__ __device__ __forceinline__ void plan_dims(Plan& g, const KernelParam& p) {
   g.N = p.n; g.C = p.c; g.H = p.h; g.W = p.w; g.K = p.k; g.R = p.r; g.S = p.s;
@@ -194,7 +195,7 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg) {
     long long best_t = -1;
     for (int nb = 128; nb >= 32; nb >>= 1) {
       const long long tiles = (g.npos + TM - 1) / TM, un = tiles * ((g.Kp + nb - 1) / nb);
-      const long long t = ((un + NSM - 1) / NSM) * mma_cycles(g.Kp < nb ? g.Kp : nb);
+      const long long t = ((un + NSM - 1) / NSM) * mma_cycles(1, g.Kp < nb ? g.Kp : nb);
       if (best_t < 0 || t < best_t) { best_t = t; g.NB = nb; }
     }
   }
@@ -209,13 +210,17 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg) {
   const long long imgs = lines / g.GY + 2;
   const long long q = px / 4 + 2 + ((g.H * g.W) % 4 ? imgs : 0);
   g.qmax = (int)(q < 4096 ? q : 4096);
-  // several 16-channel blocks a stage where a block has few taps
-  int cps = g.taps >= 6 ? 1 : g.taps >= 3 ? 2 : 4;
+  // Several 16-channel blocks a stage where a block has few taps, and two of a
+  // 3x3 filter's where four stages still fit (at most 64 output channels a
+  // CTA): the producers' and the MMA thread's work per stage then covers twice
+  // the MMAs.
+  int cps = g.taps >= 3 ? 2 : 4;
   while (cps > 1 && (cps >> 1) >= g.CB) cps >>= 1;
   for (;; cps >>= 1) {
     g.lcps = cps == 4 ? 2 : cps == 2 ? 1 : 0;
     plan_finish(g, cg);
-    if (cps == 1 || (2 * cps * g.qmax <= 3 * NPROD && 3 * (g.stageA + g.stageB) <= SMEM_STAGES)) break;
+    const int items = g.taps >= 6 ? 2 * NPROD : 3 * NPROD, stages = g.taps >= 6 ? 4 : 3;
+    if (cps == 1 || (2 * cps * g.qmax <= items && stages * (g.stageA + g.stageB) <= SMEM_STAGES)) break;
   }
   const int fit = SMEM_STAGES / (g.stageA + g.stageB);
   g.nstage = fit < MAXSTAGE ? fit : MAXSTAGE;
@@ -607,27 +612,30 @@ __device__ __forceinline__ int tap_row(const Plan& g, int r, int s) {
 
 // MMA issue: per stage and 16-channel block one MMA a tap, all on the same
 // staged input.  The whole warp runs the loop and one elected lane issues, so
-// the descriptors stay in uniform registers.  TAPS > 0: that many taps,
-// their shifts kept in registers and the taps unrolled, so
-// that an MMA costs the warp a couple of adds: one warp feeds the tensor
-// pipe, and with the shifts read from shared memory inside the loop it
-// managed one N = 64 MMA per 92 cycles against the pipe's 56.
+// descriptors stay in uniform registers (from one lane's branch a stage of
+// nine took 960 cycles to issue against 800).  An MMA here costs its shared-memory reads: 64 cycles
+// for the 128 rows of A, which a shift takes off the 128-byte lines, plus a
+// cycle per 4 rows of B (N = 64: 80 cycles a CTA; a pair's N = 256 is at its
+// arithmetic 128).  The pipe takes an MMA ahead at most, so what the thread
+// does between stages shows: the next stage's barrier is polled in the middle
+// of a stage, and only if it was not ready then is it waited for.  TAPS > 0:
+// that many taps, their shifts kept in registers.
 template <int CG, int TAPS>
 __device__ __forceinline__ void issue_mmas(const Plan& g, Shared& sh, uint32_t sbase, uint32_t tmem, int u0, int ustep,
                                            int cnt, uint32_t* err) {
   constexpr uint16_t BOTH = 3;
   constexpr int NOFF = TAPS > 0 ? TAPS : 1;
   volatile int* abort_flag = &sh.abort_flag;
-  const bool leader = elect_one();
   const uint32_t stage16 = (uint32_t)(g.stageA + g.stageB) >> 4, a16 = (uint32_t)g.stageA >> 4;
   const uint64_t adesc0 = smem_desc(sbase, (uint32_t)g.rows * 16, 128), bdesc0 = smem_desc(sbase, 128, 256) + a16;
   const uint32_t qstep = (uint32_t)g.rows * 2;
+  const bool leader = elect_one();
   uint32_t off[NOFF];
 #pragma unroll
   for (int t = 0; t < NOFF; ++t) off[t] = (uint32_t)__shfl_sync(0xffffffffu, sh.aoff[t], 0);
   int st = 0;
   uint32_t phase = 0, s16 = 0;
-  bool ok = true;
+  bool ok = true, ready = false;
   for (int i = 0; ok && i < cnt; ++i) {
     int pt, k0;
     unit_of(g, u0 + i * ustep, pt, k0);
@@ -648,16 +656,27 @@ __device__ __forceinline__ void issue_mmas(const Plan& g, Shared& sh, uint32_t s
       }
     };
     for (int j = 0; j < g.nst; ++j) {
-      ok = wait_all_lanes<CG == 2>(&sh.full[st], phase, abort_flag, err, ERR_WAIT_FULL);
-      if (!ok) break;
+      if (!ready) {
+        ok = wait_all_lanes<CG == 2>(&sh.full[st], phase, abort_flag, err, ERR_WAIT_FULL);
+        if (!ok) break;
+      }
       tc_fence_after();
       const int nk = min(g.cps, g.CB - j * g.cps);
+      const int nst_ = st + 1 == g.nstage ? 0 : st + 1;
+      const uint32_t nphase = nst_ == 0 ? phase ^ 1 : phase;
+      auto poll = [&]() {
+        ready = __all_sync(0xffffffffu, mbar_test_wait<CG == 2>(&sh.full[nst_], nphase)) != 0;
+      };
       uint64_t aq = adesc0 + s16, bd = bdesc0 + s16;
       for (int q = 0; q < nk; ++q, aq += qstep) {
         if (TAPS > 0) {
 #pragma unroll
-          for (int t = 0; t < TAPS; ++t, bd += bstep) mma(aq + off[t], bd, t > 0 || j > 0 || q > 0 ? 1u : 0u);
+          for (int t = 0; t < TAPS; ++t, bd += bstep) {
+            mma(aq + off[t], bd, t > 0 || j > 0 || q > 0 ? 1u : 0u);
+            if (t == TAPS / 2 && q + 1 == nk) poll();
+          }
         } else {
+          if (q + 1 == nk) poll();
 #pragma unroll 4
           for (int t = 0; t < g.taps; ++t, bd += bstep)
             mma(aq + (uint32_t)sh.aoff[t], bd, t > 0 || j > 0 || q > 0 ? 1u : 0u);
@@ -667,8 +686,9 @@ __device__ __forceinline__ void issue_mmas(const Plan& g, Shared& sh, uint32_t s
         if (CG == 2) mma_commit_pair(&sh.empty[st], BOTH);
         else mma_commit(&sh.empty[st]);
       }
-      s16 += stage16;
-      if (++st == g.nstage) { st = 0; s16 = 0; phase ^= 1; }
+      st = nst_;
+      phase = nphase;
+      s16 = st == 0 ? 0 : s16 + stage16;
     }
     if (ok && leader) {
       if (CG == 2) mma_commit_pair(&sh.accfull[ab], BOTH);
@@ -726,8 +746,8 @@ __device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint
   extern __shared__ __align__(128) uint8_t shift_smem[];
   __shared__ Shared sh;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(shift_smem) + 127) & ~uintptr_t(127));
-  // a warp-uniform warp index (and below tensor memory base), so that what
-  // the MMA warp derives stays in uniform registers
+  // a warp-uniform warp index, so that what the MMA warp derives stays in
+  // uniform registers
   const int warp = __shfl_sync(0xffffffffu, (int)warp_id(), 0), lane = lane_id();
   const Plan g = unpack_plan(p, CG);
   const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
@@ -765,34 +785,33 @@ __device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint
     regs_dec<REGS_MMA>();
     setup_sync<CG>();
     if (warp == WARP_LOAD) {
-      // weight pieces of a stage: (16-channel block, tap), one bulk copy each
-      // from its own lane; this CTA's rows of the unit's output channels
-      int st = 0;
-      uint32_t phase = 1;
-      bool ok = true;
-      int issued = 0;
-      for (int i = 0; ok && i < cnt && !*abort_flag; ++i) {
-        int pt, k0;
-        unit_of(g, u0 + i * ustep, pt, k0);
-        const uint32_t piece = (uint32_t)(unit_n(g, CG, k0) / CG) * 32;      // one tap of 16 channels
-        const uint8_t* src = wop + (size_t)k0 * g.NKS * 32 + (size_t)rank * piece * g.NKS;
-        for (int j = 0; j < g.nst; ++j) {
-          if (!mbar_wait_warp(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY, 0)) { ok = false; break; }
-          const uint32_t np = (uint32_t)(min(g.cps, g.CB - j * g.cps) * g.taps);
-          if (lane == 0) mbar_arrive_expect_tx(&sh.full[st], piece * np);
-          __syncwarp();
-          uint8_t* dst = smem + st * stage_bytes + g.stageA;
-          const uint8_t* from = src + (size_t)j * g.cps * g.taps * piece;
-          const uint32_t a = piece * (np * lane / NCOPY), b = piece * (np * (lane + 1) / NCOPY);
-          if (lane < NCOPY && b > a) bulk_g2s(dst + a, from + a, b - a, &sh.full[st]);
-          ++issued;
-          if (++st == g.nstage) { st = 0; phase ^= 1; }
+      // the stages' weights, one bulk copy each: this CTA's rows of the unit's
+      // output channels
+      if (lane == 0) {
+        int st = 0, issued = 0;
+        uint32_t phase = 1;
+        bool ok = true;
+        uint8_t* dst = smem + g.stageA;
+        for (int i = 0; ok && i < cnt; ++i) {
+          int pt, k0;
+          unit_of(g, u0 + i * ustep, pt, k0);
+          const uint32_t piece = (uint32_t)(unit_n(g, CG, k0) / CG) * 32;      // one tap of 16 channels
+          const uint32_t block = piece * (uint32_t)g.taps;
+          const uint8_t* src = wop + (size_t)k0 * g.NKS * 32 + (size_t)rank * piece * g.NKS;
+          for (int cb = 0; cb < g.CB; cb += g.cps) {
+            if (!mbar_wait(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY)) { ok = false; break; }
+            const uint32_t bytes = block * (uint32_t)min(g.cps, g.CB - cb);
+            mbar_arrive_expect_tx(&sh.full[st], bytes);
+            bulk_g2s(dst, src, bytes, &sh.full[st]);
+            src += bytes;
+            dst += stage_bytes;
+            ++issued;
+            if (++st == g.nstage) { st = 0; dst = smem + g.stageA; phase ^= 1; }
+          }
         }
-      }
-      // copies still in flight land before the CTA leaves (an abort may have
-      // kept the MMA side from waiting for them)
-      if (*abort_flag) {
-        if (lane == 0)
+        // copies still in flight land before the CTA leaves (an abort may have
+        // kept the MMA side from waiting for them)
+        if (*abort_flag)
           for (int b = issued > g.nstage ? issued - g.nstage : 0; b < issued; ++b)
             mbar_wait(&sh.full[b % g.nstage], (b / g.nstage) & 1, nullptr, err, ERR_WAIT_FULL);
       }
