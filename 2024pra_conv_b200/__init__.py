@@ -113,6 +113,9 @@ def lib():
             "wino_batch_graph_launch": ([vp, vp], i),
             "wino_conv2d_variant": ([i, vp, vp, vp, vp, i, i, i, i, i, vp], i),
             "wino_conv2d_fused_ws": ([vp, vp, vp, vp, i, i, i, i, i, vp], i),
+            "wino_fused_conv_workspace_bytes": ([i, i, i, i, i], sz),
+            "wino_conv2d_fused_ws_sized": ([vp, vp, vp, sz, vp, i, i, i, i, i, vp], i),
+            "wino_conv2d_fused_epilogue_sized": ([vp, vp, vp, sz, vp, vp, vp, i, i, i, i, i, i, vp], i),
             "wino_launch_kernelinfo": ([vp, vp, vp], i),
             "wino_filter_transform_unfused": ([vp, vp, i, i, vp], i),
             "wino_unfused_workspace_bytes": ([i, i, i, i, i, ctypes.POINTER(sz), ctypes.POINTER(sz)], i),
@@ -243,6 +246,12 @@ def fused_workspace_bytes(n, c, h, w) -> int:
     return int(lib().wino_fused_workspace_bytes(n, c, h, w))
 
 
+def fused_conv_workspace_bytes(n, c, h, w, k) -> int:
+    """Workspace with which the fused conv and epilogue take their fastest
+    kernel at any shape (fused_workspace_bytes is enough to run them)."""
+    return int(lib().wino_fused_conv_workspace_bytes(n, c, h, w, k))
+
+
 def input_layout(x, workspace, stream=None):
     """The fused path's pre-pass alone: NCHW input -> channel-blocked workspace."""
     n, c, h, wd = x.shape
@@ -264,10 +273,10 @@ def conv2d_fused(x, ucache, k, out=None, stream=None, workspace=True):
                "conv2d_fused")
         return y
     if workspace is True:
-        workspace = torch.empty(fused_workspace_bytes(n, c, h, wd), dtype=torch.uint8, device=x.device)
-    _check(lib().wino_conv2d_fused_ws(ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(ucache.data_ptr()),
-                                      ctypes.c_void_p(workspace.data_ptr()),
-                                      ctypes.c_void_p(y.data_ptr()), n, c, h, wd, k, _stream(stream)),
+        workspace = torch.empty(fused_conv_workspace_bytes(n, c, h, wd, k), dtype=torch.uint8, device=x.device)
+    _check(lib().wino_conv2d_fused_ws_sized(ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(ucache.data_ptr()),
+                                            ctypes.c_void_p(workspace.data_ptr()), workspace.nbytes,
+                                            ctypes.c_void_p(y.data_ptr()), n, c, h, wd, k, _stream(stream)),
            "conv2d_fused_ws")
     return y
 
@@ -281,11 +290,11 @@ def conv2d_fused_epilogue(x, ucache, k, bias=None, residual=None, relu=False, ou
     n, c, h, wd = x.shape
     y = out if out is not None else torch.empty((n, k, h, wd), dtype=torch.float16, device=x.device)
     if workspace is None:
-        workspace = torch.empty(fused_workspace_bytes(n, c, h, wd), dtype=torch.uint8, device=x.device)
+        workspace = torch.empty(fused_conv_workspace_bytes(n, c, h, wd, k), dtype=torch.uint8, device=x.device)
     ptr = lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr())
-    _check(lib().wino_conv2d_fused_epilogue(ptr(x), ptr(ucache), ptr(workspace), ptr(y), ptr(bias),
-                                            ptr(residual), 1 if relu else 0, n, c, h, wd, k, _stream(stream)),
-           "conv2d_fused_epilogue")
+    _check(lib().wino_conv2d_fused_epilogue_sized(ptr(x), ptr(ucache), ptr(workspace), workspace.nbytes, ptr(y),
+                                                  ptr(bias), ptr(residual), 1 if relu else 0, n, c, h, wd, k,
+                                                  _stream(stream)), "conv2d_fused_epilogue")
     return y
 
 

@@ -13,14 +13,44 @@ __global__ void __launch_bounds__(256) shift_weight_pair_kernel(KernelParam p) {
   shift_weight_body<2>(p, static_cast<uint8_t*>(p.transform_filter));
 }
 
+// The operand from a fused U cache (p.pweight).
+template <int CG>
+__global__ void __launch_bounds__(128) shift_weight_u_kernel(KernelParam p) {
+  shift_weight_from_u<CG>(p, static_cast<const __half*>(p.pweight), static_cast<uint8_t*>(p.transform_filter),
+                          blockIdx.x * 128 + threadIdx.x);
+}
+// ... of every layer of a table (grid y).
+__global__ void __launch_bounds__(128) shift_weight_u_batch_kernel(const __grid_constant__ ShiftTable t) {
+  const KernelParam& p = t.layer[blockIdx.y].p;
+  shift_weight_from_u<2>(p, static_cast<const __half*>(p.pweight), static_cast<uint8_t*>(p.transform_filter),
+                         blockIdx.x * 128 + threadIdx.x);
+}
+
 // One CTA a unit (128 positions, up to 128 output channels).
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_kernel(KernelParam p) {
-  shift_conv_body<1>(p, static_cast<const uint8_t*>(p.transform_filter), &g_shift_err);
+  shift_conv_body<1, false>(sc::OneConv{p}, sc::Epi{}, &g_shift_err);
 }
 
 // A pair of CTAs a unit (256 positions, up to 256 output channels).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_pair_kernel(KernelParam p) {
-  shift_conv_body<2>(p, static_cast<const uint8_t*>(p.transform_filter), &g_shift_err);
+  shift_conv_body<2, false>(sc::OneConv{p}, sc::Epi{}, &g_shift_err);
+}
+
+// The same with the fused epilogue.
+__global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_epi_kernel(KernelParam p, sc::Epi e) {
+  shift_conv_body<1, true>(sc::OneConv{p}, e, &g_shift_err);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
+    shift_conv_epi_pair_kernel(KernelParam p, sc::Epi e) {
+  shift_conv_body<2, true>(sc::OneConv{p}, e, &g_shift_err);
+}
+
+// A table of layers, passed by value: the roles read their layers' dims from
+// the constant bank (from a table in memory every role kept them in registers
+// and spilled).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
+    shift_conv_batch_kernel(const __grid_constant__ ShiftTable t) {
+  shift_conv_body<2, false>(sc::ConvTable{t}, sc::Epi{}, &g_shift_err);
 }
 
 }  // namespace wino
@@ -47,9 +77,8 @@ int wino_shift_cg(const KernelParam* p) {
   if (p->u > 2 || p->v > 2 || p->r * p->s > sc::MAXTAP) return 0;
   const sc::Plan g1 = sc::make_plan(*p, 1), g2 = sc::make_plan(*p, 2);
   if (g1.npos + 4096 >= (1LL << 31) || g1.GX >= (1 << 15) || g1.GY >= (1 << 15)) return 0;
-  // element offsets of one unit: the images its rows touch, all channels
-  const long long per = (long long)g1.GX * g1.GY;
-  if (((long long)g1.rows / per + 3) * g1.C * g1.H * g1.W >= (1LL << 31)) return 0;
+  // byte offsets into the input in 32 bits
+  if ((long long)g1.N * g1.C * g1.H * g1.W >= (1LL << 31)) return 0;
   const bool aligned = (p->h * p->w) % 4 == 0 && (reinterpret_cast<uintptr_t>(p->pin) & 7) == 0;
   const bool strided = p->u > 1 || p->v > 1;
   const int items = (!aligned ? sc::MAXITEM_ODD : strided ? sc::MAXITEM_STRIDED : sc::MAXITEM) * sc::NPROD;
@@ -79,7 +108,9 @@ int wino_shift_prepare() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 1;
   if (dev >= 0 && dev < 64 && done[dev]) return 0;
-  for (const void* f : {(const void*)shift_conv_kernel, (const void*)shift_conv_pair_kernel}) {
+  for (const void* f : {(const void*)shift_conv_kernel, (const void*)shift_conv_pair_kernel,
+                        (const void*)shift_conv_epi_kernel, (const void*)shift_conv_epi_pair_kernel,
+                        (const void*)shift_conv_batch_kernel}) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sc::SMEM_BYTES) != cudaSuccess) return 1;
     // the warpgroups split exactly the registers the block launches with
     cudaFuncAttributes fa{};
@@ -99,11 +130,113 @@ void wino_shift_plan(const KernelParam* p, int cg, int* out) {
   for (int i = 0; i < 14; ++i) out[i] = v[i];
 }
 
+// Launch with programmatic stream serialization: the kernel may start while
+// the one before it, which makes its weight operand, still runs (the operand
+// is waited for in the kernel).
+int wino_launch_dependent(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 // Launches the kernel on a problem whose weight operand is at
-// p->transform_filter and packed plan in p->transform_pin.
+// p->transform_filter and packed plan in p->transform_pin; the launch before
+// it on the stream is the one that makes the operand.
 int wino_launch_shift(const KernelParam* p, int cg, int sms, cudaStream_t stream) {
   void* args[] = {const_cast<KernelParam*>(p)};
-  return (int)cudaLaunchKernel(wino_shift_kernel_ptr(cg), dim3(wino_shift_grid(p, cg, sms)), dim3(sc::NTHREAD), args,
+  return wino_launch_dependent(wino_shift_kernel_ptr(cg), dim3(wino_shift_grid(p, cg, sms)), dim3(sc::NTHREAD), args,
+                               (size_t)sc::SMEM_BYTES, stream);
+}
+
+// ---- convolutions on a fused U cache ------------------------------------
+// Direct-conv FLOPs from which the fused entry points (conv, epilogue, batch)
+// recover the filter from U and take this kernel: below it the fused Winograd
+// kernel's configurations stay bit-identical to one another, and the two
+// launches cost what the kernel gains.
+static constexpr double kFusedMinFlops = 512e6;
+
+// CTAs a unit for a problem (dims and tensors set), or 0 when it stays with
+// the fused kernel.  `cg` 2: for a table of layers (pairs).
+int wino_shift_fused_cg(const KernelParam* p, int cg) {
+  if (p->c % 16 || p->k % 16 || 2.0 * p->n * p->k * p->h * p->w * p->c * 9 < kFusedMinFlops) return 0;
+  const int best = wino_shift_cg(p);       // (0 when either plan does not fit)
+  if (best == 0 || cg == 0) return best;
+  const sc::Plan g = sc::make_plan(*p, 2, true);
+  const bool aligned = (p->h * p->w) % 4 == 0 && (reinterpret_cast<uintptr_t>(p->pin) & 7) == 0;
+  return 2 * g.cps * g.qmax <= (aligned ? 2 : 1) * sc::NPROD ? 2 : 0;
+}
+
+int wino_launch_shift_weight_u(const KernelParam* p, int cg, cudaStream_t stream) {
+  const size_t items = wino_shift_weight_bytes(p, cg) / (9 * 16);
+  void* args[] = {const_cast<KernelParam*>(p)};
+  return (int)cudaLaunchKernel(cg == 2 ? (void*)shift_weight_u_kernel<2> : (void*)shift_weight_u_kernel<1>,
+                               dim3((unsigned)((items + 127) / 128)), dim3(128), args, 0, stream);
+}
+
+// y = relu?(conv + bias + residual) on the U cache `u`; wop holds
+// wino_shift_weight_bytes.
+int wino_launch_shift_fused(const KernelParam* p0, const void* u, void* wop, int cg, const VariantArgs* va, int sms,
+                            cudaStream_t stream) {
+  if (wino_shift_prepare() != 0) return (int)cudaErrorInvalidValue;
+  KernelParam p = *p0;
+  p.pweight = const_cast<void*>(u);
+  p.transform_filter = wop;
+  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg));
+  const int rc = wino_launch_shift_weight_u(&p, cg, stream);
+  if (rc != 0) return rc;
+  if (!va || (!va->bias && !va->residual && !va->relu)) return wino_launch_shift(&p, cg, sms, stream);
+  sc::Epi e{va->bias, static_cast<const __half*>(va->residual), va->relu};
+  void* args[] = {&p, &e};
+  return wino_launch_dependent(cg == 2 ? (void*)shift_conv_epi_pair_kernel : (void*)shift_conv_epi_kernel,
+                               dim3(wino_shift_grid(&p, cg, sms)), dim3(sc::NTHREAD), args, (size_t)sc::SMEM_BYTES,
+                               stream);
+}
+
+// Completes a table whose layers have dims, tensors, U cache (pweight) and
+// operand buffer (transform_filter): plans, unit numbers, the common ring.
+void wino_shift_table_finish(ShiftTable* t) {
+  t->units = t->pitch = 0;
+  for (int l = 0; l < t->nlayers; ++l) {
+    ShiftLayer& d = t->layer[l];
+    const sc::Plan g = sc::make_plan(d.p, 2, true);
+    d.p.transform_pin = reinterpret_cast<void*>(sc::pack_plan(g));
+    d.unit_begin = t->units;
+    d.units = g.units;
+    t->units += g.units;
+    if (g.pitch > t->pitch) t->pitch = g.pitch;
+  }
+  const int fit = t->pitch > 0 ? sc::SMEM_STAGES / t->pitch : 0;
+  t->nstage = fit < sc::MAXSTAGE ? fit : sc::MAXSTAGE;
+}
+
+// Cost of one unit of a layer in MMA cycles (to order a table by).
+double wino_shift_unit_cost(const KernelParam* p) {
+  const sc::Plan g = sc::make_plan(*p, 2);
+  return (double)g.NKS * sc::mma_cycles(2, g.Kp < 256 ? (g.Kp + 31) / 32 * 32 : 256);
+}
+
+// The operands of a table's layers, then one launch over all of them.
+int wino_launch_shift_batch(const ShiftTable* t, int sms, cudaStream_t stream) {
+  size_t items = 0;
+  for (int l = 0; l < t->nlayers; ++l) {
+    const size_t i = wino_shift_weight_bytes(&t->layer[l].p, 2) / (9 * 16);
+    if (i > items) items = i;
+  }
+  void* args[] = {const_cast<ShiftTable*>(t)};
+  cudaError_t e = cudaLaunchKernel((void*)shift_weight_u_batch_kernel,
+                                   dim3((unsigned)((items + 127) / 128), (unsigned)t->nlayers), dim3(128), args, 0,
+                                   stream);
+  if (e != cudaSuccess) return (int)e;
+  const int pairs = sms / 2, grid = 2 * (t->units < pairs ? t->units : pairs);
+  return wino_launch_dependent((void*)shift_conv_batch_kernel, dim3((unsigned)grid), dim3(sc::NTHREAD), args,
                                (size_t)sc::SMEM_BYTES, stream);
 }
 
@@ -129,7 +262,11 @@ int wino_conv2d_shift(const void* x, const void* weight, void* wprep, void* y, i
                                  args, 0, (cudaStream_t)stream) != cudaSuccess)
     return 3;
   if (!x) return 0;
-  return wino_launch_shift(&p, cg, 148, (cudaStream_t)stream) == 0 ? 0 : 3;
+  if (weight) return wino_launch_shift(&p, cg, 148, (cudaStream_t)stream) == 0 ? 0 : 3;
+  return cudaLaunchKernel(wino_shift_kernel_ptr(cg), dim3(wino_shift_grid(&p, cg, 148)), dim3(sc::NTHREAD), args,
+                          (size_t)sc::SMEM_BYTES, (cudaStream_t)stream) == cudaSuccess
+             ? 0
+             : 3;
 }
 
 uint32_t wino_shift_error_read_clear() {

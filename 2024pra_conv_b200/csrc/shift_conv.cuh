@@ -62,7 +62,9 @@
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include "tc_sm100.cuh"
+#include "wino_common.cuh"
 #include "wino_param.h"
+#include "wino_batch.h"
 
 namespace wino {
 namespace sc {
@@ -83,9 +85,11 @@ constexpr int NWARP_E = 4, WARP_MMA = 4, WARP_LOAD = 5, WARP_Z0 = 6, NWARP_Z = 2
 constexpr int NTHREAD = (WARP_P0 + NGROUP * NWARP_P) * 32;
 constexpr int NPROD = NWARP_P * 32;       // producers of one stage
 constexpr int REGS_LAUNCH = 128, REGS_EPI = 112, REGS_MMA = 64, REGS_PROD = 168;
+static_assert(NGROUP == 2, "stages alternate between two groups");
 static_assert(128 * REGS_EPI + 128 * REGS_MMA + NGROUP * NPROD * REGS_PROD == NTHREAD * REGS_LAUNCH,
               "the warpgroups' register limits add up to the launch allocation");
 constexpr uint32_t SLEEP_NS = 32;
+constexpr int BYUNIT = 2;                 // stages a unit up to which producer groups alternate by unit
 // Items (a quad of pixels, eight channels) a producer thread may own per
 // stage, and operand rows whose padding it looks after.
 constexpr int MAXITEM = 4, MAXITEM_STRIDED = 6, MAXITEM_ODD = 2, MAXROWS = 1024;
@@ -114,6 +118,7 @@ struct Plan {
   int NB, nKU;         // output channels per unit, units per position tile
   int units;
   int stageA, stageB, nstage;
+  int pitch;           // bytes from stage to stage
   int qmax, qpi;       // quads of pixels a tile's rows may touch, quads per image
   long long npos;
 };
@@ -149,9 +154,17 @@ __host__ __device__ __forceinline__ int mma_cycles(int cg, int n) {
   return reads > math ? reads : math;
 }
 
+template <bool K33 = false>
 __host__ __device__ __forceinline__ void plan_dims(Plan& g, const KernelParam& p) {
-  g.N = p.n; g.C = p.c; g.H = p.h; g.W = p.w; g.K = p.k; g.R = p.r; g.S = p.s;
-  g.U = p.u; g.V = p.v; g.P = p.p; g.Q = p.q; g.OH = p.Oh; g.OW = p.Ow;
+  g.N = p.n; g.C = p.c; g.H = p.h; g.W = p.w; g.K = p.k;
+  if (K33) {                              // 3x3 / stride 1 / pad 1 known to the compiler
+    g.R = g.S = 3;
+    g.U = g.V = g.P = g.Q = 1;
+    g.OH = g.H; g.OW = g.W;
+  } else {
+    g.R = p.r; g.S = p.s;
+    g.U = p.u; g.V = p.v; g.P = p.p; g.Q = p.q; g.OH = p.Oh; g.OW = p.Ow;
+  }
   g.nu = g.U < g.R ? g.U : g.R;
   g.nv = g.V < g.S ? g.V : g.S;
   g.taps = g.R * g.S;
@@ -176,10 +189,13 @@ __host__ __device__ __forceinline__ void plan_finish(Plan& g, int cg) {
   // one more row: where producers drop pixels of a quad that are not the tile's
   g.stageA = (g.cps * g.rows * 32 + 16 + 127) & ~127;
   g.stageB = g.cps * g.taps * rows_b * 32;
+  g.pitch = g.stageA + g.stageB;
 }
 
-// Plan of a problem for CG CTAs a unit (host; the rules).
-__host__ inline Plan make_plan(const KernelParam& p, int cg) {
+// Plan of a problem for CG CTAs a unit (host; the rules).  `table`: for the
+// kernel over a table of layers, whose producers own one unaligned quad a
+// thread (two spilled there: 100 us against 37 for N32 C512 7x7 K512).
+__host__ inline Plan make_plan(const KernelParam& p, int cg, bool table = false) {
   Plan g;
   plan_dims(g, p);
   g.GX = grid_extent(g.OW, g.S, g.V, g.Q, g.W);
@@ -219,7 +235,8 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg) {
   for (;; cps >>= 1) {
     g.lcps = cps == 4 ? 2 : cps == 2 ? 1 : 0;
     plan_finish(g, cg);
-    const int items = g.taps >= 6 ? 2 * NPROD : 3 * NPROD, stages = g.taps >= 6 ? 4 : 3;
+    const bool odd = ((g.H * g.W) & 3) != 0;
+    const int items = table && odd ? NPROD : g.taps >= 6 ? 2 * NPROD : 3 * NPROD, stages = g.taps >= 6 ? 4 : 3;
     if (cps == 1 || (2 * cps * g.qmax <= items && stages * (g.stageA + g.stageB) <= SMEM_STAGES)) break;
   }
   const int fit = SMEM_STAGES / (g.stageA + g.stageB);
@@ -232,9 +249,10 @@ __host__ inline unsigned long long pack_plan(const Plan& g) {
          (unsigned long long)g.lcps << 40 | (unsigned long long)g.nstage << 44 | (unsigned long long)g.qmax << 48;
 }
 
+template <bool K33 = false>
 __device__ __forceinline__ Plan unpack_plan(const KernelParam& p, int cg) {
   Plan g;
-  plan_dims(g, p);
+  plan_dims<K33>(g, p);
   const unsigned long long w = reinterpret_cast<unsigned long long>(p.transform_pin);
   g.GX = (int)(w & 0xffff);
   g.GY = (int)(w >> 16 & 0xffff);
@@ -245,6 +263,65 @@ __device__ __forceinline__ Plan unpack_plan(const KernelParam& p, int cg) {
   plan_finish(g, cg);
   return g;
 }
+
+// One convolution of a launch as one CTA sees it: its plan and tensors, this
+// CTA's first unit and number of units.
+struct Conv {
+  Plan g;
+  const unsigned short* x;
+  __half* y;
+  const uint8_t* wop;      // weight operand
+  int u0, cnt;
+};
+
+// A launch over one convolution (its argument carries the packed plan).
+struct OneConv {
+  static constexpr bool k33 = false;
+  const KernelParam& p;
+  __device__ __forceinline__ int layers() const { return 1; }
+  __device__ __forceinline__ bool get(int, int cg, int u, int step, Conv& c) const {
+    c.g = unpack_plan(p, cg);
+    c.x = static_cast<const unsigned short*>(p.pin);
+    c.y = static_cast<__half*>(p.pout);
+    c.wop = static_cast<const uint8_t*>(p.transform_filter);
+    c.u0 = u;
+    c.cnt = u < c.g.units ? (c.g.units - 1 - u) / step + 1 : 0;
+    return c.cnt > 0;
+  }
+};
+
+// ... and over a table of them, units numbered through (wino_batch.h): the
+// ring of stages runs on across layers, so its pitch is the largest stage's.
+struct ConvTable {
+  static constexpr bool k33 = true;       // 3x3 / stride 1 / pad 1 layers only
+  const ShiftTable& t;                    // the kernel's argument (constant bank)
+  __device__ __forceinline__ int layers() const { return t.nlayers; }
+  __device__ __forceinline__ bool get(int l, int cg, int u, int step, Conv& c) const {
+    const ShiftLayer& d = t.layer[l];
+    // first unit of the layer that is u modulo step
+    const int begin = d.unit_begin, skip = (u - begin % step + step) % step;
+    c.u0 = skip;
+    c.cnt = skip < d.units ? (d.units - 1 - skip) / step + 1 : 0;
+    if (c.cnt == 0) return false;
+    c.g = unpack_plan<true>(d.p, cg);
+    c.g.pitch = t.pitch;
+    c.g.nstage = t.nstage;
+    c.x = static_cast<const unsigned short*>(d.p.pin);
+    c.y = static_cast<__half*>(d.p.pout);
+    c.wop = static_cast<const uint8_t*>(d.p.transform_filter);
+    return true;
+  }
+};
+
+// Position in the ring of stages; a waiter for empty stages starts in phase
+// 1 (the first pass over the ring is free), one for full stages in phase 0.
+struct RingPos {
+  int st;
+  uint32_t phase;
+  __device__ __forceinline__ void next(int nstage, int by = 1) {
+    for (st += by; st >= nstage; st -= nstage) phase ^= 1;
+  }
+};
 
 // Rows of the weight operand one CTA of a unit holds (the unit's output
 // channels k0 .., padded to the MMA's granularity).
@@ -344,23 +421,29 @@ struct Slot {
 // are 256-byte runs of a channel's plane.  ALIGNED: a quad is one 8-byte
 // word of every channel (input 8-byte aligned, H * W a multiple of 4);
 // otherwise the two words around it and a shift.
+// The two groups take alternate stages, or with few stages a unit alternate
+// units (each then works out every other unit's addresses only): a group's
+// stages are `run` in a row, then `run` skipped.
 template <int CG, int NI, int DEPTH, bool ALIGNED, bool STRIDED>
-__device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uint8_t* smem, Shared& sh, int tid,
-                                        int group, int u0, int ustep, int cnt, int tile_pos, int tile_stride,
-                                        uint32_t* err) {
+__device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int done,
+                                        int ustep, int tile_pos, int tile_stride, bool& set, uint32_t* err) {
+  const Plan& g = cv.g;
+  const int u0 = cv.u0, cnt = cv.cnt;
   constexpr int NW = ALIGNED ? 1 : 2;     // 8-byte words per channel
   volatile int* abort_flag = &sh.abort_flag;
-  const unsigned short* X = static_cast<const unsigned short*>(p.pin);
+  const unsigned short* X = cv.x;
   const int HW = g.H * g.W, ngrp = 2 * g.cps;
   const uint32_t trash = (uint32_t)(ngrp * g.rows);
   const Grid gr = make_grid(g);
   const float rw = 1.0f / (float)g.W, rqpi = 1.0f / (float)g.qpi;
   const int ushift = STRIDED ? g.U - 1 : 0, vshift = STRIDED ? g.V - 1 : 0;      // strides 1 and 2
-  // Pixel order of this lane's stores: pixel k ^ rot first, so that the eight
-  // lanes of a 16-byte store phase, whose quads are 64 bytes apart, fill one
-  // 128-byte line (no bank conflicts).
-  const int rot = (tid >> 1) & 3;
-  const uint32_t sel0 = rot & 1 ? 0x7632u : 0x5410u, sel1 = rot & 1 ? 0x5410u : 0x7632u;
+  // Pixel order of this lane's stores: pixel k ^ rot k-th, so that the eight
+  // lanes of a 16-byte store phase, whose quads are 64 bytes apart, meet in
+  // pairs on a bank rather than in fours (all four orders would part them, at
+  // 16 selects an item; a producer warp's instructions are what this role
+  // waits for).
+  const int rot = (tid >> 1) & 1;
+  const uint32_t sel0 = rot ? 0x7632u : 0x5410u, sel1 = rot ? 0x5410u : 0x7632u;
   int iq[NI], ich[NI];                    // quad (-1: none) and first channel of the stage
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
@@ -382,20 +465,28 @@ __device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uin
       r += prow[pl];
     }
   }
-  // load side: element offset from the unit's first image (-1: no loads), the
-  // quad's pixels inside the image, rows of its pixels, padding rows
-  int off[NI], npx[NI];
+  uint32_t off[NI];                       // byte offset of the quad in the input, channel 0
+  int npx[NI];                            // its pixels inside the image (0: no pixel of the tile's)
   uint2 row_l[NI];
-  int lu = 0, lj = group;                 // this group's stages: every NGROUP-th
+  // load and store cursors: stage of the layer (unit lu, stage lj), ring slot
+  const bool by_unit = g.nst <= BYUNIT;
+  const int stages = cnt * g.nst;
+  const int run = by_unit ? g.nst : 1, first = by_unit ? group * g.nst : (group + done) & 1;
+  int lu = 0, lj = first;
   while (lj >= g.nst) { lj -= g.nst; ++lu; }
+  int s_left = run, l_left = run;         // stages left of the run
+  RingPos pos;
+  pos.st = (done + first) % g.nstage;
+  pos.phase = 1u ^ (uint32_t)(((done + first) / g.nstage) & 1);
   int entered = -1;
-  const unsigned short* base = X;
+  const bool whole = (g.C & 15) == 0;     // no channel of a block is missing
+  const char* XB = reinterpret_cast<const char*>(X);
   Slot<NI, NW> ring[DEPTH];
   auto enter = [&]() {
     int pt, k0;
     unit_of(g, u0 + lu * ustep, pt, k0);
     const Base b0 = tile_base(gr, pt * tile_stride + tile_pos);
-    base = X + (size_t)b0.n * g.C * HW;
+    const uint32_t img = (uint32_t)(b0.n * g.C) * (uint32_t)HW * 2u;
     // the range starts with the first position's pixel (stride 1) or the
     // first pixel row of its grid row
     const int y0 = (b0.gy << ushift) - g.P;
@@ -405,7 +496,7 @@ __device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uin
     const int q0 = lo >> 2, yb = max(y0, 0);
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      off[i] = -1;
+      off[i] = img;                       // (a quad without pixels loads what is there)
       npx[i] = 0;
       row_l[i].x = row_l[i].y = trash | trash << 16;
       if (iq[i] < 0) continue;
@@ -425,74 +516,95 @@ __device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uin
       while (x < 0) { x += g.W; --y; }    // images narrower than the overhang
       bool any = false;
       uint32_t d[4];
+      if (!STRIDED) {
+        // rows of consecutive pixels are consecutive but for the padding
+        // between image rows (at stride 1 the grid has room for every pixel:
+        // GX >= W + Q, GY >= H + P)
+        const int r0 = (dn * g.GY + y + g.P - b0.gy) * g.GX + x + g.Q - b0.gx;
+        const int first_row = (ich[i] >> 3) * g.rows;
 #pragma unroll
-      for (int px = 0; px < 4; ++px) {
-        d[px] = trash;
-        int r = -1, pr = g.rows, pb = 0;
-        bool in = i0 + px < HW;
-        if (!STRIDED) {
-          r = (dn * g.GY + y + g.P - b0.gy) * g.GX + x + g.Q - b0.gx;
-          in = in && x + g.Q < g.GX && y + g.P < g.GY;
-        } else {
+        for (int px = 0; px < 4; ++px) {
+          int r = r0 + px;
+          if (g.W >= 4) {
+            if (px >= g.W - x) r += g.GX - g.W;
+          } else {
+            r += (x + px) / g.W * (g.GX - g.W);
+          }
+          const bool in = (unsigned)r < (unsigned)g.rows && (ALIGNED || i0 + px < HW);
+          d[px] = in ? (uint32_t)(first_row + r) : trash;
+          any = any || in;
+        }
+      } else {
+#pragma unroll
+        for (int px = 0; px < 4; ++px) {
+          d[px] = trash;
           const int yy = y + g.P, xx = x + g.Q;
           const int gy = yy >> ushift, gx = xx >> vshift;
           const int pl = ((yy & ushift) << vshift) | (xx & vshift);
-          pb = pbase[0];
-          pr = prow[0];
+          int pb = pbase[0], pr = prow[0];
 #pragma unroll
           for (int z = 1; z < NPL; ++z)
             if (pl == z) { pb = pbase[z]; pr = prow[z]; }
-          r = (dn * g.GY + gy - b0.gy) * g.GX + gx - b0.gx;
-          in = in && gx < g.GX && gy < g.GY;
+          const int r = (dn * g.GY + gy - b0.gy) * g.GX + gx - b0.gx;
+          if (i0 + px < HW && gx < g.GX && gy < g.GY && r >= 0 && r < pr) {
+            d[px] = (uint32_t)((ich[i] >> 3) * g.rows + pb + r);
+            any = true;
+          }
+          if (++x == g.W) { x = 0; ++y; }
         }
-        if (in && r >= 0 && r < pr) {
-          d[px] = (uint32_t)((ich[i] >> 3) * g.rows + pb + r);
-          any = true;
-        }
-        if (++x == g.W) { x = 0; ++y; }
       }
       // stored in the order px ^ rot
-      const uint32_t w0 = d[0] | d[1] << 16, w1 = d[2] | d[3] << 16;
-      const uint32_t v0 = rot & 2 ? w1 : w0, v1 = rot & 2 ? w0 : w1;
-      row_l[i] = make_uint2(__byte_perm(v0, v0, rot & 1 ? 0x1032 : 0x3210), __byte_perm(v1, v1, rot & 1 ? 0x1032 : 0x3210));
-      npx[i] = min(4, HW - i0);
-      if (any) off[i] = dn * g.C * HW + i0;
+      row_l[i] = make_uint2(__byte_perm(d[0], d[1], rot ? 0x1054 : 0x5410), __byte_perm(d[2], d[3], rot ? 0x1054 : 0x5410));
+      if (any) {
+        npx[i] = min(4, HW - i0);
+        off[i] = img + (uint32_t)(dn * g.C * HW + i0) * 2u;
+      }
     }
   };
   auto issue = [&](Slot<NI, NW>& s) {
     const int c0 = lj << (g.lcps + 4);
+    const uint32_t plane = (uint32_t)HW * 2u;
     uint32_t shifts = 0;
+    if (ALIGNED && whole) {
+      // Channels past C are those of a block no MMA reads.
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const int c = c0 + ich[i], nc = off[i] >= 0 ? g.C - c : 0;   // channels to load
-      const unsigned short* src = base + (off[i] + c * HW);
-      s.row[i] = row_l[i];
-      if (!ALIGNED) shifts |= ((uint32_t)(reinterpret_cast<uintptr_t>(src) >> 1) & 3u) << (4 * i);
+      for (int i = 0; i < NI; ++i) {
+        const int c = c0 + ich[i];
+        uint32_t o = off[i] + (c < g.C ? (uint32_t)c * plane : 0u);
+        s.row[i] = row_l[i];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const bool on = e < nc;
-        if (ALIGNED) {
-          s.w[i][e][0] = on ? __ldg(reinterpret_cast<const uint2*>(src + e * HW)) : make_uint2(0, 0);
-        } else {
-          const uintptr_t ad = reinterpret_cast<uintptr_t>(src + e * HW);
-          const uint2* wp = reinterpret_cast<const uint2*>(ad & ~uintptr_t(7));
-          s.w[i][e][0] = on ? __ldg(wp) : make_uint2(0, 0);
-          // the next word only where it holds a pixel of the quad
-          s.w[i][e][NW - 1] = on && ((int)(ad >> 1) & 3) + npx[i] > 4 ? __ldg(wp + 1) : make_uint2(0, 0);
+        for (int e = 0; e < 8; ++e, o += plane) s.w[i][e][0] = __ldg(reinterpret_cast<const uint2*>(XB + o));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        const int c = c0 + ich[i], nc = npx[i] > 0 ? g.C - c : 0;   // channels to load
+        uint32_t o = off[i] + (nc > 0 ? (uint32_t)c * plane : 0u);
+        s.row[i] = row_l[i];
+        if (!ALIGNED) shifts |= ((uint32_t)(reinterpret_cast<uintptr_t>(XB + o) >> 1) & 3u) << (4 * i);
+#pragma unroll
+        for (int e = 0; e < 8; ++e, o += plane) {
+          const bool on = e < nc;
+          if (ALIGNED) {
+            s.w[i][e][0] = on ? __ldg(reinterpret_cast<const uint2*>(XB + o)) : make_uint2(0, 0);
+          } else {
+            const uintptr_t ad = reinterpret_cast<uintptr_t>(XB + o);
+            const uint2* wp = reinterpret_cast<const uint2*>(ad & ~uintptr_t(7));
+            s.w[i][e][0] = on ? __ldg(wp) : make_uint2(0, 0);
+            // the next word only where it holds a pixel of the quad
+            s.w[i][e][NW - 1] = on && ((int)(ad >> 1) & 3) + npx[i] > 4 ? __ldg(wp + 1) : make_uint2(0, 0);
+          }
         }
       }
     }
     s.shifts = shifts;
   };
-  const int stage_bytes = g.stageA + g.stageB;
-  int st = group;
-  uint32_t phase = 1;                     // empty waits: the first pass over the ring is free
   auto consume = [&](const Slot<NI, NW>& s) -> bool {
-    if (!wait_all_lanes(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
-    uint8_t* dst = smem + st * stage_bytes;
+    if (!wait_all_lanes(&sh.empty[pos.st], pos.phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
+    uint8_t* dst = smem + pos.st * g.pitch;
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      uint32_t lo[8], hi[8];              // pixels (rot & 2, + 1) and the other two, of eight channels
+      uint32_t lo[8], hi[8];              // pixels 0, 1 and 2, 3 of eight channels
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         uint32_t a = s.w[i][e][0].x, b = s.w[i][e][0].y;
@@ -503,8 +615,8 @@ __device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uin
           a = sh16 & 1u ? __byte_perm(t0, t1, 0x5432) : t0;
           b = sh16 & 1u ? __byte_perm(t1, t2, 0x5432) : t1;
         }
-        lo[e] = rot & 2 ? b : a;
-        hi[e] = rot & 2 ? a : b;
+        lo[e] = a;
+        hi[e] = b;
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -518,21 +630,22 @@ __device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uin
     }
     fence_proxy_async_shared();
     __syncwarp();
-    if ((tid & 31) == 0) mbar_arrive(&sh.full[st]);
-    st += NGROUP;
-    if (st >= g.nstage) { st -= g.nstage; phase ^= 1; }
+    if ((tid & 31) == 0) mbar_arrive(&sh.full[pos.st]);
+    int by = 1;
+    if (--s_left == 0) { s_left = run; by += run; }
+    pos.next(g.nstage, by);
     return true;
   };
   // Turn t stores the loads of DEPTH turns ago from its ring slot and issues
   // new ones into it.  One loop body with a case per slot: unrolled over the
   // slots, the unit entry above was compiled in seven times and its first
   // pass through the instruction cache held the first stage up by 10 us.
-  const int total = (cnt * g.nst - group + NGROUP - 1) / NGROUP;
+  const int total = by_unit ? (cnt - group + 1) / 2 * g.nst : (stages - first + 1) / 2;
   // the first loads go out before the block's setup is complete
   int slot = 0;
-  bool set = false;
-  for (int t = 0; t < total + DEPTH; ++t) {
-    if (t == DEPTH) {
+  bool ok = true;
+  for (int t = 0; ok && t < total + DEPTH; ++t) {
+    if (t == DEPTH && !set) {
       setup_sync<CG>();
       set = true;
     }
@@ -541,7 +654,6 @@ __device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uin
       enter();
       entered = lu;
     }
-    bool ok = true;
     auto turn = [&](Slot<NI, NW>& s) {
       if (t >= DEPTH) ok = consume(s);
       if (more && ok) issue(s);
@@ -550,28 +662,27 @@ __device__ __forceinline__ void produce(const Plan& g, const KernelParam& p, uin
     if (DEPTH > 1 && slot == 1) turn(ring[DEPTH > 1 ? 1 : 0]);
     if (DEPTH > 2 && slot == 2) turn(ring[DEPTH > 2 ? 2 : 0]);
     if (DEPTH > 3 && slot == 3) turn(ring[DEPTH > 3 ? 3 : 0]);
-    if (!ok) break;
     if (++slot == DEPTH) slot = 0;
-    lj += NGROUP;
-    while (lj >= g.nst) { lj -= g.nst; ++lu; }
+    int by = 1;
+    if (--l_left == 0) { l_left = run; by += run; }
+    for (lj += by; lj >= g.nst; lj -= g.nst) ++lu;
   }
-  if (!set) setup_sync<CG>();             // no stage for this group
+  return ok;
 }
 
 // Padding rows of the operand (two warps): the zero columns and rows of a
 // tile's positions, written to every stage (a slot's last tile had them
 // elsewhere).
-__device__ __forceinline__ void pad_rows(const Plan& g, uint8_t* smem, Shared& sh, int tid, int u0, int ustep, int cnt,
-                                         int tile_pos, int tile_stride, uint32_t* err) {
+__device__ __forceinline__ bool pad_rows(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int ustep, int tile_pos,
+                                         int tile_stride, RingPos& pos, uint32_t* err) {
+  const Plan& g = cv.g;
   constexpr int NT = NWARP_Z * 32;
   volatile int* abort_flag = &sh.abort_flag;
   const Grid gr = make_grid(g);
-  const int ngrp = 2 * g.cps, stage_bytes = g.stageA + g.stageB;
-  int st = 0;
-  uint32_t phase = 1;
-  for (int i = 0; i < cnt; ++i) {
+  const int ngrp = 2 * g.cps;
+  for (int i = 0; i < cv.cnt; ++i) {
     int pt, k0;
-    unit_of(g, u0 + i * ustep, pt, k0);
+    unit_of(g, cv.u0 + i * ustep, pt, k0);
     const Base b0 = tile_base(gr, pt * tile_stride + tile_pos);
     uint32_t zero = 0;                    // bit z: row tid + z * NT is padding
     int pbase = 0;
@@ -587,17 +698,18 @@ __device__ __forceinline__ void pad_rows(const Plan& g, uint8_t* smem, Shared& s
         pbase += pr;
       }
     for (int j = 0; j < g.nst; ++j) {
-      if (!wait_all_lanes(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY)) return;
-      uint8_t* dst = smem + st * stage_bytes + tid * 16;
+      if (!wait_all_lanes(&sh.empty[pos.st], pos.phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
+      uint8_t* dst = smem + pos.st * g.pitch + tid * 16;
       for (uint32_t m = zero; m != 0; m &= m - 1)
         for (int grp = 0; grp < ngrp; ++grp)
           *reinterpret_cast<uint4*>(dst + (grp * g.rows + (__ffs(m) - 1) * NT) * 16) = make_uint4(0, 0, 0, 0);
       fence_proxy_async_shared();
       __syncwarp();
-      if ((tid & 31) == 0) mbar_arrive(&sh.full[st]);
-      if (++st == g.nstage) { st = 0; phase ^= 1; }
+      if ((tid & 31) == 0) mbar_arrive(&sh.full[pos.st]);
+      pos.next(g.nstage);
     }
   }
+  return true;
 }
 
 // Operand row at which tap (r, s) starts reading a stage: its plane's first
@@ -613,38 +725,38 @@ __device__ __forceinline__ int tap_row(const Plan& g, int r, int s) {
 // MMA issue: per stage and 16-channel block one MMA a tap, all on the same
 // staged input.  The whole warp runs the loop and one elected lane issues, so
 // descriptors stay in uniform registers (from one lane's branch a stage of
-// nine took 960 cycles to issue against 800).  An MMA here costs its shared-memory reads: 64 cycles
-// for the 128 rows of A, which a shift takes off the 128-byte lines, plus a
-// cycle per 4 rows of B (N = 64: 80 cycles a CTA; a pair's N = 256 is at its
-// arithmetic 128).  The pipe takes an MMA ahead at most, so what the thread
+// nine took 960 cycles to issue against 800).  An MMA here costs its
+// shared-memory reads: 64 cycles for the 128 rows of A, which a shift takes
+// off the 128-byte lines, plus a cycle per 4 rows of B (N = 64: 80 cycles a
+// CTA; a pair's N = 256 is at its arithmetic 128).  The pipe takes an MMA ahead at most, so what the thread
 // does between stages shows: the next stage's barrier is polled in the middle
 // of a stage, and only if it was not ready then is it waited for.  TAPS > 0:
 // that many taps, their shifts kept in registers.
 template <int CG, int TAPS>
-__device__ __forceinline__ void issue_mmas(const Plan& g, Shared& sh, uint32_t sbase, uint32_t tmem, int u0, int ustep,
-                                           int cnt, uint32_t* err) {
+__device__ __forceinline__ bool issue_mmas(const Conv& cv, Shared& sh, uint32_t sbase, uint32_t tmem, int ustep,
+                                           bool leader, RingPos& pos, int& unit, bool& ready, uint32_t* err) {
+  const Plan& g = cv.g;
   constexpr uint16_t BOTH = 3;
   constexpr int NOFF = TAPS > 0 ? TAPS : 1;
   volatile int* abort_flag = &sh.abort_flag;
-  const uint32_t stage16 = (uint32_t)(g.stageA + g.stageB) >> 4, a16 = (uint32_t)g.stageA >> 4;
+  const uint32_t stage16 = (uint32_t)g.pitch >> 4, a16 = (uint32_t)g.stageA >> 4;
   const uint64_t adesc0 = smem_desc(sbase, (uint32_t)g.rows * 16, 128), bdesc0 = smem_desc(sbase, 128, 256) + a16;
   const uint32_t qstep = (uint32_t)g.rows * 2;
-  const bool leader = elect_one();
   uint32_t off[NOFF];
 #pragma unroll
   for (int t = 0; t < NOFF; ++t) off[t] = (uint32_t)__shfl_sync(0xffffffffu, sh.aoff[t], 0);
-  int st = 0;
-  uint32_t phase = 0, s16 = 0;
-  bool ok = true, ready = false;
-  for (int i = 0; ok && i < cnt; ++i) {
+  int st = pos.st;
+  uint32_t phase = pos.phase, s16 = (uint32_t)st * stage16;
+  bool ok = true;
+  for (int i = 0; ok && i < cv.cnt; ++i, ++unit) {
     int pt, k0;
-    unit_of(g, u0 + i * ustep, pt, k0);
+    unit_of(g, cv.u0 + i * ustep, pt, k0);
     const int nn = unit_n(g, CG, k0);
     const uint32_t idesc = instr_desc(CG * 128, (uint32_t)nn, 0, 0, 0, 0);
     const uint32_t bstep = (uint32_t)((nn / CG) * 32) >> 4;
-    const int ab = i & 1;
-    if (i >= 2) {
-      ok = wait_all_lanes<CG == 2>(&sh.accempty[ab], ((i >> 1) - 1) & 1, abort_flag, err, ERR_WAIT_DRAIN);
+    const int ab = unit & 1;
+    if (unit >= 2) {
+      ok = wait_all_lanes<CG == 2>(&sh.accempty[ab], ((unit >> 1) - 1) & 1, abort_flag, err, ERR_WAIT_DRAIN);
       if (!ok) break;
     }
     tc_fence_after();
@@ -695,11 +807,69 @@ __device__ __forceinline__ void issue_mmas(const Plan& g, Shared& sh, uint32_t s
       else mma_commit(&sh.accfull[ab]);
     }
   }
-  // every MMA issued (also on an abort) has finished before TMEM is freed
-  if (leader) {
-    if (CG == 2) mma_commit_pair(&sh.mmadone, 1);
-    else mma_commit(&sh.mmadone);
-    mbar_wait(&sh.mmadone, 0, nullptr, err, ERR_WAIT_ACCUM);
+  pos.st = st;
+  pos.phase = phase;
+  return ok;
+}
+
+// Epilogue operands of the fused form: y = relu?(conv + bias[k] + residual).
+struct Epi {
+  const float* bias;
+  const __half* residual;  // y's layout
+  int relu;
+};
+
+// store_cols_f16 with the fused epilogue: conv + bias is rounded to fp16, the
+// residual added in fp32, ReLU last.  `res`: the residual's element of this
+// row and column 0 (or null); bias: of column 0 (or null).
+template <int NC>
+__device__ __forceinline__ void store_cols_epi(__half* row, const __half* res, const float* bias, int relu,
+                                               size_t stride, const float* v, int lim, bool live, bool pair) {
+  const bool odd = (threadIdx.x & 1) != 0;
+  auto finish = [&](__half2 h, __half2 r) {
+    float2 f = __half22float2(h);
+    if (res) {
+      const float2 g = __half22float2(r);
+      f.x += g.x;
+      f.y += g.y;
+    }
+    if (relu) {
+      f.x = fmaxf(f.x, 0.f);
+      f.y = fmaxf(f.y, 0.f);
+    }
+    return __floats2half2_rn(f.x, f.y);
+  };
+  if (pair) {
+    __half* first = row - (odd ? 1 : 0);
+    const __half* rfirst = res ? res - (odd ? 1 : 0) : nullptr;
+#pragma unroll
+    for (int j0 = 0; j0 < NC / 2; j0 += 8) {
+      __half2 rv[8];
+      float bv[8], other[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int col = 2 * (j0 + j) + (odd ? 1 : 0);
+        const bool on = live && col < lim;
+        rv[j] = on && res ? *reinterpret_cast<const __half2*>(rfirst + (size_t)col * stride) : __half2{};
+        bv[j] = on && bias ? __ldg(bias + col) : 0.f;
+        other[j] = __shfl_xor_sync(0xffffffffu, odd ? v[2 * (j0 + j)] : v[2 * (j0 + j) + 1], 1);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c = 2 * (j0 + j), col = c + (odd ? 1 : 0);
+        const __half2 h = odd ? __floats2half2_rn(other[j] + bv[j], v[c + 1] + bv[j])
+                              : __floats2half2_rn(v[c] + bv[j], other[j] + bv[j]);
+        if (live && col < lim) *reinterpret_cast<__half2*>(first + (size_t)col * stride) = finish(h, rv[j]);
+      }
+    }
+  } else if (live) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      if (c < lim) {
+        const __half h = __float2half_rn(v[c] + (bias ? __ldg(bias + c) : 0.f));
+        const __half r = res ? res[(size_t)c * stride] : __half{};
+        row[(size_t)c * stride] = __low2half(finish(__half2half2(h), __half2half2(r)));
+      }
   }
 }
 
@@ -710,18 +880,19 @@ __device__ __forceinline__ void issue_mmas(const Plan& g, Shared& sh, uint32_t s
 template <int CG>
 __device__ __forceinline__ void shift_weight_body(const KernelParam& p, uint8_t* wop) {
   using namespace sc;
+  grid_dep_launch();
   const Plan g = unpack_plan(p, CG);
-  const long long nword = (long long)(weight_bytes(g, CG) >> 4);
-  const long long wi = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (wi >= nword) return;
+  const unsigned wi = blockIdx.x * blockDim.x + threadIdx.x;
+  if (wi >= (unsigned)(weight_bytes(g, CG) >> 4)) return;
   // (row of the operand, 16-channel block, tap, half), halves fastest, so
   // neighbouring threads read one output channel's weights
   const int hh = (int)(wi & 1);
-  const long long r2 = wi >> 1;
-  const int row = (int)(r2 / g.NKS), ks = (int)(r2 - (long long)row * g.NKS);
-  const int cb = ks / g.taps, tap = ks - cb * g.taps;
-  const int k0 = row / g.NB * g.NB, rk = row - k0;
-  const int rows = unit_n(g, CG, k0) / CG, rank = rk / rows, rr = rk - rank * rows;
+  const unsigned r2 = wi >> 1;
+  const int row = (int)(r2 / (unsigned)g.NKS), ks = (int)(r2 - (unsigned)row * (unsigned)g.NKS);
+  const int cb = (int)((unsigned)ks / (unsigned)g.taps), tap = ks - cb * g.taps;
+  // NB is a power of two
+  const int k0 = row & ~(g.NB - 1), rk = row - k0;
+  const int rows = unit_n(g, CG, k0) / CG, rank = CG == 2 && rk >= rows ? 1 : 0, rr = rk - rank * rows;
   const unsigned short* w = static_cast<const unsigned short*>(p.pweight);
   uint32_t v[4];
 #pragma unroll
@@ -737,11 +908,67 @@ __device__ __forceinline__ void shift_weight_body(const KernelParam& p, uint8_t*
   *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-// The kernel body.  CG = 2: clusters of two CTAs (__cluster_dims__(2, 1, 1)),
-// a unit is 256 positions, rank 0 issues the pair's MMAs.  `wop`: the weight
-// operand.
+// The weight operand from a fused U cache (u_offset's layout): the 3x3 filter
+// back from U = G g G^T, one thread an output channel's eight input channels.
+// With G's rows e0, (e0 + e1 + e2) / 2, (e0 - e1 + e2) / 2, e2 a vector's
+// inverse is (u0, u1 - u2, u3): the corner taps are U's own fp16 values, the
+// others sums of two or four, formed in fp32 and rounded to the fp16 grid the
+// filter came from (more than half of them land on it exactly; 2.2e-4 of the
+// filter in the 2-norm, against the 2.9e-4 to which U itself was rounded).
 template <int CG>
-__device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint8_t* wop, uint32_t* err) {
+__device__ __forceinline__ void shift_weight_from_u(const KernelParam& p, const __half* u, uint8_t* wop, unsigned item) {
+  using namespace sc;
+  grid_dep_launch();
+  const Plan g = unpack_plan<true>(p, CG);
+  // rows fastest: neighbouring threads read and write neighbouring 16-byte rows
+  const int last = (g.nKU - 1) * g.NB, nrow = last + unit_n(g, CG, last);
+  const int grp = (int)(item / (unsigned)nrow), row = (int)(item - (unsigned)grp * (unsigned)nrow), c = grp * 8;
+  if (c >= g.C) return;
+  // NB is a power of two
+  const int k0 = row & ~(g.NB - 1), rk = row - k0;
+  const int rows = unit_n(g, CG, k0) / CG, rank = CG == 2 && rk >= rows ? 1 : 0, rr = rk - rank * rows;
+  uint8_t* dst = wop + ((size_t)(k0 + rank * rows) * g.NKS + (size_t)(c >> 4) * 9 * rows) * 32 + (rr >> 3) * 256 +
+                 ((c >> 3) & 1) * 128 + (rr & 7) * 16;
+  uint4 uw[16];
+#pragma unroll
+  for (int t = 0; t < 16; ++t)
+    uw[t] = row < g.K ? __ldg(reinterpret_cast<const uint4*>(u + u_offset(t, row, c, g.K, g.C))) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        auto at = [&](int a, int b) {
+          const uint4& w = uw[4 * a + b];
+          const uint32_t x = e == 0 ? w.x : e == 1 ? w.y : e == 2 ? w.z : w.w;
+          return __half22float2(*reinterpret_cast<const __half2*>(&x));
+        };
+        auto col = [&](int a) {
+          if (s != 1) return at(a, s == 0 ? 0 : 3);
+          const float2 m = at(a, 1), n = at(a, 2);
+          return make_float2(m.x - n.x, m.y - n.y);
+        };
+        float2 v;
+        if (r != 1) {
+          v = col(r == 0 ? 0 : 3);
+        } else {
+          const float2 m = col(1), n = col(2);
+          v = make_float2(m.x - n.x, m.y - n.y);
+        }
+        const __half2 h = __floats2half2_rn(v.x, v.y);
+        o[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      *reinterpret_cast<uint4*>(dst + (size_t)(r * 3 + s) * rows * 32) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
+// The kernel body.  CG = 2: clusters of two CTAs (__cluster_dims__(2, 1, 1)),
+// a unit is 256 positions, rank 0 issues the pair's MMAs.  Every role walks
+// the source's layers and its own units of each.
+template <int CG, bool EPI, class Src>
+__device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& epi, uint32_t* err) {
   using namespace sc;
   extern __shared__ __align__(128) uint8_t shift_smem[];
   __shared__ Shared sh;
@@ -749,12 +976,11 @@ __device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint
   // a warp-uniform warp index, so that what the MMA warp derives stays in
   // uniform registers
   const int warp = __shfl_sync(0xffffffffu, (int)warp_id(), 0), lane = lane_id();
-  const Plan g = unpack_plan(p, CG);
   const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
   const int u0 = CG == 2 ? (int)cluster_id_x() : (int)blockIdx.x;
   const int ustep = CG == 2 ? (int)cluster_count_x() : (int)gridDim.x;
-  const int cnt = u0 < g.units ? (g.units - 1 - u0) / ustep + 1 : 0;
-  const int stage_bytes = g.stageA + g.stageB;
+  constexpr int TS = TM * CG;             // positions of a unit
+  const int tp = rank * TM;               // this CTA's first of them
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAXSTAGE; ++s) {
@@ -773,13 +999,11 @@ __device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint
   if (warp == WARP_MMA) {
     if (CG == 2) { tmem_alloc_pair(&sh.tmem_base, 512); tmem_relinquish_pair(); }
     else { tmem_alloc(&sh.tmem_base, 512); tmem_relinquish(); }
-    for (int t = lane; t < g.taps; t += 32) {
-      const int r = t / g.S, s = t - r * g.S;
-      sh.aoff[t] = tap_row(g, r, s);
-    }
   }
   volatile int* abort_flag = &sh.abort_flag;
   const uint32_t sbase = smem_u32(smem);
+  const int nl = src.layers();
+  bool ok = true;
 
   if (warp >= WARP_MMA && warp < WARP_P0) {
     regs_dec<REGS_MMA>();
@@ -788,53 +1012,82 @@ __device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint
       // the stages' weights, one bulk copy each: this CTA's rows of the unit's
       // output channels
       if (lane == 0) {
-        int st = 0, issued = 0;
-        uint32_t phase = 1;
-        bool ok = true;
-        uint8_t* dst = smem + g.stageA;
-        for (int i = 0; ok && i < cnt; ++i) {
-          int pt, k0;
-          unit_of(g, u0 + i * ustep, pt, k0);
-          const uint32_t piece = (uint32_t)(unit_n(g, CG, k0) / CG) * 32;      // one tap of 16 channels
-          const uint32_t block = piece * (uint32_t)g.taps;
-          const uint8_t* src = wop + (size_t)k0 * g.NKS * 32 + (size_t)rank * piece * g.NKS;
-          for (int cb = 0; cb < g.CB; cb += g.cps) {
-            if (!mbar_wait(&sh.empty[st], phase, abort_flag, err, ERR_WAIT_EMPTY)) { ok = false; break; }
-            const uint32_t bytes = block * (uint32_t)min(g.cps, g.CB - cb);
-            mbar_arrive_expect_tx(&sh.full[st], bytes);
-            bulk_g2s(dst, src, bytes, &sh.full[st]);
-            src += bytes;
-            dst += stage_bytes;
-            ++issued;
-            if (++st == g.nstage) { st = 0; dst = smem + g.stageA; phase ^= 1; }
+        RingPos pos{0, 1};
+        int issued = 0, nstage = 1;
+        // the operand is the kernel before's (programmatic launch); setup and
+        // the first input loads overlap with it
+        grid_dep_wait();
+        for (int l = 0; ok && l < nl; ++l) {
+          Conv cv;
+          if (!src.get(l, CG, u0, ustep, cv)) continue;
+          const Plan& g = cv.g;
+          nstage = g.nstage;
+          for (int i = 0; ok && i < cv.cnt; ++i) {
+            int pt, k0;
+            unit_of(g, cv.u0 + i * ustep, pt, k0);
+            const uint32_t piece = (uint32_t)(unit_n(g, CG, k0) / CG) * 32;      // one tap of 16 channels
+            const uint32_t block = piece * (uint32_t)g.taps;
+            const uint8_t* from = cv.wop + (size_t)k0 * g.NKS * 32 + (size_t)rank * piece * g.NKS;
+            for (int cb = 0; cb < g.CB; cb += g.cps) {
+              ok = mbar_wait(&sh.empty[pos.st], pos.phase, abort_flag, err, ERR_WAIT_EMPTY);
+              if (!ok) break;
+              const uint32_t bytes = block * (uint32_t)min(g.cps, g.CB - cb);
+              mbar_arrive_expect_tx(&sh.full[pos.st], bytes);
+              bulk_g2s(smem + pos.st * g.pitch + g.stageA, from, bytes, &sh.full[pos.st]);
+              from += bytes;
+              ++issued;
+              pos.next(nstage);
+            }
           }
         }
         // copies still in flight land before the CTA leaves (an abort may have
         // kept the MMA side from waiting for them)
         if (*abort_flag)
-          for (int b = issued > g.nstage ? issued - g.nstage : 0; b < issued; ++b)
-            mbar_wait(&sh.full[b % g.nstage], (b / g.nstage) & 1, nullptr, err, ERR_WAIT_FULL);
+          for (int b = issued > nstage ? issued - nstage : 0; b < issued; ++b)
+            mbar_wait(&sh.full[b % nstage], (b / nstage) & 1, nullptr, err, ERR_WAIT_FULL);
       }
     } else if (warp >= WARP_Z0) {
-      pad_rows(g, smem, sh, threadIdx.x - WARP_Z0 * 32, u0, ustep, cnt, rank * TM, TM * CG, err);
+      RingPos pos{0, 1};
+      for (int l = 0; ok && l < nl; ++l) {
+        Conv cv;
+        if (src.get(l, CG, u0, ustep, cv))
+          ok = pad_rows(cv, smem, sh, threadIdx.x - WARP_Z0 * 32, ustep, tp, TS, pos, err);
+      }
     } else {
       const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem_base, 0);
+      RingPos pos{0, 0};
       if (CG == 2 && rank == 1) {
         // tell rank 0 that this CTA's half of each stage is complete
         const uint32_t lead = mapa_shared(smem_u32(&sh.full[0]), 0);
-        int st = 0;
-        uint32_t phase = 0;
-        for (int left = cnt * g.nst; left > 0; --left) {
-          if (!wait_all_lanes(&sh.full[st], phase, abort_flag, err, ERR_WAIT_FULL)) break;
-          if (lane == 0) mbar_arrive_remote(lead + st * 8);
-          if (++st == g.nstage) { st = 0; phase ^= 1; }
+        for (int l = 0; ok && l < nl; ++l) {
+          Conv cv;
+          if (!src.get(l, CG, u0, ustep, cv)) continue;
+          for (int left = cv.cnt * cv.g.nst; ok && left > 0; --left) {
+            ok = wait_all_lanes(&sh.full[pos.st], pos.phase, abort_flag, err, ERR_WAIT_FULL);
+            if (ok && lane == 0) mbar_arrive_remote(lead + pos.st * 8);
+            pos.next(cv.g.nstage);
+          }
         }
-      } else if (g.taps == 9) {
-        issue_mmas<CG, 9>(g, sh, sbase, tmem, u0, ustep, cnt, err);
-      } else if (g.taps == 1) {
-        issue_mmas<CG, 1>(g, sh, sbase, tmem, u0, ustep, cnt, err);
       } else {
-        issue_mmas<CG, 0>(g, sh, sbase, tmem, u0, ustep, cnt, err);
+        const bool leader = elect_one();
+        int unit = 0;
+        bool ready = false;
+        for (int l = 0; ok && l < nl; ++l) {
+          Conv cv;
+          if (!src.get(l, CG, u0, ustep, cv)) continue;
+          __syncwarp();
+          for (int t = lane; t < cv.g.taps; t += 32) sh.aoff[t] = tap_row(cv.g, t / cv.g.S, t % cv.g.S);
+          __syncwarp();
+          if (Src::k33 || cv.g.taps == 9) ok = issue_mmas<CG, 9>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
+          else if (cv.g.taps == 1) ok = issue_mmas<CG, 1>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
+          else ok = issue_mmas<CG, 0>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
+        }
+        // every MMA issued (also on an abort) has finished before TMEM is freed
+        if (leader) {
+          if (CG == 2) mma_commit_pair(&sh.mmadone, 1);
+          else mma_commit(&sh.mmadone);
+          mbar_wait(&sh.mmadone, 0, nullptr, err, ERR_WAIT_ACCUM);
+        }
       }
     }
     __syncwarp();
@@ -844,74 +1097,94 @@ __device__ __forceinline__ void shift_conv_body(const KernelParam& p, const uint
     const uint32_t tmem = sh.tmem_base;
     // epilogue: TMEM lane 32 * quarter + lane = position of this CTA's tile
     const int quarter = warp;
-    __half* Y = static_cast<__half*>(p.pout);
-    const int OHOW = g.OH * g.OW;
-    const Grid gr = make_grid(g);
-    // even output rows sit on an even grid: neighbouring outputs on lanes 2i,
-    // 2i + 1 share 4-byte stores
-    const bool pair = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 3) == 0;
     const uint32_t lead_accempty = mapa_shared(smem_u32(&sh.accempty[0]), 0);
-    for (int ui = 0; ui < cnt; ++ui) {
-      int pt, k0;
-      unit_of(g, u0 + ui * ustep, pt, k0);
-      const int nrows = min(g.NB, g.Kp - k0);
-      const int kval = min(nrows, g.K - k0);             // output channels that exist
-      const int ab = ui & 1;
-      const Base c = advance(gr, tile_base(gr, pt * (TM * CG) + rank * TM), quarter * 32 + lane);
-      const bool live = c.n < g.N && c.gy < g.OH && c.gx < g.OW;
-      __half* yb = live ? Y + ((size_t)c.n * g.K + k0) * OHOW + (size_t)c.gy * g.OW + c.gx : Y;
-      if (!mbar_wait_warp(&sh.accfull[ab], (ui >> 1) & 1, abort_flag, err, ERR_WAIT_ACCUM, SLEEP_NS)) break;
-      tc_fence_after();
-      const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + ab * 256;
-      auto ld = [&](int cc, float* v) {
-        tmem_ld16(taddr + cc, v);
-        if (cc + 16 < nrows) tmem_ld16(taddr + cc + 16, v + 16);
-      };
-      auto stc = [&](int cc, const float* v) {
-        store_cols_f16<32>(yb + (size_t)cc * OHOW, (size_t)OHOW, v, kval - cc, live, pair);
-      };
-      float va[32], vb[32];
-      ld(0, va);
-      tmem_ld_wait();
-      for (int cc = 0; cc < nrows; cc += 64) {
-        if (cc + 32 < nrows) ld(cc + 32, vb);
-        stc(cc, va);
+    int unit = 0;
+    for (int l = 0; ok && l < nl; ++l) {
+      Conv cv;
+      if (!src.get(l, CG, u0, ustep, cv)) continue;
+      const Plan& g = cv.g;
+      __half* Y = cv.y;
+      const int OHOW = g.OH * g.OW;
+      const Grid gr = make_grid(g);
+      // even output rows sit on an even grid: neighbouring outputs on lanes
+      // 2i, 2i + 1 share 4-byte stores
+      const bool pair = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 3) == 0;
+      for (int i = 0; i < cv.cnt; ++i, ++unit) {
+        int pt, k0;
+        unit_of(g, cv.u0 + i * ustep, pt, k0);
+        const int nrows = min(g.NB, g.Kp - k0);
+        const int kval = min(nrows, g.K - k0);             // output channels that exist
+        const int ab = unit & 1;
+        const Base c = advance(gr, tile_base(gr, pt * TS + tp), quarter * 32 + lane);
+        const bool live = c.n < g.N && c.gy < g.OH && c.gx < g.OW;
+        const size_t at = live ? ((size_t)c.n * g.K + k0) * OHOW + (size_t)c.gy * g.OW + c.gx : 0;
+        ok = mbar_wait_warp(&sh.accfull[ab], (unit >> 1) & 1, abort_flag, err, ERR_WAIT_ACCUM, SLEEP_NS);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + ab * 256;
+        auto ld = [&](int cc, float* v) {
+          tmem_ld16(taddr + cc, v);
+          if (cc + 16 < nrows) tmem_ld16(taddr + cc + 16, v + 16);
+        };
+        auto stc = [&](int cc, const float* v) {
+          const size_t o = at + (size_t)cc * OHOW;
+          if (EPI)
+            store_cols_epi<32>(Y + o, epi.residual ? epi.residual + o : nullptr,
+                               epi.bias ? epi.bias + k0 + cc : nullptr, epi.relu, (size_t)OHOW, v, kval - cc, live, pair);
+          else
+            store_cols_f16<32>(Y + o, (size_t)OHOW, v, kval - cc, live, pair);
+        };
+        float va[32], vb[32];
+        ld(0, va);
         tmem_ld_wait();
-        if (cc + 32 >= nrows) break;
-        if (cc + 64 < nrows) ld(cc + 64, va);
-        stc(cc + 32, vb);
-        tmem_ld_wait();
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (CG == 2) mbar_arrive_peer(lead_accempty + ab * 8);
-        else mbar_arrive(&sh.accempty[ab]);
+        for (int cc = 0; cc < nrows; cc += 64) {
+          if (cc + 32 < nrows) ld(cc + 32, vb);
+          stc(cc, va);
+          tmem_ld_wait();
+          if (cc + 32 >= nrows) break;
+          if (cc + 64 < nrows) ld(cc + 64, va);
+          stc(cc + 32, vb);
+          tmem_ld_wait();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (CG == 2) mbar_arrive_peer(lead_accempty + ab * 8);
+          else mbar_arrive(&sh.accempty[ab]);
+        }
       }
     }
   } else {
     regs_inc<REGS_PROD>();
     const int group = (warp - WARP_P0) / NWARP_P, tid = threadIdx.x - (WARP_P0 + group * NWARP_P) * 32;
-    const int nitem = 2 * g.cps * g.qmax;
-    const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(p.pin) & 7) == 0;
-    const int tp = rank * TM, ts = TM * CG;
-    const bool strided = g.U > 1 || g.V > 1;
-#define SC_PRODUCE(ni, depth, al, strd) produce<CG, ni, depth, al, strd>(g, p, smem, sh, tid, group, u0, ustep, cnt, tp, ts, err)
-    if (aligned && !strided) {
-      if (nitem <= NPROD) SC_PRODUCE(1, 2, true, false);
-      else if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, false);
-      else SC_PRODUCE(4, 1, true, false);
-    } else if (aligned) {
-      if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, true);
-      else if (nitem <= 4 * NPROD) SC_PRODUCE(4, 1, true, true);
-      else SC_PRODUCE(6, 1, true, true);
-    } else if (!strided) {
-      if (nitem <= NPROD) SC_PRODUCE(1, 2, false, false);
-      else SC_PRODUCE(2, 1, false, false);
-    } else {
-      SC_PRODUCE(2, 1, false, true);
-    }
+    int done = 0;                         // stages of the layers before
+    bool set = false;                     // setup_sync passed
+    for (int l = 0; ok && l < nl; ++l) {
+      Conv cv;
+      if (!src.get(l, CG, u0, ustep, cv)) continue;
+      const Plan& g = cv.g;
+      const int nitem = 2 * g.cps * g.qmax;
+      const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(cv.x) & 7) == 0;
+      const bool strided = g.U > 1 || g.V > 1;
+#define SC_PRODUCE(ni, depth, al, strd) \
+  ok = produce<CG, ni, depth, al, strd>(cv, smem, sh, tid, group, done, ustep, tp, TS, set, err)
+      if (aligned && !strided) {
+        if (nitem <= NPROD) SC_PRODUCE(1, 2, true, false);
+        else if (Src::k33 || nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, false);
+        else SC_PRODUCE(4, 1, true, false);
+      } else if (!strided) {
+        if (Src::k33 || nitem <= NPROD) SC_PRODUCE(1, 2, false, false);
+        else SC_PRODUCE(2, 1, false, false);
+      } else if constexpr (!Src::k33) {
+        if (!aligned) SC_PRODUCE(2, 1, false, true);
+        else if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, true);
+        else if (nitem <= 4 * NPROD) SC_PRODUCE(4, 1, true, true);
+        else SC_PRODUCE(6, 1, true, true);
+      }
 #undef SC_PRODUCE
+      done += cv.cnt * g.nst;
+    }
+    if (!set) setup_sync<CG>();           // no stage for this group
   }
   tc_fence_before();
   __syncthreads();

@@ -241,6 +241,14 @@ __device__ __forceinline__ uint64_t policy_evict_first() {
   return p;
 }
 
+// ------------------------------------------------ programmatic launches ---
+// A kernel launched with programmatic stream serialization may start before
+// the kernel ahead of it has finished: grid_dep_wait returns once that kernel
+// is complete and its writes are visible (at once after an ordinary launch);
+// grid_dep_launch, in the kernel ahead, lets the next one start.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- cluster ---
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;

@@ -122,6 +122,10 @@ int wino_shift_threads();
 int wino_shift_smem_bytes();
 int wino_shift_prepare();
 uint32_t wino_shift_error_read_clear();
+int wino_shift_fused_cg(const wino::KernelParam* p, int cg);
+int wino_launch_dependent(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream);
+int wino_launch_shift_fused(const wino::KernelParam* p0, const void* u, void* wop, int cg, const wino::VariantArgs* va,
+                            int sms, cudaStream_t stream);
 }
 
 namespace {
@@ -584,12 +588,36 @@ extern "C" int wino_input_layout(const void* x, void* workspace, int n, int c, i
   return wino_launch_xb_layout(&p, (cudaStream_t)stream) == 0 ? WINO_OK : WINO_ECUDA;
 }
 
-extern "C" int wino_conv2d_fused_ws(const void* x, const void* ucache, void* workspace, void* y,
-                                    int n, int c, int h, int w, int k, void* stream) {
+// Workspace bytes of the fused entry points: the pre-pass records, and no less
+// than the shift kernel's weight operand where that kernel serves the shape.
+extern "C" size_t wino_fused_conv_workspace_bytes(int n, int c, int h, int w, int k) {
+  if (wino_check_shape(n, c, h, w, k) != WINO_OK) return 0;
+  const wino::KernelParam p = make_param(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, n, c, h, w, k);
+  const int cg = wino_shift_fused_cg(&p, 0);
+  const size_t xb = wino_xb_bytes(n, c, h, w), wop = cg ? wino_shift_weight_bytes(&p, cg) : 0;
+  return xb > wop ? xb : wop;
+}
+
+// The fused conv by the shift-reuse implicit GEMM, the filter recovered from
+// the U cache into the workspace: a WINO_* code, or -1 when the problem stays
+// with the fused Winograd kernel (too small, or no room for the operand).
+static int fused_shift(const void* x, const void* ucache, void* workspace, size_t workspace_bytes, void* y,
+                       const wino::VariantArgs* va, int n, int c, int h, int w, int k, cudaStream_t s) {
+  const wino::KernelParam p = make_param(x, nullptr, y, nullptr, nullptr, nullptr, n, c, h, w, k);
+  const int cg = wino_shift_fused_cg(&p, 0);
+  if (cg == 0 || wino_shift_weight_bytes(&p, cg) > workspace_bytes) return -1;
+  return wino_launch_shift_fused(&p, ucache, workspace, cg, va, sm_count(), s) == 0 ? WINO_OK : WINO_ECUDA;
+}
+
+extern "C" int wino_conv2d_fused_ws_sized(const void* x, const void* ucache, void* workspace, size_t workspace_bytes,
+                                          void* y, int n, int c, int h, int w, int k, void* stream) {
   if (!x || !ucache || !y || !workspace) return WINO_EINVAL;
   if ((reinterpret_cast<uintptr_t>(workspace) & 15) != 0) return WINO_EINVAL;
   const int st = wino_check_shape(n, c, h, w, k);
   if (st != WINO_OK) return st;
+  if (workspace_bytes < wino_xb_bytes(n, c, h, w)) return WINO_ESCRATCH;
+  const int rc = fused_shift(x, ucache, workspace, workspace_bytes, y, nullptr, n, c, h, w, k, (cudaStream_t)stream);
+  if (rc >= 0) return rc;
   if (!xb_items_ok(n, c, h, w)) return WINO_EUNSUPPORTED;
   if (wino_fused_prepare() != 0) return WINO_ECUDA;
   wino::KernelParam p = make_param(x, nullptr, y, workspace, const_cast<void*>(ucache), nullptr, n,
@@ -600,6 +628,12 @@ extern "C" int wino_conv2d_fused_ws(const void* x, const void* ucache, void* wor
                                          dim3(wino_fused_threads()), args,
                                          (size_t)wino_fused_smem_bytes(), (cudaStream_t)stream);
   return e == cudaSuccess ? WINO_OK : WINO_ECUDA;
+}
+
+extern "C" int wino_conv2d_fused_ws(const void* x, const void* ucache, void* workspace, void* y,
+                                    int n, int c, int h, int w, int k, void* stream) {
+  return wino_conv2d_fused_ws_sized(x, ucache, workspace, wino_fused_workspace_bytes(n, c, h, w), y, n, c, h, w, k,
+                                    stream);
 }
 
 // ------------------------------------------------ precision variants ----
@@ -694,20 +728,31 @@ extern "C" int wino_conv2d_variant(int variant, const void* x, const void* weigh
 extern "C" int wino_conv2d_fused_epilogue(const void* x, const void* ucache, void* workspace, void* y,
                                           const float* bias, const void* residual, int relu, int n, int c,
                                           int h, int w, int k, void* stream) {
+  return wino_conv2d_fused_epilogue_sized(x, ucache, workspace, wino_fused_workspace_bytes(n, c, h, w), y, bias, residual,
+                                          relu, n, c, h, w, k, stream);
+}
+
+extern "C" int wino_conv2d_fused_epilogue_sized(const void* x, const void* ucache, void* workspace,
+                                                size_t workspace_bytes, void* y, const float* bias,
+                                                const void* residual, int relu, int n, int c, int h, int w, int k,
+                                                void* stream) {
   if (!x || !ucache || !y || !workspace) return WINO_EINVAL;
   if ((reinterpret_cast<uintptr_t>(workspace) & 15) != 0) return WINO_EINVAL;
   if (residual && (reinterpret_cast<uintptr_t>(residual) & 3) != 0) return WINO_EINVAL;
   const int st = wino_check_shape(n, c, h, w, k);
   if (st != WINO_OK) return st;
-  if (!xb_items_ok(n, c, h, w)) return WINO_EUNSUPPORTED;
+  if (workspace_bytes < wino_xb_bytes(n, c, h, w)) return WINO_ESCRATCH;
   const cudaStream_t s = (cudaStream_t)stream;
-  wino::KernelParam p = make_param(x, nullptr, y, workspace, const_cast<void*>(ucache), nullptr, n, c, h,
-                                   w, k);
-  if (wino_launch_xb_layout(&p, s) != 0) return WINO_ECUDA;
   wino::VariantArgs va{};
   va.bias = bias;
   va.residual = residual;
   va.relu = relu ? 1 : 0;
+  const int rc = fused_shift(x, ucache, workspace, workspace_bytes, y, &va, n, c, h, w, k, s);
+  if (rc >= 0) return rc;
+  if (!xb_items_ok(n, c, h, w)) return WINO_EUNSUPPORTED;
+  wino::KernelParam p = make_param(x, nullptr, y, workspace, const_cast<void*>(ucache), nullptr, n, c, h,
+                                   w, k);
+  if (wino_launch_xb_layout(&p, s) != 0) return WINO_ECUDA;
   return wino_fused_launch_variant(WINO_VAR_F16, &p, &va, 0, fused_grid(n, h, w, k), s) == 0 ? WINO_OK
                                                                                           : WINO_ECUDA;
 }
@@ -789,9 +834,14 @@ extern "C" int wino_launch_kernelinfo(const void* kiv, void* param, void* stream
   for (int i = 0; i < 4; ++i) {
     if (fns[i] == wino_noop_kernel_ptr() || (no_m && fns[i] == wino_twostage_output_kernel_ptr())) continue;
     const unsigned* b = slots[i];
-    const cudaError_t e = cudaLaunchKernel(fns[i], dim3(b[0], b[1], b[2]), dim3(b[3], b[4], b[5]),
-                                           (void**)&param, (size_t)b[6], (cudaStream_t)stream);
-    if (e != cudaSuccess) return WINO_ECUDA;
+    const dim3 grid(b[0], b[1], b[2]), block(b[3], b[4], b[5]);
+    // the shift kernel starts beside the weight kernel launched right before
+    // it and waits for the weights itself
+    const bool dependent = i == 2 && (fns[0] == wino_shift_weight_kernel_ptr(1) || fns[0] == wino_shift_weight_kernel_ptr(2));
+    const int e = dependent ? wino_launch_dependent(fns[i], grid, block, (void**)&param, (size_t)b[6], (cudaStream_t)stream)
+                            : (int)cudaLaunchKernel(fns[i], grid, block, (void**)&param, (size_t)b[6],
+                                                    (cudaStream_t)stream);
+    if (e != (int)cudaSuccess) return WINO_ECUDA;
   }
   return WINO_OK;
 }

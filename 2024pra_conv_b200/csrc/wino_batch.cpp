@@ -40,6 +40,14 @@ long long wino_fused_nblocks_cfg(int n, int c, int h, int w, int k, int cfg);
 int wino_fused_cfg_splits(int c, int cfg);
 int wino_launch_y32_to_f16(const float* y32, void* y, long long count, cudaStream_t stream);
 int wino_launch_u_to_u2(const void* u, void* u2, int K, int C, cudaStream_t stream);
+int wino_shift_fused_cg(const wino::KernelParam* p, int cg);
+size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
+double wino_shift_unit_cost(const wino::KernelParam* p);
+void wino_shift_table_finish(wino::ShiftTable* t);
+int wino_shift_prepare();
+int wino_launch_shift_fused(const wino::KernelParam* p0, const void* u, void* wop, int cg, const wino::VariantArgs* va,
+                            int sms, cudaStream_t stream);
+int wino_launch_shift_batch(const wino::ShiftTable* t, int sms, cudaStream_t stream);
 size_t wino_twostage_workspace_bytes(int n, int c, int h, int w, int k);
 int wino_twostage_stage(int stage, const void* x, const void* ucache2, void* workspace, void* y, int n, int c,
                         int h, int w, int k, void* stream);
@@ -153,6 +161,8 @@ struct Layer {
   float twostage_us = -1.f; // the two-stage route alone (-1: not timed or not applicable)
   void* u2 = nullptr;       // U in the two-stage GEMM's layout (batch-owned)
   void* ws2 = nullptr;      // two-stage workspace (batch-owned)
+  bool shift = false;       // fused route on the shift-reuse implicit GEMM
+  size_t wop = 0;           // offset of its weight operand in the batch's buffer
   // U2 and the workspace for the two-stage route, made on first use from the
   // layer's fused U cache (synchronous: not inside a stream capture)
   int ensure_twostage() {
@@ -182,6 +192,9 @@ struct Batch {
   std::vector<Layer> layers;
   std::vector<int> order;        // table order of the layers
   BatchTable* table_dev = nullptr;
+  wino::ShiftTable shift{};      // layers on the shift kernel (a kernel argument)
+  void* operands = nullptr;      // their weight operands
+  size_t operand_bytes = 0;
   long long total = 0;
   bool dirty = true;
   cudaGraph_t graph = nullptr;
@@ -217,6 +230,25 @@ struct Batch {
     graph = nullptr;
   }
 
+  // Room for the shift layers' weight operands, which every run makes from the
+  // layers' U caches (not inside a stream capture).
+  int ensure_operands() {
+    size_t need = 0;
+    for (Layer& L : layers)
+      if (L.shift) {
+        L.wop = need;
+        need += align256(wino_shift_weight_bytes(&L.p, 2));
+      }
+    if (need <= operand_bytes) return WINO_OK;
+    if (settle() != WINO_OK) return WINO_ECUDA;  // no launch still reads the old buffer
+    if (operands) cudaFree(operands);
+    operands = nullptr;
+    operand_bytes = 0;
+    if (cudaMalloc(&operands, need) != cudaSuccess) return WINO_ECUDA;
+    operand_bytes = need;
+    return WINO_OK;
+  }
+
   // Build the table in `order` and copy it to the device (synchronous: never
   // called inside a stream capture).
   int commit() {
@@ -228,7 +260,7 @@ struct Batch {
     int nt = 0;
     for (size_t i = 0; i < order.size(); ++i) {
       const Layer& L = layers[order[i]];
-      if (L.route != ROUTE_FUSED) continue;     // launched on its own before the table
+      if (L.route != ROUTE_FUSED || L.shift) continue;     // not in this table
       LayerDesc& d = t.layer[nt++];
       d.p = L.p;
       int cfg = L.cfg;
@@ -241,6 +273,27 @@ struct Batch {
     t.nlayers = nt;
     t.total = begin;
     total = begin;
+    const int have = ensure_operands();
+    if (have != WINO_OK) return have;
+    // the shift kernel's table: the costliest units first, so that what is
+    // left at the end of the launch is small
+    std::vector<int> heavy;
+    for (int li : order)
+      if (layers[li].route == ROUTE_FUSED && layers[li].shift) heavy.push_back(li);
+    std::stable_sort(heavy.begin(), heavy.end(), [&](int a, int b) {
+      return wino_shift_unit_cost(&layers[a].p) > wino_shift_unit_cost(&layers[b].p);
+    });
+    wino::ShiftTable ht;
+    std::memset(&ht, 0, sizeof(ht));
+    for (int li : heavy) {
+      wino::ShiftLayer& d = ht.layer[ht.nlayers++];
+      d.p = layers[li].p;
+      d.p.pweight = layers[li].p.transform_filter;
+      d.p.transform_filter = static_cast<uint8_t*>(operands) + layers[li].wop;
+    }
+    wino_shift_table_finish(&ht);
+    if (ht.nlayers > 0 && wino_shift_prepare() != 0) return WINO_ECUDA;
+    shift = ht;
     if (settle() != WINO_OK) return WINO_ECUDA;  // no launch still reads the old table
     if (cudaMemcpy(table_dev, &t, sizeof(t), cudaMemcpyHostToDevice) != cudaSuccess) return WINO_ECUDA;
     dirty = false;
@@ -257,10 +310,11 @@ struct Batch {
         if (rc != WINO_OK) return rc;
         continue;
       }
-      if (L.p.transform_pin && !(L.cfg & wino::CFG_DIRECT) && wino_launch_xb_layout(&L.p, s) != 0)
+      if (!L.shift && L.p.transform_pin && !(L.cfg & wino::CFG_DIRECT) && wino_launch_xb_layout(&L.p, s) != 0)
         return WINO_ECUDA;
     }
-    if (total == 0) return WINO_OK;           // every layer on the two-stage route
+    if (shift.nlayers > 0 && wino_launch_shift_batch(&shift, sm_count(), s) != 0) return WINO_ECUDA;
+    if (total == 0) return WINO_OK;           // no layer on the fused Winograd kernel
     return wino_fused_launch_batch(table_dev, total, grid_for(total), s) == 0 ? WINO_OK : WINO_ECUDA;
   }
 };
@@ -341,6 +395,7 @@ int wino_batch_destroy(void* h) {
   b->drop_graph();
   for (Layer& L : b->layers) L.release();
   if (b->table_dev) cudaFree(b->table_dev);
+  if (b->operands) cudaFree(b->operands);
   if (b->done) cudaEventDestroy(b->done);
   delete b;
   return WINO_OK;
@@ -359,6 +414,9 @@ int wino_batch_add_layer(void* h, const void* x, const void* ucache, void* xb_ws
   L.p = layer_param(x, ucache, xb_ws, y, n, c, hh, w, k);
   L.blocks = wino_fused_nblocks(n, hh, w, k);
   L.cfg = xb_ws ? 0 : wino::CFG_DIRECT;
+  // the kernel wino_conv2d_fused_ws takes with room for its operand (a layer
+  // without a workspace stays with the direct fused kernel)
+  L.shift = xb_ws && wino_shift_fused_cg(&L.p, 2) == 2;
   b->order.push_back((int)b->layers.size());
   b->layers.push_back(L);
   b->dirty = true;
@@ -458,6 +516,8 @@ int wino_batch_tune(void* h, int reps, float* layer_us, float* order_us, void* s
   if (!b || b->layers.empty()) return WINO_EINVAL;
   const cudaStream_t s = (cudaStream_t)stream;
   const int nl = (int)b->layers.size();
+  const int have = b->ensure_operands();
+  if (have != WINO_OK) return have;
   for (int i = 0; i < nl; ++i) {
     Layer& L = b->layers[i];
     float us[wino::NCFG];
@@ -469,7 +529,15 @@ int wino_batch_tune(void* h, int reps, float* layer_us, float* order_us, void* s
       if (wino::cfg_split_level(cfg) != 0) continue;
       if (!L.p.transform_pin && !(cfg & wino::CFG_DIRECT)) continue;
       float t = 0.f;
-      const int rc = time_us([&] { return run_layer_cfg(L.p, L.p.transform_pin, cfg, s); }, reps, s, &t);
+      // (a layer on the shift kernel runs the same under every configuration)
+      auto one = [&] {
+        if (!L.shift) return run_layer_cfg(L.p, L.p.transform_pin, cfg, s);
+        KernelParam p = L.p;
+        p.transform_filter = nullptr;
+        return wino_launch_shift_fused(&p, L.p.transform_filter, static_cast<uint8_t*>(b->operands) + L.wop, 2, nullptr,
+                                       sm_count(), s) == 0 ? (int)WINO_OK : (int)WINO_ECUDA;
+      };
+      const int rc = time_us(one, reps, s, &t);
       if (rc != WINO_OK) return rc;
       us[cfg] = t;
       if (best < 0 || t < us[best]) best = cfg;

@@ -37,6 +37,20 @@ struct LayerDesc {
   int pad;
 };
 
+// Layers of the shift-reuse implicit GEMM (shift_conv.cuh) in one launch of
+// CTA pairs: p.transform_filter is the layer's weight operand,
+// p.transform_pin its packed plan, p.pweight the U cache the operand is made
+// from.  Units are numbered through the layers.
+struct ShiftLayer {
+  KernelParam p;
+  int unit_begin, units;
+};
+
+struct ShiftTable {
+  int nlayers, pitch, nstage, units;   // ring of stages: bytes from stage to stage, stages
+  ShiftLayer layer[BATCH_MAX];
+};
+
 struct BatchTable {
   int nlayers, pad;
   long long total;

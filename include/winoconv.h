@@ -115,6 +115,17 @@ int wino_input_layout(const void* x, void* workspace, int n, int c, int h, int w
 int wino_conv2d_fused_ws(const void* x, const void* ucache, void* workspace, void* y, int n, int c,
                          int h, int w, int k, void* stream);
 
+/* The same with the workspace's size stated (at least
+ * wino_fused_workspace_bytes, else WINO_ESCRATCH).  From 512 MFLOP on (direct
+ * count) the conv runs on the shift-reuse implicit GEMM instead of the fused
+ * Winograd kernel when the filter, recovered from the U cache, fits the
+ * workspace as that kernel's operand: wino_fused_conv_workspace_bytes is the
+ * size that always suffices (wino_fused_workspace_bytes, the size the entry
+ * point above assumes, does whenever 9 * k is at most about n * h * w). */
+size_t wino_fused_conv_workspace_bytes(int n, int c, int h, int w, int k);
+int wino_conv2d_fused_ws_sized(const void* x, const void* ucache, void* workspace, size_t workspace_bytes, void* y,
+                               int n, int c, int h, int w, int k, void* stream);
+
 /* The fast path with the step that follows a conv in a ResNet block folded
  * into its output transform (the reference stops at the conv, writing M and
  * transforming it in a separate kernel, src/conv2d.cpp:17-250):
@@ -126,6 +137,9 @@ int wino_conv2d_fused_ws(const void* x, const void* ucache, void* workspace, voi
 int wino_conv2d_fused_epilogue(const void* x, const void* ucache, void* workspace, void* y,
                                const float* bias, const void* residual, int relu, int n, int c, int h,
                                int w, int k, void* stream);
+int wino_conv2d_fused_epilogue_sized(const void* x, const void* ucache, void* workspace, size_t workspace_bytes, void* y,
+                                     const float* bias, const void* residual, int relu, int n, int c, int h, int w,
+                                     int k, void* stream);
 
 /* Direct convolution for any filter size r x s, stride (u, v) and padding
  * (p, q) and any channel counts (implicit GEMM on CUDA cores, fp32

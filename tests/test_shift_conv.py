@@ -234,3 +234,82 @@ def test_dropin_takes_the_shift_route(wino, cuda, shape, pin):
     torch.cuda.synchronize()
     assert wino.error_read_clear() == 0
     _check(y, x, wt, 1, 1, 1)
+
+
+def _fused_case(cuda, shape, seed):
+    import torch
+    n, c, h, w, k = shape
+    gen = torch.Generator(device=cuda).manual_seed(seed)
+    x = torch.randn((n, c, h, w), device=cuda, generator=gen).relu_().half()
+    wt = (torch.randn((k, c, 3, 3), device=cuda, generator=gen) * (2 / (9 * c)) ** 0.5).half()
+    bias = torch.randn(k, device=cuda, generator=gen) * 0.5
+    res = (torch.randn((n, k, h, w), device=cuda, generator=gen) * 0.5).half()
+    return x, wt, bias, res
+
+
+# At least 512 MFLOP: one CTA a unit, pairs, odd rows (2-byte stores), a K
+# block of 16 beside a full one.
+FUSED = [(8, 128, 28, 28, 128), (48, 128, 28, 28, 256), (16, 128, 15, 15, 144), (40, 64, 30, 22, 272)]
+# The filter from the fp16 U is off by 2.2e-4 in the 2-norm, y's rounding by at
+# most 2.8e-4, twice with a residual.
+FUSED_REL = 5e-4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["plain", "bias_relu", "residual", "all_in_place"])
+@pytest.mark.parametrize("shape", FUSED)
+def test_fused_conv_on_a_u_cache(wino, cuda, shape, mode):
+    import torch
+    x, wt, bias, res = _fused_case(cuda, shape, 3)
+    k = shape[4]
+    p = wino.fused_conv_workspace_bytes(*shape)
+    ws = torch.empty(p, dtype=torch.uint8, device=cuda)
+    u = wino.filter_transform(wt)
+    ref = torch.nn.functional.conv2d(x.double(), wt.double(), padding=1)
+    if mode == "plain":
+        y = wino.conv2d_fused(x, u, k, workspace=ws)
+    elif mode == "bias_relu":
+        y = wino.conv2d_fused_epilogue(x, u, k, bias=bias, relu=True, workspace=ws)
+        ref = torch.relu(ref + bias.double().view(1, -1, 1, 1))
+    elif mode == "residual":
+        y = wino.conv2d_fused_epilogue(x, u, k, residual=res, workspace=ws)
+        ref = ref + res.double()
+    else:
+        ref = torch.relu(ref + bias.double().view(1, -1, 1, 1) + res.double())
+        y = wino.conv2d_fused_epilogue(x, u, k, bias=bias, residual=res, relu=True, workspace=ws, out=res)
+    torch.cuda.synchronize()
+    assert wino.error_read_clear() == 0
+    assert float((y.double() - ref).norm() / ref.norm()) <= FUSED_REL
+
+
+@pytest.mark.gpu
+def test_batch_mixes_kernels(wino, cuda):
+    """Layers of at least 512 MFLOP run in one launch of the shift kernel, the
+    others in the fused kernel's; both equal the single-layer calls, from
+    capture too and after the U cache was rewritten in place."""
+    import torch
+    cases = [_fused_case(cuda, s, 4 + i) for i, s in enumerate(FUSED + [(2, 32, 14, 14, 32)])]
+    b, outs = wino.Batch(), []
+    for x, wt, _, res in cases:
+        u = wino.filter_transform(wt)
+        n, c, h, w = x.shape
+        ws = torch.empty(wino.fused_conv_workspace_bytes(n, c, h, w, wt.shape[0]), dtype=torch.uint8, device=cuda)
+        y = torch.full_like(res, float("nan"))
+        b.add(x, u, wt.shape[0], y, workspace=ws)
+        outs.append((x, u, wt, y))
+    torch.cuda.synchronize()
+    b.run()
+    b.capture()
+    for round_ in range(2):
+        torch.cuda.synchronize()
+        for x, u, wt, y in outs:
+            assert torch.equal(y, wino.conv2d_fused(x, u, wt.shape[0]))
+            y.fill_(float("nan"))
+            if round_ == 0:
+                u.copy_(wino.filter_transform(wt * 0.5))
+        b.launch()
+    torch.cuda.synchronize()
+    for x, u, wt, y in outs:
+        assert torch.equal(y, wino.conv2d_fused(x, u, wt.shape[0]))
+    b.close()
+    assert wino.error_read_clear() == 0
