@@ -28,21 +28,29 @@ __global__ void __launch_bounds__(128) shift_weight_u_batch_kernel(const __grid_
 
 // One CTA a unit (128 positions, up to 128 output channels).
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_kernel(KernelParam p) {
-  shift_conv_body<1, false>(sc::OneConv{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // A pair of CTAs a unit (256 positions, up to 256 output channels).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_pair_kernel(KernelParam p) {
-  shift_conv_body<2, false>(sc::OneConv{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
+}
+
+// The same for problems whose filter columns became channels.
+__global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_kernel(KernelParam p) {
+  shift_conv_body<1, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_pair_kernel(KernelParam p) {
+  shift_conv_body<2, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same with the fused epilogue.
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_epi_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<1, true>(sc::OneConv{p}, e, &g_shift_err);
+  shift_conv_body<1, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_epi_pair_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<2, true>(sc::OneConv{p}, e, &g_shift_err);
+  shift_conv_body<2, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
 }
 
 // A table of layers, passed by value: the roles read their layers' dims from
@@ -59,7 +67,10 @@ using namespace wino;
 
 extern "C" {
 
-void* wino_shift_kernel_ptr(int cg) { return cg == 2 ? (void*)shift_conv_pair_kernel : (void*)shift_conv_kernel; }
+void* wino_shift_kernel_ptr(const KernelParam* p, int cg) {
+  if (sc::folds(p->c, p->s)) return cg == 2 ? (void*)shift_conv_fold_pair_kernel : (void*)shift_conv_fold_kernel;
+  return cg == 2 ? (void*)shift_conv_pair_kernel : (void*)shift_conv_kernel;
+}
 void* wino_shift_weight_kernel_ptr(int cg) {
   return cg == 2 ? (void*)shift_weight_pair_kernel : (void*)shift_weight_kernel;
 }
@@ -78,12 +89,14 @@ int wino_shift_cg(const KernelParam* p) {
   const sc::Plan g1 = sc::make_plan(*p, 1), g2 = sc::make_plan(*p, 2);
   if (g1.npos + 4096 >= (1LL << 31) || g1.GX >= (1 << 15) || g1.GY >= (1 << 15)) return 0;
   // byte offsets into the input in 32 bits
-  if ((long long)g1.N * g1.C * g1.H * g1.W >= (1LL << 31)) return 0;
+  if ((long long)p->n * p->c * p->h * p->w >= (1LL << 31)) return 0;
   const bool aligned = (p->h * p->w) % 4 == 0 && (reinterpret_cast<uintptr_t>(p->pin) & 7) == 0;
   const bool strided = p->u > 1 || p->v > 1;
   const int items = (!aligned ? sc::MAXITEM_ODD : strided ? sc::MAXITEM_STRIDED : sc::MAXITEM) * sc::NPROD;
   for (const sc::Plan* g : {&g1, &g2})
-    if (2 * g->cps * g->qmax > items || g->nstage < 2 || g->rows > sc::MAXROWS) return 0;
+    if ((!g->fold && 2 * g->cps * g->qmax > items) || g->nstage < 2 || g->rows > sc::MAXROWS || g->nu > 2 ||
+        (g->fold && g->nst > 1))
+      return 0;
   const long long w1 = (g1.units + sc::NSM - 1) / sc::NSM, w2 = (g2.units + sc::NSM / 2 - 1) / (sc::NSM / 2);
   const int n2 = g2.Kp < 256 ? (g2.Kp + 31) / 32 * 32 : 256;
   // a pair needs work for every pair of SMs
@@ -109,6 +122,7 @@ int wino_shift_prepare() {
   if (cudaGetDevice(&dev) != cudaSuccess) return 1;
   if (dev >= 0 && dev < 64 && done[dev]) return 0;
   for (const void* f : {(const void*)shift_conv_kernel, (const void*)shift_conv_pair_kernel,
+                        (const void*)shift_conv_fold_kernel, (const void*)shift_conv_fold_pair_kernel,
                         (const void*)shift_conv_epi_kernel, (const void*)shift_conv_epi_pair_kernel,
                         (const void*)shift_conv_batch_kernel}) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sc::SMEM_BYTES) != cudaSuccess) return 1;
@@ -152,7 +166,7 @@ int wino_launch_dependent(const void* fn, dim3 grid, dim3 block, void** args, si
 // it on the stream is the one that makes the operand.
 int wino_launch_shift(const KernelParam* p, int cg, int sms, cudaStream_t stream) {
   void* args[] = {const_cast<KernelParam*>(p)};
-  return wino_launch_dependent(wino_shift_kernel_ptr(cg), dim3(wino_shift_grid(p, cg, sms)), dim3(sc::NTHREAD), args,
+  return wino_launch_dependent(wino_shift_kernel_ptr(p, cg), dim3(wino_shift_grid(p, cg, sms)), dim3(sc::NTHREAD), args,
                                (size_t)sc::SMEM_BYTES, stream);
 }
 
@@ -263,7 +277,7 @@ int wino_conv2d_shift(const void* x, const void* weight, void* wprep, void* y, i
     return 3;
   if (!x) return 0;
   if (weight) return wino_launch_shift(&p, cg, 148, (cudaStream_t)stream) == 0 ? 0 : 3;
-  return cudaLaunchKernel(wino_shift_kernel_ptr(cg), dim3(wino_shift_grid(&p, cg, 148)), dim3(sc::NTHREAD), args,
+  return cudaLaunchKernel(wino_shift_kernel_ptr(&p, cg), dim3(wino_shift_grid(&p, cg, 148)), dim3(sc::NTHREAD), args,
                           (size_t)sc::SMEM_BYTES, (cudaStream_t)stream) == cudaSuccess
              ? 0
              : 3;

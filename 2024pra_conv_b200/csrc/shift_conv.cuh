@@ -121,7 +121,17 @@ struct Plan {
   int pitch;           // bytes from stage to stage
   int qmax, qpi;       // quads of pixels a tile's rows may touch, quads per image
   long long npos;
+  // Few input channels (a network's stem): the filter's columns become
+  // channels, virtual channel c * S + s being input channel c at column offset
+  // s, so that C * S channels and R taps fill K-steps which C channels and R * S
+  // taps would leave mostly empty (3 of 16 for an RGB stem).  C, S, V, Q and W
+  // above are then the virtual problem's (C * S, 1, 1, 0, OW) and these the real ones.
+  bool fold;
+  int fC, fS, fV, fQ, fW;
 };
+
+// Whether a problem folds: two K-steps hold its virtual channels.
+__host__ __device__ __forceinline__ bool folds(int c, int s) { return c <= 8 && s > 1 && s <= 16 && c * s <= 32; }
 
 // Smallest grid extent for `o` outputs with filter extent f, stride st, pad
 // pd over an input extent e: a shift past the end must find zero padding on
@@ -154,16 +164,27 @@ __host__ __device__ __forceinline__ int mma_cycles(int cg, int n) {
   return reads > math ? reads : math;
 }
 
-template <bool K33 = false>
+// What a kernel knows of its problems at compile time.
+enum Kind : int { ANY, PLAIN, FOLDED, CONV33 };   // CONV33: 3x3 / stride 1 / pad 1
+
+template <int KIND = ANY>
 __host__ __device__ __forceinline__ void plan_dims(Plan& g, const KernelParam& p) {
   g.N = p.n; g.C = p.c; g.H = p.h; g.W = p.w; g.K = p.k;
-  if (K33) {                              // 3x3 / stride 1 / pad 1 known to the compiler
+  if (KIND == CONV33) {
     g.R = g.S = 3;
     g.U = g.V = g.P = g.Q = 1;
     g.OH = g.H; g.OW = g.W;
   } else {
     g.R = p.r; g.S = p.s;
     g.U = p.u; g.V = p.v; g.P = p.p; g.Q = p.q; g.OH = p.Oh; g.OW = p.Ow;
+  }
+  g.fold = KIND == FOLDED || (KIND == ANY && folds(g.C, g.S));
+  if (g.fold) {
+    g.fC = g.C; g.fS = g.S; g.fV = g.V; g.fQ = g.Q; g.fW = g.W;
+    g.C *= g.S;
+    g.S = g.V = 1;
+    g.Q = 0;
+    g.W = g.OW;
   }
   g.nu = g.U < g.R ? g.U : g.R;
   g.nv = g.V < g.S ? g.V : g.S;
@@ -230,14 +251,15 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg, bool table = false)
   // 3x3 filter's where four stages still fit (at most 64 output channels a
   // CTA): the producers' and the MMA thread's work per stage then covers twice
   // the MMAs.
-  int cps = g.taps >= 3 ? 2 : 4;
+  int cps = g.fold ? 2 : g.taps >= 3 ? 2 : 4;
   while (cps > 1 && (cps >> 1) >= g.CB) cps >>= 1;
   for (;; cps >>= 1) {
     g.lcps = cps == 4 ? 2 : cps == 2 ? 1 : 0;
     plan_finish(g, cg);
     const bool odd = ((g.H * g.W) & 3) != 0;
     const int items = table && odd ? NPROD : g.taps >= 6 ? 2 * NPROD : 3 * NPROD, stages = g.taps >= 6 ? 4 : 3;
-    if (cps == 1 || (2 * cps * g.qmax <= items && stages * (g.stageA + g.stageB) <= SMEM_STAGES)) break;
+    // (a folded problem's unit is one stage)
+    if (cps == 1 || g.fold || (2 * cps * g.qmax <= items && stages * (g.stageA + g.stageB) <= SMEM_STAGES)) break;
   }
   const int fit = SMEM_STAGES / (g.stageA + g.stageB);
   g.nstage = fit < MAXSTAGE ? fit : MAXSTAGE;
@@ -249,10 +271,10 @@ __host__ inline unsigned long long pack_plan(const Plan& g) {
          (unsigned long long)g.lcps << 40 | (unsigned long long)g.nstage << 44 | (unsigned long long)g.qmax << 48;
 }
 
-template <bool K33 = false>
+template <int KIND = ANY>
 __device__ __forceinline__ Plan unpack_plan(const KernelParam& p, int cg) {
   Plan g;
-  plan_dims<K33>(g, p);
+  plan_dims<KIND>(g, p);
   const unsigned long long w = reinterpret_cast<unsigned long long>(p.transform_pin);
   g.GX = (int)(w & 0xffff);
   g.GY = (int)(w >> 16 & 0xffff);
@@ -275,12 +297,13 @@ struct Conv {
 };
 
 // A launch over one convolution (its argument carries the packed plan).
+template <int KIND>
 struct OneConv {
-  static constexpr bool k33 = false;
+  static constexpr int kind = KIND;
   const KernelParam& p;
   __device__ __forceinline__ int layers() const { return 1; }
   __device__ __forceinline__ bool get(int, int cg, int u, int step, Conv& c) const {
-    c.g = unpack_plan(p, cg);
+    c.g = unpack_plan<KIND>(p, cg);
     c.x = static_cast<const unsigned short*>(p.pin);
     c.y = static_cast<__half*>(p.pout);
     c.wop = static_cast<const uint8_t*>(p.transform_filter);
@@ -293,7 +316,7 @@ struct OneConv {
 // ... and over a table of them, units numbered through (wino_batch.h): the
 // ring of stages runs on across layers, so its pitch is the largest stage's.
 struct ConvTable {
-  static constexpr bool k33 = true;       // 3x3 / stride 1 / pad 1 layers only
+  static constexpr int kind = CONV33;
   const ShiftTable& t;                    // the kernel's argument (constant bank)
   __device__ __forceinline__ int layers() const { return t.nlayers; }
   __device__ __forceinline__ bool get(int l, int cg, int u, int step, Conv& c) const {
@@ -303,7 +326,7 @@ struct ConvTable {
     c.u0 = skip;
     c.cnt = skip < d.units ? (d.units - 1 - skip) / step + 1 : 0;
     if (c.cnt == 0) return false;
-    c.g = unpack_plan<true>(d.p, cg);
+    c.g = unpack_plan<CONV33>(d.p, cg);
     c.g.pitch = t.pitch;
     c.g.nstage = t.nstage;
     c.x = static_cast<const unsigned short*>(d.p.pin);
@@ -670,6 +693,77 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   return ok;
 }
 
+// Producers of a folded problem (Plan): thread = operand row, a position's
+// C * S values gathered with 2-byte loads (lanes on neighbouring output
+// columns) into up to four 16-byte words.  N32 224x224 RGB 7x7 / 2
+// K64 takes 72 us, waiting on these gathers (CUDA-core direct kernel: 590 us;
+// its bytes take 9).  A unit is one stage and the groups
+// take alternate units.  FC, FS: channels and columns known at compile time
+// (0: as the plan says).
+template <int CG, int FC, int FS>
+__device__ __forceinline__ bool produce_fold(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int ustep,
+                                             int tile_pos, int tile_stride, uint32_t* err) {
+  const Plan& g = cv.g;
+  volatile int* abort_flag = &sh.abort_flag;
+  const int C = FC ? FC : g.fC, S = FC ? FS : g.fS, HW = g.H * g.fW, ngrp = 2 * g.cps;
+  const Grid gr = make_grid(g);
+  const int plane0 = plane_rows(g, 0, 0);
+  RingPos pos{group % g.nstage, 1u ^ (uint32_t)((group / g.nstage) & 1)};
+  for (int i = group; i < cv.cnt; i += NGROUP, pos.next(g.nstage, NGROUP)) {
+    int pt, k0;
+    unit_of(g, cv.u0 + i * ustep, pt, k0);
+    const Base b0 = tile_base(gr, pt * tile_stride + tile_pos);
+    if (!wait_all_lanes(&sh.empty[pos.st], pos.phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
+    uint8_t* dst = smem + pos.st * g.pitch;
+#pragma unroll 2
+    for (int r = tid; r < g.rows; r += NPROD) {
+      const int a = r >= plane0 ? 1 : 0;
+      const Base c = advance(gr, b0, r - (a ? plane0 : 0));
+      const int y = c.gy * g.U + a - g.P, x0 = c.gx * g.fV - g.fQ;
+      // columns s of the filter that lie in the image
+      const int lo = max(0, -x0), hi = min(S, g.fW - x0);
+      uint32_t in = c.n < g.N && (unsigned)y < (unsigned)g.H && c.gx < g.OW && hi > lo
+                        ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
+      const unsigned short* src = cv.x + ((long long)(c.n * C) * HW + (long long)y * g.fW + x0);
+      if (FC) {
+        uint32_t v[32];
+#pragma unroll
+        for (int ch = 0; ch < FC; ++ch)
+#pragma unroll
+          for (int s = 0; s < FS; ++s) {
+            uint32_t e = 0;
+            if (in >> s & 1u) e = __ldg(src + ch * HW + s);
+            v[ch * FS + s] = e;
+          }
+#pragma unroll
+        for (int e = FC * FS; e < 32; ++e) v[e] = 0;
+#pragma unroll
+        for (int grp = 0; grp < 4; ++grp)
+          if (grp < ngrp)
+            *reinterpret_cast<uint4*>(dst + (grp * g.rows + r) * 16) =
+                make_uint4(v[8 * grp] | v[8 * grp + 1] << 16, v[8 * grp + 2] | v[8 * grp + 3] << 16,
+                           v[8 * grp + 4] | v[8 * grp + 5] << 16, v[8 * grp + 6] | v[8 * grp + 7] << 16);
+      } else {
+        int ch = 0, s = 0;
+        for (int grp = 0; grp < ngrp; ++grp) {
+          uint32_t v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            v[e] = ch < C && (in >> s & 1u) ? (uint32_t)__ldg(src + ch * HW + s) : 0u;
+            if (++s == S) { s = 0; ++ch; }
+          }
+          *reinterpret_cast<uint4*>(dst + (grp * g.rows + r) * 16) =
+              make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+        }
+      }
+    }
+    fence_proxy_async_shared();
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(&sh.full[pos.st]);
+  }
+  return true;
+}
+
 // Padding rows of the operand (two warps): the zero columns and rows of a
 // tile's positions, written to every stage (a slot's last tile had them
 // elsewhere).
@@ -898,10 +992,13 @@ __device__ __forceinline__ void shift_weight_body(const KernelParam& p, uint8_t*
 #pragma unroll
   for (int e = 0; e < 8; e += 2) {
     const int c = cb * 16 + hh * 8 + e;
-    uint32_t lo = 0, hi = 0;
-    if (row < g.K && c < g.C) lo = w[((size_t)row * g.C + c) * g.taps + tap];
-    if (row < g.K && c + 1 < g.C) hi = w[((size_t)row * g.C + c + 1) * g.taps + tap];
-    v[e >> 1] = lo | (hi << 16);
+    auto at = [&](int ch) {
+      if (row >= g.K || ch >= g.C) return 0u;
+      if (!g.fold) return (uint32_t)w[((size_t)row * g.C + ch) * g.taps + tap];
+      const int rc = ch / g.fS;           // virtual channel -> input channel, filter column
+      return (uint32_t)w[(((size_t)row * g.fC + rc) * g.R + tap) * g.fS + ch - rc * g.fS];
+    };
+    v[e >> 1] = at(c) | at(c + 1) << 16;
   }
   uint8_t* dst = wop + ((size_t)(k0 + rank * rows) * g.NKS + (size_t)ks * rows) * 32 + (rr >> 3) * 256 + hh * 128 +
                  (rr & 7) * 16;
@@ -919,7 +1016,7 @@ template <int CG>
 __device__ __forceinline__ void shift_weight_from_u(const KernelParam& p, const __half* u, uint8_t* wop, unsigned item) {
   using namespace sc;
   grid_dep_launch();
-  const Plan g = unpack_plan<true>(p, CG);
+  const Plan g = unpack_plan<CONV33>(p, CG);
   // rows fastest: neighbouring threads read and write neighbouring 16-byte rows
   const int last = (g.nKU - 1) * g.NB, nrow = last + unit_n(g, CG, last);
   const int grp = (int)(item / (unsigned)nrow), row = (int)(item - (unsigned)grp * (unsigned)nrow), c = grp * 8;
@@ -1078,8 +1175,8 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
           __syncwarp();
           for (int t = lane; t < cv.g.taps; t += 32) sh.aoff[t] = tap_row(cv.g, t / cv.g.S, t % cv.g.S);
           __syncwarp();
-          if (Src::k33 || cv.g.taps == 9) ok = issue_mmas<CG, 9>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
-          else if (cv.g.taps == 1) ok = issue_mmas<CG, 1>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
+          if (Src::kind == CONV33 || (Src::kind != FOLDED && cv.g.taps == 9)) ok = issue_mmas<CG, 9>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
+          else if (Src::kind != FOLDED && cv.g.taps == 1) ok = issue_mmas<CG, 1>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
           else ok = issue_mmas<CG, 0>(cv, sh, sbase, tmem, ustep, leader, pos, unit, ready, err);
         }
         // every MMA issued (also on an abort) has finished before TMEM is freed
@@ -1163,25 +1260,33 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       Conv cv;
       if (!src.get(l, CG, u0, ustep, cv)) continue;
       const Plan& g = cv.g;
-      const int nitem = 2 * g.cps * g.qmax;
-      const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(cv.x) & 7) == 0;
-      const bool strided = g.U > 1 || g.V > 1;
+      if constexpr (Src::kind == FOLDED) {
+        setup_sync<CG>();
+        set = true;
+        if (g.fC == 3 && g.fS == 7) ok = produce_fold<CG, 3, 7>(cv, smem, sh, tid, group, ustep, tp, TS, err);
+        else ok = produce_fold<CG, 0, 0>(cv, smem, sh, tid, group, ustep, tp, TS, err);
+      } else {
+        const int nitem = 2 * g.cps * g.qmax;
+        const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(cv.x) & 7) == 0;
+        const bool strided = g.U > 1 || g.V > 1;
+        constexpr bool k33 = Src::kind == CONV33;
 #define SC_PRODUCE(ni, depth, al, strd) \
   ok = produce<CG, ni, depth, al, strd>(cv, smem, sh, tid, group, done, ustep, tp, TS, set, err)
-      if (aligned && !strided) {
-        if (nitem <= NPROD) SC_PRODUCE(1, 2, true, false);
-        else if (Src::k33 || nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, false);
-        else SC_PRODUCE(4, 1, true, false);
-      } else if (!strided) {
-        if (Src::k33 || nitem <= NPROD) SC_PRODUCE(1, 2, false, false);
-        else SC_PRODUCE(2, 1, false, false);
-      } else if constexpr (!Src::k33) {
-        if (!aligned) SC_PRODUCE(2, 1, false, true);
-        else if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, true);
-        else if (nitem <= 4 * NPROD) SC_PRODUCE(4, 1, true, true);
-        else SC_PRODUCE(6, 1, true, true);
-      }
+        if (aligned && !strided) {
+          if (nitem <= NPROD) SC_PRODUCE(1, 2, true, false);
+          else if (k33 || nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, false);
+          else SC_PRODUCE(4, 1, true, false);
+        } else if (!strided) {
+          if (k33 || nitem <= NPROD) SC_PRODUCE(1, 2, false, false);
+          else SC_PRODUCE(2, 1, false, false);
+        } else if constexpr (!k33) {
+          if (!aligned) SC_PRODUCE(2, 1, false, true);
+          else if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, true);
+          else if (nitem <= 4 * NPROD) SC_PRODUCE(4, 1, true, true);
+          else SC_PRODUCE(6, 1, true, true);
+        }
 #undef SC_PRODUCE
+      }
       done += cv.cnt * g.nst;
     }
     if (!set) setup_sync<CG>();           // no stage for this group

@@ -1186,7 +1186,7 @@ __global__ void __launch_bounds__(TMAV && F8 ? trs::NTHREAD_V : trs::NTHREAD, 1)
   static_assert(trs::NTHREAD == sc::NTHREAD && sc::SMEM_BYTES <= 227 * 1024, "one kernel hosts both schedules");
   if constexpr (TMAV && F8 == 0) {
     if (p.mid_result == nullptr) {
-      shift_conv_body<1, false>(sc::OneConv{p}, sc::Epi{}, &g_twostage_err);
+      shift_conv_body<1, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_twostage_err);
       return;
     }
   }

@@ -117,7 +117,7 @@ unsigned wino_shift_grid(const wino::KernelParam* p, int cg, int sms);
 size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
 unsigned wino_shift_weight_grid(const wino::KernelParam* p, int cg);
 void* wino_shift_weight_kernel_ptr(int cg);
-void* wino_shift_kernel_ptr(int cg);
+void* wino_shift_kernel_ptr(const wino::KernelParam* p, int cg);
 int wino_shift_threads();
 int wino_shift_smem_bytes();
 int wino_shift_prepare();
@@ -368,7 +368,7 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
     const bool hosted = shift.cg == 1 && pr.c <= 256 && wino_contract(pr) && two_stage_fits(pr);
     set_slot(kernelInfo, 3, wino_shift_grid(kp, shift.cg, sm_count()), 1, 1, (unsigned)wino_shift_threads(), 1, 1,
              (unsigned)wino_shift_smem_bytes(),
-             hosted ? wino_twostage_gemm_kernel_ptr_for((int)pr.c) : wino_shift_kernel_ptr(shift.cg));
+             hosted ? wino_twostage_gemm_kernel_ptr_for((int)pr.c) : wino_shift_kernel_ptr(kp, shift.cg));
     if (hosted)
       set_slot(kernelInfo, 4, 1, 1, 1, (unsigned)wino_twostage_output_threads(), 1, 1, 0,
                wino_twostage_output_kernel_ptr());

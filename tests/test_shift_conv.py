@@ -206,6 +206,41 @@ def test_shift_conv(wino, cuda, shape, cg):
     _check(_conv(wino, x, wt, stride, p, q, cg), x, wt, stride, p, q)
 
 
+# few channels: the filter's columns become channels
+FOLDED = [
+    (2, 3, 32, 32, 64, 7, 7, 2, 3, 3),       # RGB stem
+    (3, 3, 37, 45, 40, 7, 7, 2, 3, 3),       # odd height and width, ragged K
+    (2, 3, 64, 60, 96, 7, 7, 2, 3, 3),       # several units
+    (1, 3, 9, 8, 16, 7, 7, 2, 3, 3),         # image smaller than the filter's reach
+    (3, 5, 20, 17, 24, 3, 3, 1, 1, 1),       # 15 of 16 virtual channels, stride 1
+    (2, 8, 15, 15, 32, 3, 3, 2, 1, 1),       # 24 virtual channels
+    (2, 4, 12, 18, 16, 2, 5, 1, 0, 2),       # 2x5 filter
+    (2, 2, 21, 19, 32, 3, 3, 1, 1, 1),       # one K-step
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cg", [1, 2])
+@pytest.mark.parametrize("shape", FOLDED)
+def test_folded_conv(wino, cuda, shape, cg):
+    test_shift_conv(wino, cuda, shape, cg)
+
+
+@pytest.mark.gpu
+def test_dropin_stem(wino, cuda):
+    """A stem's operand does not fit transform_filter and goes to
+    transform_pin; without one the direct kernel runs."""
+    import torch
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    x = torch.randn((4, 3, 112, 112), device=cuda, generator=gen).half()
+    wt = (torch.randn((64, 3, 7, 7), device=cuda, generator=gen) / 12).half()
+    for pin in (True, False):
+        y = wino.dropin_conv2d(x, wt, transform_pin=pin, stride=2, pad=3)
+        torch.cuda.synchronize()
+        assert wino.error_read_clear() == 0
+        _check(y, x, wt, 2, 3, 3)
+
+
 @pytest.mark.gpu
 def test_shift_conv_unaligned_input(wino, cuda):
     """An input 2 bytes off its allocation takes the unaligned quads."""
