@@ -88,8 +88,9 @@ int wino_shift_cg(const KernelParam* p) {
   if (p->u > 2 || p->v > 2 || p->r * p->s > sc::MAXTAP) return 0;
   const sc::Plan g1 = sc::make_plan(*p, 1), g2 = sc::make_plan(*p, 2);
   if (g1.npos + 4096 >= (1LL << 31) || g1.GX >= (1 << 15) || g1.GY >= (1 << 15)) return 0;
-  // byte offsets into the input in 32 bits
-  if ((long long)p->n * p->c * p->h * p->w >= (1LL << 31)) return 0;
+  // byte offsets into input and output in 32 bits
+  if ((long long)p->n * p->c * p->h * p->w >= (1LL << 31) || (long long)p->n * p->k * p->Oh * p->Ow >= (1LL << 31))
+    return 0;
   const bool aligned = (p->h * p->w) % 4 == 0 && (reinterpret_cast<uintptr_t>(p->pin) & 7) == 0;
   const bool strided = p->u > 1 || p->v > 1;
   const int items = (!aligned ? sc::MAXITEM_ODD : strided ? sc::MAXITEM_STRIDED : sc::MAXITEM) * sc::NPROD;

@@ -913,56 +913,72 @@ struct Epi {
   int relu;
 };
 
-// store_cols_f16 with the fused epilogue: conv + bias is rounded to fp16, the
-// residual added in fp32, ReLU last.  `res`: the residual's element of this
-// row and column 0 (or null); bias: of column 0 (or null).
-template <int NC>
-__device__ __forceinline__ void store_cols_epi(__half* row, const __half* res, const float* bias, int relu,
-                                               size_t stride, const float* v, int lim, bool live, bool pair) {
-  const bool odd = (threadIdx.x & 1) != 0;
+// Stores NC accumulator columns (output channels) of a position per lane:
+// column c < lim of this lane goes to byte offset o + c * step of Y (32-bit
+// offsets: an output of 4 GB or more is not this kernel's).  With `pair` the
+// lanes 2i and 2i + 1 hold neighbouring outputs of one row, live together:
+// two columns are rounded into one word, the pair swaps words, and each lane
+// stores one column of both -- a conversion, a shuffle, a byte permute, an
+// add and a 4-byte store for two columns (40 -> 25 cycles a column of a 128 x
+// 256 unit against float shuffles and 64-bit addresses).
+// EPI: + bias (rounded to fp16), + residual in fp32, ReLU last.  All 32 lanes call.
+template <int NC, bool EPI>
+__device__ __forceinline__ void store_cols(const Epi& epi, const float* bias, char* Y, uint32_t o, uint32_t step,
+                                           const float* v, int lim, bool live, bool pair) {
+  const char* R = EPI ? reinterpret_cast<const char*>(epi.residual) : nullptr;
   auto finish = [&](__half2 h, __half2 r) {
     float2 f = __half22float2(h);
-    if (res) {
+    if (R) {
       const float2 g = __half22float2(r);
       f.x += g.x;
       f.y += g.y;
     }
-    if (relu) {
+    if (epi.relu) {
       f.x = fmaxf(f.x, 0.f);
       f.y = fmaxf(f.y, 0.f);
     }
     return __floats2half2_rn(f.x, f.y);
   };
   if (pair) {
-    __half* first = row - (odd ? 1 : 0);
-    const __half* rfirst = res ? res - (odd ? 1 : 0) : nullptr;
+    const bool odd = (threadIdx.x & 1) != 0;
+    const uint32_t sel = odd ? 0x3276u : 0x5410u;
+    // the pair's even position, this lane's column of the first two
+    uint32_t at = o - (odd ? 2u : 0u) + (odd ? step : 0u);
+    const int mine = odd ? 1 : 0;
+    __half2 rv[EPI ? NC / 2 : 1];
+    if (EPI && R) {
+      uint32_t ra = at;
 #pragma unroll
-    for (int j0 = 0; j0 < NC / 2; j0 += 8) {
-      __half2 rv[8];
-      float bv[8], other[8];
+      for (int j = 0; j < NC / 2; ++j, ra += 2 * step)
+        rv[j] = live && 2 * j + mine < lim ? *reinterpret_cast<const __half2*>(R + ra) : __half2{};
+    }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int col = 2 * (j0 + j) + (odd ? 1 : 0);
-        const bool on = live && col < lim;
-        rv[j] = on && res ? *reinterpret_cast<const __half2*>(rfirst + (size_t)col * stride) : __half2{};
-        bv[j] = on && bias ? __ldg(bias + col) : 0.f;
-        other[j] = __shfl_xor_sync(0xffffffffu, odd ? v[2 * (j0 + j)] : v[2 * (j0 + j) + 1], 1);
+    for (int j = 0; j < NC / 2; ++j, at += 2 * step) {
+      float a = v[2 * j], b = v[2 * j + 1];
+      if (EPI && bias) {
+        // (bias of channels past K is not read: lim)
+        a += 2 * j < lim ? __ldg(bias + 2 * j) : 0.f;
+        b += 2 * j + 1 < lim ? __ldg(bias + 2 * j + 1) : 0.f;
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int c = 2 * (j0 + j), col = c + (odd ? 1 : 0);
-        const __half2 h = odd ? __floats2half2_rn(other[j] + bv[j], v[c + 1] + bv[j])
-                              : __floats2half2_rn(v[c] + bv[j], other[j] + bv[j]);
-        if (live && col < lim) *reinterpret_cast<__half2*>(first + (size_t)col * stride) = finish(h, rv[j]);
-      }
+      const __half2 h = __floats2half2_rn(a, b);
+      const uint32_t own = *reinterpret_cast<const uint32_t*>(&h);
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+      const uint32_t w = __byte_perm(own, other, sel);
+      __half2 out = *reinterpret_cast<const __half2*>(&w);
+      if (EPI) out = finish(out, rv[j]);
+      if (live && 2 * j + mine < lim) *reinterpret_cast<__half2*>(Y + at) = out;
     }
   } else if (live) {
+    uint32_t at = o;
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
+    for (int c = 0; c < NC; ++c, at += step)
       if (c < lim) {
-        const __half h = __float2half_rn(v[c] + (bias ? __ldg(bias + c) : 0.f));
-        const __half r = res ? res[(size_t)c * stride] : __half{};
-        row[(size_t)c * stride] = __low2half(finish(__half2half2(h), __half2half2(r)));
+        __half h = __float2half_rn(v[c] + (EPI && bias ? __ldg(bias + c) : 0.f));
+        if (EPI) {
+          const __half r = R ? *reinterpret_cast<const __half*>(R + at) : __half{};
+          h = __low2half(finish(__half2half2(h), __half2half2(r)));
+        }
+        *reinterpret_cast<__half*>(Y + at) = h;
       }
   }
 }
@@ -1202,6 +1218,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       const Plan& g = cv.g;
       __half* Y = cv.y;
       const int OHOW = g.OH * g.OW;
+      const uint32_t step = (uint32_t)OHOW * 2u;
       const Grid gr = make_grid(g);
       // even output rows sit on an even grid: neighbouring outputs on lanes
       // 2i, 2i + 1 share 4-byte stores
@@ -1214,7 +1231,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         const int ab = unit & 1;
         const Base c = advance(gr, tile_base(gr, pt * TS + tp), quarter * 32 + lane);
         const bool live = c.n < g.N && c.gy < g.OH && c.gx < g.OW;
-        const size_t at = live ? ((size_t)c.n * g.K + k0) * OHOW + (size_t)c.gy * g.OW + c.gx : 0;
+        const uint32_t at = live ? ((uint32_t)(c.n * g.K + k0) * (uint32_t)OHOW + (uint32_t)(c.gy * g.OW + c.gx)) * 2u : 0u;
         ok = mbar_wait_warp(&sh.accfull[ab], (unit >> 1) & 1, abort_flag, err, ERR_WAIT_ACCUM, SLEEP_NS);
         if (!ok) break;
         tc_fence_after();
@@ -1224,12 +1241,8 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
           if (cc + 16 < nrows) tmem_ld16(taddr + cc + 16, v + 16);
         };
         auto stc = [&](int cc, const float* v) {
-          const size_t o = at + (size_t)cc * OHOW;
-          if (EPI)
-            store_cols_epi<32>(Y + o, epi.residual ? epi.residual + o : nullptr,
-                               epi.bias ? epi.bias + k0 + cc : nullptr, epi.relu, (size_t)OHOW, v, kval - cc, live, pair);
-          else
-            store_cols_f16<32>(Y + o, (size_t)OHOW, v, kval - cc, live, pair);
+          store_cols<32, EPI>(epi, EPI && epi.bias ? epi.bias + k0 + cc : nullptr, reinterpret_cast<char*>(Y),
+                              at + (uint32_t)cc * step, step, v, kval - cc, live, pair);
         };
         float va[32], vb[32];
         ld(0, va);
