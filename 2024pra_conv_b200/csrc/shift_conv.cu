@@ -28,29 +28,29 @@ __global__ void __launch_bounds__(128) shift_weight_u_batch_kernel(const __grid_
 
 // One CTA a unit (128 positions, up to 128 output channels).
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_kernel(KernelParam p) {
-  shift_conv_body<1, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, sc::Wide, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // A pair of CTAs a unit (256 positions, up to 256 output channels).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_pair_kernel(KernelParam p) {
-  shift_conv_body<2, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::Wide, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same for problems whose filter columns became channels.
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_kernel(KernelParam p) {
-  shift_conv_body<1, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, sc::Wide, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_pair_kernel(KernelParam p) {
-  shift_conv_body<2, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::Wide, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same with the fused epilogue.
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_epi_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<1, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
+  shift_conv_body<1, sc::Wide, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_epi_pair_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<2, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
+  shift_conv_body<2, sc::Wide, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
 }
 
 // A table of layers, passed by value: the roles read their layers' dims from
@@ -58,7 +58,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
 // and spilled).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_batch_kernel(const __grid_constant__ ShiftTable t) {
-  shift_conv_body<2, false>(sc::ConvTable{t}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::Wide, false>(sc::ConvTable{t}, sc::Epi{}, &g_shift_err);
 }
 
 }  // namespace wino
@@ -78,7 +78,7 @@ size_t wino_shift_weight_bytes(const KernelParam* p, int cg) { return sc::weight
 unsigned wino_shift_weight_grid(const KernelParam* p, int cg) {
   return (unsigned)((wino_shift_weight_bytes(p, cg) / 16 + 255) / 256);
 }
-int wino_shift_threads() { return sc::NTHREAD; }
+int wino_shift_threads(int hosted) { return hosted ? sc::NTHREAD_HOSTED : sc::NTHREAD; }
 int wino_shift_smem_bytes() { return sc::SMEM_BYTES; }
 
 // CTAs a unit for a problem (1 or 2), or 0 when the kernel does not take it:
@@ -92,22 +92,26 @@ int wino_shift_cg(const KernelParam* p) {
   if ((long long)p->n * p->c * p->h * p->w >= (1LL << 31) || (long long)p->n * p->k * p->Oh * p->Ow >= (1LL << 31))
     return 0;
   const bool aligned = (p->h * p->w) % 4 == 0 && (reinterpret_cast<uintptr_t>(p->pin) & 7) == 0;
-  const bool strided = p->u > 1 || p->v > 1;
-  const int items = (!aligned ? sc::MAXITEM_ODD : strided ? sc::MAXITEM_STRIDED : sc::MAXITEM) * sc::NPROD;
   for (const sc::Plan* g : {&g1, &g2})
-    if ((!g->fold && 2 * g->cps * g->qmax > items) || g->nstage < 2 || g->rows > sc::MAXROWS || g->nu > 2 ||
+    if ((!g->fold && sc::stage_items(*g, aligned, false) > sc::MAXITEMS) || g->nstage < 2 || g->rows > sc::MAXROWS || g->nu > 2 ||
         (g->fold && g->nst > 1))
       return 0;
   const long long w1 = (g1.units + sc::NSM - 1) / sc::NSM, w2 = (g2.units + sc::NSM / 2 - 1) / (sc::NSM / 2);
   const int n2 = g2.Kp < 256 ? (g2.Kp + 31) / 32 * 32 : 256;
   // a pair needs work for every pair of SMs
   if (g2.units < sc::NSM / 2) return 1;
+  // narrow outputs: a pair's halved weights gain nothing there and the tiles of
+  // one CTA balance better (3x3 N32 C64 56x56 K64 20.2 us alone, 22.6 in
+  // pairs; 1x1 N32 C512 28x28 K128 16.3 / 20.6)
+  if (g1.Kp <= (g1.taps == 1 ? 128 : 64)) return 1;
   const long long t1 = w1 * sc::mma_cycles(1, g1.Kp < g1.NB ? g1.Kp : g1.NB), t2 = w2 * sc::mma_cycles(2, n2);
   return t2 <= t1 ? 2 : 1;
 }
 
 // The packed plan the kernels read from the argument's transform_pin.
-unsigned long long wino_shift_pack(const KernelParam* p, int cg) { return sc::pack_plan(sc::make_plan(*p, cg)); }
+unsigned long long wino_shift_pack(const KernelParam* p, int cg, int hosted) {
+  return sc::pack_plan(sc::make_plan(*p, cg, hosted != 0));
+}
 
 unsigned wino_shift_grid(const KernelParam* p, int cg, int sms) {
   const sc::Plan g = sc::make_plan(*p, cg);
@@ -127,9 +131,6 @@ int wino_shift_prepare() {
                         (const void*)shift_conv_epi_kernel, (const void*)shift_conv_epi_pair_kernel,
                         (const void*)shift_conv_batch_kernel}) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sc::SMEM_BYTES) != cudaSuccess) return 1;
-    // the warpgroups split exactly the registers the block launches with
-    cudaFuncAttributes fa{};
-    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess || fa.numRegs != sc::REGS_LAUNCH) return 1;
   }
   if (dev >= 0 && dev < 64) done[dev] = 1;
   return 0;
@@ -183,10 +184,7 @@ static constexpr double kFusedMinFlops = 512e6;
 int wino_shift_fused_cg(const KernelParam* p, int cg) {
   if (p->c % 16 || p->k % 16 || 2.0 * p->n * p->k * p->h * p->w * p->c * 9 < kFusedMinFlops) return 0;
   const int best = wino_shift_cg(p);       // (0 when either plan does not fit)
-  if (best == 0 || cg == 0) return best;
-  const sc::Plan g = sc::make_plan(*p, 2, true);
-  const bool aligned = (p->h * p->w) % 4 == 0 && (reinterpret_cast<uintptr_t>(p->pin) & 7) == 0;
-  return 2 * g.cps * g.qmax <= (aligned ? 2 : 1) * sc::NPROD ? 2 : 0;
+  return best == 0 || cg == 0 ? best : cg;
 }
 
 int wino_launch_shift_weight_u(const KernelParam* p, int cg, cudaStream_t stream) {
@@ -204,7 +202,7 @@ int wino_launch_shift_fused(const KernelParam* p0, const void* u, void* wop, int
   KernelParam p = *p0;
   p.pweight = const_cast<void*>(u);
   p.transform_filter = wop;
-  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg));
+  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg, 0));
   const int rc = wino_launch_shift_weight_u(&p, cg, stream);
   if (rc != 0) return rc;
   if (!va || (!va->bias && !va->residual && !va->relu)) return wino_launch_shift(&p, cg, sms, stream);
@@ -221,7 +219,7 @@ void wino_shift_table_finish(ShiftTable* t) {
   t->units = t->pitch = 0;
   for (int l = 0; l < t->nlayers; ++l) {
     ShiftLayer& d = t->layer[l];
-    const sc::Plan g = sc::make_plan(d.p, 2, true);
+    const sc::Plan g = sc::make_plan(d.p, 2);
     d.p.transform_pin = reinterpret_cast<void*>(sc::pack_plan(g));
     d.unit_begin = t->units;
     d.units = g.units;
@@ -271,7 +269,7 @@ int wino_conv2d_shift(const void* x, const void* weight, void* wprep, void* y, i
   if (wino_shift_cg(&p) == 0) return 2;
   if (cg == 0) cg = wino_shift_cg(&p);
   if (wino_shift_prepare() != 0) return 3;
-  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg));
+  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg, 0));
   void* args[] = {&p};
   if (weight && cudaLaunchKernel(wino_shift_weight_kernel_ptr(cg), dim3(wino_shift_weight_grid(&p, cg)), dim3(256),
                                  args, 0, (cudaStream_t)stream) != cudaSuccess)

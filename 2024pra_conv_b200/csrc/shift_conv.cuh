@@ -75,24 +75,41 @@ constexpr int MAXSTAGE = 8;
 constexpr int SMEM_STAGES = 225 * 1024;   // dynamic shared memory of the stages
 constexpr int SMEM_BYTES = SMEM_STAGES + 128;
 constexpr int NSM = 148;                  // SMs of a B200 (the rules below count units against them)
-// Four warpgroups: warps 0-3 epilogue, 4 MMA issue, 5 weight copies, 6-7
-// padding rows, 8-15 input producers in two groups of four that take alternate
-// stages (a warp's own latency, not the issue slots, sets its pace, so two
-// groups bring twice the stages).  Launched with 128 registers a thread (the
-// whole register file); the MMA and epilogue warpgroups hand registers to the
-// producers, which hold the loads of the stages ahead.
-constexpr int NWARP_E = 4, WARP_MMA = 4, WARP_LOAD = 5, WARP_Z0 = 6, NWARP_Z = 2, WARP_P0 = 8, NWARP_P = 4, NGROUP = 2;
-constexpr int NTHREAD = (WARP_P0 + NGROUP * NWARP_P) * 32;
-constexpr int NPROD = NWARP_P * 32;       // producers of one stage
-constexpr int REGS_LAUNCH = 128, REGS_EPI = 112, REGS_MMA = 64, REGS_PROD = 168;
-static_assert(NGROUP == 2, "stages alternate between two groups");
-static_assert(128 * REGS_EPI + 128 * REGS_MMA + NGROUP * NPROD * REGS_PROD == NTHREAD * REGS_LAUNCH,
+constexpr int NWARP_Z = 2;
+// Warp roles: EW epilogue warps, then MMA issue, weight copies and two warps
+// for padding rows, then input producers in two groups of PW warps that take
+// alternate stages (or, strided, alternate channel halves of every stage).
+// Epilogue and producers are a few hundred instructions a turn which one warp
+// issues every ten cycles or so, so their number sets the pace: Wide runs 28
+// warps of 72 registers.  Hosted shares a kernel of 512 threads and 128
+// registers (twostage_conv.cu) and moves registers to its eight producer
+// warps, which own more and keep DEPTH stages of loads in flight.
+// Conv alone back to back, 16 warps -> 28: 1x1 N128 C64 56x56 K256 94 -> 66 us,
+// N32 C512 28x28 K128 23 -> 16, 3x3 N32 C64 56x56 K64 21.5 -> 20.2.
+struct Wide {
+  static constexpr int EW = 8, PW = 8, DEPTH = 1;
+  static constexpr bool SPLIT_REGS = false;
+};
+struct Hosted {
+  static constexpr int EW = 4, PW = 4, DEPTH = 2;
+  static constexpr bool SPLIT_REGS = true;
+  static constexpr int REGS_LAUNCH = 128, REGS_EPI = 112, REGS_MMA = 64, REGS_PROD = 168;
+};
+template <class F>
+struct Roles : F {
+  static constexpr int MMA = F::EW, LOAD = F::EW + 1, Z0 = F::EW + 2, P0 = F::EW + 4;
+  static constexpr int NPROD = F::PW * 32;   // producers of a group
+  static constexpr int NTHREAD = (P0 + 2 * F::PW) * 32;
+};
+constexpr int NTHREAD = Roles<Wide>::NTHREAD, NTHREAD_HOSTED = Roles<Hosted>::NTHREAD;
+static_assert(128 * Hosted::REGS_EPI + 128 * Hosted::REGS_MMA + 256 * Hosted::REGS_PROD ==
+                  NTHREAD_HOSTED * Hosted::REGS_LAUNCH,
               "the warpgroups' register limits add up to the launch allocation");
 constexpr uint32_t SLEEP_NS = 32;
 constexpr int BYUNIT = 2;                 // stages a unit up to which producer groups alternate by unit
-// Items (a quad of pixels, eight channels) a producer thread may own per
-// stage, and operand rows whose padding it looks after.
-constexpr int MAXITEM = 4, MAXITEM_STRIDED = 6, MAXITEM_ODD = 2, MAXROWS = 1024;
+// Producer items (a quad of pixels and eight channels, four where the input is
+// not aligned) a group may own per stage, and operand rows.
+constexpr int MAXITEMS = 512, MAXROWS = 1024;
 
 struct Shared {
   uint64_t full[MAXSTAGE], empty[MAXSTAGE];
@@ -213,10 +230,15 @@ __host__ __device__ __forceinline__ void plan_finish(Plan& g, int cg) {
   g.pitch = g.stageA + g.stageB;
 }
 
-// Plan of a problem for CG CTAs a unit (host; the rules).  `table`: for the
-// kernel over a table of layers, whose producers own one unaligned quad a
-// thread (two spilled there: 100 us against 37 for N32 C512 7x7 K512).
-__host__ inline Plan make_plan(const KernelParam& p, int cg, bool table = false) {
+// Items of a producer group and stage.
+__host__ __device__ __forceinline__ int stage_items(const Plan& g, bool aligned, bool hosted) {
+  const int eights = g.cps * g.qmax * (g.U > 1 || g.V > 1 ? 1 : 2);
+  return aligned || hosted ? eights : 2 * eights;
+}
+
+// Plan of a problem for CG CTAs a unit (host; the rules); `hosted`: for the
+// Hosted roles.
+__host__ inline Plan make_plan(const KernelParam& p, int cg, bool hosted = false) {
   Plan g;
   plan_dims(g, p);
   g.GX = grid_extent(g.OW, g.S, g.V, g.Q, g.W);
@@ -245,7 +267,10 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg, bool table = false)
   const long long px = g.U == 1 && g.V == 1 ? longest : lines * g.U * g.W;
   // (images end in a partial quad when H * W is not a multiple of 4)
   const long long imgs = lines / g.GY + 2;
-  const long long q = px / 4 + 2 + ((g.H * g.W) % 4 ? imgs : 0);
+  // (a grid without padding, 1x1: tiles are whole quads)
+  const bool odd = (g.H * g.W) % 4 != 0;
+  const long long q = g.taps == 1 && g.GX == g.W && g.GY == g.H && !odd && g.U == 1 && g.V == 1
+                          ? px / 4 : px / 4 + 2 + (odd ? imgs : 0);
   g.qmax = (int)(q < 4096 ? q : 4096);
   // Several 16-channel blocks a stage where a block has few taps, and two of a
   // 3x3 filter's where four stages still fit (at most 64 output channels a
@@ -256,10 +281,11 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg, bool table = false)
   for (;; cps >>= 1) {
     g.lcps = cps == 4 ? 2 : cps == 2 ? 1 : 0;
     plan_finish(g, cg);
-    const bool odd = ((g.H * g.W) & 3) != 0;
-    const int items = table && odd ? NPROD : g.taps >= 6 ? 2 * NPROD : 3 * NPROD, stages = g.taps >= 6 ? 4 : 3;
-    // (a folded problem's unit is one stage)
-    if (cps == 1 || g.fold || (2 * cps * g.qmax <= items && stages * (g.stageA + g.stageB) <= SMEM_STAGES)) break;
+    // (a folded problem's unit is one stage; else an item a Wide producer, two
+    // of the smaller unaligned ones: N32 C512 7x7 K512 28.0 -> 25.1 us)
+    if (cps == 1 || g.fold || (stage_items(g, !odd, hosted) <= (odd && !hosted ? 512 : 256) &&
+                               (g.taps >= 6 ? 4 : 3) * (g.stageA + g.stageB) <= SMEM_STAGES))
+      break;
   }
   const int fit = SMEM_STAGES / (g.stageA + g.stageB);
   g.nstage = fit < MAXSTAGE ? fit : MAXSTAGE;
@@ -302,6 +328,7 @@ struct OneConv {
   static constexpr int kind = KIND;
   const KernelParam& p;
   __device__ __forceinline__ int layers() const { return 1; }
+  __device__ __forceinline__ bool strided() const { return KIND == PLAIN && (p.u > 1 || p.v > 1); }
   __device__ __forceinline__ bool get(int, int cg, int u, int step, Conv& c) const {
     c.g = unpack_plan<KIND>(p, cg);
     c.x = static_cast<const unsigned short*>(p.pin);
@@ -319,6 +346,7 @@ struct ConvTable {
   static constexpr int kind = CONV33;
   const ShiftTable& t;                    // the kernel's argument (constant bank)
   __device__ __forceinline__ int layers() const { return t.nlayers; }
+  __device__ __forceinline__ bool strided() const { return false; }
   __device__ __forceinline__ bool get(int l, int cg, int u, int step, Conv& c) const {
     const ShiftLayer& d = t.layer[l];
     // first unit of the layer that is u modulo step
@@ -431,9 +459,9 @@ __device__ __forceinline__ bool wait_all_lanes(uint64_t* bar, uint32_t parity, v
 }
 
 // One stage's loads of a producer thread, and where they go.
-template <int NI, int NW>
+template <int NI, int NW, int CH>
 struct Slot {
-  uint2 w[NI][8][NW];
+  uint2 w[NI][CH][NW];
   uint2 row[NI];                          // 16-byte rows of the stage its pixels go to, 16 bits each, store order
   uint32_t shifts;                        // unaligned quads: first pixel's place in its 8-byte word, 4 bits an item
 };
@@ -447,12 +475,17 @@ struct Slot {
 // The two groups take alternate stages, or with few stages a unit alternate
 // units (each then works out every other unit's addresses only): a group's
 // stages are `run` in a row, then `run` skipped.
-template <int CG, int NI, int DEPTH, bool ALIGNED, bool STRIDED>
+// Strided, a stage's pixels are many and each group takes one channel half of
+// every stage.
+template <int CG, class F, int NI, bool ALIGNED, bool STRIDED>
 __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int done,
                                         int ustep, int tile_pos, int tile_stride, bool& set, uint32_t* err) {
   const Plan& g = cv.g;
   const int u0 = cv.u0, cnt = cv.cnt;
   constexpr int NW = ALIGNED ? 1 : 2;     // 8-byte words per channel
+  constexpr int DEPTH = F::DEPTH, NPROD = Roles<F>::NPROD;
+  // channels of an item: two words a channel are many registers for Wide
+  constexpr int CH = ALIGNED || F::SPLIT_REGS ? 8 : 4;
   volatile int* abort_flag = &sh.abort_flag;
   const unsigned short* X = cv.x;
   const int HW = g.H * g.W, ngrp = 2 * g.cps;
@@ -470,9 +503,9 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   int iq[NI], ich[NI];                    // quad (-1: none) and first channel of the stage
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
-    const int idx = tid + i * NPROD, grp = idx / g.qmax;
-    iq[i] = grp < ngrp ? idx - grp * g.qmax : -1;
-    ich[i] = grp * 8;
+    const int idx = tid + i * NPROD, grp = idx / g.qmax;   // channel group of the stage (strided: of its half)
+    iq[i] = grp < (STRIDED ? g.cps : ngrp) * (8 / CH) ? idx - grp * g.qmax : -1;
+    ich[i] = STRIDED ? (grp * CH >> 3) * 16 + group * 8 + (grp * CH & 7) : grp * CH;
   }
   // planes by (row parity, column parity): first operand row, rows (0: none)
   constexpr int NPL = STRIDED ? 4 : 1;
@@ -494,7 +527,8 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   // load and store cursors: stage of the layer (unit lu, stage lj), ring slot
   const bool by_unit = g.nst <= BYUNIT;
   const int stages = cnt * g.nst;
-  const int run = by_unit ? g.nst : 1, first = by_unit ? group * g.nst : (group + done) & 1;
+  const int run = STRIDED ? stages : by_unit ? g.nst : 1;
+  const int first = STRIDED ? 0 : by_unit ? group * g.nst : (group + done) & 1;
   int lu = 0, lj = first;
   while (lj >= g.nst) { lj -= g.nst; ++lu; }
   int s_left = run, l_left = run;         // stages left of the run
@@ -504,7 +538,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   int entered = -1;
   const bool whole = (g.C & 15) == 0;     // no channel of a block is missing
   const char* XB = reinterpret_cast<const char*>(X);
-  Slot<NI, NW> ring[DEPTH];
+  Slot<NI, NW, CH> ring[DEPTH];
   auto enter = [&]() {
     int pt, k0;
     unit_of(g, u0 + lu * ustep, pt, k0);
@@ -584,7 +618,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
       }
     }
   };
-  auto issue = [&](Slot<NI, NW>& s) {
+  auto issue = [&](Slot<NI, NW, CH>& s) {
     const int c0 = lj << (g.lcps + 4);
     const uint32_t plane = (uint32_t)HW * 2u;
     uint32_t shifts = 0;
@@ -596,7 +630,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
         uint32_t o = off[i] + (c < g.C ? (uint32_t)c * plane : 0u);
         s.row[i] = row_l[i];
 #pragma unroll
-        for (int e = 0; e < 8; ++e, o += plane) s.w[i][e][0] = __ldg(reinterpret_cast<const uint2*>(XB + o));
+        for (int e = 0; e < CH; ++e, o += plane) s.w[i][e][0] = __ldg(reinterpret_cast<const uint2*>(XB + o));
       }
     } else {
 #pragma unroll
@@ -606,7 +640,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
         s.row[i] = row_l[i];
         if (!ALIGNED) shifts |= ((uint32_t)(reinterpret_cast<uintptr_t>(XB + o) >> 1) & 3u) << (4 * i);
 #pragma unroll
-        for (int e = 0; e < 8; ++e, o += plane) {
+        for (int e = 0; e < CH; ++e, o += plane) {
           const bool on = e < nc;
           if (ALIGNED) {
             s.w[i][e][0] = on ? __ldg(reinterpret_cast<const uint2*>(XB + o)) : make_uint2(0, 0);
@@ -622,14 +656,14 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
     }
     s.shifts = shifts;
   };
-  auto consume = [&](const Slot<NI, NW>& s) -> bool {
+  auto consume = [&](const Slot<NI, NW, CH>& s) -> bool {
     if (!wait_all_lanes(&sh.empty[pos.st], pos.phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
     uint8_t* dst = smem + pos.st * g.pitch;
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      uint32_t lo[8], hi[8];              // pixels 0, 1 and 2, 3 of eight channels
+      uint32_t lo[CH], hi[CH];            // pixels 0, 1 and 2, 3 of the channels
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
+      for (int e = 0; e < CH; ++e) {
         uint32_t a = s.w[i][e][0].x, b = s.w[i][e][0].y;
         if (!ALIGNED) {
           const uint32_t sh16 = ((s.shifts >> (4 * i)) + (uint32_t)(e * HW)) & 3u;
@@ -646,9 +680,12 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
         const uint32_t rw2 = k < 2 ? s.row[i].x : s.row[i].y, r = k & 1 ? rw2 >> 16 : rw2 & 0xffffu;
         const uint32_t sel = k & 1 ? sel1 : sel0;
         const uint32_t* v = k < 2 ? lo : hi;
-        *reinterpret_cast<uint4*>(dst + r * 16) =
-            make_uint4(__byte_perm(v[0], v[1], sel), __byte_perm(v[2], v[3], sel), __byte_perm(v[4], v[5], sel),
-                       __byte_perm(v[6], v[7], sel));
+        const uint32_t a = __byte_perm(v[0], v[1], sel), b = __byte_perm(v[2], v[3], sel);
+        if (CH == 8)
+          *reinterpret_cast<uint4*>(dst + r * 16) =
+              make_uint4(a, b, __byte_perm(v[CH - 4], v[CH - 3], sel), __byte_perm(v[CH - 2], v[CH - 1], sel));
+        else
+          *reinterpret_cast<uint2*>(dst + r * 16 + (ich[i] & 4) * 2) = make_uint2(a, b);
       }
     }
     fence_proxy_async_shared();
@@ -663,7 +700,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   // new ones into it.  One loop body with a case per slot: unrolled over the
   // slots, the unit entry above was compiled in seven times and its first
   // pass through the instruction cache held the first stage up by 10 us.
-  const int total = by_unit ? (cnt - group + 1) / 2 * g.nst : (stages - first + 1) / 2;
+  const int total = STRIDED ? stages : by_unit ? (cnt - group + 1) / 2 * g.nst : (stages - first + 1) / 2;
   // the first loads go out before the block's setup is complete
   int slot = 0;
   bool ok = true;
@@ -677,7 +714,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
       enter();
       entered = lu;
     }
-    auto turn = [&](Slot<NI, NW>& s) {
+    auto turn = [&](Slot<NI, NW, CH>& s) {
       if (t >= DEPTH) ok = consume(s);
       if (more && ok) issue(s);
     };
@@ -700,7 +737,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
 // its bytes take 9).  A unit is one stage and the groups
 // take alternate units.  FC, FS: channels and columns known at compile time
 // (0: as the plan says).
-template <int CG, int FC, int FS>
+template <int CG, class F, int FC, int FS>
 __device__ __forceinline__ bool produce_fold(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int ustep,
                                              int tile_pos, int tile_stride, uint32_t* err) {
   const Plan& g = cv.g;
@@ -709,14 +746,14 @@ __device__ __forceinline__ bool produce_fold(const Conv& cv, uint8_t* smem, Shar
   const Grid gr = make_grid(g);
   const int plane0 = plane_rows(g, 0, 0);
   RingPos pos{group % g.nstage, 1u ^ (uint32_t)((group / g.nstage) & 1)};
-  for (int i = group; i < cv.cnt; i += NGROUP, pos.next(g.nstage, NGROUP)) {
+  for (int i = group; i < cv.cnt; i += 2, pos.next(g.nstage, 2)) {
     int pt, k0;
     unit_of(g, cv.u0 + i * ustep, pt, k0);
     const Base b0 = tile_base(gr, pt * tile_stride + tile_pos);
     if (!wait_all_lanes(&sh.empty[pos.st], pos.phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
     uint8_t* dst = smem + pos.st * g.pitch;
-#pragma unroll 2
-    for (int r = tid; r < g.rows; r += NPROD) {
+#pragma unroll 1
+    for (int r = tid; r < g.rows; r += Roles<F>::NPROD) {
       const int a = r >= plane0 ? 1 : 0;
       const Base c = advance(gr, b0, r - (a ? plane0 : 0));
       const int y = c.gy * g.U + a - g.P, x0 = c.gx * g.fV - g.fQ;
@@ -1080,9 +1117,10 @@ __device__ __forceinline__ void shift_weight_from_u(const KernelParam& p, const 
 // The kernel body.  CG = 2: clusters of two CTAs (__cluster_dims__(2, 1, 1)),
 // a unit is 256 positions, rank 0 issues the pair's MMAs.  Every role walks
 // the source's layers and its own units of each.
-template <int CG, bool EPI, class Src>
+template <int CG, class F, bool EPI, class Src>
 __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& epi, uint32_t* err) {
   using namespace sc;
+  using Ro = Roles<F>;
   extern __shared__ __align__(128) uint8_t shift_smem[];
   __shared__ Shared sh;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(shift_smem) + 127) & ~uintptr_t(127));
@@ -1098,18 +1136,18 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAXSTAGE; ++s) {
       // producers, padding, weights (and at a pair's rank 0 the peer's whole stage)
-      mbar_init(&sh.full[s], NWARP_P + NWARP_Z + 1 + (CG == 2 && rank == 0 ? 1 : 0));
+      mbar_init(&sh.full[s], (src.strided() ? 2 : 1) * Ro::PW + NWARP_Z + 1 + (CG == 2 && rank == 0 ? 1 : 0));
       mbar_init(&sh.empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&sh.accfull[a], 1);
-      mbar_init(&sh.accempty[a], CG * NWARP_E);
+      mbar_init(&sh.accempty[a], CG * Ro::EW);
     }
     mbar_init(&sh.mmadone, 1);
     sh.abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == WARP_MMA) {
+  if (warp == Ro::MMA) {
     if (CG == 2) { tmem_alloc_pair(&sh.tmem_base, 512); tmem_relinquish_pair(); }
     else { tmem_alloc(&sh.tmem_base, 512); tmem_relinquish(); }
   }
@@ -1118,10 +1156,10 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
   const int nl = src.layers();
   bool ok = true;
 
-  if (warp >= WARP_MMA && warp < WARP_P0) {
-    regs_dec<REGS_MMA>();
+  if (warp >= Ro::MMA && warp < Ro::P0) {
+    if constexpr (F::SPLIT_REGS) regs_dec<F::REGS_MMA>();
     setup_sync<CG>();
-    if (warp == WARP_LOAD) {
+    if (warp == Ro::LOAD) {
       // the stages' weights, one bulk copy each: this CTA's rows of the unit's
       // output channels
       if (lane == 0) {
@@ -1159,12 +1197,12 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
           for (int b = issued > nstage ? issued - nstage : 0; b < issued; ++b)
             mbar_wait(&sh.full[b % nstage], (b / nstage) & 1, nullptr, err, ERR_WAIT_FULL);
       }
-    } else if (warp >= WARP_Z0) {
+    } else if (warp >= Ro::Z0) {
       RingPos pos{0, 1};
       for (int l = 0; ok && l < nl; ++l) {
         Conv cv;
         if (src.get(l, CG, u0, ustep, cv))
-          ok = pad_rows(cv, smem, sh, threadIdx.x - WARP_Z0 * 32, ustep, tp, TS, pos, err);
+          ok = pad_rows(cv, smem, sh, threadIdx.x - Ro::Z0 * 32, ustep, tp, TS, pos, err);
       }
     } else {
       const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem_base, 0);
@@ -1204,12 +1242,14 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       }
     }
     __syncwarp();
-  } else if (warp < NWARP_E) {
-    regs_dec<REGS_EPI>();
+  } else if (warp < Ro::EW) {
+    if constexpr (F::SPLIT_REGS) regs_dec<F::REGS_EPI>();
     setup_sync<CG>();
     const uint32_t tmem = sh.tmem_base;
-    // epilogue: TMEM lane 32 * quarter + lane = position of this CTA's tile
-    const int quarter = warp;
+    // epilogue: TMEM lane 32 * quarter + lane = position of this CTA's tile;
+    // a quarter's warps take alternate 32-column chunks
+    const int quarter = warp & 3, part = warp >> 2;
+    constexpr int PARTS = Ro::EW / 4;
     const uint32_t lead_accempty = mapa_shared(smem_u32(&sh.accempty[0]), 0);
     int unit = 0;
     for (int l = 0; ok && l < nl; ++l) {
@@ -1244,17 +1284,12 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
           store_cols<32, EPI>(epi, EPI && epi.bias ? epi.bias + k0 + cc : nullptr, reinterpret_cast<char*>(Y),
                               at + (uint32_t)cc * step, step, v, kval - cc, live, pair);
         };
-        float va[32], vb[32];
-        ld(0, va);
-        tmem_ld_wait();
-        for (int cc = 0; cc < nrows; cc += 64) {
-          if (cc + 32 < nrows) ld(cc + 32, vb);
+#pragma unroll 1
+        for (int cc = part * 32; cc < nrows; cc += 32 * PARTS) {
+          float va[32];
+          ld(cc, va);
+          tmem_ld_wait();
           stc(cc, va);
-          tmem_ld_wait();
-          if (cc + 32 >= nrows) break;
-          if (cc + 64 < nrows) ld(cc + 64, va);
-          stc(cc + 32, vb);
-          tmem_ld_wait();
         }
         tc_fence_before();
         __syncwarp();
@@ -1265,8 +1300,8 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       }
     }
   } else {
-    regs_inc<REGS_PROD>();
-    const int group = (warp - WARP_P0) / NWARP_P, tid = threadIdx.x - (WARP_P0 + group * NWARP_P) * 32;
+    if constexpr (F::SPLIT_REGS) regs_inc<F::REGS_PROD>();
+    const int group = (warp - Ro::P0) / Ro::PW, tid = threadIdx.x - (Ro::P0 + group * Ro::PW) * 32;
     int done = 0;                         // stages of the layers before
     bool set = false;                     // setup_sync passed
     for (int l = 0; ok && l < nl; ++l) {
@@ -1276,28 +1311,29 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       if constexpr (Src::kind == FOLDED) {
         setup_sync<CG>();
         set = true;
-        if (g.fC == 3 && g.fS == 7) ok = produce_fold<CG, 3, 7>(cv, smem, sh, tid, group, ustep, tp, TS, err);
-        else ok = produce_fold<CG, 0, 0>(cv, smem, sh, tid, group, ustep, tp, TS, err);
+        if (g.fC == 3 && g.fS == 7) ok = produce_fold<CG, F, 3, 7>(cv, smem, sh, tid, group, ustep, tp, TS, err);
+        else ok = produce_fold<CG, F, 0, 0>(cv, smem, sh, tid, group, ustep, tp, TS, err);
       } else {
-        const int nitem = 2 * g.cps * g.qmax;
         const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(cv.x) & 7) == 0;
-        const bool strided = g.U > 1 || g.V > 1;
-        constexpr bool k33 = Src::kind == CONV33;
-#define SC_PRODUCE(ni, depth, al, strd) \
-  ok = produce<CG, ni, depth, al, strd>(cv, smem, sh, tid, group, done, ustep, tp, TS, set, err)
-        if (aligned && !strided) {
-          if (nitem <= NPROD) SC_PRODUCE(1, 2, true, false);
-          else if (k33 || nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, false);
-          else SC_PRODUCE(4, 1, true, false);
-        } else if (!strided) {
-          if (k33 || nitem <= NPROD) SC_PRODUCE(1, 2, false, false);
-          else SC_PRODUCE(2, 1, false, false);
-        } else if constexpr (!k33) {
-          if (!aligned) SC_PRODUCE(2, 1, false, true);
-          else if (nitem <= 2 * NPROD) SC_PRODUCE(2, 2, true, true);
-          else if (nitem <= 4 * NPROD) SC_PRODUCE(4, 1, true, true);
-          else SC_PRODUCE(6, 1, true, true);
+        const bool one = stage_items(g, aligned, F::SPLIT_REGS) <= Ro::NPROD;
+        constexpr int MORE = MAXITEMS / Ro::NPROD;   // items a producer may own
+#define SC_PRODUCE(ni, al, strd) ok = produce<CG, F, ni, al, strd>(cv, smem, sh, tid, group, done, ustep, tp, TS, set, err)
+        if constexpr (Src::kind == PLAIN) {
+          if (src.strided()) {
+            if (aligned && one) SC_PRODUCE(1, true, true);
+            else if (aligned) SC_PRODUCE(MORE, true, true);
+            else if (one) SC_PRODUCE(1, false, true);
+            else SC_PRODUCE(MORE, false, true);
+            continue;
+          }
         }
+        if (F::SPLIT_REGS && !one && stage_items(g, aligned, true) <= 2 * Ro::NPROD) {
+          if (aligned) SC_PRODUCE(2, true, false);
+          else SC_PRODUCE(2, false, false);
+        } else if (aligned && one) SC_PRODUCE(1, true, false);
+        else if (aligned) SC_PRODUCE(MORE, true, false);
+        else if (F::SPLIT_REGS || one) SC_PRODUCE(1, false, false);
+        else SC_PRODUCE(MORE, false, false);
 #undef SC_PRODUCE
       }
       done += cv.cnt * g.nst;
@@ -1309,7 +1345,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
   // the peer may still read this CTA's shared memory or arrive on its
   // barriers until both CTAs get here
   if (CG == 2) cluster_sync();
-  if (warp == WARP_MMA) {
+  if (warp == Ro::MMA) {
     tc_fence_after();
     if (CG == 2) tmem_dealloc_pair(sh.tmem_base, 512);
     else tmem_dealloc(sh.tmem_base, 512);

@@ -1183,10 +1183,10 @@ __device__ __forceinline__ Prod prod(const Geo& g, const uint8_t* xr, int t, int
 template <bool TMAV, int F8 = 0>
 __global__ void __launch_bounds__(TMAV && F8 ? trs::NTHREAD_V : trs::NTHREAD, 1) twostage_res_kernel_t(KernelParam p) {
   static_assert(F8 == 0 || TMAV, "the fp8 variants read V2 by bulk copy");
-  static_assert(trs::NTHREAD == sc::NTHREAD && sc::SMEM_BYTES <= 227 * 1024, "one kernel hosts both schedules");
+  static_assert(trs::NTHREAD == sc::NTHREAD_HOSTED && sc::SMEM_BYTES <= 227 * 1024, "one kernel hosts both schedules");
   if constexpr (TMAV && F8 == 0) {
     if (p.mid_result == nullptr) {
-      shift_conv_body<1, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_twostage_err);
+      shift_conv_body<1, sc::Hosted, false>(sc::OneConv<sc::CONV33>{p}, sc::Epi{}, &g_twostage_err);
       return;
     }
   }
@@ -2144,7 +2144,7 @@ int wino_twostage_prepare() {
   cudaFuncAttributes fa{};
   if (cudaFuncGetAttributes(&fa, twostage_res_kernel_t<false>) != cudaSuccess || fa.numRegs != trs::REGS_LAUNCH)
     return 1;
-  if (cudaFuncGetAttributes(&fa, twostage_res_kernel_t<true>) != cudaSuccess || fa.numRegs != sc::REGS_LAUNCH)
+  if (cudaFuncGetAttributes(&fa, twostage_res_kernel_t<true>) != cudaSuccess || fa.numRegs != sc::Hosted::REGS_LAUNCH)
     return 1;
   return (int)cudaFuncSetAttribute(twostage_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    tp::SMEM_BYTES);

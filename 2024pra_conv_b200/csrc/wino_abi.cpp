@@ -112,13 +112,13 @@ int wino_igemm_shape_ok(int n, int c, int h, int w, int k, int oh, int ow);
 int wino_igemm_prepare();
 uint32_t wino_igemm_error_read_clear();
 int wino_shift_cg(const wino::KernelParam* p);
-unsigned long long wino_shift_pack(const wino::KernelParam* p, int cg);
+unsigned long long wino_shift_pack(const wino::KernelParam* p, int cg, int hosted);
 unsigned wino_shift_grid(const wino::KernelParam* p, int cg, int sms);
 size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
 unsigned wino_shift_weight_grid(const wino::KernelParam* p, int cg);
 void* wino_shift_weight_kernel_ptr(int cg);
 void* wino_shift_kernel_ptr(const wino::KernelParam* p, int cg);
-int wino_shift_threads();
+int wino_shift_threads(int hosted);
 int wino_shift_smem_bytes();
 int wino_shift_prepare();
 uint32_t wino_shift_error_read_clear();
@@ -352,21 +352,20 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
 
   if (shift.cg != 0) {
     if (wino_shift_prepare() != 0 || wino_twostage_prepare() != 0) return WINO_ECUDA;
+    // Problems of the two-stage route keep its slot 3 and 4 kernels, by which
+    // callers tell the route: given no mid_result, its GEMM kernel runs the
+    // one-CTA shift schedule and its output transform has nothing to do.
+    const bool hosted = shift.cg == 1 && pr.c <= 256 && wino_contract(pr) && two_stage_fits(pr);
     a->transform_filter = static_cast<_Float16*>(shift.wop);
     a->mid_result = nullptr;
     wino::KernelParam* kp = static_cast<wino::KernelParam*>(param);
     // the packed plan travels in transform_pin, which the kernels need no
     // pointer in
-    kp->transform_pin = nullptr;
-    kp->transform_pin = reinterpret_cast<void*>(wino_shift_pack(kp, shift.cg));
+    kp->transform_pin = reinterpret_cast<void*>(wino_shift_pack(kp, shift.cg, hosted));
     set_slot(kernelInfo, 1, wino_shift_weight_grid(kp, shift.cg), 1, 1, 256, 1, 1, 0,
              wino_shift_weight_kernel_ptr(shift.cg));
     set_slot(kernelInfo, 2, 1, 1, 1, 32, 1, 1, 0, wino_noop_kernel_ptr());
-    // Problems of the two-stage route keep its slot 3 and 4 kernels, by which
-    // callers tell the route: given no mid_result, its GEMM kernel runs the
-    // one-CTA shift schedule and its output transform has nothing to do.
-    const bool hosted = shift.cg == 1 && pr.c <= 256 && wino_contract(pr) && two_stage_fits(pr);
-    set_slot(kernelInfo, 3, wino_shift_grid(kp, shift.cg, sm_count()), 1, 1, (unsigned)wino_shift_threads(), 1, 1,
+    set_slot(kernelInfo, 3, wino_shift_grid(kp, shift.cg, sm_count()), 1, 1, (unsigned)wino_shift_threads(hosted), 1, 1,
              (unsigned)wino_shift_smem_bytes(),
              hosted ? wino_twostage_gemm_kernel_ptr_for((int)pr.c) : wino_shift_kernel_ptr(kp, shift.cg));
     if (hosted)

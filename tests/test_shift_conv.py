@@ -34,6 +34,10 @@ SHAPES = [
     (3, 32, 7, 7, 48, 1, 3, 1, 0, 1),        # 1x3
     (2, 48, 10, 12, 24, 5, 5, 1, 2, 2),      # 25 taps
     (2, 32, 9, 11, 48, 2, 2, 1, 0, 0),       # two 16-channel blocks a stage
+    (3, 96, 10, 14, 40, 1, 1, 1, 0, 0),      # 1x1: the grid has no padding
+    (3, 72, 7, 9, 40, 1, 1, 1, 0, 0),
+    (2, 64, 15, 15, 64, 3, 3, 2, 1, 1),      # stride 2, unaligned quads
+    (1, 32, 14, 126, 32, 3, 3, 2, 1, 1),     # stride 2, long rows
 ]
 
 
