@@ -543,7 +543,9 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
     int pt, k0;
     unit_of(g, u0 + lu * ustep, pt, k0);
     const Base b0 = tile_base(gr, pt * tile_stride + tile_pos);
-    const uint32_t img = (uint32_t)(b0.n * g.C) * (uint32_t)HW * 2u;
+    // (a pair's second tile may start past the last image: its loads, of which
+    // no row is stored, stay inside)
+    const uint32_t img = (uint32_t)(min(b0.n, g.N - 1) * g.C) * (uint32_t)HW * 2u;
     // the range starts with the first position's pixel (stride 1) or the
     // first pixel row of its grid row
     const int y0 = (b0.gy << ushift) - g.P;
