@@ -458,6 +458,10 @@ __device__ __forceinline__ bool wait_all_lanes(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait_impl<kCluster>(bar, parity, abort, err, code)) != 0;
 }
 
+// Whether producer groups alternate by unit (a run of nst stages; two rounds of
+// the ring are apart as long as that is not all of it).
+__device__ __forceinline__ bool runs_by_unit(const Plan& g) { return g.nst <= BYUNIT && g.nst < g.nstage; }
+
 // One stage's loads of a producer thread, and where they go.
 template <int NI, int NW, int CH>
 struct Slot {
@@ -474,11 +478,14 @@ struct Slot {
 // otherwise the two words around it and a shift.
 // The two groups take alternate stages, or with few stages a unit alternate
 // units (each then works out every other unit's addresses only): a group's
-// stages are `run` in a row, then `run` skipped.
+// stages are `run` in a row, then `run` skipped, from layer to layer too
+// (`turn`: the group whose turn the layer's first run is; done: stages of the
+// layers before).  A group must not skip a whole round of the ring: the empty
+// barrier's parity it then waits for could be two rounds old.
 // Strided, a stage's pixels are many and each group takes one channel half of
 // every stage.
 template <int CG, class F, int NI, bool ALIGNED, bool STRIDED>
-__device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int done,
+__device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int done, int turn,
                                         int ustep, int tile_pos, int tile_stride, bool& set, uint32_t* err) {
   const Plan& g = cv.g;
   const int u0 = cv.u0, cnt = cv.cnt;
@@ -525,10 +532,10 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   int npx[NI];                            // its pixels inside the image (0: no pixel of the tile's)
   uint2 row_l[NI];
   // load and store cursors: stage of the layer (unit lu, stage lj), ring slot
-  const bool by_unit = g.nst <= BYUNIT;
+  const bool by_unit = runs_by_unit(g);
   const int stages = cnt * g.nst;
   const int run = STRIDED ? stages : by_unit ? g.nst : 1;
-  const int first = STRIDED ? 0 : by_unit ? group * g.nst : (group + done) & 1;
+  const int first = STRIDED ? 0 : (group ^ turn) * run;
   int lu = 0, lj = first;
   while (lj >= g.nst) { lj -= g.nst; ++lu; }
   int s_left = run, l_left = run;         // stages left of the run
@@ -702,7 +709,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   // new ones into it.  One loop body with a case per slot: unrolled over the
   // slots, the unit entry above was compiled in seven times and its first
   // pass through the instruction cache held the first stage up by 10 us.
-  const int total = STRIDED ? stages : by_unit ? (cnt - group + 1) / 2 * g.nst : (stages - first + 1) / 2;
+  const int total = STRIDED ? stages : ((by_unit ? cnt : stages) - (group ^ turn) + 1) / 2 * run;
   // the first loads go out before the block's setup is complete
   int slot = 0;
   bool ok = true;
@@ -1304,7 +1311,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
   } else {
     if constexpr (F::SPLIT_REGS) regs_inc<F::REGS_PROD>();
     const int group = (warp - Ro::P0) / Ro::PW, tid = threadIdx.x - (Ro::P0 + group * Ro::PW) * 32;
-    int done = 0;                         // stages of the layers before
+    int done = 0, turn = 0;               // stages of the layers before, whose turn the next run is
     bool set = false;                     // setup_sync passed
     for (int l = 0; ok && l < nl; ++l) {
       Conv cv;
@@ -1319,7 +1326,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(cv.x) & 7) == 0;
         const bool one = stage_items(g, aligned, F::SPLIT_REGS) <= Ro::NPROD;
         constexpr int MORE = MAXITEMS / Ro::NPROD;   // items a producer may own
-#define SC_PRODUCE(ni, al, strd) ok = produce<CG, F, ni, al, strd>(cv, smem, sh, tid, group, done, ustep, tp, TS, set, err)
+#define SC_PRODUCE(ni, al, strd) ok = produce<CG, F, ni, al, strd>(cv, smem, sh, tid, group, done, turn, ustep, tp, TS, set, err)
         if constexpr (Src::kind == PLAIN) {
           if (src.strided()) {
             if (aligned && one) SC_PRODUCE(1, true, true);
@@ -1339,6 +1346,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
 #undef SC_PRODUCE
       }
       done += cv.cnt * g.nst;
+      turn ^= (runs_by_unit(g) ? cv.cnt : cv.cnt * g.nst) & 1;
     }
     if (!set) setup_sync<CG>();           // no stage for this group
   }

@@ -33,6 +33,7 @@ SHAPES = [
     (2, 64, 112, 112, 64, 3, 3, 2, 1, 1),
     (3, 32, 7, 7, 48, 1, 3, 1, 0, 1),        # 1x3
     (2, 48, 10, 12, 24, 5, 5, 1, 2, 2),      # 25 taps
+    (12, 32, 72, 72, 256, 5, 5, 1, 2, 2),    # a ring of two stages, two a unit
     (2, 32, 9, 11, 48, 2, 2, 1, 0, 0),       # two 16-channel blocks a stage
     (3, 96, 10, 14, 40, 1, 1, 1, 0, 0),      # 1x1: the grid has no padding
     (3, 72, 7, 9, 40, 1, 1, 1, 0, 0),
@@ -289,6 +290,8 @@ def _fused_case(cuda, shape, seed):
 # At least 512 MFLOP: one CTA a unit, pairs, odd rows (2-byte stores), a K
 # block of 16 beside a full one.
 FUSED = [(8, 128, 28, 28, 128), (48, 128, 28, 28, 256), (16, 128, 15, 15, 144), (40, 64, 30, 22, 272)]
+# short units one producer group takes, between layers of many stages
+RING = [(8, c, h, h, c) for c, h in ((64, 56), (128, 28), (256, 14), (512, 7)) for _ in range(2)]
 # The filter from the fp16 U is off by 2.2e-4 in the 2-norm, y's rounding by at
 # most 2.8e-4, twice with a residual.
 FUSED_REL = 5e-4
@@ -322,12 +325,13 @@ def test_fused_conv_on_a_u_cache(wino, cuda, shape, mode):
 
 
 @pytest.mark.gpu
-def test_batch_mixes_kernels(wino, cuda):
+@pytest.mark.parametrize("shapes", [FUSED + [(2, 32, 14, 14, 32)], RING])
+def test_batch_mixes_kernels(wino, cuda, shapes):
     """Layers of at least 512 MFLOP run in one launch of the shift kernel, the
     others in the fused kernel's; both equal the single-layer calls, from
     capture too and after the U cache was rewritten in place."""
     import torch
-    cases = [_fused_case(cuda, s, 4 + i) for i, s in enumerate(FUSED + [(2, 32, 14, 14, 32)])]
+    cases = [_fused_case(cuda, s, 4 + i) for i, s in enumerate(shapes)]
     b, outs = wino.Batch(), []
     for x, wt, _, res in cases:
         u = wino.filter_transform(wt)
