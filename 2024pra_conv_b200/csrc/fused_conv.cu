@@ -769,6 +769,9 @@ template __global__ void fused_wino_var_kernel<VAR_F16_HILO>(KernelParam, Varian
 __global__ void __launch_bounds__(NTHREAD, 1) fused_wino_batch_kernel(const BatchTable* t, long long total) {
   const LayerTable lt{t, total};
   fused_body<VAR_F16>(lt, VariantArgs{nullptr, nullptr, nullptr});
+  // (launched beside the kernel ahead, whose work it needs nothing of: complete
+  // only when that is)
+  grid_dep_wait();
 }
 
 }  // namespace wino
@@ -836,7 +839,13 @@ int wino_fused_prepare_batch() {
                                    fused::SMEM_BYTES);
 }
 
-int wino_fused_launch_batch(const void* table_dev, long long total_blocks, unsigned grid,
+int wino_launch_dependent(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream);
+
+// `beside`: the launch ahead on the stream is the shift kernel's over other
+// layers, which lets this one start on the SMs it has no use for.  Small
+// batches of both kinds leave most SMs idle (N2, C64 K64 57x57 to C256 15x15: 58 us one
+// after the other, 41 beside).
+int wino_fused_launch_batch(const void* table_dev, long long total_blocks, unsigned grid, bool beside,
                             cudaStream_t stream) {
   static const int prepared = wino_fused_prepare_batch();
   if (prepared != 0) return prepared;
@@ -844,6 +853,9 @@ int wino_fused_launch_batch(const void* table_dev, long long total_blocks, unsig
   const BatchTable* t = static_cast<const BatchTable*>(table_dev);
   long long tot = total_blocks;
   void* args[] = {&t, &tot};
+  if (beside)
+    return wino_launch_dependent((void*)fused_wino_batch_kernel, dim3(grid), dim3(fused::NTHREAD), args,
+                                 (size_t)fused::SMEM_BYTES, stream);
   e = cudaLaunchKernel((void*)fused_wino_batch_kernel, dim3(grid), dim3(fused::NTHREAD), args,
                        (size_t)fused::SMEM_BYTES, stream);
   return (int)e;

@@ -91,7 +91,7 @@ int wino_shift_cg(const KernelParam* p) {
   // byte offsets into input and output in 32 bits
   if ((long long)p->n * p->c * p->h * p->w >= (1LL << 31) || (long long)p->n * p->k * p->Oh * p->Ow >= (1LL << 31))
     return 0;
-  const bool aligned = (p->h * p->w) % 4 == 0 && (reinterpret_cast<uintptr_t>(p->pin) & 7) == 0;
+  const bool aligned = sc::input_aligned(p->h * p->w, p->pin);
   for (const sc::Plan* g : {&g1, &g2})
     if ((!g->fold && sc::stage_items(*g, aligned, false) > sc::MAXITEMS) || g->nstage < 2 || g->rows > sc::MAXROWS || g->nu > 2 ||
         (g->fold && g->nst > 1))
@@ -110,7 +110,7 @@ int wino_shift_cg(const KernelParam* p) {
 
 // The packed plan the kernels read from the argument's transform_pin.
 unsigned long long wino_shift_pack(const KernelParam* p, int cg, int hosted) {
-  return sc::pack_plan(sc::make_plan(*p, cg, hosted != 0));
+  return sc::pack_plan(sc::make_plan(*p, cg, hosted ? sc::TWOSTAGE : sc::OWN));
 }
 
 unsigned wino_shift_grid(const KernelParam* p, int cg, int sms) {
@@ -180,11 +180,16 @@ int wino_launch_shift(const KernelParam* p, int cg, int sms, cudaStream_t stream
 static constexpr double kFusedMinFlops = 512e6;
 
 // CTAs a unit for a problem (dims and tensors set), or 0 when it stays with
-// the fused kernel.  `cg` 2: for a table of layers (pairs).
-int wino_shift_fused_cg(const KernelParam* p, int cg) {
+// the fused kernel.
+int wino_shift_fused_cg(const KernelParam* p) {
   if (p->c % 16 || p->k % 16 || 2.0 * p->n * p->k * p->h * p->w * p->c * 9 < kFusedMinFlops) return 0;
-  const int best = wino_shift_cg(p);       // (0 when either plan does not fit)
-  return best == 0 || cg == 0 ? best : cg;
+  return wino_shift_cg(p);
+}
+// Whether a batch's table can hold a problem that wino_shift_fused_cg takes
+// (pairs): its producers own one item each.
+int wino_shift_in_table(const KernelParam* p) {
+  return sc::stage_items(sc::make_plan(*p, 2, sc::TABLE), sc::input_aligned(p->h * p->w, p->pin), false) <=
+         sc::Roles<sc::Wide>::NPROD;
 }
 
 int wino_launch_shift_weight_u(const KernelParam* p, int cg, cudaStream_t stream) {
@@ -219,7 +224,7 @@ void wino_shift_table_finish(ShiftTable* t) {
   t->units = t->pitch = 0;
   for (int l = 0; l < t->nlayers; ++l) {
     ShiftLayer& d = t->layer[l];
-    const sc::Plan g = sc::make_plan(d.p, 2);
+    const sc::Plan g = sc::make_plan(d.p, 2, sc::TABLE);
     d.p.transform_pin = reinterpret_cast<void*>(sc::pack_plan(g));
     d.unit_begin = t->units;
     d.units = g.units;

@@ -182,6 +182,7 @@ __host__ __device__ __forceinline__ int mma_cycles(int cg, int n) {
 }
 
 // What a kernel knows of its problems at compile time.
+enum Host : int { OWN, TWOSTAGE, TABLE };   // kernels the schedule runs in
 enum Kind : int { ANY, PLAIN, FOLDED, CONV33 };   // CONV33: 3x3 / stride 1 / pad 1
 
 template <int KIND = ANY>
@@ -236,9 +237,8 @@ __host__ __device__ __forceinline__ int stage_items(const Plan& g, bool aligned,
   return aligned || hosted ? eights : 2 * eights;
 }
 
-// Plan of a problem for CG CTAs a unit (host; the rules); `hosted`: for the
-// Hosted roles.
-__host__ inline Plan make_plan(const KernelParam& p, int cg, bool hosted = false) {
+// Plan of a problem for CG CTAs a unit (host; the rules).
+__host__ inline Plan make_plan(const KernelParam& p, int cg, Host host = OWN) {
   Plan g;
   plan_dims(g, p);
   g.GX = grid_extent(g.OW, g.S, g.V, g.Q, g.W);
@@ -283,13 +283,18 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg, bool hosted = false
     plan_finish(g, cg);
     // (a folded problem's unit is one stage; else an item a Wide producer, two
     // of the smaller unaligned ones: N32 C512 7x7 K512 28.0 -> 25.1 us)
-    if (cps == 1 || g.fold || (stage_items(g, !odd, hosted) <= (odd && !hosted ? 512 : 256) &&
+    if (cps == 1 || g.fold || (stage_items(g, !odd, host == TWOSTAGE) <= (odd && host == OWN ? 512 : 256) &&
                                (g.taps >= 6 ? 4 : 3) * (g.stageA + g.stageB) <= SMEM_STAGES))
       break;
   }
   const int fit = SMEM_STAGES / (g.stageA + g.stageB);
   g.nstage = fit < MAXSTAGE ? fit : MAXSTAGE;
   return g;
+}
+
+// Whether every channel's quads of pixels are 8-byte words.
+__host__ __device__ __forceinline__ bool input_aligned(int hw, const void* x) {
+  return (hw & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0;
 }
 
 __host__ inline unsigned long long pack_plan(const Plan& g) {
@@ -326,6 +331,7 @@ struct Conv {
 template <int KIND>
 struct OneConv {
   static constexpr int kind = KIND;
+  static constexpr bool table = false;
   const KernelParam& p;
   __device__ __forceinline__ int layers() const { return 1; }
   __device__ __forceinline__ bool strided() const { return KIND == PLAIN && (p.u > 1 || p.v > 1); }
@@ -344,6 +350,10 @@ struct OneConv {
 // ring of stages runs on across layers, so its pitch is the largest stage's.
 struct ConvTable {
   static constexpr int kind = CONV33;
+  // An item a producer: with two for some layers too, the producers' variants
+  // spilled into an L1 cache that the stages leave little of (N32 C512 7x7
+  // K512 with its operand 69 -> 37 us, the set's eight layers N32 186 -> 130).
+  static constexpr bool table = true;
   const ShiftTable& t;                    // the kernel's argument (constant bank)
   __device__ __forceinline__ int layers() const { return t.nlayers; }
   __device__ __forceinline__ bool strided() const { return false; }
@@ -1177,6 +1187,8 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         // the operand is the kernel before's (programmatic launch); setup and
         // the first input loads overlap with it
         grid_dep_wait();
+        // what a batch launches next works on other layers
+        grid_dep_launch();
         for (int l = 0; ok && l < nl; ++l) {
           Conv cv;
           if (!src.get(l, CG, u0, ustep, cv)) continue;
@@ -1323,7 +1335,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         if (g.fC == 3 && g.fS == 7) ok = produce_fold<CG, F, 3, 7>(cv, smem, sh, tid, group, ustep, tp, TS, err);
         else ok = produce_fold<CG, F, 0, 0>(cv, smem, sh, tid, group, ustep, tp, TS, err);
       } else {
-        const bool aligned = ((g.H * g.W) & 3) == 0 && (reinterpret_cast<uintptr_t>(cv.x) & 7) == 0;
+        const bool aligned = input_aligned(g.H * g.W, cv.x);
         const bool one = stage_items(g, aligned, F::SPLIT_REGS) <= Ro::NPROD;
         constexpr int MORE = MAXITEMS / Ro::NPROD;   // items a producer may own
 #define SC_PRODUCE(ni, al, strd) ok = produce<CG, F, ni, al, strd>(cv, smem, sh, tid, group, done, turn, ustep, tp, TS, set, err)
@@ -1336,7 +1348,10 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
             continue;
           }
         }
-        if (F::SPLIT_REGS && !one && stage_items(g, aligned, true) <= 2 * Ro::NPROD) {
+        if (Src::table) {
+          if (aligned) SC_PRODUCE(1, true, false);
+          else SC_PRODUCE(1, false, false);
+        } else if (F::SPLIT_REGS && !one && stage_items(g, aligned, true) <= 2 * Ro::NPROD) {
           if (aligned) SC_PRODUCE(2, true, false);
           else SC_PRODUCE(2, false, false);
         } else if (aligned && one) SC_PRODUCE(1, true, false);

@@ -122,7 +122,7 @@ int wino_shift_threads(int hosted);
 int wino_shift_smem_bytes();
 int wino_shift_prepare();
 uint32_t wino_shift_error_read_clear();
-int wino_shift_fused_cg(const wino::KernelParam* p, int cg);
+int wino_shift_fused_cg(const wino::KernelParam* p);
 int wino_launch_dependent(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream);
 int wino_launch_shift_fused(const wino::KernelParam* p0, const void* u, void* wop, int cg, const wino::VariantArgs* va,
                             int sms, cudaStream_t stream);
@@ -595,7 +595,7 @@ extern "C" int wino_input_layout(const void* x, void* workspace, int n, int c, i
 extern "C" size_t wino_fused_conv_workspace_bytes(int n, int c, int h, int w, int k) {
   if (wino_check_shape(n, c, h, w, k) != WINO_OK) return 0;
   const wino::KernelParam p = make_param(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, n, c, h, w, k);
-  const int cg = wino_shift_fused_cg(&p, 0);
+  const int cg = wino_shift_fused_cg(&p);
   const size_t xb = wino_xb_bytes(n, c, h, w), wop = cg ? wino_shift_weight_bytes(&p, cg) : 0;
   return xb > wop ? xb : wop;
 }
@@ -606,7 +606,7 @@ extern "C" size_t wino_fused_conv_workspace_bytes(int n, int c, int h, int w, in
 static int fused_shift(const void* x, const void* ucache, void* workspace, size_t workspace_bytes, void* y,
                        const wino::VariantArgs* va, int n, int c, int h, int w, int k, cudaStream_t s) {
   const wino::KernelParam p = make_param(x, nullptr, y, nullptr, nullptr, nullptr, n, c, h, w, k);
-  const int cg = wino_shift_fused_cg(&p, 0);
+  const int cg = wino_shift_fused_cg(&p);
   if (cg == 0 || wino_shift_weight_bytes(&p, cg) > workspace_bytes) return -1;
   return wino_launch_shift_fused(&p, ucache, workspace, cg, va, sm_count(), s) == 0 ? WINO_OK : WINO_ECUDA;
 }

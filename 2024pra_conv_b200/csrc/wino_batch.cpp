@@ -28,7 +28,7 @@
 extern "C" {
 int wino_fused_launch_variant(int variant, const wino::KernelParam* p, const wino::VariantArgs* va,
                               int cfg, unsigned grid, cudaStream_t stream);
-int wino_fused_launch_batch(const void* table_dev, long long total_blocks, unsigned grid,
+int wino_fused_launch_batch(const void* table_dev, long long total_blocks, unsigned grid, bool beside,
                             cudaStream_t stream);
 int wino_launch_xb_layout(const wino::KernelParam* p, cudaStream_t stream);
 int wino_fused_prepare_batch();
@@ -40,7 +40,8 @@ long long wino_fused_nblocks_cfg(int n, int c, int h, int w, int k, int cfg);
 int wino_fused_cfg_splits(int c, int cfg);
 int wino_launch_y32_to_f16(const float* y32, void* y, long long count, cudaStream_t stream);
 int wino_launch_u_to_u2(const void* u, void* u2, int K, int C, cudaStream_t stream);
-int wino_shift_fused_cg(const wino::KernelParam* p, int cg);
+int wino_shift_fused_cg(const wino::KernelParam* p);
+int wino_shift_in_table(const wino::KernelParam* p);
 size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
 double wino_shift_unit_cost(const wino::KernelParam* p);
 void wino_shift_table_finish(wino::ShiftTable* t);
@@ -161,7 +162,8 @@ struct Layer {
   float twostage_us = -1.f; // the two-stage route alone (-1: not timed or not applicable)
   void* u2 = nullptr;       // U in the two-stage GEMM's layout (batch-owned)
   void* ws2 = nullptr;      // two-stage workspace (batch-owned)
-  bool shift = false;       // fused route on the shift-reuse implicit GEMM
+  int shift = 0;            // the fused route's CTAs a unit on the shift-reuse implicit GEMM (0: not on it)
+  bool table = false;       // ... in the launch over a table of layers (pairs)
   size_t wop = 0;           // offset of its weight operand in the batch's buffer
   // U2 and the workspace for the two-stage route, made on first use from the
   // layer's fused U cache (synchronous: not inside a stream capture)
@@ -192,7 +194,7 @@ struct Batch {
   std::vector<Layer> layers;
   std::vector<int> order;        // table order of the layers
   BatchTable* table_dev = nullptr;
-  wino::ShiftTable shift{};      // layers on the shift kernel (a kernel argument)
+  wino::ShiftTable shift{};      // layers of the shift kernel's table (a kernel argument)
   void* operands = nullptr;      // their weight operands
   size_t operand_bytes = 0;
   long long total = 0;
@@ -230,6 +232,15 @@ struct Batch {
     graph = nullptr;
   }
 
+  bool on_shift(const Layer& L) const { return L.route == ROUTE_FUSED && L.shift; }
+  // One layer by itself on the shift kernel.
+  int run_shift(const Layer& L, cudaStream_t s) const {
+    KernelParam p = L.p;
+    p.transform_filter = nullptr;
+    return wino_launch_shift_fused(&p, L.p.transform_filter, static_cast<uint8_t*>(operands) + L.wop, L.shift, nullptr,
+                                   sm_count(), s) == 0 ? (int)WINO_OK : (int)WINO_ECUDA;
+  }
+
   // Room for the shift layers' weight operands, which every run makes from the
   // layers' U caches (not inside a stream capture).
   int ensure_operands() {
@@ -237,7 +248,7 @@ struct Batch {
     for (Layer& L : layers)
       if (L.shift) {
         L.wop = need;
-        need += align256(wino_shift_weight_bytes(&L.p, 2));
+        need += align256(wino_shift_weight_bytes(&L.p, L.shift));
       }
     if (need <= operand_bytes) return WINO_OK;
     if (settle() != WINO_OK) return WINO_ECUDA;  // no launch still reads the old buffer
@@ -260,7 +271,7 @@ struct Batch {
     int nt = 0;
     for (size_t i = 0; i < order.size(); ++i) {
       const Layer& L = layers[order[i]];
-      if (L.route != ROUTE_FUSED || L.shift) continue;     // not in this table
+      if (L.route != ROUTE_FUSED || on_shift(L)) continue;     // not in this table
       LayerDesc& d = t.layer[nt++];
       d.p = L.p;
       int cfg = L.cfg;
@@ -279,7 +290,7 @@ struct Batch {
     // left at the end of the launch is small
     std::vector<int> heavy;
     for (int li : order)
-      if (layers[li].route == ROUTE_FUSED && layers[li].shift) heavy.push_back(li);
+      if (on_shift(layers[li]) && layers[li].table) heavy.push_back(li);
     std::stable_sort(heavy.begin(), heavy.end(), [&](int a, int b) {
       return wino_shift_unit_cost(&layers[a].p) > wino_shift_unit_cost(&layers[b].p);
     });
@@ -310,12 +321,21 @@ struct Batch {
         if (rc != WINO_OK) return rc;
         continue;
       }
-      if (!L.shift && L.p.transform_pin && !(L.cfg & wino::CFG_DIRECT) && wino_launch_xb_layout(&L.p, s) != 0)
+      if (!on_shift(L) && L.p.transform_pin && !(L.cfg & wino::CFG_DIRECT) && wino_launch_xb_layout(&L.p, s) != 0)
         return WINO_ECUDA;
     }
-    if (shift.nlayers > 0 && wino_launch_shift_batch(&shift, sm_count(), s) != 0) return WINO_ECUDA;
+    bool beside = false;
+    for (int li : order)
+      if (on_shift(layers[li]) && !layers[li].table) {
+        if (run_shift(layers[li], s) != WINO_OK) return WINO_ECUDA;
+        beside = true;
+      }
+    if (shift.nlayers > 0) {
+      if (wino_launch_shift_batch(&shift, sm_count(), s) != 0) return WINO_ECUDA;
+      beside = true;
+    }
     if (total == 0) return WINO_OK;           // no layer on the fused Winograd kernel
-    return wino_fused_launch_batch(table_dev, total, grid_for(total), s) == 0 ? WINO_OK : WINO_ECUDA;
+    return wino_fused_launch_batch(table_dev, total, grid_for(total), beside, s) == 0 ? WINO_OK : WINO_ECUDA;
   }
 };
 
@@ -416,7 +436,11 @@ int wino_batch_add_layer(void* h, const void* x, const void* ucache, void* xb_ws
   L.cfg = xb_ws ? 0 : wino::CFG_DIRECT;
   // the kernel wino_conv2d_fused_ws takes with room for its operand (a layer
   // without a workspace stays with the direct fused kernel)
-  L.shift = xb_ws && wino_shift_fused_cg(&L.p, 2) == 2;
+  L.shift = xb_ws ? wino_shift_fused_cg(&L.p) : 0;
+  if (L.shift && wino_shift_in_table(&L.p)) {
+    L.table = true;
+    L.shift = 2;
+  }
   b->order.push_back((int)b->layers.size());
   b->layers.push_back(L);
   b->dirty = true;
@@ -531,11 +555,7 @@ int wino_batch_tune(void* h, int reps, float* layer_us, float* order_us, void* s
       float t = 0.f;
       // (a layer on the shift kernel runs the same under every configuration)
       auto one = [&] {
-        if (!L.shift) return run_layer_cfg(L.p, L.p.transform_pin, cfg, s);
-        KernelParam p = L.p;
-        p.transform_filter = nullptr;
-        return wino_launch_shift_fused(&p, L.p.transform_filter, static_cast<uint8_t*>(b->operands) + L.wop, 2, nullptr,
-                                       sm_count(), s) == 0 ? (int)WINO_OK : (int)WINO_ECUDA;
+        return L.shift ? b->run_shift(L, s) : run_layer_cfg(L.p, L.p.transform_pin, cfg, s);
       };
       const int rc = time_us(one, reps, s, &t);
       if (rc != WINO_OK) return rc;

@@ -33,7 +33,7 @@ SHAPES = [
     (2, 64, 112, 112, 64, 3, 3, 2, 1, 1),
     (3, 32, 7, 7, 48, 1, 3, 1, 0, 1),        # 1x3
     (2, 48, 10, 12, 24, 5, 5, 1, 2, 2),      # 25 taps
-    (12, 32, 72, 72, 256, 5, 5, 1, 2, 2),    # a ring of two stages, two a unit
+    (24, 32, 56, 56, 256, 5, 5, 1, 2, 2),    # a ring of two stages, two a unit
     (2, 32, 9, 11, 48, 2, 2, 1, 0, 0),       # two 16-channel blocks a stage
     (3, 96, 10, 14, 40, 1, 1, 1, 0, 0),      # 1x1: the grid has no padding
     (3, 72, 7, 9, 40, 1, 1, 1, 0, 0),
