@@ -28,29 +28,31 @@ __global__ void __launch_bounds__(128) shift_weight_u_batch_kernel(const __grid_
 
 // One CTA a unit (128 positions, up to 128 output channels).
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_kernel(KernelParam p) {
-  shift_conv_body<1, sc::Wide, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // A pair of CTAs a unit (256 positions, up to 256 output channels).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_pair_kernel(KernelParam p) {
-  shift_conv_body<2, sc::Wide, false>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same for problems whose filter columns became channels.
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_kernel(KernelParam p) {
-  shift_conv_body<1, sc::Wide, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, sc::Wide, sc::NOEPI>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_pair_kernel(KernelParam p) {
-  shift_conv_body<2, sc::Wide, false>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same with the fused epilogue.
+template <int EPI>
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_epi_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<1, sc::Wide, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
+  shift_conv_body<1, sc::Wide, EPI>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
 }
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_epi_pair_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<2, sc::Wide, true>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
+  shift_conv_body<2, sc::Wide, EPI>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
 }
 
 // A table of layers, passed by value: the roles read their layers' dims from
@@ -58,7 +60,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
 // and spilled).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_batch_kernel(const __grid_constant__ ShiftTable t) {
-  shift_conv_body<2, sc::Wide, false>(sc::ConvTable{t}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::ConvTable{t}, sc::Epi{}, &g_shift_err);
 }
 
 }  // namespace wino
@@ -128,7 +130,9 @@ int wino_shift_prepare() {
   if (dev >= 0 && dev < 64 && done[dev]) return 0;
   for (const void* f : {(const void*)shift_conv_kernel, (const void*)shift_conv_pair_kernel,
                         (const void*)shift_conv_fold_kernel, (const void*)shift_conv_fold_pair_kernel,
-                        (const void*)shift_conv_epi_kernel, (const void*)shift_conv_epi_pair_kernel,
+                        (const void*)shift_conv_epi_kernel<sc::EPI_PAIR>, (const void*)shift_conv_epi_kernel<sc::EPI_ODD>,
+                        (const void*)shift_conv_epi_pair_kernel<sc::EPI_PAIR>,
+                        (const void*)shift_conv_epi_pair_kernel<sc::EPI_ODD>,
                         (const void*)shift_conv_batch_kernel}) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sc::SMEM_BYTES) != cudaSuccess) return 1;
   }
@@ -213,8 +217,12 @@ int wino_launch_shift_fused(const KernelParam* p0, const void* u, void* wop, int
   if (!va || (!va->bias && !va->residual && !va->relu)) return wino_launch_shift(&p, cg, sms, stream);
   sc::Epi e{va->bias, static_cast<const __half*>(va->residual), va->relu};
   void* args[] = {&p, &e};
-  return wino_launch_dependent(cg == 2 ? (void*)shift_conv_epi_pair_kernel : (void*)shift_conv_epi_kernel,
-                               dim3(wino_shift_grid(&p, cg, sms)), dim3(sc::NTHREAD), args, (size_t)sc::SMEM_BYTES,
+  const bool even = sc::store_pairs(p.Ow, p.pout, va->residual);
+  const void* fn = cg == 2 ? (even ? (const void*)shift_conv_epi_pair_kernel<sc::EPI_PAIR>
+                                   : (const void*)shift_conv_epi_pair_kernel<sc::EPI_ODD>)
+                           : (even ? (const void*)shift_conv_epi_kernel<sc::EPI_PAIR>
+                                   : (const void*)shift_conv_epi_kernel<sc::EPI_ODD>);
+  return wino_launch_dependent(fn, dim3(wino_shift_grid(&p, cg, sms)), dim3(sc::NTHREAD), args, (size_t)sc::SMEM_BYTES,
                                stream);
 }
 

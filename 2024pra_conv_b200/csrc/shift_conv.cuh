@@ -962,6 +962,11 @@ __device__ __forceinline__ bool issue_mmas(const Conv& cv, Shared& sh, uint32_t 
   return ok;
 }
 
+// Whether outputs (and residuals) are stored in pairs.
+__host__ __device__ __forceinline__ bool store_pairs(int ow, const void* y, const void* residual) {
+  return (ow & 1) == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) & 3) == 0;
+}
+
 // Epilogue operands of the fused form: y = relu?(conv + bias[k] + residual).
 struct Epi {
   const float* bias;
@@ -977,14 +982,36 @@ struct Epi {
 // stores one column of both -- a conversion, a shuffle, a byte permute, an
 // add and a 4-byte store for two columns (40 -> 25 cycles a column of a 128 x
 // 256 unit against float shuffles and 64-bit addresses).
-// EPI: + bias (rounded to fp16), + residual in fp32, ReLU last.  All 32 lanes call.
-template <int NC, bool EPI>
+// Epilogue: + bias (rounded to fp16), + residual in fp32, ReLU last; a kernel
+// for even rows of 4-byte aligned outputs and one for others.  The residuals
+// `rv` of the columns come from load_cols, ahead of the accumulators.  All 32
+// lanes call.
+enum EpiKind : int { NOEPI, EPI_PAIR, EPI_ODD };
+template <int NC>
+__device__ __forceinline__ void load_cols(const Epi& epi, uint32_t o, uint32_t step, int lim, bool live, bool pair,
+                                          __half2* rv) {
+  const char* R = reinterpret_cast<const char*>(epi.residual);
+  if (!R) return;
+  if (pair) {
+    const bool odd = (threadIdx.x & 1) != 0;
+    uint32_t ra = o - (odd ? 2u : 0u) + (odd ? step : 0u);
+#pragma unroll
+    for (int j = 0; j < NC / 2; ++j, ra += 2 * step)
+      rv[j] = live && 2 * j + odd < lim ? *reinterpret_cast<const __half2*>(R + ra) : __half2{};
+  } else {
+    uint32_t ra = o;
+#pragma unroll
+    for (int j = 0; j < NC / 2; ++j, ra += 2 * step)
+      rv[j] = __halves2half2(live && 2 * j < lim ? *reinterpret_cast<const __half*>(R + ra) : __half{},
+                             live && 2 * j + 1 < lim ? *reinterpret_cast<const __half*>(R + ra + step) : __half{});
+  }
+}
+template <int NC, int EPI>
 __device__ __forceinline__ void store_cols(const Epi& epi, const float* bias, char* Y, uint32_t o, uint32_t step,
-                                           const float* v, int lim, bool live, bool pair) {
-  const char* R = EPI ? reinterpret_cast<const char*>(epi.residual) : nullptr;
+                                           const float* v, const __half2* rv, int lim, bool live, bool pair) {
   auto finish = [&](__half2 h, __half2 r) {
     float2 f = __half22float2(h);
-    if (R) {
+    if (epi.residual) {
       const float2 g = __half22float2(r);
       f.x += g.x;
       f.y += g.y;
@@ -995,28 +1022,24 @@ __device__ __forceinline__ void store_cols(const Epi& epi, const float* bias, ch
     }
     return __floats2half2_rn(f.x, f.y);
   };
+  auto rounded = [&](int j) {
+    float a = v[2 * j], b = v[2 * j + 1];
+    if (EPI && bias) {
+      // (bias of channels past K is not read: lim)
+      a += 2 * j < lim ? __ldg(bias + 2 * j) : 0.f;
+      b += 2 * j + 1 < lim ? __ldg(bias + 2 * j + 1) : 0.f;
+    }
+    return __floats2half2_rn(a, b);
+  };
   if (pair) {
     const bool odd = (threadIdx.x & 1) != 0;
     const uint32_t sel = odd ? 0x3276u : 0x5410u;
     // the pair's even position, this lane's column of the first two
     uint32_t at = o - (odd ? 2u : 0u) + (odd ? step : 0u);
     const int mine = odd ? 1 : 0;
-    __half2 rv[EPI ? NC / 2 : 1];
-    if (EPI && R) {
-      uint32_t ra = at;
-#pragma unroll
-      for (int j = 0; j < NC / 2; ++j, ra += 2 * step)
-        rv[j] = live && 2 * j + mine < lim ? *reinterpret_cast<const __half2*>(R + ra) : __half2{};
-    }
 #pragma unroll
     for (int j = 0; j < NC / 2; ++j, at += 2 * step) {
-      float a = v[2 * j], b = v[2 * j + 1];
-      if (EPI && bias) {
-        // (bias of channels past K is not read: lim)
-        a += 2 * j < lim ? __ldg(bias + 2 * j) : 0.f;
-        b += 2 * j + 1 < lim ? __ldg(bias + 2 * j + 1) : 0.f;
-      }
-      const __half2 h = __floats2half2_rn(a, b);
+      const __half2 h = rounded(j);
       const uint32_t own = *reinterpret_cast<const uint32_t*>(&h);
       const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
       const uint32_t w = __byte_perm(own, other, sel);
@@ -1027,15 +1050,12 @@ __device__ __forceinline__ void store_cols(const Epi& epi, const float* bias, ch
   } else if (live) {
     uint32_t at = o;
 #pragma unroll
-    for (int c = 0; c < NC; ++c, at += step)
-      if (c < lim) {
-        __half h = __float2half_rn(v[c] + (EPI && bias ? __ldg(bias + c) : 0.f));
-        if (EPI) {
-          const __half r = R ? *reinterpret_cast<const __half*>(R + at) : __half{};
-          h = __low2half(finish(__half2half2(h), __half2half2(r)));
-        }
-        *reinterpret_cast<__half*>(Y + at) = h;
-      }
+    for (int j = 0; j < NC / 2; ++j, at += 2 * step) {
+      __half2 h = rounded(j);
+      if (EPI) h = finish(h, rv[j]);
+      if (2 * j < lim) *reinterpret_cast<__half*>(Y + at) = __low2half(h);
+      if (2 * j + 1 < lim) *reinterpret_cast<__half*>(Y + at + step) = __high2half(h);
+    }
   }
 }
 
@@ -1136,7 +1156,7 @@ __device__ __forceinline__ void shift_weight_from_u(const KernelParam& p, const 
 // The kernel body.  CG = 2: clusters of two CTAs (__cluster_dims__(2, 1, 1)),
 // a unit is 256 positions, rank 0 issues the pair's MMAs.  Every role walks
 // the source's layers and its own units of each.
-template <int CG, class F, bool EPI, class Src>
+template <int CG, class F, int EPI, class Src>
 __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& epi, uint32_t* err) {
   using namespace sc;
   using Ro = Roles<F>;
@@ -1283,7 +1303,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       const Grid gr = make_grid(g);
       // even output rows sit on an even grid: neighbouring outputs on lanes
       // 2i, 2i + 1 share 4-byte stores
-      const bool pair = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 3) == 0;
+      const bool pair = EPI == NOEPI ? store_pairs(g.OW, Y, nullptr) : EPI == EPI_PAIR;
       for (int i = 0; i < cv.cnt; ++i, ++unit) {
         int pt, k0;
         unit_of(g, cv.u0 + i * ustep, pt, k0);
@@ -1293,6 +1313,11 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         const Base c = advance(gr, tile_base(gr, pt * TS + tp), quarter * 32 + lane);
         const bool live = c.n < g.N && c.gy < g.OH && c.gx < g.OW;
         const uint32_t at = live ? ((uint32_t)(c.n * g.K + k0) * (uint32_t)OHOW + (uint32_t)(c.gy * g.OW + c.gx)) * 2u : 0u;
+        __half2 rv[EPI ? 16 : 1];
+        auto res = [&](int cc) {
+          if (EPI) load_cols<32>(epi, at + (uint32_t)cc * step, step, kval - cc, live, pair, rv);
+        };
+        res(part * 32);
         ok = mbar_wait_warp(&sh.accfull[ab], (unit >> 1) & 1, abort_flag, err, ERR_WAIT_ACCUM, SLEEP_NS);
         if (!ok) break;
         tc_fence_after();
@@ -1303,7 +1328,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         };
         auto stc = [&](int cc, const float* v) {
           store_cols<32, EPI>(epi, EPI && epi.bias ? epi.bias + k0 + cc : nullptr, reinterpret_cast<char*>(Y),
-                              at + (uint32_t)cc * step, step, v, kval - cc, live, pair);
+                              at + (uint32_t)cc * step, step, v, rv, kval - cc, live, pair);
         };
 #pragma unroll 1
         for (int cc = part * 32; cc < nrows; cc += 32 * PARTS) {
@@ -1311,6 +1336,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
           ld(cc, va);
           tmem_ld_wait();
           stc(cc, va);
+          if (cc + 32 * PARTS < nrows) res(cc + 32 * PARTS);
         }
         tc_fence_before();
         __syncwarp();

@@ -1186,7 +1186,7 @@ __global__ void __launch_bounds__(TMAV && F8 ? trs::NTHREAD_V : trs::NTHREAD, 1)
   static_assert(trs::NTHREAD == sc::NTHREAD_HOSTED && sc::SMEM_BYTES <= 227 * 1024, "one kernel hosts both schedules");
   if constexpr (TMAV && F8 == 0) {
     if (p.mid_result == nullptr) {
-      shift_conv_body<1, sc::Hosted, false>(sc::OneConv<sc::CONV33>{p}, sc::Epi{}, &g_twostage_err);
+      shift_conv_body<1, sc::Hosted, sc::NOEPI>(sc::OneConv<sc::CONV33>{p}, sc::Epi{}, &g_twostage_err);
       return;
     }
   }
