@@ -111,23 +111,24 @@ int wino_shift_cg(const KernelParam* p) {
 }
 
 // The packed plan the kernels read from the argument's transform_pin.
-unsigned long long wino_shift_pack(const KernelParam* p, int cg, int hosted) {
-  return sc::pack_plan(sc::make_plan(*p, cg, hosted ? sc::TWOSTAGE : sc::OWN));
-}
+unsigned long long wino_shift_pack(const KernelParam* p, int cg) { return sc::pack_plan(sc::make_plan(*p, cg)); }
 
-unsigned wino_shift_grid(const KernelParam* p, int cg, int sms) {
-  const sc::Plan g = sc::make_plan(*p, cg);
+static unsigned units_grid(const sc::Plan& g, int cg, int sms) {
   const long long cap = sms / cg;
   return (unsigned)(cg * (g.units < cap ? g.units : cap));
 }
+unsigned wino_shift_grid(const KernelParam* p, int cg, int sms) { return units_grid(sc::make_plan(*p, cg), cg, sms); }
 
-int wino_shift_prepare() {
-  // attributes are per function and device: set them once per device (a
-  // repeated set from another thread is harmless)
-  static int done[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
-  if (dev >= 0 && dev < 64 && done[dev]) return 0;
+// Packed plan and both kernels' grids of a drop-in problem.
+unsigned long long wino_shift_slots(const KernelParam* p, int cg, int hosted, int sms, unsigned* grid,
+                                    unsigned* weight_grid) {
+  const sc::Plan g = sc::make_plan(*p, cg, hosted ? sc::TWOSTAGE : sc::OWN);
+  *grid = units_grid(g, cg, sms);
+  *weight_grid = (unsigned)((sc::weight_bytes(g, cg) / 16 + 255) / 256);
+  return sc::pack_plan(g);
+}
+
+static int shift_prepare_device() {
   for (const void* f : {(const void*)shift_conv_kernel, (const void*)shift_conv_pair_kernel,
                         (const void*)shift_conv_fold_kernel, (const void*)shift_conv_fold_pair_kernel,
                         (const void*)shift_conv_epi_kernel<sc::EPI_PAIR>, (const void*)shift_conv_epi_kernel<sc::EPI_ODD>,
@@ -136,8 +137,11 @@ int wino_shift_prepare() {
                         (const void*)shift_conv_batch_kernel}) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sc::SMEM_BYTES) != cudaSuccess) return 1;
   }
-  if (dev >= 0 && dev < 64) done[dev] = 1;
   return 0;
+}
+int wino_shift_prepare() {
+  static OncePerDevice once;
+  return once.run(shift_prepare_device);
 }
 
 // The plan's numbers (host tests): GX, GY, operand rows, blocks per stage,
@@ -211,7 +215,7 @@ int wino_launch_shift_fused(const KernelParam* p0, const void* u, void* wop, int
   KernelParam p = *p0;
   p.pweight = const_cast<void*>(u);
   p.transform_filter = wop;
-  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg, 0));
+  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg));
   const int rc = wino_launch_shift_weight_u(&p, cg, stream);
   if (rc != 0) return rc;
   if (!va || (!va->bias && !va->residual && !va->relu)) return wino_launch_shift(&p, cg, sms, stream);
@@ -282,7 +286,7 @@ int wino_conv2d_shift(const void* x, const void* weight, void* wprep, void* y, i
   if (wino_shift_cg(&p) == 0) return 2;
   if (cg == 0) cg = wino_shift_cg(&p);
   if (wino_shift_prepare() != 0) return 3;
-  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg, 0));
+  p.transform_pin = reinterpret_cast<void*>(wino_shift_pack(&p, cg));
   void* args[] = {&p};
   if (weight && cudaLaunchKernel(wino_shift_weight_kernel_ptr(cg), dim3(wino_shift_weight_grid(&p, cg)), dim3(256),
                                  args, 0, (cudaStream_t)stream) != cudaSuccess)

@@ -2123,7 +2123,7 @@ int wino_twostage_smem_bytes_for(int c) {
 int wino_twostage_output_smem_bytes() { return ot::SMEM_BYTES; }
 int wino_twostage_output_threads() { return ot::NTHREAD; }
 
-int wino_twostage_prepare() {
+static int twostage_prepare_device() {
   if (cudaFuncSetAttribute(twostage_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            ot::SMEM_BYTES) != cudaSuccess)
     return 1;
@@ -2148,6 +2148,10 @@ int wino_twostage_prepare() {
     return 1;
   return (int)cudaFuncSetAttribute(twostage_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    tp::SMEM_BYTES);
+}
+int wino_twostage_prepare() {
+  static OncePerDevice once;
+  return once.run(twostage_prepare_device);
 }
 
 // The two-stage pre-pass: row-transformed records (XR) for the resident-U

@@ -112,10 +112,9 @@ int wino_igemm_shape_ok(int n, int c, int h, int w, int k, int oh, int ow);
 int wino_igemm_prepare();
 uint32_t wino_igemm_error_read_clear();
 int wino_shift_cg(const wino::KernelParam* p);
-unsigned long long wino_shift_pack(const wino::KernelParam* p, int cg, int hosted);
-unsigned wino_shift_grid(const wino::KernelParam* p, int cg, int sms);
+unsigned long long wino_shift_slots(const wino::KernelParam* p, int cg, int hosted, int sms, unsigned* grid,
+                                    unsigned* weight_grid);
 size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
-unsigned wino_shift_weight_grid(const wino::KernelParam* p, int cg);
 void* wino_shift_weight_kernel_ptr(int cg);
 void* wino_shift_kernel_ptr(const wino::KernelParam* p, int cg);
 int wino_shift_threads(int hosted);
@@ -364,11 +363,13 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
     wino::KernelParam* kp = static_cast<wino::KernelParam*>(param);
     // the packed plan travels in transform_pin, which the kernels need no
     // pointer in
-    kp->transform_pin = reinterpret_cast<void*>(wino_shift_pack(kp, shift.cg, hosted));
-    set_slot(kernelInfo, 1, wino_shift_weight_grid(kp, shift.cg), 1, 1, 256, 1, 1, 0,
+    unsigned grid = 0, weight_grid = 0;
+    kp->transform_pin =
+        reinterpret_cast<void*>(wino_shift_slots(kp, shift.cg, hosted, sm_count(), &grid, &weight_grid));
+    set_slot(kernelInfo, 1, weight_grid, 1, 1, 256, 1, 1, 0,
              wino_shift_weight_kernel_ptr(shift.cg));
     set_slot(kernelInfo, 2, 1, 1, 1, 32, 1, 1, 0, wino_noop_kernel_ptr());
-    set_slot(kernelInfo, 3, wino_shift_grid(kp, shift.cg, sm_count()), 1, 1, (unsigned)wino_shift_threads(hosted), 1, 1,
+    set_slot(kernelInfo, 3, grid, 1, 1, (unsigned)wino_shift_threads(hosted), 1, 1,
              (unsigned)wino_shift_smem_bytes(),
              hosted ? wino_twostage_gemm_kernel_ptr_for((int)pr.c) : wino_shift_kernel_ptr(kp, shift.cg));
     if (hosted)
@@ -846,6 +847,29 @@ extern "C" int wino_launch_kernelinfo(const void* kiv, void* param, void* stream
     if (e != (int)cudaSuccess) return WINO_ECUDA;
   }
   return WINO_OK;
+}
+
+// One drop-in call of the harness: getkernelInfo on a parameter block of its
+// own, then the four slots.  WINO_* of getkernelInfo, or 256 more of the launch.
+extern "C" int wino_dropin_conv2d(void* in, void* weight, void* out, void* transform_pin, void* transform_filter,
+                                  void* mid_result, unsigned n, unsigned c, unsigned h, unsigned w, unsigned k,
+                                  unsigned r, unsigned s, unsigned stride, unsigned pad, void* stream) {
+  problem_t pr{};
+  pr.in = static_cast<decltype(pr.in)>(in);
+  pr.weight = static_cast<decltype(pr.weight)>(weight);
+  pr.out = static_cast<decltype(pr.out)>(out);
+  pr.transform_pin = static_cast<decltype(pr.transform_pin)>(transform_pin);
+  pr.transform_filter = static_cast<decltype(pr.transform_filter)>(transform_filter);
+  pr.mid_result = static_cast<decltype(pr.mid_result)>(mid_result);
+  pr.n = n; pr.c = c; pr.h = h; pr.w = w; pr.k = k; pr.r = r; pr.s = s;
+  pr.u = pr.v = stride;
+  pr.p = pr.q = pad;
+  kernelInfo_t ki;
+  mykernelParamType param{};
+  int rc = getkernelInfo(&pr, &ki, &param);
+  if (rc != WINO_OK) return rc;
+  rc = wino_launch_kernelinfo(&ki, &param, stream);
+  return rc == WINO_OK ? WINO_OK : 256 + rc;
 }
 
 extern "C" int wino_error_read_clear(uint32_t* code) {

@@ -12,7 +12,9 @@
 // zero outside the image (pad = 1).  Tiles are numbered flat over
 // (n, ty, tx) with tx fastest; an image has ceil(H/2) * ceil(W/2) tiles.
 #pragma once
+#include <atomic>
 #include <cstdint>
+#include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -112,6 +114,21 @@ __host__ __device__ __forceinline__ void filter_tile(const float g[9], float u[1
     u[4 * a + 3] = tmp[a][2];
   }
 }
+
+// Kernel attributes are per function and device: set once for each, as a call
+// took a microsecond for every few of them.  A repeat by another thread is harmless.
+struct OncePerDevice {
+  std::atomic<bool> done[64] = {};
+  int run(int (*prepare)()) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    const bool kept = dev >= 0 && dev < 64;
+    if (kept && done[dev].load(std::memory_order_acquire)) return 0;
+    const int rc = prepare();
+    if (rc == 0 && kept) done[dev].store(true, std::memory_order_release);
+    return rc;
+  }
+};
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
