@@ -23,6 +23,7 @@ LIB_PATH = os.path.join(HERE, "_build", "libwinoconv.so")
 WINO_OK, WINO_EINVAL, WINO_EUNSUPPORTED, WINO_ECUDA, WINO_EDEVICE = 0, 1, 2, 3, 4
 WINO_ESCRATCH, WINO_ESTALE, WINO_EIO = 5, 6, 7
 VAR_F16, VAR_BF16, VAR_F8, VAR_F16_HILO = 0, 1, 2, 3
+ROUTE_IGEMM, ROUTE_SHIFT = 4, 5   # of wino_dropin_route
 
 
 class WinoError(RuntimeError):

@@ -553,7 +553,10 @@ int wino_batch_tune(void* h, int reps, float* layer_us, float* order_us, void* s
       if (wino::cfg_split_level(cfg) != 0) continue;
       if (!L.p.transform_pin && !(cfg & wino::CFG_DIRECT)) continue;
       float t = 0.f;
-      // (a layer on the shift kernel runs the same under every configuration)
+      if (L.shift && best >= 0) {           // the shift kernel runs the same under every configuration
+        us[cfg] = us[best];
+        continue;
+      }
       auto one = [&] {
         return L.shift ? b->run_shift(L, s) : run_layer_cfg(L.p, L.p.transform_pin, cfg, s);
       };

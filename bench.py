@@ -5,20 +5,21 @@ One step = one forward conv of the single-large-layer workload
 (N=128, C=K=256, H=W=28, 3x3, stride 1, pad 1; x = ReLU(N(0,1)),
 w ~ N(0, 2/(9C)), seed 0), run through the drop-in ABI exactly as the
 reference harness runs it: getkernelInfo once, then per step the four launch
-slots (for this even-sized layer: filter transform, input pre-pass writing
-the transformed tiles to transform_pin, tap GEMM writing M to mid_result,
-output transform).
+slots (for this layer: weights laid out as a tensor-core operand in
+transform_filter, then the shift-reuse implicit GEMM on NCHW input and output;
+the other two slots are empty and not launched).
 
 Printed (rank 0, one JSON line):
   value      direct-conv-equivalent TFLOP/s (2*N*K*C*P*Q*9 / time), whole job,
              inputs resident in HBM, L2 flushed between steps
   e2e        the same metric through the C-ABI with host buffers: each step
-             copies x host->device, runs the four slots, copies y back
+             copies x host->device, runs the slots, copies y back
   roofline   the step's slowest kernel against its own roofline (the slower
-             of Winograd GEMM FLOPs 2*16*K*C*N*ceil(P/2)*ceil(Q/2) over the
+             of the GEMM FLOPs it computes -- 2*N*K*C*P*Q*9 for the implicit
+             GEMM, 2*16*K*C*N*ceil(P/2)*ceil(Q/2) for Winograd -- over the
              measured bf16 GEMM peak and its compulsory DRAM bytes over the
              measured copy bandwidth, MEASURED_PEAKS.json), each kernel timed
-             alone by CUDA events; roofline.kernels lists all three
+             alone by CUDA events; roofline.kernels lists them
   cpu_baseline  the reference's own conv2dcpu (oracle/_ref) on this host's
              cores over a bounded sample of images
 plus the fused-vs-unfused comparison and the error against FP64.
@@ -85,6 +86,8 @@ def committed_traffic(kernel):
     """DRAM bytes per launch of `kernel` from the committed ncu summaries, if any."""
     if kernel == "fused_wino_f16_kernel":
         name = "fused_conv_n128_c256_h28.json"
+    elif kernel == "shift_conv":
+        name = "shift_conv_n128_c256_h28.json"
     else:
         name = "twostage_conv_n128_c256_h28.json"
     try:
@@ -383,15 +386,22 @@ def run_ours(args, rank, world, local_rank):
     unf_rel = float(torch.linalg.vector_norm(yu.double() - y.double()) /
                     torch.linalg.vector_norm(y.double()))
     del ws
-    fused_us = fused_ms / iters * 1e3          # pre-pass + fused kernel
+    fused_us = fused_ms / iters * 1e3          # conv on a cached U with a workspace
     layout_us = layout_ms / iters * 1e3         # pre-pass alone
-    kernel_us = max(fused_us - layout_us, 1e-3)  # the fused kernel
+    # the route getkernelInfo chose for the timed drop-in step
+    shift = wino.lib().wino_dropin_route(ctypes.byref(pr)) == wino.ROUTE_SHIFT
+    if shift:                                    # slot 3 alone, on the operand the steps left
+        conv = wino.KernelInfo.from_buffer_copy(ki)
+        conv.kernelPtr1 = ki.kernelPtr2          # the empty slot's kernel: not launched
+        conv_ms, _ = timed(lambda: wino.launch_kernel_info(conv, param, stream), iters)
+        kernel_us = conv_ms / iters * 1e3
+    else:
+        kernel_us = max(fused_us - layout_us, 1e-3)  # the fused kernel
     unfused_us = unf_ms / iters * 1e3
     ft_us = ft_ms / iters * 1e3
     ts_us, ts_pre_us, ts_gemm_us, ts_out_us = (ts_ms / iters * 1e3, ts_pre_ms / iters * 1e3,
                                                ts_gemm_ms / iters * 1e3, ts_out_ms / iters * 1e3)
-    # the route getkernelInfo chose for the timed drop-in step
-    two_stage = ki.slot(3)["kernel"] == wino.lib().wino_twostage_gemm_kernel_ptr_for(c)
+    two_stage = not shift and ki.slot(3)["kernel"] == wino.lib().wino_twostage_gemm_kernel_ptr_for(c)
 
     # --- end to end through the C-ABI with host buffers.  Every step uploads
     # its input from pinned host memory, runs the drop-in slots and downloads
@@ -467,7 +477,9 @@ def run_ours(args, rank, world, local_rank):
     tiles = n * ((h + 1) // 2) * ((w + 1) // 2)
     x_bytes, y_bytes = n * c * h * w * 2, n * k * h * w * 2
     m_bytes, u_bytes = 16 * k * tiles * 2, 16 * k * c * 2
-    if two_stage:
+    if shift:
+        kern = [kernel_roofline("shift_conv", kernel_us, dflops, x_bytes + y_bytes + 2 * 9 * k * c, peaks)]
+    elif two_stage:
         pre_bytes = L.wino_twostage_prepass_bytes(n, c, h, w)
         gk = L.wino_twostage_gemm_kernel_ptr_for(c)
         gname = ("twostage_res_kernel_t<1>" if gk == L.wino_twostage_resv_kernel_ptr() else
@@ -483,7 +495,7 @@ def run_ours(args, rank, world, local_rank):
     roofline = {k2: dom[k2] for k2 in ("bound", "achieved", "peak", "unit", "frac", "traffic", "peak_source",
                                        "kernel")}
     roofline["algorithmic"] = (f"{dom['bytes'] / 1e6:.1f} MB compulsory DRAM bytes and {dom['flops'] / 1e9:.2f} "
-                               "Winograd GEMM GFLOP per launch; the bound is the slower of the two")
+                               "GEMM GFLOP per launch; the bound is the slower of the two")
     roofline["kernels"] = kern
     roofline["step_floor_us"] = sum(r["floor_us"] for r in kern)
     roofline["step_frac_of_kernel_floors"] = roofline["step_floor_us"] / (max_ms / args.steps * 1e3)
@@ -506,7 +518,8 @@ def run_ours(args, rank, world, local_rank):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f16",
         "data": "synthetic (seeded ReLU(N(0,1)) input, N(0,2/(9C)) weights)",
         "config": {"workload": WORKLOAD_NAME, **W, "parallelism": f"replicas x{world}",
-                   "step": ("drop-in ABI: filter transform + input pre-pass (transformed tiles) + tap GEMM + "
+                   "step": ("drop-in ABI: weight re-layout + shift-reuse implicit GEMM" if shift else
+                            "drop-in ABI: filter transform + input pre-pass (transformed tiles) + tap GEMM + "
                             "output transform" if two_stage else
                             "drop-in ABI: filter transform + input re-layout + fused conv + 1 empty slot"),
                    "l2": "flushed between steps (256 MB write)"},
@@ -528,7 +541,7 @@ def run_ours(args, rank, world, local_rank):
         "e2e": {"value": e2e_value, "unit": "TFLOP/s", "h2d_bytes_per_step": x.numel() * 2,
                 "d2h_bytes_per_step": y.numel() * 2, "rel_l2_of_downloaded_output": e2e_err,
                 "pipelining": "2 buffer sets, upload / compute / download streams"},
-        "gpu_launches": 4 * args.steps,
+        "gpu_launches": (2 if shift else 4) * args.steps,
         "clocks": clocks,
     }
     if world == 1 and not args.no_extras:
@@ -600,13 +613,13 @@ def extension_legs(wino, dev, flush, ev, peaks, steps):
     for (x, wt, u, ws, y, c, k, h) in layers:
         y64 = torch.nn.functional.conv2d(x.double(), wt.double(), padding=1)
         worst = max(worst, float(torch.linalg.vector_norm(y.double() - y64) / torch.linalg.vector_norm(y64)))
-    # each layer alone with its tuned configuration (pre-pass + fused kernel),
-    # against its own roofline, to show which layer classes lose the time
+    # each layer alone, as the single-layer call runs it, against its own
+    # roofline, to show which layer classes lose the time
     per_layer = []
     for i, (x, wt, u, ws, y, c, k, h) in enumerate(layers):
         cfg = b.config(i)
-        cws = wino._aligned_ws(wino.cfg_workspace_bytes(n, c, h, h, k, cfg), dev)
-        us = timed(lambda: wino.conv2d_fused_cfg(x, u, k, cfg, workspace=cws, out=y), steps)
+        cws = torch.empty(wino.fused_conv_workspace_bytes(n, c, h, h, k), dtype=torch.uint8, device=dev)
+        us = timed(lambda: wino.conv2d_fused(x, u, k, workspace=cws, out=y), steps)
         byt = 2.0 * (n * c * h * h + n * k * h * h + 16 * k * c)
         t_hbm = byt / (peaks["hbm_gbs"] * 1e9) * 1e6
         t_tc = wino_flops(n, c, h, h, k) / (peaks["tflops"] * 1e12) * 1e6
@@ -620,7 +633,7 @@ def extension_legs(wino, dev, flush, ev, peaks, steps):
         "us_graph_tuned": graph_us, "us_persistent_untuned": untuned_us, "us_sequential_launches": seq_us,
         "direct_equiv_tflops": dfl / (graph_us * 1e-6) / 1e12,
         "configs": [b.config(i) for i in range(len(layers))], "order": b.order(),
-        # the tuner's route per layer (0 fused tile blocks of 128 k x 32 tiles, 1 two-stage
+        # the tuner's route per layer (0 shift kernel or fused tile blocks, 1 two-stage
         # tap-GEMM units of 128 tiles x 256 k) with each layer's time alone on both routes
         "routes": [b.route(i)[0] for i in range(len(layers))],
         "alone_us_fused_twostage": [[round(b.route(i)[1], 1), round(b.route(i)[2], 1)] for i in range(len(layers))],
