@@ -25,8 +25,8 @@
 // 8-row groups follow each other without a gap (SBO = 128), so any row may
 // start a tile.  Against one staged operand per tap that is 9 * 128 = 1152
 // rows down to 128 + 2 GX + 2 per 16 channels of a 3x3 layer (190 at 28x28),
-// few enough that four warps bring them in from NCHW and no pre-pass over the
-// input is needed.
+// few enough that the block's own warps bring them in from NCHW and no pre-pass
+// over the input is needed.
 //
 // Those producers read the input as quads of pixels: a channel's plane is
 // contiguous, so four consecutive pixels of eight channels are eight 8-byte
@@ -42,10 +42,11 @@
 // two CTAs, M = 256 positions) halves that stream per SM: each CTA holds half
 // of the weights' rows and the pair's MMA reads both halves.
 //
-// Measured (B200, L2 flushed, conv alone): N128 C256 28x28 K256 92 us = 1284
-// TFLOP/s direct (the Winograd two-stage kernels it replaces there: 61 + 79 +
-// 54 us); N64 C256 14x14 K256 30 us; N32 C512 7x7 K512 31 us; N32 C128 56x56
-// K128 stride 2 37 us (gathering implicit GEMM: 69 us).
+// Measured (B200): N128 C256 28x28 K256 94 us for the conv alone with L2
+// flushed = 1253 TFLOP/s direct (the Winograd two-stage kernels it replaces
+// there: 61 + 79 + 54 us).  Whole drop-in calls against the kernels replaced: N64
+// C256 14x14 K256 27 us (55), N32 C512 7x7 K512 29 (62), N32 C128 56x56 K128
+// stride 2 31 (74, gathering implicit GEMM), N32 C64 56x56 K256 1x1 25 (53).
 //
 // The weight operand (shift_weight_kernel) is laid out as the stages read it:
 // per unit block of output channels and CTA of the unit, 16-channel block by
@@ -752,7 +753,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
 // Producers of a folded problem (Plan): thread = operand row, a position's
 // C * S values gathered with 2-byte loads (lanes on neighbouring output
 // columns) into up to four 16-byte words.  N32 224x224 RGB 7x7 / 2
-// K64 takes 72 us, waiting on these gathers (CUDA-core direct kernel: 590 us;
+// K64 takes 61 us, waiting on these gathers (CUDA-core direct kernel: 590 us;
 // its bytes take 9).  A unit is one stage and the groups
 // take alternate units.  FC, FS: channels and columns known at compile time
 // (0: as the plan says).
@@ -984,8 +985,9 @@ struct Epi {
 // 256 unit against float shuffles and 64-bit addresses).
 // Epilogue: + bias (rounded to fp16), + residual in fp32, ReLU last; a kernel
 // for even rows of 4-byte aligned outputs and one for others.  The residuals
-// `rv` of the columns come from load_cols, ahead of the accumulators.  All 32
-// lanes call.
+// `rv` of the columns come from load_cols, ahead of the accumulators: a load
+// between stores waits for them, as they may alias (N8 C32 51x51 K528 197 us,
+// so 67).  All 32 lanes call.
 enum EpiKind : int { NOEPI, EPI_PAIR, EPI_ODD };
 template <int NC>
 __device__ __forceinline__ void load_cols(const Epi& epi, uint32_t o, uint32_t step, int lim, bool live, bool pair,
