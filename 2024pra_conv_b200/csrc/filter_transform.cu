@@ -49,6 +49,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) filter_transform_kernel(const __half* __restrict__ w,
                                                                T* __restrict__ u, T* __restrict__ lo,
                                                                int K, int C, int layout) {
+  grid_dep_launch();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)K * C) return;
   int k, c;
@@ -72,6 +73,7 @@ __global__ void __launch_bounds__(256) filter_transform_kernel(const __half* __r
 
 // Drop-in slot-1 kernel: weight -> transform_filter (fp16 U cache).
 __global__ void __launch_bounds__(256) dropin_filter_kernel(KernelParam p) {
+  grid_dep_launch();
   const int K = p.k, C = p.c;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)K * C) return;

@@ -20,6 +20,7 @@
 // checks N*(C/16)*rows*entries < 2^31).
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
+#include "tc_sm100.cuh"
 #include "wino_param.h"
 #include "vgen.cuh"
 
@@ -27,6 +28,7 @@ namespace wino {
 
 template <bool AMAX>
 __global__ void __launch_bounds__(256) xb_layout_kernel(KernelParam p) {
+  grid_dep_launch();
   const int C = p.c, H = p.h, W = p.w;
   const int CB = C >> 4, HP = xb_rows(H), E = xb_entries(W);
   const uint32_t items = (uint32_t)p.n * CB * HP * E;
@@ -94,6 +96,8 @@ __global__ void __launch_bounds__(256) xb_layout_kernel(KernelParam p) {
         out[(2 + hh) * E] = make_uint4(0u, 0u, 0u, 0u);
     }
   }
+  // (launched beside the filter transform ahead of it: complete only when that is)
+  grid_dep_wait();
 }
 
 // fp8 scales from the per-channel input maxima: |V| <= 4 max|x_c| (each
@@ -153,6 +157,15 @@ int wino_launch_xb_layout(const KernelParam* p, cudaStream_t stream) {
   void* args[] = {const_cast<KernelParam*>(p)};
   return (int)cudaLaunchKernel((void*)xb_layout_kernel<false>,
                                dim3(wino_xb_layout_grid(p->n, p->c, p->h, p->w)), dim3(256), args, 0, stream);
+}
+
+// ... beside the filter transform launched right before it, whose work it needs
+// nothing of.
+int wino_launch_dependent(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream);
+int wino_launch_xb_layout_beside(const KernelParam* p, cudaStream_t stream) {
+  void* args[] = {const_cast<KernelParam*>(p)};
+  return wino_launch_dependent((void*)xb_layout_kernel<false>, dim3(wino_xb_layout_grid(p->n, p->c, p->h, p->w)),
+                               dim3(256), args, 0, stream);
 }
 
 // The fp8 variant's pre-pass: also the per-channel max |x| into p->mid_result

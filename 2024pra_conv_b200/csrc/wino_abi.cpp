@@ -63,6 +63,7 @@ size_t wino_xb_bytes(int n, int c, int h, int w);
 unsigned wino_xb_layout_grid(int n, int c, int h, int w);
 long long wino_xb_items(int n, int c, int h, int w);
 int wino_launch_xb_layout(const wino::KernelParam* p, cudaStream_t stream);
+int wino_launch_xb_layout_beside(const wino::KernelParam* p, cudaStream_t stream);
 int wino_launch_xb_layout_amax(const wino::KernelParam* p, cudaStream_t stream);
 int wino_launch_xb_f8_scales(const unsigned* amax, float* sv, uint32_t* inv_sv2, int C,
                              cudaStream_t stream);
@@ -627,10 +628,10 @@ extern "C" int wino_conv2d_fused_ws_sized(const void* x, const void* ucache, voi
                                    c, h, w, k);
   if (wino_launch_xb_layout(&p, (cudaStream_t)stream) != 0) return WINO_ECUDA;
   void* args[] = {&p};
-  const cudaError_t e = cudaLaunchKernel(wino_fused_kernel_ptr(), dim3(fused_grid(n, h, w, k)),
-                                         dim3(wino_fused_threads()), args,
-                                         (size_t)wino_fused_smem_bytes(), (cudaStream_t)stream);
-  return e == cudaSuccess ? WINO_OK : WINO_ECUDA;
+  return wino_launch_dependent(wino_fused_kernel_ptr(), dim3(fused_grid(n, h, w, k)), dim3(wino_fused_threads()), args,
+                               (size_t)wino_fused_smem_bytes(), (cudaStream_t)stream) == 0
+             ? WINO_OK
+             : WINO_ECUDA;
 }
 
 extern "C" int wino_conv2d_fused_ws(const void* x, const void* ucache, void* workspace, void* y,
@@ -721,7 +722,7 @@ extern "C" int wino_conv2d_variant(int variant, const void* x, const void* weigh
     }
   }
   if (rc != 0) return WINO_ECUDA;
-  if (variant != WINO_VAR_F8 && wino_launch_xb_layout(&p, s) != 0) return WINO_ECUDA;
+  if (variant != WINO_VAR_F8 && wino_launch_xb_layout_beside(&p, s) != 0) return WINO_ECUDA;
   return wino_fused_launch_variant(variant, &p, &va, 0, fused_grid(n, h, w, k), s) == 0 ? WINO_OK
                                                                                          : WINO_ECUDA;
 }
@@ -839,8 +840,12 @@ extern "C" int wino_launch_kernelinfo(const void* kiv, void* param, void* stream
     const unsigned* b = slots[i];
     const dim3 grid(b[0], b[1], b[2]), block(b[3], b[4], b[5]);
     // the shift kernel starts beside the weight kernel launched right before
-    // it and waits for the weights itself
-    const bool dependent = i == 2 && (fns[0] == wino_shift_weight_kernel_ptr(1) || fns[0] == wino_shift_weight_kernel_ptr(2));
+    // it and waits for the weights itself; the fused route's pre-pass needs
+    // nothing of its filter transform, and the fused kernel waits for both
+    const bool xb = fns[1] == wino_xb_layout_kernel_ptr() && fns[0] == wino_dropin_filter_kernel_ptr();
+    const bool dependent =
+        (i == 2 && (fns[0] == wino_shift_weight_kernel_ptr(1) || fns[0] == wino_shift_weight_kernel_ptr(2))) ||
+        (xb && (i == 1 || (i == 2 && fns[2] == wino_fused_kernel_ptr())));
     const int e = dependent ? wino_launch_dependent(fns[i], grid, block, (void**)&param, (size_t)b[6], (cudaStream_t)stream)
                             : (int)cudaLaunchKernel(fns[i], grid, block, (void**)&param, (size_t)b[6],
                                                     (cudaStream_t)stream);
