@@ -86,7 +86,7 @@ int wino_shift_smem_bytes() { return sc::SMEM_BYTES; }
 // CTAs a unit for a problem (1 or 2), or 0 when the kernel does not take it:
 // strides past 2, more than MAXTAP taps, a position tile whose pixels exceed
 // the producers' items, fewer than two stages, or indices past 32 bits.
-int wino_shift_cg(const KernelParam* p) {
+static int shift_cg(const KernelParam* p, bool full_pairs) {
   if (p->u > 2 || p->v > 2 || p->r * p->s > sc::MAXTAP) return 0;
   const sc::Plan g1 = sc::make_plan(*p, 1), g2 = sc::make_plan(*p, 2);
   if (g1.npos + 4096 >= (1LL << 31) || g1.GX >= (1 << 15) || g1.GY >= (1 << 15)) return 0;
@@ -100,8 +100,11 @@ int wino_shift_cg(const KernelParam* p) {
       return 0;
   const long long w1 = (g1.units + sc::NSM - 1) / sc::NSM, w2 = (g2.units + sc::NSM / 2 - 1) / (sc::NSM / 2);
   const int n2 = g2.Kp < 256 ? (g2.Kp + 31) / 32 * 32 : 256;
-  // a pair needs work for every pair of SMs
-  if (g2.units < sc::NSM / 2) return 1;
+  // one wave of single CTAs beats pairs that leave SMs idle (3x3 N20 C128 28x28
+  // K128 14.1 us alone, 15.5 in pairs); from the second wave on pairs win though
+  // some idle (N64 C256 14x14 K256 31.2 / 24.7; N64 C256 28x28 K256 stride 2
+  // 55.5 / 34.9; N128 C512 7x7 K512 52.3 / 36.1)
+  if (g2.units < sc::NSM / 2 && (w1 == 1 || full_pairs)) return 1;
   // narrow outputs: a pair's halved weights gain nothing there and the tiles of
   // one CTA balance better (3x3 N32 C64 56x56 K64 20.2 us alone, 22.6 in
   // pairs; 1x1 N32 C512 28x28 K128 16.3 / 20.6)
@@ -109,6 +112,11 @@ int wino_shift_cg(const KernelParam* p) {
   const long long t1 = w1 * sc::mma_cycles(1, g1.Kp < g1.NB ? g1.Kp : g1.NB), t2 = w2 * sc::mma_cycles(2, n2);
   return t2 <= t1 ? 2 : 1;
 }
+
+int wino_shift_cg(const KernelParam* p) { return shift_cg(p, false); }
+// ... where the one-CTA schedule runs in the kernel callers know the route by:
+// pairs only when they fill the device.
+int wino_shift_cg_hosted(const KernelParam* p) { return shift_cg(p, true); }
 
 // The packed plan the kernels read from the argument's transform_pin.
 unsigned long long wino_shift_pack(const KernelParam* p, int cg) { return sc::pack_plan(sc::make_plan(*p, cg)); }

@@ -113,6 +113,7 @@ int wino_igemm_shape_ok(int n, int c, int h, int w, int k, int oh, int ow);
 int wino_igemm_prepare();
 uint32_t wino_igemm_error_read_clear();
 int wino_shift_cg(const wino::KernelParam* p);
+int wino_shift_cg_hosted(const wino::KernelParam* p);
 unsigned long long wino_shift_slots(const wino::KernelParam* p, int cg, int hosted, int sms, unsigned* grid,
                                     unsigned* weight_grid);
 size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
@@ -251,33 +252,6 @@ struct ShiftPlan {
 // wino_conv2d_twostage there.
 constexpr double kShiftMinFlops = 64e6;
 
-static ShiftPlan plan_shift(const problem_t& pr, int oh, int ow) {
-  const ShiftPlan none{0, nullptr};
-  if (!pr.transform_filter) return none;
-  // strided 1x1 stays with the gathering implicit GEMM, which reads only the
-  // rows it needs (N32 C256 56x56 K128 / 2: 23 us against 29)
-  if (pr.r * pr.s == 1 && (pr.u > 1 || pr.v > 1)) return none;
-  if (2.0 * pr.n * pr.k * oh * ow * pr.c * pr.r * pr.s < kShiftMinFlops) return none;
-  wino::KernelParam p{};
-  p.pin = pr.in;
-  p.n = (short)pr.n; p.c = (short)pr.c; p.h = (short)pr.h; p.w = (short)pr.w; p.k = (short)pr.k;
-  p.r = (short)pr.r; p.s = (short)pr.s; p.u = (short)pr.u; p.v = (short)pr.v; p.p = (short)pr.p; p.q = (short)pr.q;
-  p.Oh = (short)oh; p.Ow = (short)ow;
-  int cg = wino_shift_cg(&p);
-  if (cg == 0) return none;
-  // weight operand: the caller's transform_filter (16*k*c fp16), else its
-  // transform_pin (4*h*h*n*c fp16); reference src/main.cpp:36-38
-  const size_t filter_bytes = (size_t)16 * pr.k * pr.c * 2, pin_bytes = (size_t)4 * pr.h * pr.h * pr.n * pr.c * 2;
-  for (; cg >= 1; --cg) {
-    const size_t need = wino_shift_weight_bytes(&p, cg);
-    if (need <= filter_bytes && (reinterpret_cast<uintptr_t>(pr.transform_filter) & 15) == 0)
-      return ShiftPlan{cg, pr.transform_filter};
-    if (pr.transform_pin && need <= pin_bytes && (reinterpret_cast<uintptr_t>(pr.transform_pin) & 15) == 0)
-      return ShiftPlan{cg, pr.transform_pin};
-  }
-  return none;
-}
-
 // Two-stage route (input transform fused into full-width tap GEMMs, M in the
 // caller's mid_result, output transform in slot 4): M fits the reference's
 // mid_result size of 4*k*h*w*n fp16 elements (even H and W) and the pre-pass
@@ -296,6 +270,37 @@ static bool wino_contract(const problem_t& pr) {
   return pr.r == 3 && pr.s == 3 && pr.u == 1 && pr.v == 1 && pr.p == 1 && pr.q == 1 &&
          wino_check_shape((int)pr.n, (int)pr.c, (int)pr.h, (int)pr.w, (int)pr.k) == WINO_OK &&
          pr.transform_filter != nullptr;
+}
+
+// Problems whose slot 3 keeps the two-stage route's kernel, which hosts the
+// one-CTA shift schedule.
+static bool hosts_shift(const problem_t& pr) { return pr.c <= 256 && wino_contract(pr) && two_stage_fits(pr); }
+
+static ShiftPlan plan_shift(const problem_t& pr, int oh, int ow) {
+  const ShiftPlan none{0, nullptr};
+  if (!pr.transform_filter) return none;
+  // strided 1x1 stays with the gathering implicit GEMM, which reads only the
+  // rows it needs (N32 C256 56x56 K128 / 2: 23 us against 29)
+  if (pr.r * pr.s == 1 && (pr.u > 1 || pr.v > 1)) return none;
+  if (2.0 * pr.n * pr.k * oh * ow * pr.c * pr.r * pr.s < kShiftMinFlops) return none;
+  wino::KernelParam p{};
+  p.pin = pr.in;
+  p.n = (short)pr.n; p.c = (short)pr.c; p.h = (short)pr.h; p.w = (short)pr.w; p.k = (short)pr.k;
+  p.r = (short)pr.r; p.s = (short)pr.s; p.u = (short)pr.u; p.v = (short)pr.v; p.p = (short)pr.p; p.q = (short)pr.q;
+  p.Oh = (short)oh; p.Ow = (short)ow;
+  int cg = hosts_shift(pr) ? wino_shift_cg_hosted(&p) : wino_shift_cg(&p);
+  if (cg == 0) return none;
+  // weight operand: the caller's transform_filter (16*k*c fp16), else its
+  // transform_pin (4*h*h*n*c fp16); reference src/main.cpp:36-38
+  const size_t filter_bytes = (size_t)16 * pr.k * pr.c * 2, pin_bytes = (size_t)4 * pr.h * pr.h * pr.n * pr.c * 2;
+  for (; cg >= 1; --cg) {
+    const size_t need = wino_shift_weight_bytes(&p, cg);
+    if (need <= filter_bytes && (reinterpret_cast<uintptr_t>(pr.transform_filter) & 15) == 0)
+      return ShiftPlan{cg, pr.transform_filter};
+    if (pr.transform_pin && need <= pin_bytes && (reinterpret_cast<uintptr_t>(pr.transform_pin) & 15) == 0)
+      return ShiftPlan{cg, pr.transform_pin};
+  }
+  return none;
 }
 
 // Route of getkernelInfo for a validated problem (no CUDA calls).
@@ -358,7 +363,7 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
     // Problems of the two-stage route keep its slot 3 and 4 kernels, by which
     // callers tell the route: given no mid_result, its GEMM kernel runs the
     // one-CTA shift schedule and its output transform has nothing to do.
-    const bool hosted = shift.cg == 1 && pr.c <= 256 && wino_contract(pr) && two_stage_fits(pr);
+    const bool hosted = shift.cg == 1 && hosts_shift(pr);
     a->transform_filter = static_cast<_Float16*>(shift.wop);
     a->mid_result = nullptr;
     wino::KernelParam* kp = static_cast<wino::KernelParam*>(param);
