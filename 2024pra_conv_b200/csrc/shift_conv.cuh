@@ -265,7 +265,10 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg, Host host = OWN) {
   for (int a = 0; a < g.nu; ++a)
     for (int b = 0; b < g.nv; ++b) longest = plane_rows(g, a, b) > longest ? plane_rows(g, a, b) : longest;
   const long long lines = (longest + 2 * g.GX - 2) / g.GX;
-  const long long px = g.U == 1 && g.V == 1 ? longest : lines * g.U * g.W;
+  // (strided, an image may end in rows that no output reads -- 2x2 / 2 without
+  // padding over odd H -- which a tile that runs into the next image steps over)
+  const int unread = g.H > g.GY * g.U - g.P ? g.H - (g.GY * g.U - g.P) : 0;
+  const long long px = g.U == 1 && g.V == 1 ? longest : (lines * g.U + (lines / g.GY + 1) * unread) * g.W;
   // (images end in a partial quad when H * W is not a multiple of 4)
   const long long imgs = lines / g.GY + 2;
   // (a grid without padding, 1x1: tiles are whole quads)
