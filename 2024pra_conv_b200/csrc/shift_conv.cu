@@ -27,13 +27,15 @@ __global__ void __launch_bounds__(128) shift_weight_u_batch_kernel(const __grid_
 }
 
 // One CTA a unit (128 positions, up to 128 output channels).
+template <bool EDGES>
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_kernel(KernelParam p) {
-  shift_conv_body<1, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // A pair of CTAs a unit (256 positions, up to 256 output channels).
+template <bool EDGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_pair_kernel(KernelParam p) {
-  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same for problems whose filter columns became channels.
@@ -45,14 +47,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shif
 }
 
 // The same with the fused epilogue.
-template <int EPI>
+template <int EPI, bool EDGES>
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_epi_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<1, sc::Wide, EPI>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
+  shift_conv_body<1, sc::Wide, EPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, e, &g_shift_err);
 }
-template <int EPI>
+template <int EPI, bool EDGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_epi_pair_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<2, sc::Wide, EPI>(sc::OneConv<sc::PLAIN>{p}, e, &g_shift_err);
+  shift_conv_body<2, sc::Wide, EPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, e, &g_shift_err);
+}
+template <int CG, bool EDGES>
+static const void* epi_kernel(bool even) {
+  if (CG == 2)
+    return even ? (const void*)shift_conv_epi_pair_kernel<sc::EPI_PAIR, EDGES>
+                : (const void*)shift_conv_epi_pair_kernel<sc::EPI_ODD, EDGES>;
+  return even ? (const void*)shift_conv_epi_kernel<sc::EPI_PAIR, EDGES>
+              : (const void*)shift_conv_epi_kernel<sc::EPI_ODD, EDGES>;
 }
 
 // A table of layers, passed by value: the roles read their layers' dims from
@@ -71,7 +81,12 @@ extern "C" {
 
 void* wino_shift_kernel_ptr(const KernelParam* p, int cg) {
   if (sc::folds(p->c, p->s)) return cg == 2 ? (void*)shift_conv_fold_pair_kernel : (void*)shift_conv_fold_kernel;
-  return cg == 2 ? (void*)shift_conv_pair_kernel : (void*)shift_conv_kernel;
+  if (sc::input_edges(*p)) return cg == 2 ? (void*)shift_conv_pair_kernel<true> : (void*)shift_conv_kernel<true>;
+  return cg == 2 ? (void*)shift_conv_pair_kernel<false> : (void*)shift_conv_kernel<false>;
+}
+// Host tests: item_at_edge for an item of `ch` channels.
+int wino_shift_item_at_edge(unsigned o, unsigned head, unsigned total, unsigned plane, int ch) {
+  return sc::item_at_edge(o, head, total, sc::item_span(plane, ch)) ? 1 : 0;
 }
 void* wino_shift_weight_kernel_ptr(int cg) {
   return cg == 2 ? (void*)shift_weight_pair_kernel : (void*)shift_weight_kernel;
@@ -137,12 +152,13 @@ unsigned long long wino_shift_slots(const KernelParam* p, int cg, int hosted, in
 }
 
 static int shift_prepare_device() {
-  for (const void* f : {(const void*)shift_conv_kernel, (const void*)shift_conv_pair_kernel,
-                        (const void*)shift_conv_fold_kernel, (const void*)shift_conv_fold_pair_kernel,
-                        (const void*)shift_conv_epi_kernel<sc::EPI_PAIR>, (const void*)shift_conv_epi_kernel<sc::EPI_ODD>,
-                        (const void*)shift_conv_epi_pair_kernel<sc::EPI_PAIR>,
-                        (const void*)shift_conv_epi_pair_kernel<sc::EPI_ODD>,
-                        (const void*)shift_conv_batch_kernel}) {
+  for (const void* f :
+       {(const void*)shift_conv_kernel<false>, (const void*)shift_conv_kernel<true>,
+        (const void*)shift_conv_pair_kernel<false>, (const void*)shift_conv_pair_kernel<true>,
+        (const void*)shift_conv_fold_kernel, (const void*)shift_conv_fold_pair_kernel, epi_kernel<1, false>(true),
+        epi_kernel<1, false>(false), epi_kernel<1, true>(true), epi_kernel<1, true>(false), epi_kernel<2, false>(true),
+        epi_kernel<2, false>(false), epi_kernel<2, true>(true), epi_kernel<2, true>(false),
+        (const void*)shift_conv_batch_kernel}) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sc::SMEM_BYTES) != cudaSuccess) return 1;
   }
   return 0;
@@ -202,9 +218,9 @@ int wino_shift_fused_cg(const KernelParam* p) {
   return wino_shift_cg(p);
 }
 // Whether a batch's table can hold a problem that wino_shift_fused_cg takes
-// (pairs): its producers own one item each.
+// (pairs): its producers own one item each, of words inside the input.
 int wino_shift_in_table(const KernelParam* p) {
-  return sc::stage_items(sc::make_plan(*p, 2, sc::TABLE), sc::input_aligned(p->h * p->w, p->pin), false) <=
+  return !sc::input_edges(*p) && sc::stage_items(sc::make_plan(*p, 2, sc::TABLE), sc::input_aligned(p->h * p->w, p->pin), false) <=
          sc::Roles<sc::Wide>::NPROD;
 }
 
@@ -230,10 +246,8 @@ int wino_launch_shift_fused(const KernelParam* p0, const void* u, void* wop, int
   sc::Epi e{va->bias, static_cast<const __half*>(va->residual), va->relu};
   void* args[] = {&p, &e};
   const bool even = sc::store_pairs(p.Ow, p.pout, va->residual);
-  const void* fn = cg == 2 ? (even ? (const void*)shift_conv_epi_pair_kernel<sc::EPI_PAIR>
-                                   : (const void*)shift_conv_epi_pair_kernel<sc::EPI_ODD>)
-                           : (even ? (const void*)shift_conv_epi_kernel<sc::EPI_PAIR>
-                                   : (const void*)shift_conv_epi_kernel<sc::EPI_ODD>);
+  const void* fn = sc::input_edges(p) ? (cg == 2 ? epi_kernel<2, true>(even) : epi_kernel<1, true>(even))
+                                      : (cg == 2 ? epi_kernel<2, false>(even) : epi_kernel<1, false>(even));
   return wino_launch_dependent(fn, dim3(wino_shift_grid(&p, cg, sms)), dim3(sc::NTHREAD), args, (size_t)sc::SMEM_BYTES,
                                stream);
 }

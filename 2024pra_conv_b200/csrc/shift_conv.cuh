@@ -301,6 +301,26 @@ __host__ __device__ __forceinline__ bool input_aligned(int hw, const void* x) {
   return (hw & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0;
 }
 
+// Whether the 8-byte words around unaligned quads may reach outside the input:
+// it starts or ends inside such a word.
+__host__ inline bool input_edges(const KernelParam& p) {
+  const unsigned long long total = 2ull * p.n * p.c * p.h * p.w;
+  return ((reinterpret_cast<uintptr_t>(p.pin) | total) & 7) != 0;
+}
+
+// Bytes from the first pixel of an item of `ch` channels to the end of the last
+// word it loads (saturated: more than any input).
+__host__ __device__ __forceinline__ uint32_t item_span(uint32_t plane, int ch) {
+  const unsigned long long b = (unsigned long long)(ch - 1) * plane + 16;
+  return b < 0xffffffffull ? (uint32_t)b : 0xffffffffu;
+}
+
+// Whether an unaligned item's words, the first pixel `o` bytes into an input of
+// `total` bytes that starts `head` bytes past a word, may be such ones.
+__host__ __device__ __forceinline__ bool item_at_edge(uint32_t o, uint32_t head, uint32_t total, uint32_t span) {
+  return total - o < span || (head != 0 && o < 8);
+}
+
 __host__ inline unsigned long long pack_plan(const Plan& g) {
   return (unsigned long long)g.GX | (unsigned long long)g.GY << 16 | (unsigned long long)(g.NB / 16) << 32 |
          (unsigned long long)g.lcps << 40 | (unsigned long long)g.nstage << 44 | (unsigned long long)g.qmax << 48;
@@ -331,10 +351,14 @@ struct Conv {
   int u0, cnt;
 };
 
-// A launch over one convolution (its argument carries the packed plan).
-template <int KIND>
+// A launch over one convolution (its argument carries the packed plan).  EDGES:
+// its input starts or ends inside an 8-byte word (input_edges), whose pixels the
+// producers then load one by one; kernels of their own, as the few more
+// registers cost the others 5 % (N32 C512 7x7 K512 29.3 -> 30.7 us).
+template <int KIND, bool EDGES = false>
 struct OneConv {
   static constexpr int kind = KIND;
+  static constexpr bool edges = EDGES;
   static constexpr bool table = false;
   const KernelParam& p;
   __device__ __forceinline__ int layers() const { return 1; }
@@ -357,7 +381,7 @@ struct ConvTable {
   // An item a producer: with two for some layers too, the producers' variants
   // spilled into an L1 cache that the stages leave little of (N32 C512 7x7
   // K512 with its operand 69 -> 37 us, the set's eight layers N32 186 -> 130).
-  static constexpr bool table = true;
+  static constexpr bool table = true, edges = false;
   const ShiftTable& t;                    // the kernel's argument (constant bank)
   __device__ __forceinline__ int layers() const { return t.nlayers; }
   __device__ __forceinline__ bool strided() const { return false; }
@@ -498,7 +522,8 @@ struct Slot {
 // barrier's parity it then waits for could be two rounds old.
 // Strided, a stage's pixels are many and each group takes one channel half of
 // every stage.
-template <int CG, class F, int NI, bool ALIGNED, bool STRIDED>
+// EDGES: items whose words may reach outside the input load pixel by pixel.
+template <int CG, class F, int NI, bool ALIGNED, bool STRIDED, bool EDGES>
 __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int done, int turn,
                                         int ustep, int tile_pos, int tile_stride, bool& set, uint32_t* err) {
   const Plan& g = cv.g;
@@ -662,6 +687,25 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
         uint32_t o = off[i] + (nc > 0 ? (uint32_t)c * plane : 0u);
         s.row[i] = row_l[i];
         if (!ALIGNED) shifts |= ((uint32_t)(reinterpret_cast<uintptr_t>(XB + o) >> 1) & 3u) << (4 * i);
+        if constexpr (EDGES) {
+          const uint32_t head = (uint32_t)reinterpret_cast<uintptr_t>(XB) & 7u;
+          if (nc > 0 && item_at_edge(o, head, (uint32_t)(g.N * g.C) * plane, item_span(plane, CH))) {
+#pragma unroll
+            for (int e = 0; e < CH; ++e, o += plane) {
+              unsigned long long px = 0;
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                if (e < nc && k < npx[i])
+                  px |= (unsigned long long)__ldg(reinterpret_cast<const unsigned short*>(XB + o) + k) << (16 * k);
+              // where the two words around them would hold them
+              const uint32_t by = ((head + o) & 6u) * 8u;
+              const unsigned long long w0 = px << by, w1 = by ? px >> (64 - by) : 0;
+              s.w[i][e][0] = make_uint2((uint32_t)w0, (uint32_t)(w0 >> 32));
+              s.w[i][e][NW - 1] = make_uint2((uint32_t)w1, (uint32_t)(w1 >> 32));
+            }
+            continue;
+          }
+        }
 #pragma unroll
         for (int e = 0; e < CH; ++e, o += plane) {
           const bool on = e < nc;
@@ -1366,10 +1410,11 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         if (g.fC == 3 && g.fS == 7) ok = produce_fold<CG, F, 3, 7>(cv, smem, sh, tid, group, ustep, tp, TS, err);
         else ok = produce_fold<CG, F, 0, 0>(cv, smem, sh, tid, group, ustep, tp, TS, err);
       } else {
-        const bool aligned = input_aligned(g.H * g.W, cv.x);
+        const bool aligned = !Src::edges && input_aligned(g.H * g.W, cv.x);
         const bool one = stage_items(g, aligned, F::SPLIT_REGS) <= Ro::NPROD;
         constexpr int MORE = MAXITEMS / Ro::NPROD;   // items a producer may own
-#define SC_PRODUCE(ni, al, strd) ok = produce<CG, F, ni, al, strd>(cv, smem, sh, tid, group, done, turn, ustep, tp, TS, set, err)
+#define SC_PRODUCE(ni, al, strd) \
+  ok = produce<CG, F, ni, al, strd, Src::edges && !al>(cv, smem, sh, tid, group, done, turn, ustep, tp, TS, set, err)
         if constexpr (Src::kind == PLAIN) {
           if (src.strided()) {
             if (aligned && one) SC_PRODUCE(1, true, true);

@@ -273,8 +273,10 @@ static bool wino_contract(const problem_t& pr) {
 }
 
 // Problems whose slot 3 keeps the two-stage route's kernel, which hosts the
-// one-CTA shift schedule.
-static bool hosts_shift(const problem_t& pr) { return pr.c <= 256 && wino_contract(pr) && two_stage_fits(pr); }
+// one-CTA shift schedule (for inputs of whole 8-byte words).
+static bool hosts_shift(const problem_t& pr) {
+  return pr.c <= 256 && (reinterpret_cast<uintptr_t>(pr.in) & 7) == 0 && wino_contract(pr) && two_stage_fits(pr);
+}
 
 static ShiftPlan plan_shift(const problem_t& pr, int oh, int ow) {
   const ShiftPlan none{0, nullptr};
