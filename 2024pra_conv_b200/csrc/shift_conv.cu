@@ -29,32 +29,32 @@ __global__ void __launch_bounds__(128) shift_weight_u_batch_kernel(const __grid_
 // One CTA a unit (128 positions, up to 128 output channels).
 template <bool EDGES>
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_kernel(KernelParam p) {
-  shift_conv_body<1, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, sc::NOEPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // A pair of CTAs a unit (256 positions, up to 256 output channels).
 template <bool EDGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_pair_kernel(KernelParam p) {
-  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::NOEPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same for problems whose filter columns became channels.
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_kernel(KernelParam p) {
-  shift_conv_body<1, sc::Wide, sc::NOEPI>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<1, sc::NOEPI>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1) shift_conv_fold_pair_kernel(KernelParam p) {
-  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::NOEPI>(sc::OneConv<sc::FOLDED>{p}, sc::Epi{}, &g_shift_err);
 }
 
 // The same with the fused epilogue.
 template <int EPI, bool EDGES>
 __global__ void __launch_bounds__(sc::NTHREAD, 1) shift_conv_epi_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<1, sc::Wide, EPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, e, &g_shift_err);
+  shift_conv_body<1, EPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, e, &g_shift_err);
 }
 template <int EPI, bool EDGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_epi_pair_kernel(KernelParam p, sc::Epi e) {
-  shift_conv_body<2, sc::Wide, EPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, e, &g_shift_err);
+  shift_conv_body<2, EPI>(sc::OneConv<sc::PLAIN, EDGES>{p}, e, &g_shift_err);
 }
 template <int CG, bool EDGES>
 static const void* epi_kernel(bool even) {
@@ -70,7 +70,7 @@ static const void* epi_kernel(bool even) {
 // and spilled).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(sc::NTHREAD, 1)
     shift_conv_batch_kernel(const __grid_constant__ ShiftTable t) {
-  shift_conv_body<2, sc::Wide, sc::NOEPI>(sc::ConvTable{t}, sc::Epi{}, &g_shift_err);
+  shift_conv_body<2, sc::NOEPI>(sc::ConvTable{t}, sc::Epi{}, &g_shift_err);
 }
 
 }  // namespace wino
@@ -95,13 +95,13 @@ size_t wino_shift_weight_bytes(const KernelParam* p, int cg) { return sc::weight
 unsigned wino_shift_weight_grid(const KernelParam* p, int cg) {
   return (unsigned)((wino_shift_weight_bytes(p, cg) / 16 + 255) / 256);
 }
-int wino_shift_threads(int hosted) { return hosted ? sc::NTHREAD_HOSTED : sc::NTHREAD; }
+int wino_shift_threads() { return sc::NTHREAD; }
 int wino_shift_smem_bytes() { return sc::SMEM_BYTES; }
 
 // CTAs a unit for a problem (1 or 2), or 0 when the kernel does not take it:
 // strides past 2, more than MAXTAP taps, a position tile whose pixels exceed
 // the producers' items, fewer than two stages, or indices past 32 bits.
-static int shift_cg(const KernelParam* p, bool full_pairs) {
+int wino_shift_cg(const KernelParam* p) {
   if (p->u > 2 || p->v > 2 || p->r * p->s > sc::MAXTAP) return 0;
   const sc::Plan g1 = sc::make_plan(*p, 1), g2 = sc::make_plan(*p, 2);
   if (g1.npos + 4096 >= (1LL << 31) || g1.GX >= (1 << 15) || g1.GY >= (1 << 15)) return 0;
@@ -110,7 +110,7 @@ static int shift_cg(const KernelParam* p, bool full_pairs) {
     return 0;
   const bool aligned = sc::input_aligned(p->h * p->w, p->pin);
   for (const sc::Plan* g : {&g1, &g2})
-    if ((!g->fold && sc::stage_items(*g, aligned, false) > sc::MAXITEMS) || g->nstage < 2 || g->rows > sc::MAXROWS || g->nu > 2 ||
+    if ((!g->fold && sc::stage_items(*g, aligned) > sc::MAXITEMS) || g->nstage < 2 || g->rows > sc::MAXROWS || g->nu > 2 ||
         (g->fold && g->nst > 1))
       return 0;
   const long long w1 = (g1.units + sc::NSM - 1) / sc::NSM, w2 = (g2.units + sc::NSM / 2 - 1) / (sc::NSM / 2);
@@ -119,7 +119,7 @@ static int shift_cg(const KernelParam* p, bool full_pairs) {
   // K128 14.1 us alone, 15.5 in pairs); from the second wave on pairs win though
   // some idle (N64 C256 14x14 K256 31.2 / 24.7; N64 C256 28x28 K256 stride 2
   // 55.5 / 34.9; N128 C512 7x7 K512 52.3 / 36.1)
-  if (g2.units < sc::NSM / 2 && (w1 == 1 || full_pairs)) return 1;
+  if (g2.units < sc::NSM / 2 && w1 == 1) return 1;
   // narrow outputs: a pair's halved weights gain nothing there and the tiles of
   // one CTA balance better (3x3 N32 C64 56x56 K64 20.2 us alone, 22.6 in
   // pairs; 1x1 N32 C512 28x28 K128 16.3 / 20.6)
@@ -127,11 +127,6 @@ static int shift_cg(const KernelParam* p, bool full_pairs) {
   const long long t1 = w1 * sc::mma_cycles(1, g1.Kp < g1.NB ? g1.Kp : g1.NB), t2 = w2 * sc::mma_cycles(2, n2);
   return t2 <= t1 ? 2 : 1;
 }
-
-int wino_shift_cg(const KernelParam* p) { return shift_cg(p, false); }
-// ... where the one-CTA schedule runs in the kernel callers know the route by:
-// pairs only when they fill the device.
-int wino_shift_cg_hosted(const KernelParam* p) { return shift_cg(p, true); }
 
 // The packed plan the kernels read from the argument's transform_pin.
 unsigned long long wino_shift_pack(const KernelParam* p, int cg) { return sc::pack_plan(sc::make_plan(*p, cg)); }
@@ -143,9 +138,8 @@ static unsigned units_grid(const sc::Plan& g, int cg, int sms) {
 unsigned wino_shift_grid(const KernelParam* p, int cg, int sms) { return units_grid(sc::make_plan(*p, cg), cg, sms); }
 
 // Packed plan and both kernels' grids of a drop-in problem.
-unsigned long long wino_shift_slots(const KernelParam* p, int cg, int hosted, int sms, unsigned* grid,
-                                    unsigned* weight_grid) {
-  const sc::Plan g = sc::make_plan(*p, cg, hosted ? sc::TWOSTAGE : sc::OWN);
+unsigned long long wino_shift_slots(const KernelParam* p, int cg, int sms, unsigned* grid, unsigned* weight_grid) {
+  const sc::Plan g = sc::make_plan(*p, cg);
   *grid = units_grid(g, cg, sms);
   *weight_grid = (unsigned)((sc::weight_bytes(g, cg) / 16 + 255) / 256);
   return sc::pack_plan(g);
@@ -220,8 +214,8 @@ int wino_shift_fused_cg(const KernelParam* p) {
 // Whether a batch's table can hold a problem that wino_shift_fused_cg takes
 // (pairs): its producers own one item each, of words inside the input.
 int wino_shift_in_table(const KernelParam* p) {
-  return !sc::input_edges(*p) && sc::stage_items(sc::make_plan(*p, 2, sc::TABLE), sc::input_aligned(p->h * p->w, p->pin), false) <=
-         sc::Roles<sc::Wide>::NPROD;
+  return !sc::input_edges(*p) && sc::stage_items(sc::make_plan(*p, 2, sc::TABLE),
+                                                 sc::input_aligned(p->h * p->w, p->pin)) <= sc::NPROD;
 }
 
 int wino_launch_shift_weight_u(const KernelParam* p, int cg, cudaStream_t stream) {

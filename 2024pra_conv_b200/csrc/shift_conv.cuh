@@ -81,31 +81,13 @@ constexpr int NWARP_Z = 2;
 // for padding rows, then input producers in two groups of PW warps that take
 // alternate stages (or, strided, alternate channel halves of every stage).
 // Epilogue and producers are a few hundred instructions a turn which one warp
-// issues every ten cycles or so, so their number sets the pace: Wide runs 28
-// warps of 72 registers.  Hosted shares a kernel of 512 threads and 128
-// registers (twostage_conv.cu) and moves registers to its eight producer
-// warps, which own more and keep DEPTH stages of loads in flight.
-// Conv alone back to back, 16 warps -> 28: 1x1 N128 C64 56x56 K256 94 -> 66 us,
-// N32 C512 28x28 K128 23 -> 16, 3x3 N32 C64 56x56 K64 21.5 -> 20.2.
-struct Wide {
-  static constexpr int EW = 8, PW = 8, DEPTH = 1;
-  static constexpr bool SPLIT_REGS = false;
-};
-struct Hosted {
-  static constexpr int EW = 4, PW = 4, DEPTH = 2;
-  static constexpr bool SPLIT_REGS = true;
-  static constexpr int REGS_LAUNCH = 128, REGS_EPI = 112, REGS_MMA = 64, REGS_PROD = 168;
-};
-template <class F>
-struct Roles : F {
-  static constexpr int MMA = F::EW, LOAD = F::EW + 1, Z0 = F::EW + 2, P0 = F::EW + 4;
-  static constexpr int NPROD = F::PW * 32;   // producers of a group
-  static constexpr int NTHREAD = (P0 + 2 * F::PW) * 32;
-};
-constexpr int NTHREAD = Roles<Wide>::NTHREAD, NTHREAD_HOSTED = Roles<Hosted>::NTHREAD;
-static_assert(128 * Hosted::REGS_EPI + 128 * Hosted::REGS_MMA + 256 * Hosted::REGS_PROD ==
-                  NTHREAD_HOSTED * Hosted::REGS_LAUNCH,
-              "the warpgroups' register limits add up to the launch allocation");
+// issues every ten cycles or so, so their number sets the pace: 28 warps of 72
+// registers.  Conv alone back to back, 16 warps -> 28: 1x1 N128 C64 56x56 K256
+// 94 -> 66 us, N32 C512 28x28 K128 23 -> 16, 3x3 N32 C64 56x56 K64 21.5 -> 20.2.
+constexpr int EW = 8, PW = 8;
+constexpr int W_MMA = EW, W_LOAD = EW + 1, W_Z0 = EW + 2, W_P0 = EW + 4;
+constexpr int NPROD = PW * 32;            // producers of a group
+constexpr int NTHREAD = (W_P0 + 2 * PW) * 32;
 constexpr uint32_t SLEEP_NS = 32;
 constexpr int BYUNIT = 2;                 // stages a unit up to which producer groups alternate by unit
 // Producer items (a quad of pixels and eight channels, four where the input is
@@ -183,7 +165,7 @@ __host__ __device__ __forceinline__ int mma_cycles(int cg, int n) {
 }
 
 // What a kernel knows of its problems at compile time.
-enum Host : int { OWN, TWOSTAGE, TABLE };   // kernels the schedule runs in
+enum Host : int { OWN, TABLE };       // kernels the schedule runs in: one convolution's, a table's
 enum Kind : int { ANY, PLAIN, FOLDED, CONV33 };   // CONV33: 3x3 / stride 1 / pad 1
 
 template <int KIND = ANY>
@@ -233,9 +215,9 @@ __host__ __device__ __forceinline__ void plan_finish(Plan& g, int cg) {
 }
 
 // Items of a producer group and stage.
-__host__ __device__ __forceinline__ int stage_items(const Plan& g, bool aligned, bool hosted) {
+__host__ __device__ __forceinline__ int stage_items(const Plan& g, bool aligned) {
   const int eights = g.cps * g.qmax * (g.U > 1 || g.V > 1 ? 1 : 2);
-  return aligned || hosted ? eights : 2 * eights;
+  return aligned ? eights : 2 * eights;
 }
 
 // Plan of a problem for CG CTAs a unit (host; the rules).
@@ -285,9 +267,9 @@ __host__ inline Plan make_plan(const KernelParam& p, int cg, Host host = OWN) {
   for (;; cps >>= 1) {
     g.lcps = cps == 4 ? 2 : cps == 2 ? 1 : 0;
     plan_finish(g, cg);
-    // (a folded problem's unit is one stage; else an item a Wide producer, two
-    // of the smaller unaligned ones: N32 C512 7x7 K512 28.0 -> 25.1 us)
-    if (cps == 1 || g.fold || (stage_items(g, !odd, host == TWOSTAGE) <= (odd && host == OWN ? 512 : 256) &&
+    // (a folded problem's unit is one stage; else an item a producer, two of the
+    // smaller unaligned ones: N32 C512 7x7 K512 28.0 -> 25.1 us)
+    if (cps == 1 || g.fold || (stage_items(g, !odd) <= (odd && host == OWN ? 512 : 256) &&
                                (g.taps >= 6 ? 4 : 3) * (g.stageA + g.stageB) <= SMEM_STAGES))
       break;
   }
@@ -508,8 +490,8 @@ struct Slot {
   uint32_t shifts;                        // unaligned quads: first pixel's place in its 8-byte word, 4 bits an item
 };
 
-// Input producers with NI items a thread and stage, the loads of DEPTH (at
-// most four) of the group's stages in flight.  An item is (8-channel group of the
+// Input producers with NI items a thread and stage, one stage of loads ahead
+// of the stores.  An item is (8-channel group of the
 // stage, quad of the tile's pixel range), quads fastest, so a warp's loads
 // are 256-byte runs of a channel's plane.  ALIGNED: a quad is one 8-byte
 // word of every channel (input 8-byte aligned, H * W a multiple of 4);
@@ -523,15 +505,14 @@ struct Slot {
 // Strided, a stage's pixels are many and each group takes one channel half of
 // every stage.
 // EDGES: items whose words may reach outside the input load pixel by pixel.
-template <int CG, class F, int NI, bool ALIGNED, bool STRIDED, bool EDGES>
+template <int CG, int NI, bool ALIGNED, bool STRIDED, bool EDGES>
 __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int done, int turn,
                                         int ustep, int tile_pos, int tile_stride, bool& set, uint32_t* err) {
   const Plan& g = cv.g;
   const int u0 = cv.u0, cnt = cv.cnt;
   constexpr int NW = ALIGNED ? 1 : 2;     // 8-byte words per channel
-  constexpr int DEPTH = F::DEPTH, NPROD = Roles<F>::NPROD;
-  // channels of an item: two words a channel are many registers for Wide
-  constexpr int CH = ALIGNED || F::SPLIT_REGS ? 8 : 4;
+  // channels of an item: two words a channel are many registers
+  constexpr int CH = ALIGNED ? 8 : 4;
   volatile int* abort_flag = &sh.abort_flag;
   const unsigned short* X = cv.x;
   const int HW = g.H * g.W, ngrp = 2 * g.cps;
@@ -584,7 +565,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
   int entered = -1;
   const bool whole = (g.C & 15) == 0;     // no channel of a block is missing
   const char* XB = reinterpret_cast<const char*>(X);
-  Slot<NI, NW, CH> ring[DEPTH];
+  Slot<NI, NW, CH> slot;
   auto enter = [&]() {
     int pt, k0;
     unit_of(g, u0 + lu * ustep, pt, k0);
@@ -763,16 +744,14 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
     pos.next(g.nstage, by);
     return true;
   };
-  // Turn t stores the loads of DEPTH turns ago from its ring slot and issues
-  // new ones into it.  One loop body with a case per slot: unrolled over the
-  // slots, the unit entry above was compiled in seven times and its first
-  // pass through the instruction cache held the first stage up by 10 us.
+  // Turn t stores the loads of the turn before and issues new ones.  One loop
+  // body: unrolled, the unit entry above was compiled in several times and its
+  // first pass through the instruction cache held the first stage up by 10 us.
   const int total = STRIDED ? stages : ((by_unit ? cnt : stages) - (group ^ turn) + 1) / 2 * run;
-  // the first loads go out before the block's setup is complete
-  int slot = 0;
   bool ok = true;
-  for (int t = 0; ok && t < total + DEPTH; ++t) {
-    if (t == DEPTH && !set) {
+  for (int t = 0; ok && t <= total; ++t) {
+    // the first loads go out before the block's setup is complete
+    if (t == 1 && !set) {
       setup_sync<CG>();
       set = true;
     }
@@ -781,15 +760,8 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
       enter();
       entered = lu;
     }
-    auto turn = [&](Slot<NI, NW, CH>& s) {
-      if (t >= DEPTH) ok = consume(s);
-      if (more && ok) issue(s);
-    };
-    if (slot == 0) turn(ring[0]);
-    if (DEPTH > 1 && slot == 1) turn(ring[DEPTH > 1 ? 1 : 0]);
-    if (DEPTH > 2 && slot == 2) turn(ring[DEPTH > 2 ? 2 : 0]);
-    if (DEPTH > 3 && slot == 3) turn(ring[DEPTH > 3 ? 3 : 0]);
-    if (++slot == DEPTH) slot = 0;
+    if (t > 0) ok = consume(slot);
+    if (more && ok) issue(slot);
     int by = 1;
     if (--l_left == 0) { l_left = run; by += run; }
     for (lj += by; lj >= g.nst; lj -= g.nst) ++lu;
@@ -804,7 +776,7 @@ __device__ __forceinline__ bool produce(const Conv& cv, uint8_t* smem, Shared& s
 // its bytes take 9).  A unit is one stage and the groups
 // take alternate units.  FC, FS: channels and columns known at compile time
 // (0: as the plan says).
-template <int CG, class F, int FC, int FS>
+template <int CG, int FC, int FS>
 __device__ __forceinline__ bool produce_fold(const Conv& cv, uint8_t* smem, Shared& sh, int tid, int group, int ustep,
                                              int tile_pos, int tile_stride, uint32_t* err) {
   const Plan& g = cv.g;
@@ -820,7 +792,7 @@ __device__ __forceinline__ bool produce_fold(const Conv& cv, uint8_t* smem, Shar
     if (!wait_all_lanes(&sh.empty[pos.st], pos.phase, abort_flag, err, ERR_WAIT_EMPTY)) return false;
     uint8_t* dst = smem + pos.st * g.pitch;
 #pragma unroll 1
-    for (int r = tid; r < g.rows; r += Roles<F>::NPROD) {
+    for (int r = tid; r < g.rows; r += NPROD) {
       const int a = r >= plane0 ? 1 : 0;
       const Base c = advance(gr, b0, r - (a ? plane0 : 0));
       const int y = c.gy * g.U + a - g.P, x0 = c.gx * g.fV - g.fQ;
@@ -1205,10 +1177,9 @@ __device__ __forceinline__ void shift_weight_from_u(const KernelParam& p, const 
 // The kernel body.  CG = 2: clusters of two CTAs (__cluster_dims__(2, 1, 1)),
 // a unit is 256 positions, rank 0 issues the pair's MMAs.  Every role walks
 // the source's layers and its own units of each.
-template <int CG, class F, int EPI, class Src>
+template <int CG, int EPI, class Src>
 __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& epi, uint32_t* err) {
   using namespace sc;
-  using Ro = Roles<F>;
   extern __shared__ __align__(128) uint8_t shift_smem[];
   __shared__ Shared sh;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(shift_smem) + 127) & ~uintptr_t(127));
@@ -1224,18 +1195,18 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAXSTAGE; ++s) {
       // producers, padding, weights (and at a pair's rank 0 the peer's whole stage)
-      mbar_init(&sh.full[s], (src.strided() ? 2 : 1) * Ro::PW + NWARP_Z + 1 + (CG == 2 && rank == 0 ? 1 : 0));
+      mbar_init(&sh.full[s], (src.strided() ? 2 : 1) * PW + NWARP_Z + 1 + (CG == 2 && rank == 0 ? 1 : 0));
       mbar_init(&sh.empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&sh.accfull[a], 1);
-      mbar_init(&sh.accempty[a], CG * Ro::EW);
+      mbar_init(&sh.accempty[a], CG * EW);
     }
     mbar_init(&sh.mmadone, 1);
     sh.abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == Ro::MMA) {
+  if (warp == W_MMA) {
     if (CG == 2) { tmem_alloc_pair(&sh.tmem_base, 512); tmem_relinquish_pair(); }
     else { tmem_alloc(&sh.tmem_base, 512); tmem_relinquish(); }
   }
@@ -1244,10 +1215,9 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
   const int nl = src.layers();
   bool ok = true;
 
-  if (warp >= Ro::MMA && warp < Ro::P0) {
-    if constexpr (F::SPLIT_REGS) regs_dec<F::REGS_MMA>();
+  if (warp >= W_MMA && warp < W_P0) {
     setup_sync<CG>();
-    if (warp == Ro::LOAD) {
+    if (warp == W_LOAD) {
       // the stages' weights, one bulk copy each: this CTA's rows of the unit's
       // output channels
       if (lane == 0) {
@@ -1287,12 +1257,12 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
           for (int b = issued > nstage ? issued - nstage : 0; b < issued; ++b)
             mbar_wait(&sh.full[b % nstage], (b / nstage) & 1, nullptr, err, ERR_WAIT_FULL);
       }
-    } else if (warp >= Ro::Z0) {
+    } else if (warp >= W_Z0) {
       RingPos pos{0, 1};
       for (int l = 0; ok && l < nl; ++l) {
         Conv cv;
         if (src.get(l, CG, u0, ustep, cv))
-          ok = pad_rows(cv, smem, sh, threadIdx.x - Ro::Z0 * 32, ustep, tp, TS, pos, err);
+          ok = pad_rows(cv, smem, sh, threadIdx.x - W_Z0 * 32, ustep, tp, TS, pos, err);
       }
     } else {
       const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem_base, 0);
@@ -1332,14 +1302,13 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       }
     }
     __syncwarp();
-  } else if (warp < Ro::EW) {
-    if constexpr (F::SPLIT_REGS) regs_dec<F::REGS_EPI>();
+  } else if (warp < EW) {
     setup_sync<CG>();
     const uint32_t tmem = sh.tmem_base;
     // epilogue: TMEM lane 32 * quarter + lane = position of this CTA's tile;
     // a quarter's warps take alternate 32-column chunks
     const int quarter = warp & 3, part = warp >> 2;
-    constexpr int PARTS = Ro::EW / 4;
+    constexpr int PARTS = EW / 4;
     const uint32_t lead_accempty = mapa_shared(smem_u32(&sh.accempty[0]), 0);
     int unit = 0;
     for (int l = 0; ok && l < nl; ++l) {
@@ -1396,8 +1365,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       }
     }
   } else {
-    if constexpr (F::SPLIT_REGS) regs_inc<F::REGS_PROD>();
-    const int group = (warp - Ro::P0) / Ro::PW, tid = threadIdx.x - (Ro::P0 + group * Ro::PW) * 32;
+    const int group = (warp - W_P0) / PW, tid = threadIdx.x - (W_P0 + group * PW) * 32;
     int done = 0, turn = 0;               // stages of the layers before, whose turn the next run is
     bool set = false;                     // setup_sync passed
     for (int l = 0; ok && l < nl; ++l) {
@@ -1407,14 +1375,14 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
       if constexpr (Src::kind == FOLDED) {
         setup_sync<CG>();
         set = true;
-        if (g.fC == 3 && g.fS == 7) ok = produce_fold<CG, F, 3, 7>(cv, smem, sh, tid, group, ustep, tp, TS, err);
-        else ok = produce_fold<CG, F, 0, 0>(cv, smem, sh, tid, group, ustep, tp, TS, err);
+        if (g.fC == 3 && g.fS == 7) ok = produce_fold<CG, 3, 7>(cv, smem, sh, tid, group, ustep, tp, TS, err);
+        else ok = produce_fold<CG, 0, 0>(cv, smem, sh, tid, group, ustep, tp, TS, err);
       } else {
         const bool aligned = !Src::edges && input_aligned(g.H * g.W, cv.x);
-        const bool one = stage_items(g, aligned, F::SPLIT_REGS) <= Ro::NPROD;
-        constexpr int MORE = MAXITEMS / Ro::NPROD;   // items a producer may own
+        const bool one = stage_items(g, aligned) <= NPROD;
+        constexpr int MORE = MAXITEMS / NPROD;   // items a producer may own
 #define SC_PRODUCE(ni, al, strd) \
-  ok = produce<CG, F, ni, al, strd, Src::edges && !al>(cv, smem, sh, tid, group, done, turn, ustep, tp, TS, set, err)
+  ok = produce<CG, ni, al, strd, Src::edges && !al>(cv, smem, sh, tid, group, done, turn, ustep, tp, TS, set, err)
         if constexpr (Src::kind == PLAIN) {
           if (src.strided()) {
             if (aligned && one) SC_PRODUCE(1, true, true);
@@ -1427,12 +1395,9 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
         if (Src::table) {
           if (aligned) SC_PRODUCE(1, true, false);
           else SC_PRODUCE(1, false, false);
-        } else if (F::SPLIT_REGS && !one && stage_items(g, aligned, true) <= 2 * Ro::NPROD) {
-          if (aligned) SC_PRODUCE(2, true, false);
-          else SC_PRODUCE(2, false, false);
         } else if (aligned && one) SC_PRODUCE(1, true, false);
         else if (aligned) SC_PRODUCE(MORE, true, false);
-        else if (F::SPLIT_REGS || one) SC_PRODUCE(1, false, false);
+        else if (one) SC_PRODUCE(1, false, false);
         else SC_PRODUCE(MORE, false, false);
 #undef SC_PRODUCE
       }
@@ -1446,7 +1411,7 @@ __device__ __forceinline__ void shift_conv_body(const Src& src, const sc::Epi& e
   // the peer may still read this CTA's shared memory or arrive on its
   // barriers until both CTAs get here
   if (CG == 2) cluster_sync();
-  if (warp == Ro::MMA) {
+  if (warp == W_MMA) {
     tc_fence_after();
     if (CG == 2) tmem_dealloc_pair(sh.tmem_base, 512);
     else tmem_dealloc(sh.tmem_base, 512);

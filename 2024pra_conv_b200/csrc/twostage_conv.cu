@@ -66,7 +66,6 @@
 #include "tc_sm100.cuh"
 #include "wino_common.cuh"
 #include "vgen.cuh"
-#include "shift_conv.cuh"
 
 // Load instruction of the tap-pair producers' window words: through L1
 // (ld.global.nc) by default, or cached in L2 only (ld.global.cg).
@@ -1177,19 +1176,12 @@ __device__ __forceinline__ Prod prod(const Geo& g, const uint8_t* xr, int t, int
 // output channel) U scale su (p.pweight, fp32 [16][K]) before rounding M.
 // F8 = 1: single e4m3 terms (one MMA per K-step, one byte per tile and
 // channel, a K-step of 32 channels per piece).
-// The fp16 bulk-copy variant, launched without a mid_result, computes outputs
-// instead of M: the one-CTA shift-reuse implicit GEMM (shift_conv.cuh), which
-// needs no M and no pre-pass (transform_pin then carries its packed plan).
+// Launched without an M (mid_result) the fp16 bulk-copy variant has nothing to
+// do: the drop-in's shift route leaves it in its slot that way.
 template <bool TMAV, int F8 = 0>
-__global__ void __launch_bounds__(TMAV && F8 ? trs::NTHREAD_V : trs::NTHREAD, 1) twostage_res_kernel_t(KernelParam p) {
+__global__ void __launch_bounds__(TMAV ? trs::NTHREAD_V : trs::NTHREAD, 1) twostage_res_kernel_t(KernelParam p) {
   static_assert(F8 == 0 || TMAV, "the fp8 variants read V2 by bulk copy");
-  static_assert(trs::NTHREAD == sc::NTHREAD_HOSTED && sc::SMEM_BYTES <= 227 * 1024, "one kernel hosts both schedules");
-  if constexpr (TMAV && F8 == 0) {
-    if (p.mid_result == nullptr) {
-      shift_conv_body<1, sc::Hosted, sc::NOEPI>(sc::OneConv<sc::CONV33>{p}, sc::Epi{}, &g_twostage_err);
-      return;
-    }
-  }
+  if (TMAV && F8 == 0 && p.mid_result == nullptr) return;
   constexpr int TERMS = F8 == 1 ? 1 : 2;        // bytes per tile and channel in V2 and U
   using namespace trs;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1936,7 +1928,7 @@ __global__ void __launch_bounds__(ot::NTHREAD, WINO_OT_MINB) twostage_output_ker
   using namespace ts;
   extern __shared__ __align__(128) uint8_t osm[];
   __shared__ uint64_t full[ot::NBUF];
-  if (p.mid_result == nullptr) return;    // slot 3 wrote the outputs itself
+  if (p.mid_result == nullptr) return;    // the outputs are there already (the drop-in's shift route)
   const int K = p.k, P = p.Oh, Q = p.Ow;
   const int TP = (P + 1) >> 1, TQ = (Q + 1) >> 1;
   const long long NT = (long long)p.n * TP * TQ;
@@ -2133,7 +2125,7 @@ static int twostage_prepare_device() {
   if (cudaFuncSetAttribute(twostage_res_kernel_t<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            trs::SMEM_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(twostage_res_kernel_t<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           sc::SMEM_BYTES > trs::SMEM_BYTES ? sc::SMEM_BYTES : trs::SMEM_BYTES) != cudaSuccess ||
+                           trs::SMEM_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(twostage_res_kernel_t<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            trs::SMEM_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(twostage_res_kernel_t<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2143,8 +2135,6 @@ static int twostage_prepare_device() {
   // launched with; any other launch count would leave an increase waiting
   cudaFuncAttributes fa{};
   if (cudaFuncGetAttributes(&fa, twostage_res_kernel_t<false>) != cudaSuccess || fa.numRegs != trs::REGS_LAUNCH)
-    return 1;
-  if (cudaFuncGetAttributes(&fa, twostage_res_kernel_t<true>) != cudaSuccess || fa.numRegs != sc::Hosted::REGS_LAUNCH)
     return 1;
   return (int)cudaFuncSetAttribute(twostage_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    tp::SMEM_BYTES);

@@ -83,6 +83,7 @@ int wino_launch_filter_transform(const void* weight, void* ucache, void* ucache_
 void* wino_dropin_filter_u2_kernel_ptr();
 void* wino_twostage_gemm_kernel_ptr_for(int c);
 void* wino_twostage_output_kernel_ptr();
+void* wino_twostage_resv_kernel_ptr();
 int wino_twostage_threads_for(int c);
 int wino_twostage_smem_bytes_for(int c);
 int wino_twostage_prepare();
@@ -113,13 +114,11 @@ int wino_igemm_shape_ok(int n, int c, int h, int w, int k, int oh, int ow);
 int wino_igemm_prepare();
 uint32_t wino_igemm_error_read_clear();
 int wino_shift_cg(const wino::KernelParam* p);
-int wino_shift_cg_hosted(const wino::KernelParam* p);
-unsigned long long wino_shift_slots(const wino::KernelParam* p, int cg, int hosted, int sms, unsigned* grid,
-                                    unsigned* weight_grid);
+unsigned long long wino_shift_slots(const wino::KernelParam* p, int cg, int sms, unsigned* grid, unsigned* weight_grid);
 size_t wino_shift_weight_bytes(const wino::KernelParam* p, int cg);
 void* wino_shift_weight_kernel_ptr(int cg);
 void* wino_shift_kernel_ptr(const wino::KernelParam* p, int cg);
-int wino_shift_threads(int hosted);
+int wino_shift_threads();
 int wino_shift_smem_bytes();
 int wino_shift_prepare();
 uint32_t wino_shift_error_read_clear();
@@ -272,10 +271,12 @@ static bool wino_contract(const problem_t& pr) {
          pr.transform_filter != nullptr;
 }
 
-// Problems whose slot 3 keeps the two-stage route's kernel, which hosts the
-// one-CTA shift schedule (for inputs of whole 8-byte words).
-static bool hosts_shift(const problem_t& pr) {
-  return pr.c <= 256 && (reinterpret_cast<uintptr_t>(pr.in) & 7) == 0 && wino_contract(pr) && two_stage_fits(pr);
+// Problems that the shift route leaves the two-stage route's kernels in slots 3
+// and 4, by which callers tell a problem that route fits; given no mid_result
+// they have nothing to do.
+static bool keeps_two_stage_slots(const problem_t& pr) {
+  return wino_twostage_gemm_kernel_ptr_for((int)pr.c) == wino_twostage_resv_kernel_ptr() && wino_contract(pr) &&
+         two_stage_fits(pr);
 }
 
 static ShiftPlan plan_shift(const problem_t& pr, int oh, int ow) {
@@ -290,7 +291,7 @@ static ShiftPlan plan_shift(const problem_t& pr, int oh, int ow) {
   p.n = (short)pr.n; p.c = (short)pr.c; p.h = (short)pr.h; p.w = (short)pr.w; p.k = (short)pr.k;
   p.r = (short)pr.r; p.s = (short)pr.s; p.u = (short)pr.u; p.v = (short)pr.v; p.p = (short)pr.p; p.q = (short)pr.q;
   p.Oh = (short)oh; p.Ow = (short)ow;
-  int cg = hosts_shift(pr) ? wino_shift_cg_hosted(&p) : wino_shift_cg(&p);
+  int cg = wino_shift_cg(&p);
   if (cg == 0) return none;
   // weight operand: the caller's transform_filter (16*k*c fp16), else its
   // transform_pin (4*h*h*n*c fp16); reference src/main.cpp:36-38
@@ -361,11 +362,7 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
   std::memset(kernelInfo, 0, sizeof(*kernelInfo));
 
   if (shift.cg != 0) {
-    if (wino_shift_prepare() != 0 || wino_twostage_prepare() != 0) return WINO_ECUDA;
-    // Problems of the two-stage route keep its slot 3 and 4 kernels, by which
-    // callers tell the route: given no mid_result, its GEMM kernel runs the
-    // one-CTA shift schedule and its output transform has nothing to do.
-    const bool hosted = shift.cg == 1 && hosts_shift(pr);
+    if (wino_shift_prepare() != 0) return WINO_ECUDA;
     a->transform_filter = static_cast<_Float16*>(shift.wop);
     a->mid_result = nullptr;
     wino::KernelParam* kp = static_cast<wino::KernelParam*>(param);
@@ -373,18 +370,21 @@ int getkernelInfo(problem_t* problem, kernelInfo_t* kernelInfo, void* param) {
     // pointer in
     unsigned grid = 0, weight_grid = 0;
     kp->transform_pin =
-        reinterpret_cast<void*>(wino_shift_slots(kp, shift.cg, hosted, sm_count(), &grid, &weight_grid));
+        reinterpret_cast<void*>(wino_shift_slots(kp, shift.cg, sm_count(), &grid, &weight_grid));
     set_slot(kernelInfo, 1, weight_grid, 1, 1, 256, 1, 1, 0,
              wino_shift_weight_kernel_ptr(shift.cg));
-    set_slot(kernelInfo, 2, 1, 1, 1, 32, 1, 1, 0, wino_noop_kernel_ptr());
-    set_slot(kernelInfo, 3, grid, 1, 1, (unsigned)wino_shift_threads(hosted), 1, 1,
-             (unsigned)wino_shift_smem_bytes(),
-             hosted ? wino_twostage_gemm_kernel_ptr_for((int)pr.c) : wino_shift_kernel_ptr(kp, shift.cg));
-    if (hosted)
+    const bool keeps = keeps_two_stage_slots(pr);
+    set_slot(kernelInfo, keeps ? 2 : 3, grid, 1, 1, (unsigned)wino_shift_threads(), 1, 1,
+             (unsigned)wino_shift_smem_bytes(), wino_shift_kernel_ptr(kp, shift.cg));
+    if (keeps) {
+      set_slot(kernelInfo, 3, 1, 1, 1, (unsigned)wino_twostage_threads_for((int)pr.c), 1, 1, 0,
+               wino_twostage_gemm_kernel_ptr_for((int)pr.c));
       set_slot(kernelInfo, 4, 1, 1, 1, (unsigned)wino_twostage_output_threads(), 1, 1, 0,
                wino_twostage_output_kernel_ptr());
-    else
+    } else {
+      set_slot(kernelInfo, 2, 1, 1, 1, 32, 1, 1, 0, wino_noop_kernel_ptr());
       set_slot(kernelInfo, 4, 1, 1, 1, 32, 1, 1, 0, wino_noop_kernel_ptr());
+    }
     return WINO_OK;
   }
   if (route == WINO_ROUTE_IGEMM) {
@@ -840,10 +840,12 @@ extern "C" int wino_launch_kernelinfo(const void* kiv, void* param, void* stream
   const unsigned* slots[4] = {&ki->blockx1, &ki->blockx2, &ki->blockx3, &ki->blockx4};
   void* const fns[4] = {ki->kernelPtr1, ki->kernelPtr2, ki->kernelPtr3, ki->kernelPtr4};
   // slots whose kernel has nothing to do are not launched: the empty kernel,
-  // and the two-stage output transform without an M
+  // and the two-stage GEMM and output transform without an M
   const bool no_m = static_cast<const wino::KernelParam*>(param)->mid_result == nullptr;
+  const bool shift = fns[0] == wino_shift_weight_kernel_ptr(1) || fns[0] == wino_shift_weight_kernel_ptr(2);
   for (int i = 0; i < 4; ++i) {
-    if (fns[i] == wino_noop_kernel_ptr() || (no_m && fns[i] == wino_twostage_output_kernel_ptr())) continue;
+    if (fns[i] == wino_noop_kernel_ptr()) continue;
+    if (no_m && (fns[i] == wino_twostage_resv_kernel_ptr() || fns[i] == wino_twostage_output_kernel_ptr())) continue;
     const unsigned* b = slots[i];
     const dim3 grid(b[0], b[1], b[2]), block(b[3], b[4], b[5]);
     // the shift kernel starts beside the weight kernel launched right before
@@ -851,7 +853,7 @@ extern "C" int wino_launch_kernelinfo(const void* kiv, void* param, void* stream
     // nothing of its filter transform, and the fused kernel waits for both
     const bool xb = fns[1] == wino_xb_layout_kernel_ptr() && fns[0] == wino_dropin_filter_kernel_ptr();
     const bool dependent =
-        (i == 2 && (fns[0] == wino_shift_weight_kernel_ptr(1) || fns[0] == wino_shift_weight_kernel_ptr(2))) ||
+        (shift && (i == 1 || i == 2)) ||
         (xb && (i == 1 || (i == 2 && fns[2] == wino_fused_kernel_ptr())));
     const int e = dependent ? wino_launch_dependent(fns[i], grid, block, (void**)&param, (size_t)b[6], (cudaStream_t)stream)
                             : (int)cudaLaunchKernel(fns[i], grid, block, (void**)&param, (size_t)b[6],

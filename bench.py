@@ -390,9 +390,9 @@ def run_ours(args, rank, world, local_rank):
     layout_us = layout_ms / iters * 1e3         # pre-pass alone
     # the route getkernelInfo chose for the timed drop-in step
     shift = wino.lib().wino_dropin_route(ctypes.byref(pr)) == wino.ROUTE_SHIFT
-    if shift:                                    # slot 3 alone, on the operand the steps left
+    if shift:                                    # the conv alone, on the operand the steps left
         conv = wino.KernelInfo.from_buffer_copy(ki)
-        conv.kernelPtr1 = ki.kernelPtr2          # the empty slot's kernel: not launched
+        conv.kernelPtr1 = ki.kernelPtr4          # a kernel with nothing to do: not launched
         conv_ms, _ = timed(lambda: wino.launch_kernel_info(conv, param, stream), iters)
         kernel_us = conv_ms / iters * 1e3
     else:

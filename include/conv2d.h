@@ -31,7 +31,10 @@
  *         slot 1  weight -> transform_filter (tensor-core operand; to
  *                 transform_pin where it does not fit there)
  *         slot 3  shift-reuse implicit GEMM reading `in` directly -> out;
- *                 slots 2, 4 have nothing to do.
+ *                 slots 2, 4 have nothing to do.  Where the problem is one
+ *                 that the two-stage route below fits (c <= 256) the conv is
+ *                 in slot 2 instead, and slots 3 and 4 hold that route's
+ *                 kernels, which find no M and return.
  *       mid_result is left untouched, and so is transform_pin unless it holds
  *       the weights.  For smaller problems, and what this route does not
  *       take:
