@@ -282,9 +282,12 @@ static bool keeps_two_stage_slots(const problem_t& pr) {
 static ShiftPlan plan_shift(const problem_t& pr, int oh, int ow) {
   const ShiftPlan none{0, nullptr};
   if (!pr.transform_filter) return none;
-  // strided 1x1 stays with the gathering implicit GEMM, which reads only the
-  // rows it needs (N32 C256 56x56 K128 / 2: 23 us against 29)
-  if (pr.r * pr.s == 1 && (pr.u > 1 || pr.v > 1)) return none;
+  // strided filters of one or two taps stay with the gathering implicit GEMM,
+  // which reads only the pixels it needs, where this kernel loads every one for
+  // a few MMAs (1x1/2 N32 C256 56x56 K128 23 us against 29; 1x2/2 N60 C16
+  // 137x137 K64 50 against 73; 2x1/2 N29 C256 67x67 K128 58 against 83).  From
+  // three taps on it wins (3x1/2 N9 C256 42x42 K64 67 against 30)
+  if (pr.r * pr.s <= 2 && (pr.u > 1 || pr.v > 1)) return none;
   if (2.0 * pr.n * pr.k * oh * ow * pr.c * pr.r * pr.s < kShiftMinFlops) return none;
   wino::KernelParam p{};
   p.pin = pr.in;

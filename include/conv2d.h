@@ -25,7 +25,8 @@
  *     kernels go in the slots depends on the shape and on which workspaces
  *     are usable (wino_dropin_route in winoconv.h reports the choice):
  *
- *     shift route: any filter of up to 64 taps with strides 1 or 2 (1x1: 1)
+ *     shift route: any filter of up to 64 taps with strides 1 or 2 (of one or
+ *       two taps: stride 1)
  *       from 64 MFLOP on (2*n*k*Oh*Ow*c*r*s; a position tile's input must fit
  *       the kernel's shared memory, in practice w up to about 400):
  *         slot 1  weight -> transform_filter (tensor-core operand; to

@@ -56,7 +56,7 @@ int wino_check_shape(int n, int c, int h, int w, int k);
  * 4*k*h*w*n fp16 to hold 16*k*tiles, i.e. even h and w), or the tensor-core
  * implicit GEMM for shapes outside the Winograd contract (weights re-laid
  * out into transform_filter, which must hold wino_igemm_weight_bytes).
- * Problems of at least 64 MFLOP (direct count) with strides up to 2 (1x1: 1)
+ * Problems of at least 64 MFLOP (direct count) with strides up to 2 (of one or two taps: 1)
  * take the shift-reuse implicit GEMM instead (reported as
  * WINO_ROUTE_SHIFT inside the Winograd contract, as the implicit GEMM outside
  * it), whose weight operand goes to transform_filter or, where it does not

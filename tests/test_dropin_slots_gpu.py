@@ -77,3 +77,26 @@ def test_two_stage_route_below_the_threshold(wino, cuda, shape):
     ref = torch.nn.functional.conv2d(x.double(), wt.double(), padding=1)
     assert float((y.double() - ref).norm() / ref.norm()) <= 2e-3
     assert wino.error_read_clear() == 0
+
+
+@pytest.mark.parametrize("r,s,stride,shift", [(1, 1, 2, False), (1, 2, 2, False), (2, 1, 2, False), (3, 1, 2, True),
+                                              (1, 2, 1, True), (2, 1, 1, True)])
+def test_strided_filters_of_two_taps_gather(wino, cuda, r, s, stride, shift):
+    """They read few of the pixels: the implicit GEMM that gathers them serves
+    strided filters of up to two taps, the shift kernel the others."""
+    import torch
+    gen = torch.Generator(device=cuda).manual_seed(r + 8 * s)
+    x = torch.randn((10, 32, 61, 58), device=cuda, generator=gen).half()
+    wt = (torch.randn((128, 32, r, s), device=cuda, generator=gen) / (32 * r * s) ** 0.5).half()
+    ws = wino.DropinWorkspaces(10, 32, 61, 58, 128, cuda)
+    oh, ow = (61 - r) // stride + 1, (58 - s) // stride + 1
+    y = torch.empty((10, 128, oh, ow), dtype=torch.float16, device=cuda)
+    pr = wino.make_problem(x, wt, y, ws.transform_pin, ws.transform_filter, ws.mid_result, r=r, s=s, u=stride, v=stride,
+                           p=0, q=0)
+    rc, ki = wino.get_kernel_info(pr, (ctypes.c_char * wino.get_param_size(pr))())
+    assert rc == 0
+    assert (ki.slot(3)["lds"] == wino.lib().wino_shift_smem_bytes()) is shift
+    y = wino.dropin_conv2d(x, wt, ws=ws, stride=stride, pad=0)
+    torch.cuda.synchronize()
+    base._check(y, x, wt, stride, 0, 0)
+    assert wino.error_read_clear() == 0
