@@ -312,7 +312,14 @@ struct Batch {
     return WINO_OK;
   }
 
-  int run(cudaStream_t s) {
+  // Whether both the shift kernel and the fused kernel serve layers.
+  bool mixed() const {
+    return total > 0 && std::any_of(layers.begin(), layers.end(), [&](const Layer& L) { return on_shift(L); });
+  }
+
+  // All layers on `s`; the shift kernel's on `side` where that is another
+  // stream, forked from `s` and joined to it by the caller.
+  int run(cudaStream_t s, cudaStream_t side) {
     if (dirty) return WINO_EINVAL;  // commit first (outside any capture)
     for (int li : order) {
       const Layer& L = layers[li];
@@ -327,15 +334,35 @@ struct Batch {
     bool beside = false;
     for (int li : order)
       if (on_shift(layers[li]) && !layers[li].table) {
-        if (run_shift(layers[li], s) != WINO_OK) return WINO_ECUDA;
-        beside = true;
+        if (run_shift(layers[li], side) != WINO_OK) return WINO_ECUDA;
+        beside = side == s;
       }
     if (shift.nlayers > 0) {
-      if (wino_launch_shift_batch(&shift, sm_count(), s) != 0) return WINO_ECUDA;
-      beside = true;
+      if (wino_launch_shift_batch(&shift, sm_count(), side) != 0) return WINO_ECUDA;
+      beside = side == s;
     }
     if (total == 0) return WINO_OK;           // no layer on the fused Winograd kernel
     return wino_fused_launch_batch(table_dev, total, grid_for(total), beside, s) == 0 ? WINO_OK : WINO_ECUDA;
+  }
+  int run(cudaStream_t s) { return run(s, s); }
+
+  // run() into the capture that `s` is in, with the shift kernel's layers on a
+  // branch of their own beside the pre-passes and the fused kernel.  Small
+  // batches of both kinds are as long as the fused kernel's longest chain of
+  // blocks; behind the shift kernel's two launches it started late (us a
+  // replay; before this kernel took layers, one branch, two: N2, the set's 12
+  // layers 80, 88, 76; its layers 7 and 8 51, 55, 53; N1 + 1 pixel, 12 layers 70, 74, 73).
+  int run_forked(cudaStream_t s, cudaStream_t side) {
+    cudaEvent_t fork = nullptr, join = nullptr;
+    bool ok = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
+              cudaEventCreateWithFlags(&join, cudaEventDisableTiming) == cudaSuccess &&
+              cudaEventRecord(fork, s) == cudaSuccess && cudaStreamWaitEvent(side, fork, 0) == cudaSuccess;
+    const int rc = ok ? run(s, side) : (int)WINO_ECUDA;
+    // joined after a failed launch too: a capture must not end with a branch open
+    ok = ok && cudaEventRecord(join, side) == cudaSuccess && cudaStreamWaitEvent(s, join, 0) == cudaSuccess;
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    return rc != WINO_OK ? rc : ok ? (int)WINO_OK : (int)WINO_ECUDA;
   }
 };
 
@@ -637,7 +664,7 @@ int wino_batch_tune(void* h, int reps, float* layer_us, float* order_us, void* s
 }
 
 // Capture one run (pre-passes + the persistent launch) into a CUDA graph.
-// The capture uses a stream of its own (the legacy default stream cannot be
+// The capture uses streams of its own (the legacy default stream cannot be
 // captured); the graph may then be launched on any stream.  `stream` is
 // accepted for symmetry and unused.
 int wino_batch_graph_capture(void* h, void* stream) {
@@ -649,15 +676,19 @@ int wino_batch_graph_capture(void* h, void* stream) {
   if (wino_fused_prepare_batch() != 0) return WINO_ECUDA;
   if (b->settle() != WINO_OK) return WINO_ECUDA;  // the old graph may still be running
   b->drop_graph();
-  cudaStream_t s = nullptr;
+  cudaStream_t s = nullptr, side = nullptr;
+  const bool fork = b->mixed();
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return WINO_ECUDA;
-  if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+  if ((fork && cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) ||
+      cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+    if (side) cudaStreamDestroy(side);
     cudaStreamDestroy(s);
     return WINO_ECUDA;
   }
-  rc = b->run(s);
+  rc = fork ? b->run_forked(s, side) : b->run(s);
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(s, &g);
+  if (side) cudaStreamDestroy(side);
   cudaStreamDestroy(s);
   if (rc != WINO_OK || e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);

@@ -1,0 +1,46 @@
+"""Batches whose layers take both the shift kernel and the fused kernel: a capture
+runs them as two branches, which a replay joins before what follows it."""
+import pytest
+
+import test_shift_conv as base
+
+pytestmark = pytest.mark.gpu
+
+# n, c, h, w, k: 925 MFLOP (the shift kernel's table), 578 MFLOP of rows too long for
+# it (a launch of its own), small layers of the fused kernel
+SHAPES = [(2, 64, 56, 56, 128), (1, 16, 40, 224, 224), (2, 512, 7, 7, 512), (2, 32, 15, 15, 48)]
+
+
+@pytest.mark.parametrize("picks", [(0, 2, 3), (0, 1, 2), (1, 3), (0, 1)])
+def test_replays_join_before_what_follows(wino, cuda, picks):
+    import torch
+    cases = [base._fused_case(cuda, SHAPES[i], 30 + i) for i in picks]
+    b, layers = wino.Batch(), []
+    for x, wt, _, res in cases:
+        n, c, h, w = x.shape
+        k = wt.shape[0]
+        ws = torch.empty(wino.fused_conv_workspace_bytes(n, c, h, w, k), dtype=torch.uint8, device=cuda)
+        y, u = torch.empty_like(res), wino.filter_transform(wt)
+        b.add(x, u, k, y, workspace=ws)
+        layers.append((x, u, k, y))
+    torch.cuda.synchronize()
+    b.capture()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = []
+    for i in range(6):
+        # inputs rewritten and outputs read on the replay's stream, no other wait
+        s = streams[i & 1]
+        s.wait_stream(streams[1 - (i & 1)])
+        with torch.cuda.stream(s):
+            for x, _, _, _ in layers:
+                x.mul_(-0.5)
+            b.launch(stream=s)
+            got.append([(x.clone(), y.clone()) for x, _, _, y in layers])
+            for _, _, _, y in layers:
+                y.fill_(float("nan"))
+    torch.cuda.synchronize()
+    for pass_ in got:
+        for (_, u, k, _), (x, y) in zip(layers, pass_):
+            assert torch.equal(y, wino.conv2d_fused(x, u, k))
+    b.close()
+    assert wino.error_read_clear() == 0
