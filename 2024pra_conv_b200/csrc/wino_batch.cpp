@@ -164,7 +164,7 @@ struct Layer {
   void* ws2 = nullptr;      // two-stage workspace (batch-owned)
   int shift = 0;            // the fused route's CTAs a unit on the shift-reuse implicit GEMM (0: not on it)
   bool table = false;       // ... in the launch over a table of layers (pairs)
-  size_t wop = 0;           // offset of its weight operand in the batch's buffer
+  uint8_t* wop = nullptr;   // its weight operand (batch-owned)
   // U2 and the workspace for the two-stage route, made on first use from the
   // layer's fused U cache (synchronous: not inside a stream capture)
   int ensure_twostage() {
@@ -195,8 +195,8 @@ struct Batch {
   std::vector<int> order;        // table order of the layers
   BatchTable* table_dev = nullptr;
   wino::ShiftTable shift{};      // layers of the shift kernel's table (a kernel argument)
-  void* operands = nullptr;      // their weight operands
-  size_t operand_bytes = 0;
+  void* operands[wino::BATCH_MAX] = {};  // buffers of the shift layers' weight operands, one a commit that
+  int noperands = 0;                     // added any
   long long total = 0;
   bool dirty = true;
   cudaGraph_t graph = nullptr;
@@ -237,26 +237,28 @@ struct Batch {
   int run_shift(const Layer& L, cudaStream_t s) const {
     KernelParam p = L.p;
     p.transform_filter = nullptr;
-    return wino_launch_shift_fused(&p, L.p.transform_filter, static_cast<uint8_t*>(operands) + L.wop, L.shift, nullptr,
+    return wino_launch_shift_fused(&p, L.p.transform_filter, L.wop, L.shift, nullptr,
                                    sm_count(), s) == 0 ? (int)WINO_OK : (int)WINO_ECUDA;
   }
 
   // Room for the shift layers' weight operands, which every run makes from the
-  // layers' U caches (not inside a stream capture).
+  // layers' U caches (not inside a stream capture).  A layer's operand stays
+  // where it is until the batch is destroyed: a caller's own graph of a run
+  // holds its address.
   int ensure_operands() {
     size_t need = 0;
+    for (const Layer& L : layers)
+      if (L.shift && !L.wop) need += align256(wino_shift_weight_bytes(&L.p, L.shift));
+    if (need == 0) return WINO_OK;
+    void* block = nullptr;
+    if (cudaMalloc(&block, need) != cudaSuccess) return WINO_ECUDA;
+    operands[noperands++] = block;
+    uint8_t* at = static_cast<uint8_t*>(block);
     for (Layer& L : layers)
-      if (L.shift) {
-        L.wop = need;
-        need += align256(wino_shift_weight_bytes(&L.p, L.shift));
+      if (L.shift && !L.wop) {
+        L.wop = at;
+        at += align256(wino_shift_weight_bytes(&L.p, L.shift));
       }
-    if (need <= operand_bytes) return WINO_OK;
-    if (settle() != WINO_OK) return WINO_ECUDA;  // no launch still reads the old buffer
-    if (operands) cudaFree(operands);
-    operands = nullptr;
-    operand_bytes = 0;
-    if (cudaMalloc(&operands, need) != cudaSuccess) return WINO_ECUDA;
-    operand_bytes = need;
     return WINO_OK;
   }
 
@@ -288,19 +290,20 @@ struct Batch {
     if (have != WINO_OK) return have;
     // the shift kernel's table: the costliest units first, so that what is
     // left at the end of the launch is small
-    std::vector<int> heavy;
+    int heavy[wino::BATCH_MAX], nheavy = 0;
     for (int li : order)
-      if (on_shift(layers[li]) && layers[li].table) heavy.push_back(li);
-    std::stable_sort(heavy.begin(), heavy.end(), [&](int a, int b) {
+      if (on_shift(layers[li]) && layers[li].table) heavy[nheavy++] = li;
+    std::stable_sort(heavy, heavy + nheavy, [&](int a, int b) {
       return wino_shift_unit_cost(&layers[a].p) > wino_shift_unit_cost(&layers[b].p);
     });
     wino::ShiftTable ht;
     std::memset(&ht, 0, sizeof(ht));
-    for (int li : heavy) {
+    for (int i = 0; i < nheavy; ++i) {
+      const int li = heavy[i];
       wino::ShiftLayer& d = ht.layer[ht.nlayers++];
       d.p = layers[li].p;
       d.p.pweight = layers[li].p.transform_filter;
-      d.p.transform_filter = static_cast<uint8_t*>(operands) + layers[li].wop;
+      d.p.transform_filter = layers[li].wop;
     }
     wino_shift_table_finish(&ht);
     if (ht.nlayers > 0 && wino_shift_prepare() != 0) return WINO_ECUDA;
@@ -442,7 +445,7 @@ int wino_batch_destroy(void* h) {
   b->drop_graph();
   for (Layer& L : b->layers) L.release();
   if (b->table_dev) cudaFree(b->table_dev);
-  if (b->operands) cudaFree(b->operands);
+  for (int i = 0; i < b->noperands; ++i) cudaFree(b->operands[i]);
   if (b->done) cudaEventDestroy(b->done);
   delete b;
   return WINO_OK;

@@ -44,3 +44,42 @@ def test_replays_join_before_what_follows(wino, cuda, picks):
             assert torch.equal(y, wino.conv2d_fused(x, u, k))
     b.close()
     assert wino.error_read_clear() == 0
+
+
+def test_a_callers_graph_outlives_layers_added_later(wino, cuda):
+    """A run captured into the caller's own graph replays after the batch grew: the
+    operands of the layers it holds stay where they are."""
+    import torch
+    shapes = [(2, 64, 56, 56, 128), (8, 128, 28, 28, 128), (8, 256, 14, 14, 256)]
+    cases = [base._fused_case(cuda, s, 40 + i) for i, s in enumerate(shapes)]
+    b, layers = wino.Batch(), []
+
+    def add(case):
+        x, wt, _, res = case
+        n, c, h, w = x.shape
+        ws = torch.empty(wino.fused_conv_workspace_bytes(n, c, h, w, wt.shape[0]), dtype=torch.uint8, device=cuda)
+        layers.append((x, wino.filter_transform(wt), wt.shape[0], torch.empty_like(res), ws))
+        b.add(layers[-1][0], layers[-1][1], layers[-1][2], layers[-1][3], workspace=ws)
+
+    add(cases[0])
+    b.run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        b.run()
+    for case in cases[1:]:
+        add(case)
+        b.run()
+    x, u, k, y, _ = layers[0]
+    for _ in range(2):
+        x.mul_(-0.5)
+        y.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, wino.conv2d_fused(x, u, k))
+    b.run()
+    torch.cuda.synchronize()
+    for x, u, k, y, _ in layers:
+        assert torch.equal(y, wino.conv2d_fused(x, u, k))
+    b.close()
+    assert wino.error_read_clear() == 0
