@@ -557,12 +557,13 @@ int wino_batch_run(void* h, void* stream) {
   return rc != WINO_OK ? rc : b->mark((cudaStream_t)stream);
 }
 
-// Autotune: per-layer configurations (exhaustive over CFG_*) and routes
-// (the fused launch's 128 x 32 tile blocks or the two-stage path's 128 x 256
-// tap-GEMM units, the faster alone), then the layer order of the table among
+// Autotune: per-layer configurations (of the layers on the fused Winograd kernel,
+// exhaustive over CFG_* without splits; a shift layer runs once) and routes (the
+// batch's own kernel or the two-stage path's 128 x 256 tap-GEMM units, the faster
+// alone), then the layer order of the table among
 // {as added, longest first, longest/shortest interleaved}; the routes picked
 // stay only if the whole batch beats the all-fused batch in the best order.
-// layer_us: nlayers x NCFG timings (-1 = not applicable); order_us: the
+// layer_us: nlayers x NCFG timings (-1 = not run); order_us: the
 // three whole-batch timings with the picked routes.  Leaves the best choice
 // set; wino_batch_get_route reports each layer's route and both timings.
 int wino_batch_tune(void* h, int reps, float* layer_us, float* order_us, void* stream) {
@@ -583,10 +584,7 @@ int wino_batch_tune(void* h, int reps, float* layer_us, float* order_us, void* s
       if (wino::cfg_split_level(cfg) != 0) continue;
       if (!L.p.transform_pin && !(cfg & wino::CFG_DIRECT)) continue;
       float t = 0.f;
-      if (L.shift && best >= 0) {           // the shift kernel runs the same under every configuration
-        us[cfg] = us[best];
-        continue;
-      }
+      if (L.shift && best >= 0) continue;   // the shift kernel has no configurations: run under the first
       auto one = [&] {
         return L.shift ? b->run_shift(L, s) : run_layer_cfg(L.p, L.p.transform_pin, cfg, s);
       };

@@ -292,17 +292,23 @@ int wino_tune_layer(const void* x, const void* ucache, void* workspace, void* y,
 /* Batched persistent launch (no counterpart in the reference, whose harness
  * runs one hard-wired shape per launch sequence, src/main.cpp:105-124).  A
  * batch holds up to 32 fp16 layers, each with its input, cached U, output
- * and (optional) pre-pass workspace; wino_batch_run issues the pre-passes and
- * ONE persistent fused-kernel launch over all layers' work blocks (a device
- * layer table); wino_batch_graph_capture records that sequence in a CUDA
- * graph, wino_batch_graph_launch replays it.  Batch layers run unsplit.
- * wino_batch_tune runs the autotuner: per layer the route (fused or
- * two-stage, kept only if the whole batch is faster with the picks than
- * all-fused) and the fastest unsplit
- * configuration (exhaustive), then the
+ * and (optional) pre-pass workspace.  Layers with a workspace of 512 MFLOP or
+ * more (direct count) run on the shift-reuse implicit GEMM, as the single-layer
+ * calls do: one launch over a table of those whose tiles fit it, which makes
+ * their operands from the U caches first, and launches of their own for the
+ * others.  The rest run on the fused Winograd kernel: wino_batch_run issues
+ * their pre-passes and ONE persistent launch over all their work blocks (a
+ * device layer table).  wino_batch_graph_capture records that sequence in a
+ * CUDA graph, the two kernels' launches on two branches, and
+ * wino_batch_graph_launch replays it.  Batch layers run unsplit.
+ * wino_batch_tune runs the autotuner: per layer the route (the batch's own
+ * kernel or two-stage, kept only if the whole batch is faster with the picks
+ * than with none) and the fastest unsplit configuration (exhaustive), then the
  * fastest table order among {as added, longest first, longest/shortest
- * interleaved}; layer_us receives nlayers x WINO_NCFG timings, order_us the
- * three whole-batch timings (either may be NULL).  Configuration and order
+ * interleaved}; layer_us receives nlayers x WINO_NCFG timings (-1: not run),
+ * order_us the three whole-batch timings (either may be NULL).  Configurations
+ * and the order are the fused Winograd kernel's: a layer on the shift kernel is
+ * timed once, and set_config and set_order change nothing for it.  Configuration and order
  * changes invalidate a captured graph.  wino_batch_run and
  * wino_batch_graph_launch record their completion on the caller's stream;
  * the next commit (explicit, or the one a run or capture after a change
@@ -318,13 +324,13 @@ int wino_batch_add_layer(void* batch, const void* x, const void* ucache, void* w
 int wino_batch_num_layers(void* batch);
 int wino_batch_set_config(void* batch, int layer, int cfg);
 int wino_batch_get_config(void* batch, int layer, int* cfg);
-/* Route of a batch layer (a tile-shape choice): 0 inside the persistent
- * fused launch (128 output channels x 32 tiles per block), 1 the two-stage
- * path (tap-GEMM units of 128 tiles x 256 output channels, M in a
+/* Route of a batch layer: 0 the batch's own kernel for it (the shift kernel, or
+ * the persistent fused launch's blocks of 128 output channels x 32 tiles), 1 the
+ * two-stage path (tap-GEMM units of 128 tiles x 256 output channels, M in a
  * batch-owned workspace, U relaid from the layer's fused U cache) launched
  * before it.  Setting route 1 allocates those buffers (outside any stream
  * capture).  get_route also reports the tuner's timings of the layer alone
- * (fastest fused configuration, two-stage; -1 when not timed). */
+ * (route 0 in its fastest configuration, two-stage; -1 when not timed). */
 int wino_batch_set_route(void* batch, int layer, int route);
 int wino_batch_get_route(void* batch, int layer, int* route, float* fused_us, float* twostage_us);
 int wino_batch_set_order(void* batch, const int* order, int n);

@@ -83,3 +83,23 @@ def test_a_callers_graph_outlives_layers_added_later(wino, cuda):
         assert torch.equal(y, wino.conv2d_fused(x, u, k))
     b.close()
     assert wino.error_read_clear() == 0
+
+
+def test_tuner_reports_only_what_it_ran(wino, cuda):
+    """The shift kernel has no configurations: one time for its layer, the others
+    -1; the fused kernel's layer has one for each configuration without splits."""
+    import torch
+    b, keep = wino.Batch(), []
+    for i, shape in enumerate([(2, 64, 56, 56, 128), (2, 64, 14, 14, 64)]):
+        x, wt, _, res = base._fused_case(cuda, shape, 50 + i)
+        n, c, h, w, k = shape
+        ws = torch.empty(wino.fused_conv_workspace_bytes(n, c, h, w, k), dtype=torch.uint8, device=cuda)
+        keep.append((x, wino.filter_transform(wt), res, ws))
+        b.add(x, keep[-1][1], k, res, workspace=ws)
+    rows, _ = b.tune(reps=1)
+    ran = [[c for c, t in enumerate(row) if t > 0] for row in rows]
+    assert len(ran[0]) == 1 and ran[0][0] == b.config(0)
+    assert len(ran[1]) > 1 and b.config(1) in ran[1]
+    assert all(t == -1 for row, r in zip(rows, ran) for c, t in enumerate(row) if c not in r)
+    b.close()
+    assert wino.error_read_clear() == 0
