@@ -788,14 +788,14 @@ void* wino_fused_kernel_ptr() { return (void*)fused_wino_f16_kernel; }
 int wino_fused_smem_bytes() { return fused::SMEM_BYTES; }
 int wino_fused_threads() { return fused::NTHREAD; }
 
-static int fused_prepare_device() {
+static int fused_prepare_context() {
   cudaError_t e = cudaFuncSetAttribute(fused_wino_f16_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, fused::SMEM_BYTES);
   return (int)e;
 }
 int wino_fused_prepare() {
-  static OncePerDevice once;
-  return once.run(fused_prepare_device);
+  static OncePerContext once;
+  return once.run(fused_prepare_context);
 }
 
 static void* var_kernel(int variant);

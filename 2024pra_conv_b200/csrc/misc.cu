@@ -1,5 +1,6 @@
 // Small kernels shared by the drop-in ABI, and the self-test of the bounded
 // waits.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include "wino_param.h"
 #include "tc_sm100.cuh"
@@ -37,6 +38,20 @@ __global__ void wait_timeout_selftest_kernel() {
 }
 
 }  // namespace wino
+
+// Id of the calling thread's current context (wino_common.cuh).
+extern "C" unsigned long long wino_context_id() {
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const GetId get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<GetId>(f) : nullptr;
+  }();
+  unsigned long long id = 0;
+  return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
 
 extern "C" void* wino_noop_kernel_ptr() { return (void*)wino::noop_kernel; }
 

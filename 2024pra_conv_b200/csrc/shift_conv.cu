@@ -145,7 +145,7 @@ unsigned long long wino_shift_slots(const KernelParam* p, int cg, int sms, unsig
   return sc::pack_plan(g);
 }
 
-static int shift_prepare_device() {
+static int shift_prepare_context() {
   for (const void* f :
        {(const void*)shift_conv_kernel<false>, (const void*)shift_conv_kernel<true>,
         (const void*)shift_conv_pair_kernel<false>, (const void*)shift_conv_pair_kernel<true>,
@@ -158,8 +158,8 @@ static int shift_prepare_device() {
   return 0;
 }
 int wino_shift_prepare() {
-  static OncePerDevice once;
-  return once.run(shift_prepare_device);
+  static OncePerContext once;
+  return once.run(shift_prepare_context);
 }
 
 // The plan's numbers (host tests): GX, GY, operand rows, blocks per stage,

@@ -2115,7 +2115,7 @@ int wino_twostage_smem_bytes_for(int c) {
 int wino_twostage_output_smem_bytes() { return ot::SMEM_BYTES; }
 int wino_twostage_output_threads() { return ot::NTHREAD; }
 
-static int twostage_prepare_device() {
+static int twostage_prepare_context() {
   if (cudaFuncSetAttribute(twostage_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            ot::SMEM_BYTES) != cudaSuccess)
     return 1;
@@ -2140,8 +2140,8 @@ static int twostage_prepare_device() {
                                    tp::SMEM_BYTES);
 }
 int wino_twostage_prepare() {
-  static OncePerDevice once;
-  return once.run(twostage_prepare_device);
+  static OncePerContext once;
+  return once.run(twostage_prepare_context);
 }
 
 // The two-stage pre-pass: row-transformed records (XR) for the resident-U

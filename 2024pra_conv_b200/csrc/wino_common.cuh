@@ -115,17 +115,25 @@ __host__ __device__ __forceinline__ void filter_tile(const float g[9], float u[1
   }
 }
 
-// Kernel attributes are per function and device: set once for each, as a call
-// took a microsecond for every few of them.  A repeat by another thread is harmless.
-struct OncePerDevice {
-  std::atomic<bool> done[64] = {};
+// Id of the calling thread's context, unique over the process's life, or 0
+// where there is none yet (misc.cu).
+extern "C" unsigned long long wino_context_id();
+
+// Kernel attributes are per function and context: set them once for each, as a
+// call took a microsecond for every few of them.  The id tells a context made
+// after a cudaDeviceReset, or one of the caller's own, from the device's last.
+// A repeat by another thread is harmless.
+struct OncePerContext {
+  std::atomic<unsigned long long> done[64] = {};   // by device: the context last prepared
   int run(int (*prepare)()) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 1;
     const bool kept = dev >= 0 && dev < 64;
-    if (kept && done[dev].load(std::memory_order_acquire)) return 0;
+    const unsigned long long id = kept ? wino_context_id() : 0;
+    if (id != 0 && done[dev].load(std::memory_order_acquire) == id) return 0;
     const int rc = prepare();
-    if (rc == 0 && kept) done[dev].store(true, std::memory_order_release);
+    // (the first call of a process makes the context)
+    if (rc == 0 && kept) done[dev].store(wino_context_id(), std::memory_order_release);
     return rc;
   }
 };
