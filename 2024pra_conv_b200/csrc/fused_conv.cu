@@ -820,10 +820,10 @@ static void* var_kernel(int variant) {
   }
 }
 
-// Launch the fused kernel of a precision variant and schedule configuration
-// (CFG_* bits) on `grid` CTAs.
 int wino_launch_dependent(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream);
 
+// Launch the fused kernel of a precision variant and schedule configuration
+// (CFG_* bits) on `grid` CTAs.
 int wino_fused_launch_variant(int variant, const KernelParam* p, const VariantArgs* va, int cfg,
                               unsigned grid, cudaStream_t stream) {
   void* fn = var_kernel(variant);

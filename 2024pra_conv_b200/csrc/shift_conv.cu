@@ -200,9 +200,11 @@ int wino_launch_shift(const KernelParam* p, int cg, int sms, cudaStream_t stream
 
 // ---- convolutions on a fused U cache ------------------------------------
 // Direct-conv FLOPs from which the fused entry points (conv, epilogue, batch)
-// recover the filter from U and take this kernel: below it the fused Winograd
-// kernel's configurations stay bit-identical to one another, and the two
-// launches cost what the kernel gains.
+// recover the filter from U and take this kernel.  Not where the kernels cross:
+// in a graph, the conv takes 16.4 us on the fused Winograd kernel and 10.3 on this one at
+// N1 C64 14x14 K64 (14 MFLOP), 30.8 and 14.4 at N2 C256 14x14 K256 (462); the
+// epilogue 24 and 12, 37 and 16.  Below the line results are bit-identical to the fused
+// kernel's configurations (wino_conv2d_fused_cfg), which tests hold at up to 265 MFLOP.
 static constexpr double kFusedMinFlops = 512e6;
 
 // CTAs a unit for a problem (dims and tensors set), or 0 when it stays with
@@ -308,8 +310,8 @@ int wino_conv2d_shift(const void* x, const void* weight, void* wprep, void* y, i
                                  args, 0, (cudaStream_t)stream) != cudaSuccess)
     return 3;
   if (!x) return 0;
-  if (weight) return wino_launch_shift(&p, cg, 148, (cudaStream_t)stream) == 0 ? 0 : 3;
-  return cudaLaunchKernel(wino_shift_kernel_ptr(&p, cg), dim3(wino_shift_grid(&p, cg, 148)), dim3(sc::NTHREAD), args,
+  if (weight) return wino_launch_shift(&p, cg, sc::NSM, (cudaStream_t)stream) == 0 ? 0 : 3;
+  return cudaLaunchKernel(wino_shift_kernel_ptr(&p, cg), dim3(wino_shift_grid(&p, cg, sc::NSM)), dim3(sc::NTHREAD), args,
                           (size_t)sc::SMEM_BYTES, (cudaStream_t)stream) == cudaSuccess
              ? 0
              : 3;

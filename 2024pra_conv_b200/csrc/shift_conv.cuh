@@ -45,14 +45,15 @@
 // Measured (B200): N128 C256 28x28 K256 94 us for the conv alone with L2
 // flushed = 1253 TFLOP/s direct (the Winograd two-stage kernels it replaces
 // there: 61 + 79 + 54 us).  Whole drop-in calls against the kernels replaced: N64
-// C256 14x14 K256 27 us (55), N32 C512 7x7 K512 29 (62), N32 C128 56x56 K128
+// C256 14x14 K256 27 us (54), N32 C512 7x7 K512 29 (62), N32 C128 56x56 K128
 // stride 2 31 (74, gathering implicit GEMM), N32 C64 56x56 K256 1x1 25 (53).
 //
 // The weight operand (shift_weight_kernel) is laid out as the stages read it:
 // per unit block of output channels and CTA of the unit, 16-channel block by
 // 16-channel block, tap by tap, each piece the K-major core-matrix
 // interleave (row k, channel c at (k >> 3) * 256 + (c >> 3) * 128 + (k & 7)
-// * 16 + (c & 7) * 2).  A stage is then one run of up to 36 KB
+// * 16 + (c & 7) * 2).  A stage is then one run (36 KB for a 3x3
+// filter at 128 rows a CTA; as at least two stages fit, at most half of SMEM_STAGES)
 // and one bulk copy (one per tap issued no faster than a stage per 1.8 k
 // cycles; splitting the run over lanes gained nothing).
 //

@@ -245,10 +245,12 @@ struct ShiftPlan {
   void* wop;
 };
 
-// Direct-conv FLOPs from which the drop-in takes the shift kernel.  Below it
-// every route is bound by its launches (N1 C16 16x16 K16: 8 us of kernels on
-// either), and the two-stage route's results stay bit-identical to
-// wino_conv2d_twostage there.
+// Direct-conv FLOPs from which the drop-in takes the shift kernel.  Not where
+// the routes cross, which they do not: in a graph, N1 C16 16x16 K16 (1.2 MFLOP)
+// takes 14.4 us on the two-stage route and 8.2 on the shift kernel, N2 C64 20x20
+// K64 (59) 16.4 and 10.3, 3x3/2 N2 C128 14x14 K96 (22) 59 and 16, an RGB stem of
+// one 112x112 image (59) 33 and 8.  Below the line results are bit-identical to
+// wino_conv2d_twostage's, which tests hold at up to 36 MFLOP.
 constexpr double kShiftMinFlops = 64e6;
 
 // Two-stage route (input transform fused into full-width tap GEMMs, M in the

@@ -1,16 +1,17 @@
 // Batched persistent launch, schedule configurations and the autotuner.
 //
 // A batch holds the uneven 3x3 conv layers of a network (each with its own
-// input, cached U, output and XB workspace).  Running it issues the input
-// pre-pass of every layer that uses one and then ONE persistent fused-kernel
-// launch whose CTAs walk the concatenated work blocks of all layers through
-// a device-resident layer table; the whole sequence can be captured into a
-// CUDA graph and replayed.  The reference has no counterpart: its harness
+// input, cached U, output and XB workspace).  The large ones run on the
+// shift-reuse implicit GEMM (shift_conv.cuh), in one launch over a table of
+// them where their tiles fit it; for the others it issues the input pre-passes and
+// then ONE persistent fused-kernel launch whose CTAs walk the concatenated work
+// blocks of all those layers through a device-resident layer table.  The whole
+// sequence can be captured into a CUDA graph and replayed.  The reference has no counterpart: its harness
 // runs one hard-wired shape per launch sequence (src/main.cpp:105-124,
 // src/conv2d.cpp:458-494).
 //
-// The autotuner times every schedule configuration of every layer (CFG_*
-// bits of wino_batch.h) with CUDA events, keeps the fastest per layer, then
+// The autotuner times every schedule configuration (CFG_* bits of wino_batch.h)
+// of every layer on the fused kernel with CUDA events, keeps the fastest per layer, then
 // times whole-batch launches under three layer orders and keeps the fastest.
 #include <algorithm>
 #include <cstdint>

@@ -826,7 +826,8 @@ def implicit_gemm_leg(wino, dev, timed, peaks, steps):
                      "rel_l2_fp64": rl2})
         del x, wt, y, wp, xs, ys, y64
     return {"workload": "ResNet-50 layers outside the Winograd contract, N128, x ~ N(0,1), "
-                        "weights ~ N(0, 1/(c r s)); drop-in route 4 runs the same kernels",
+                        "weights ~ N(0, 1/(c r s)); wino_conv2d_igemm, which the drop-in runs for the strided "
+                        "1x1 layers only (the others are past 64 MFLOP: its shift kernel)",
             "layers": rows, "sum_us": round(t_sum, 1), "sum_floor_us": round(floor_sum, 1),
             "frac_of_floor": round(floor_sum / t_sum, 3)}
 

@@ -58,9 +58,9 @@ int wino_check_shape(int n, int c, int h, int w, int k);
  * out into transform_filter, which must hold wino_igemm_weight_bytes).
  * Problems of at least 64 MFLOP (direct count) with strides up to 2 (of one or two taps: 1)
  * take the shift-reuse implicit GEMM instead (reported as
- * WINO_ROUTE_SHIFT inside the Winograd contract, as the implicit GEMM outside
- * it), whose weight operand goes to transform_filter or, where it does not
- * fit there, to transform_pin.  Returns a WINO_ROUTE_* value, or minus a WINO_E* code for an invalid
+ * WINO_ROUTE_SHIFT inside the Winograd contract; outside it WINO_ROUTE_IGEMM
+ * stands for either implicit GEMM), whose weight operand goes to
+ * transform_filter or, where it does not fit there, to transform_pin.  Returns a WINO_ROUTE_* value, or minus a WINO_E* code for an invalid
  * problem. */
 enum {
   WINO_ROUTE_DIRECT = 0,
